@@ -31,10 +31,12 @@ __device__ __forceinline__ void load_camera(Camera& dst, const Camera* src) {
 // seen by camera cam, its SH coefficients at shv: writes the 48-byte splat to out
 // (zeros when culled) and returns the tiles it touches
 // (src/shaders/tiles.wgsl:24-35; blend tiles of 2^twl x 2^thl tiles for a batch
-// of views) and its depth's bits (0 when culled).
+// of views) and its depth's bits (all ones when culled: last in the depth order).
 struct Projected {
-  uint32_t tiles, depth_bits;
+  uint4 rect;  // the tiles it touches (empty when culled)
+  uint32_t depth_bits;
   float radius;  // 0 when culled
+  __device__ __forceinline__ uint32_t tiles() const { return (rect.z - rect.x) * (rect.w - rect.y); }
 };
 
 __device__ __forceinline__ Projected preprocess_one(const Camera& cam, const float (&g)[16], const float* shv,
@@ -45,7 +47,7 @@ __device__ __forceinline__ Projected preprocess_one(const Camera& cam, const flo
     out[0] = zero;
     out[1] = zero;
     out[2] = zero;
-    return Projected{0u, 0u, 0.0f};
+    return Projected{make_uint4(0u, 0u, 0u, 0u), ~0u, 0.0f};
   };
   if (-view_z(cam, g) <= 0.2f) return culled();
   Projection p;
@@ -92,7 +94,7 @@ __device__ __forceinline__ Projected preprocess_one(const Camera& cam, const flo
   out[1] = make_float4(p.c / p.det, -p.b / p.det, p.a / p.det, blend_cutoff(g[3]));
   out[2] = make_float4(fmaxf(color[0], 0.0f), fmaxf(color[1], 0.0f), fmaxf(color[2], 0.0f), g[3]);
   const uint4 rect = blend_rect(tile_rect(mx, my, radius, tile_grid(cam)), twl, thl);
-  return Projected{(rect.z - rect.x) * (rect.w - rect.y), __float_as_uint(p.depth), radius};
+  return Projected{rect, __float_as_uint(p.depth), radius};
 }
 
 // Stages the SH coefficients of Gaussians [first, first + n) into shared memory
@@ -115,9 +117,10 @@ __device__ __forceinline__ void load_gaussian(const float* __restrict__ gaussian
   }
 }
 
-// One thread per Gaussian, one view. When tile_counts is given, the tiles each
-// splat touches are written too (src/shaders/tiles.wgsl:24-35, fused); when
-// depth_keys is given, the depth's bits (0 when culled) and the splat's index,
+// One thread per Gaussian, one view. The tiles each splat touches are written too,
+// as a packed rectangle when rects is given (dg_bin.cu's input), else as their
+// number in tile_counts (src/shaders/tiles.wgsl:24-35, fused); when depth_keys is
+// given, the depth's bits (all ones when culled) and the splat's index,
 // the input of the depth sort; when radii is given, each splat's radius densely
 // (the training step's fused backward reads it there, not from the 48-byte
 // splat records).
@@ -133,6 +136,7 @@ __global__ void __launch_bounds__(PRE_THREADS) preprocess_kernel(const Camera* _
                                                                  const uint32_t* __restrict__ scene_params,
                                                                  float* __restrict__ splats,
                                                                  uint32_t* __restrict__ tile_counts,
+                                                                 uint32_t* __restrict__ rects,
                                                                  uint32_t* __restrict__ depth_keys,
                                                                  uint32_t* __restrict__ depth_order,
                                                                  float* __restrict__ radii) {
@@ -163,7 +167,10 @@ __global__ void __launch_bounds__(PRE_THREADS) preprocess_kernel(const Camera* _
     if (i < count) {
       const Projected pr = preprocess_one(s_cam, g, s_sh[step & 1] + threadIdx.x * SH_REST_FLOATS, basis_count,
                                           reinterpret_cast<float4*>(splats + (size_t)i * FLOATS_PER_SPLAT));
-      if (tile_counts) tile_counts[i] = pr.tiles;
+      if (rects)
+        rects[i] = pack_rect(pr.rect);
+      else
+        tile_counts[i] = pr.tiles();
       if (depth_keys) depth_keys[i] = pr.depth_bits;
       if (depth_order) depth_order[i] = i;
       if (radii) radii[i] = pr.radius;
@@ -194,8 +201,8 @@ uint32_t preprocess_grid(const dg_context* ctx, uint32_t count) {
 __global__ void __launch_bounds__(PRE_THREADS) preprocess_views_kernel(
     const Camera* __restrict__ cameras, uint32_t views, const float* __restrict__ gaussians,
     const float* __restrict__ sh, uint32_t count, const uint32_t* __restrict__ scene_params,
-    float* __restrict__ splats, uint32_t* __restrict__ tile_counts, uint2* __restrict__ depth_keys,
-    uint32_t* __restrict__ depth_order, uint32_t twl, uint32_t thl) {
+    float* __restrict__ splats, uint32_t* __restrict__ tile_counts, uint32_t* __restrict__ rects,
+    uint2* __restrict__ depth_keys, uint32_t* __restrict__ depth_order, uint32_t twl, uint32_t thl) {
   __shared__ float s_sh[PRE_THREADS * SH_REST_FLOATS];
   const uint32_t degree = scene_params[0];
   const uint32_t basis_count = (degree + 1u) * (degree + 1u) - 1u;
@@ -210,15 +217,18 @@ __global__ void __launch_bounds__(PRE_THREADS) preprocess_views_kernel(
     const size_t at = (size_t)v * count + i;
     const Projected pr = preprocess_one(cameras[v], g, s_sh + threadIdx.x * SH_REST_FLOATS, basis_count,
                                         reinterpret_cast<float4*>(splats + at * FLOATS_PER_SPLAT), twl, thl);
-    tile_counts[at] = pr.tiles;
+    if (rects)
+      rects[at] = pack_rect(pr.rect);
+    else
+      tile_counts[at] = pr.tiles();
     depth_keys[at] = make_uint2(pr.depth_bits, v);
     depth_order[at] = (uint32_t)at;
   }
 }
 
-// The depth-first tile sort (the renderer's path). The reference sorts 64-bit
-// (tile, depth) keys (src/shaders/tiles.wgsl:37-60, src/radixSort.ts:101-104).
-// Here the splats are first sorted by depth alone (stable, so equal depths keep
+// The depth-first tile sort (the renderer's path on grids that dg_bin.cu does not
+// take). The reference sorts 64-bit (tile, depth) keys
+// (src/shaders/tiles.wgsl:37-60, src/radixSort.ts:101-104). Here the splats are first sorted by depth alone (stable, so equal depths keep
 // index order), their pairs are then emitted in that order, and a stable sort on
 // the 16-bit tile index finishes the job. Within a tile the pairs end up by depth
 // with ties by splat index: exactly the reference's order, from sorting N 32-bit
@@ -882,6 +892,7 @@ __global__ void clear_target_kernel(uchar4* __restrict__ target, uint32_t pixels
 // ------------------------------------------------------------ TileRasterizer
 
 static dg_status ensure_plan(dg_tile_rasterizer* tr);
+static dg_status ensure_pair_sort(dg_tile_rasterizer* tr);
 
 static dg_status make_pairs(dg_tile_rasterizer* tr, uint32_t capacity) {
   dg_context* ctx = tr->ctx;
@@ -894,13 +905,25 @@ static dg_status make_pairs(dg_tile_rasterizer* tr, uint32_t capacity) {
   tr->plan = sort_plan(capacity, TILE_INDEX_BITS);
   tr->tile_plan = sort_plan_low_bits(capacity, TILE_INDEX_BITS);
   tr->pair_capacity = capacity;
-  DG_TRY(alloc_buffer(ctx, (size_t)capacity * 8, &tr->keys));
   DG_TRY(alloc_buffer(ctx, (size_t)capacity * 4, &tr->values));
-  DG_TRY(alloc_buffer(ctx, (size_t)capacity * 8, &tr->keys_alt));
-  DG_TRY(alloc_buffer(ctx, (size_t)capacity * 4, &tr->values_alt));
-  DG_TRY(alloc_buffer(ctx, std::max(sort_scratch_bytes(tr->plan), sort_scratch_bytes(tr->tile_plan)),
-                      &tr->sort_scratch));
+  if (!tr->depth_first) DG_TRY(ensure_pair_sort(tr));
   return ensure_plan(tr);
+}
+
+// The buffers of frames whose pairs are sorted; binned frames need none of them.
+static dg_status ensure_pair_sort(dg_tile_rasterizer* tr) {
+  if (tr->sort_scratch) return DG_OK;
+  dg_context* ctx = tr->ctx;
+  const size_t capacity = tr->pair_capacity;
+  for (dg_buffer** b : {&tr->keys, &tr->keys_alt, &tr->values_alt}) {
+    free_buffer(*b);
+    *b = nullptr;
+  }
+  DG_TRY(alloc_buffer(ctx, capacity * 8, &tr->keys));
+  DG_TRY(alloc_buffer(ctx, capacity * 8, &tr->keys_alt));
+  DG_TRY(alloc_buffer(ctx, capacity * 4, &tr->values_alt));
+  return alloc_buffer(ctx, std::max(sort_scratch_bytes(tr->plan), sort_scratch_bytes(tr->tile_plan)),
+                      &tr->sort_scratch);
 }
 
 
@@ -924,8 +947,8 @@ dg_status rasterizer_create(dg_context* ctx, dg_buffer* camera, dg_buffer* splat
     if (cudaEventCreateWithFlags(&tr->readback_events[k], cudaEventDisableTiming) != cudaSuccess)
       st = fail(DG_ERROR_CUDA, "event");
   uint32_t capacity = initial_pair_capacity ? initial_pair_capacity : std::max(1u << 16, count * 8u);
-  if (st == DG_OK) st = make_pairs(tr, capacity);
   tr->depth_first = depth_first;
+  if (st == DG_OK) st = make_pairs(tr, capacity);
   tr->coop_min = COOP_MIN;
   if (st == DG_OK && depth_first) {
     const size_t n = std::max(count, 1u);
@@ -961,6 +984,17 @@ dg_status rasterizer_prepare(dg_tile_rasterizer* tr, const float viewport[2], co
   uint32_t tile_bits = 1;
   while (tile_bits < 32 && (1u << tile_bits) < tiles) tile_bits++;
   sort_plan_key_bits(tr->tile_plan, tile_bits);
+  tr->binned = tr->depth_first && bin_fits(tiles_x, tiles_y);
+  if (tr->binned) {
+    const size_t bytes = bin_scratch_bytes(BinShape{tr->count, 1u, tiles_x, tiles_y});
+    if (!tr->bin_scratch || tr->bin_scratch->bytes < bytes) {
+      free_buffer(tr->bin_scratch);
+      tr->bin_scratch = nullptr;
+      DG_TRY(alloc_buffer(tr->ctx, bytes, &tr->bin_scratch));
+    }
+  } else {
+    DG_TRY(ensure_pair_sort(tr));
+  }
   if (!tr->ranges || tr->ranges_tiles < tiles) {
     free_buffer(tr->ranges);
     tr->ranges = nullptr;
@@ -986,6 +1020,32 @@ dg_status rasterizer_launch(dg_tile_rasterizer* tr, dg_buffer* target, bool coun
   cudaStream_t st = ctx->stream;
   const uint32_t count = tr->count;
   const auto* cam = typed<const Camera>(tr->camera);
+  tr->keys_in_ranges = false;
+  if (tr->binned && counts_ready) {
+    // tile_offsets holds each splat's rectangle of tiles; depth_keys/depth_values its
+    // depth bits and index (both written by the renderer's preprocess).
+    uint32_t* order = typed<uint32_t>(tr->depth_values);
+    if (count > 0) {
+      DG_TRY(sort_launch(ctx, tr->depth_plan, tr->depth_keys->ptr, order, tr->depth_keys_alt->ptr,
+                         typed<uint32_t>(tr->depth_values_alt), nullptr, tr->depth_scratch->ptr));
+    }
+    BinLaunch l{};
+    l.rects = typed<uint32_t>(tr->tile_offsets);
+    l.order = order;
+    l.capacity = tr->pair_capacity;
+    l.coop_min = tr->coop_min;
+    l.scratch = tr->bin_scratch->ptr;
+    l.pair_total = typed<uint32_t>(tr->scan_total);
+    l.values = typed<uint32_t>(tr->values);
+    l.ranges = typed<uint2>(tr->ranges);
+    l.plan = typed<uint32_t>(tr->work_plan);
+    l.chunks = typed<uint2>(tr->chunks);
+    l.work = typed<uint32_t>(tr->work);
+    DG_TRY(bin_launch(ctx, BinShape{count, 1u, tr->tiles_x, tr->tiles_y}, l));
+    tr->keys_in_ranges = true;
+    tr->keys_are_tiles = false;
+    return launch_rasterize(tr, target);
+  }
   DG_CUDA(cudaMemsetAsync(tr->ranges->ptr, 0, (size_t)tr->tiles_x * tr->tiles_y * 8, st));
   if (tr->depth_first && counts_ready) {
     // tile_offsets holds each splat's tile count; depth_keys/depth_values its depth
@@ -1060,6 +1120,7 @@ dg_status launch_rasterize(dg_tile_rasterizer* tr, dg_buffer* target) {
   f.blend_mask = typed<uint32_t>(tr->blend_mask);
   f.counters = typed<uint32_t>(tr->work);
   f.splat_cutoffs = tr->splat_cutoffs;
+  f.planned = tr->keys_in_ranges;
   return blend_forward(ctx, f);
 }
 
@@ -1079,9 +1140,11 @@ dg_status blend_forward(dg_context* ctx, const BlendForward& f) {
   DG_REQUIRE(sh.twl <= MAX_BLEND_TILE_LOG2 && sh.thl <= MAX_BLEND_TILE_LOG2, "blend tiles of at most 2 x 2 tiles");
   DG_REQUIRE(sh.twl + sh.thl == 0 || (!f.checkpoints && !f.blend_mask && !f.chunks),
              "blend tiles larger than 16x16 have no backward pass");
-  DG_CUDA(cudaMemsetAsync(f.counters, 0, 16, ctx->stream));
-  DG_LAUNCH(ctx, "plan",
-            plan_kernel<<<1, PLAN_THREADS, 0, ctx->stream>>>(f.ranges, f.tiles, f.coop_min, f.plan, f.chunks));
+  if (!f.planned) {
+    DG_CUDA(cudaMemsetAsync(f.counters, 0, 16, ctx->stream));
+    DG_LAUNCH(ctx, "plan",
+              plan_kernel<<<1, PLAN_THREADS, 0, ctx->stream>>>(f.ranges, f.tiles, f.coop_min, f.plan, f.chunks));
+  }
   if (sh.twl == 0 && sh.thl == 0) return launch_rasterize_kernel<0, 0>(ctx, f);
   if (sh.twl == 1 && sh.thl == 0) return launch_rasterize_kernel<1, 0>(ctx, f);
   if (sh.twl == 0 && sh.thl == 1) return launch_rasterize_kernel<0, 1>(ctx, f);
@@ -1101,10 +1164,11 @@ uint32_t blend_grid(dg_context* ctx, const void* kernel, uint32_t threads, uint3
 
 dg_status views_preprocess_launch(dg_context* ctx, const Camera* cameras, uint32_t views, const float* gaussians,
                                   const float* sh, uint32_t count, const uint32_t* scene_params, float* splats,
-                                  uint32_t* tile_counts, uint2* depth_keys, uint32_t* order, BlendShape shape) {
+                                  uint32_t* tile_counts, uint32_t* rects, uint2* depth_keys, uint32_t* order,
+                                  BlendShape shape) {
   DG_LAUNCH(ctx, "preprocess",
             preprocess_views_kernel<<<ceil_div(count, PRE_THREADS), PRE_THREADS, 0, ctx->stream>>>(
-                cameras, views, gaussians, sh, count, scene_params, splats, tile_counts, depth_keys, order,
+                cameras, views, gaussians, sh, count, scene_params, splats, tile_counts, rects, depth_keys, order,
                 shape.twl, shape.thl));
   return DG_OK;
 }
@@ -1153,12 +1217,17 @@ static dg_status ensure_plan(dg_tile_rasterizer* tr) {
 // The sorted keys in the reference's 64-bit form, rebuilt if the last frame took
 // the depth-first path.
 dg_buffer* rasterizer_sorted_keys(dg_tile_rasterizer* tr) {
-  if (!tr->keys_are_tiles) return tr->keys;
+  if (!tr->keys_are_tiles && !tr->keys_in_ranges) return ensure_pair_sort(tr) == DG_OK ? tr->keys : nullptr;
   if (!tr->keys64 || tr->keys64->bytes < (uint64_t)tr->pair_capacity * 8) {
     free_buffer(tr->keys64);
     tr->keys64 = nullptr;
     if (alloc_buffer(tr->ctx, (size_t)tr->pair_capacity * 8, &tr->keys64) != DG_OK) return nullptr;
   }
+  if (tr->keys_in_ranges)
+    return bin_keys_launch(tr->ctx, tr->tiles_x * tr->tiles_y, typed<uint2>(tr->ranges), typed<uint32_t>(tr->values),
+                           typed<float>(tr->splats), typed<uint64_t>(tr->keys64)) == DG_OK
+               ? tr->keys64
+               : nullptr;
   materialize_keys_kernel<<<std::max(1u, ceil_div(tr->pair_capacity, 256)), 256, 0, tr->ctx->stream>>>(
       typed<uint32_t>(tr->keys), typed<uint32_t>(tr->values), typed<float>(tr->splats), typed<uint32_t>(tr->scan_total),
       tr->pair_capacity, typed<uint64_t>(tr->keys64));
@@ -1267,7 +1336,9 @@ dg_status renderer_launch_forward(dg_renderer* r, dg_buffer* target) {
               preprocess_kernel<<<preprocess_grid(ctx, r->count), PRE_THREADS, 0, ctx->stream>>>(
                   typed<const Camera>(r->camera), typed<float>(r->gaussians), typed<float>(r->sh), r->count,
                   typed<uint32_t>(r->scene_params), typed<float>(r->splats),
-                  typed<uint32_t>(r->rasterizer->tile_offsets), typed<uint32_t>(r->rasterizer->depth_keys),
+                  typed<uint32_t>(r->rasterizer->tile_offsets),
+                  r->rasterizer->binned ? typed<uint32_t>(r->rasterizer->tile_offsets) : nullptr,
+                  typed<uint32_t>(r->rasterizer->depth_keys),
                   typed<uint32_t>(r->rasterizer->depth_values), typed<float>(r->radii)));
   }
   return rasterizer_launch(r->rasterizer, target, true);
@@ -1343,7 +1414,7 @@ dg_status dg_tile_rasterizer_destroy(dg_tile_rasterizer* tr) {
   for (dg_buffer* b : {tr->tile_offsets, tr->scan_total, tr->scan_scratch, tr->raster_params, tr->keys, tr->values,
                        tr->keys_alt, tr->values_alt, tr->sort_scratch, tr->ranges, tr->pixel_color, tr->pixel_last,
                        tr->depth_keys, tr->depth_values, tr->depth_keys_alt, tr->depth_values_alt, tr->depth_scratch,
-                       tr->counts_sorted, tr->keys64, tr->work, tr->work_plan, tr->chunks, tr->checkpoints,
+                       tr->counts_sorted, tr->bin_scratch, tr->keys64, tr->work, tr->work_plan, tr->chunks, tr->checkpoints,
                        tr->blend_mask})
     free_buffer(b);
   for (cudaEvent_t e : tr->readback_events)

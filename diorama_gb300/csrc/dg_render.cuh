@@ -1,5 +1,6 @@
 // Internal view of the renderer's objects, shared with the trainer.
 #pragma once
+#include "dg_bin.cuh"
 #include "dg_common.cuh"
 #include "dg_scan.cuh"
 
@@ -36,10 +37,14 @@ struct dg_tile_rasterizer {
   uint32_t last_pair_count;
   uint32_t tiles_x, tiles_y;
   float viewport[2];
-  // The depth-first tile sort (the renderer's path, dg_render.cu): splats sorted
-  // by depth, their pairs emitted in that order and sorted by tile index alone.
+  // The depth-first tile stage (the renderer's path): splats sorted by depth, then
+  // binned into tiles (dg_bin.cu), or, on a grid that bin_fits refuses, their pairs
+  // emitted in that order and sorted by tile index alone (dg_render.cu).
   bool depth_first;
+  bool binned;          // the prepared frame's tile stage
   bool keys_are_tiles;  // the last frame left u32 tile indices in `keys`
+  bool keys_in_ranges;  // the last frame was binned: it has no keys, only ranges
+  dg_buffer* bin_scratch;
   dg::SortPlan depth_plan, tile_plan;
   dg_buffer* depth_keys;
   dg_buffer* depth_values;  // splat indices, sorted by depth
@@ -108,12 +113,14 @@ struct BlendForward {
   uint32_t* counters;  // 4 words, cleared here
   BlendShape shape;
   bool splat_cutoffs;  // the splats carry their blend cutoff (this build's preprocess wrote them)
+  bool planned;        // plan, chunks and counters are ready (bin_launch wrote them)
 };
 dg_status blend_forward(dg_context* ctx, const BlendForward& f);
 // The batched views' stages (dg_render.cu; used by dg_views.cu).
 dg_status views_preprocess_launch(dg_context* ctx, const Camera* cameras, uint32_t views, const float* gaussians,
                                   const float* sh, uint32_t count, const uint32_t* scene_params, float* splats,
-                                  uint32_t* tile_counts, uint2* depth_keys, uint32_t* order, BlendShape shape);
+                                  uint32_t* tile_counts, uint32_t* rects, uint2* depth_keys, uint32_t* order,
+                                  BlendShape shape);
 dg_status duplicate_sorted_launch(dg_context* ctx, const Camera* camera, const float* splats, const uint32_t* order,
                                   const uint32_t* offsets, uint32_t count, uint32_t per_view, uint32_t view_shift,
                                   uint32_t capacity, uint32_t* keys, uint32_t* values, BlendShape shape);

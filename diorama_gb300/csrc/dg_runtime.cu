@@ -1,5 +1,6 @@
 // Context, buffers and errors: the GPUDevice / GPUQueue / GPUBuffer layer of the
 // reference (src/gpu.ts:8-46, src/readback.ts) on one CUDA device and stream.
+#include "dg_bin.cuh"
 #include "dg_common.cuh"
 #include "dg_scan.cuh"
 
@@ -151,7 +152,9 @@ dg_status dg_context_create(int32_t device, dg_context** out) {
     return cuda_fail(err, "context allocation");
   }
   ctx->staging_bytes = STAGING_BYTES;
-  if (dg_status st = sort_init(); st != DG_OK) {
+  dg_status st = sort_init();
+  if (st == DG_OK) st = bin_init();
+  if (st != DG_OK) {
     dg_context_destroy(ctx);
     return st;
   }

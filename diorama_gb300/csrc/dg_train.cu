@@ -559,7 +559,7 @@ static void drop_graph(dg_trainer* t) {
 
 static dg_status run_graph_step(dg_trainer* t) {
   dg_renderer* r = t->renderer;
-  dg_trainer::Key key{t->count, r->rasterizer->pair_capacity, r->gaussians->ptr, r->rasterizer->keys->ptr,
+  dg_trainer::Key key{t->count, r->rasterizer->pair_capacity, r->gaussians->ptr, r->rasterizer->values->ptr,
                       t->loss->pixel_grads->ptr};
   if (!t->graph_exec || !(key == t->graph_key)) {
     drop_graph(t);

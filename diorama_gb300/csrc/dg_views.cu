@@ -1,7 +1,7 @@
 // Batched rendering of many views of one scene: every stage of the frame runs
 // once over all the views of a batch (one preprocess launch projecting each
-// Gaussian into every view, one depth sort over (view, depth) keys, one tile
-// sort over the views' stacked tile numbers, one blend over all their tiles),
+// Gaussian into every view, one depth sort over (view, depth) keys, one binning of
+// every view's splats into its tiles, one blend over all their tiles),
 // and a batch whose pair count is known is replayed as one CUDA graph. Each view
 // gets exactly the pairs, order and blend of a single-view render, so its image
 // is bit-identical to GaussianRenderer.encode's. The views per batch, the
@@ -46,12 +46,15 @@ using namespace dg;
 struct dg_view_batch {
   dg_context* ctx = nullptr;
   uint32_t views = 0, count = 0, tiles_per_view = 0, pixels = 0;
+  uint32_t grid_x = 0, grid_y = 0;  // blend tiles along each side of a view
   BlendShape shape{0u, 0u};
   uint32_t pair_capacity = 0;
   dg_buffer *cameras = nullptr, *raster_params = nullptr, *splats = nullptr, *tile_counts = nullptr;
   dg_buffer *depth_keys = nullptr, *depth_keys_alt = nullptr, *order = nullptr, *order_alt = nullptr;
   dg_buffer *depth_scratch = nullptr, *counts_sorted = nullptr, *scan_scratch = nullptr, *scan_total = nullptr;
   dg_buffer *keys = nullptr, *keys_alt = nullptr, *values = nullptr, *values_alt = nullptr, *sort_scratch = nullptr;
+  bool binned = false;  // the tile stage: dg_bin.cu, or a sort where bin_fits refuses the grid
+  dg_buffer* bin_scratch = nullptr;
   dg_buffer *ranges = nullptr, *plan = nullptr, *pixel_color = nullptr, *pixel_last = nullptr, *work = nullptr;
   uint32_t* pinned_total = nullptr;
   // The captured batch (valid while its key matches).
@@ -59,10 +62,10 @@ struct dg_view_batch {
   struct Key {
     uint32_t views, count, capacity, coop_min;
     BlendShape shape;
-    const void *gaussians, *targets, *keys;
+    const void *gaussians, *targets, *values;
     bool operator==(const Key& o) const {
       return views == o.views && count == o.count && capacity == o.capacity && coop_min == o.coop_min &&
-             shape == o.shape && gaussians == o.gaussians && targets == o.targets && keys == o.keys;
+             shape == o.shape && gaussians == o.gaussians && targets == o.targets && values == o.values;
     }
   } key{};
   uint32_t last_total = 0;
@@ -75,7 +78,8 @@ void view_batch_destroy(dg_view_batch* b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   for (dg_buffer* x : {b->cameras, b->raster_params, b->splats, b->tile_counts, b->depth_keys, b->depth_keys_alt,
                        b->order, b->order_alt, b->depth_scratch, b->counts_sorted, b->scan_scratch, b->scan_total,
-                       b->keys, b->keys_alt, b->values, b->values_alt, b->sort_scratch, b->ranges, b->plan,
+                       b->keys, b->keys_alt, b->values, b->values_alt, b->sort_scratch, b->bin_scratch, b->ranges,
+                       b->plan,
                        b->pixel_color, b->pixel_last, b->work})
     free_buffer(x);
   if (b->pinned_total) cudaFreeHost(b->pinned_total);
@@ -86,25 +90,34 @@ namespace {
 
 dg_status grow_pairs(dg_view_batch* b, uint32_t capacity) {
   dg_context* ctx = b->ctx;
-  const SortPlan tile_plan = sort_plan_digits(capacity, 1, bits_for(b->tiles_per_view));
-  DG_TRY(ensure(ctx, &b->keys, (size_t)capacity * 4));
-  DG_TRY(ensure(ctx, &b->keys_alt, (size_t)capacity * 4));
   DG_TRY(ensure(ctx, &b->values, (size_t)capacity * 4));
-  DG_TRY(ensure(ctx, &b->values_alt, (size_t)capacity * 4));
-  DG_TRY(ensure(ctx, &b->sort_scratch, sort_scratch_bytes(tile_plan)));
+  if (!b->binned) {
+    const SortPlan tile_plan = sort_plan_digits(capacity, 1, bits_for(b->tiles_per_view));
+    DG_TRY(ensure(ctx, &b->keys, (size_t)capacity * 4));
+    DG_TRY(ensure(ctx, &b->keys_alt, (size_t)capacity * 4));
+    DG_TRY(ensure(ctx, &b->values_alt, (size_t)capacity * 4));
+    DG_TRY(ensure(ctx, &b->sort_scratch, sort_scratch_bytes(tile_plan)));
+  }
   b->pair_capacity = capacity;
   return DG_OK;
 }
 
 // Sizes the batch for `views` views of `count` Gaussians at `pixels` pixels in
-// tiles_per_view blend tiles each.
-dg_status prepare(dg_view_batch* b, uint32_t views, uint32_t count, uint32_t tiles_per_view, uint32_t pixels) {
+// grid_x x grid_y blend tiles each.
+dg_status prepare(dg_view_batch* b, uint32_t views, uint32_t count, uint32_t grid_x, uint32_t grid_y,
+                  uint32_t pixels) {
   dg_context* ctx = b->ctx;
+  const uint32_t tiles_per_view = grid_x * grid_y;
   const size_t n = (size_t)views * count;
   if (n >= (1ull << 31)) return fail(DG_ERROR_INVALID_ARGUMENT, "too many view x Gaussian pairs in one batch");
   if ((uint64_t)views * tiles_per_view >= (1ull << 24))
     return fail(DG_ERROR_INVALID_ARGUMENT, "too many tiles in one batch of views");
-  const bool reshaped = views != b->views || count != b->count || tiles_per_view != b->tiles_per_view;
+  const bool binned = bin_fits(grid_x, grid_y);
+  const bool reshaped = views != b->views || count != b->count || tiles_per_view != b->tiles_per_view ||
+                        binned != b->binned;
+  b->grid_x = grid_x;
+  b->grid_y = grid_y;
+  b->binned = binned;
   b->views = views;
   b->count = count;
   b->tiles_per_view = tiles_per_view;
@@ -119,8 +132,12 @@ dg_status prepare(dg_view_batch* b, uint32_t views, uint32_t count, uint32_t til
   DG_TRY(ensure(ctx, &b->order, n * 4));
   DG_TRY(ensure(ctx, &b->order_alt, n * 4));
   DG_TRY(ensure(ctx, &b->depth_scratch, sort_scratch_bytes(depth_plan)));
-  DG_TRY(ensure(ctx, &b->counts_sorted, n * 4));
-  DG_TRY(ensure(ctx, &b->scan_scratch, scan_scratch_bytes((uint32_t)n)));
+  if (binned) {
+    DG_TRY(ensure(ctx, &b->bin_scratch, bin_scratch_bytes(BinShape{count, views, grid_x, grid_y})));
+  } else {
+    DG_TRY(ensure(ctx, &b->counts_sorted, n * 4));
+    DG_TRY(ensure(ctx, &b->scan_scratch, scan_scratch_bytes((uint32_t)n)));
+  }
   DG_TRY(ensure(ctx, &b->scan_total, 16));
   DG_TRY(ensure(ctx, &b->ranges, (size_t)views * tiles_per_view * 8));
   DG_TRY(ensure(ctx, &b->plan, (PLAN_HEADER + (size_t)views * tiles_per_view) * 4));
@@ -144,31 +161,48 @@ dg_status launch_batch(dg_renderer* r, dg_view_batch* b, uchar4* targets, uint32
   const uint32_t tiles = b->views * b->tiles_per_view;
   DG_TRY(views_preprocess_launch(ctx, typed<Camera>(b->cameras), b->views, typed<float>(r->gaussians),
                                  typed<float>(r->sh), b->count, typed<uint32_t>(r->scene_params),
-                                 typed<float>(b->splats), typed<uint32_t>(b->tile_counts), typed<uint2>(b->depth_keys),
+                                 typed<float>(b->splats), typed<uint32_t>(b->tile_counts),
+                                 b->binned ? typed<uint32_t>(b->tile_counts) : nullptr, typed<uint2>(b->depth_keys),
                                  typed<uint32_t>(b->order), b->shape));
   // (view, depth) keys: 4 passes over the depth bits and one per 8 bits of view.
   const SortPlan depth_plan = sort_plan_digits(n, 2, bits_for(b->views));
   DG_TRY(sort_launch(ctx, depth_plan, b->depth_keys->ptr, typed<uint32_t>(b->order), b->depth_keys_alt->ptr,
                      typed<uint32_t>(b->order_alt), nullptr, b->depth_scratch->ptr));
   uint32_t* order = depth_plan.passes & 1 ? typed<uint32_t>(b->order_alt) : typed<uint32_t>(b->order);
-  DG_TRY(scan_launch(ctx, typed<uint32_t>(b->counts_sorted), n, nullptr, typed<uint32_t>(b->scan_total),
-                     b->scan_scratch->ptr, order, typed<uint32_t>(b->tile_counts)));
-  // Pairs in depth order, view-major, keyed view << shift | local tile: a stable
-  // sort on the local tile's bits alone leaves every (view, tile) run contiguous
-  // and in depth order, an 8-bit pass fewer than sorting global tile numbers.
-  const uint32_t shift = view_shift_for(b->tiles_per_view);
-  DG_TRY(duplicate_sorted_launch(ctx, typed<Camera>(b->cameras), typed<float>(b->splats), order,
-                                 typed<uint32_t>(b->counts_sorted), n, b->count, shift, b->pair_capacity,
-                                 typed<uint32_t>(b->keys), typed<uint32_t>(b->values), b->shape));
-  const SortPlan tile_plan = sort_plan_digits(b->pair_capacity, 1, bits_for(b->tiles_per_view));
-  DG_TRY(sort_launch(ctx, tile_plan, b->keys->ptr, typed<uint32_t>(b->values), b->keys_alt->ptr,
-                     typed<uint32_t>(b->values_alt), typed<uint32_t>(b->scan_total), b->sort_scratch->ptr));
-  const bool odd = tile_plan.passes & 1;
-  const uint32_t* tile_keys = typed<uint32_t>(odd ? b->keys_alt : b->keys);
-  const uint32_t* pair_splats = typed<uint32_t>(odd ? b->values_alt : b->values);
-  DG_CUDA(cudaMemsetAsync(b->ranges->ptr, 0, (size_t)tiles * 8, ctx->stream));
-  DG_TRY(find_view_ranges_launch(ctx, tile_keys, typed<uint32_t>(b->scan_total), b->pair_capacity, shift,
-                                 b->tiles_per_view, tiles, typed<uint2>(b->ranges)));
+  const uint32_t* pair_splats = typed<uint32_t>(b->values);
+  if (b->binned) {
+    BinLaunch l{};
+    l.rects = typed<uint32_t>(b->tile_counts);
+    l.order = order;
+    l.capacity = b->pair_capacity;
+    l.coop_min = coop_min;
+    l.scratch = b->bin_scratch->ptr;
+    l.pair_total = typed<uint32_t>(b->scan_total);
+    l.values = typed<uint32_t>(b->values);
+    l.ranges = typed<uint2>(b->ranges);
+    l.plan = typed<uint32_t>(b->plan);
+    l.work = typed<uint32_t>(b->work);
+    DG_TRY(bin_launch(ctx, BinShape{b->count, b->views, b->grid_x, b->grid_y}, l));
+  } else {
+    DG_TRY(scan_launch(ctx, typed<uint32_t>(b->counts_sorted), n, nullptr, typed<uint32_t>(b->scan_total),
+                       b->scan_scratch->ptr, order, typed<uint32_t>(b->tile_counts)));
+    // Pairs in depth order, view-major, keyed view << shift | local tile: a stable
+    // sort on the local tile's bits alone leaves every (view, tile) run contiguous
+    // and in depth order, an 8-bit pass fewer than sorting global tile numbers.
+    const uint32_t shift = view_shift_for(b->tiles_per_view);
+    DG_TRY(duplicate_sorted_launch(ctx, typed<Camera>(b->cameras), typed<float>(b->splats), order,
+                                   typed<uint32_t>(b->counts_sorted), n, b->count, shift, b->pair_capacity,
+                                   typed<uint32_t>(b->keys), typed<uint32_t>(b->values), b->shape));
+    const SortPlan tile_plan = sort_plan_digits(b->pair_capacity, 1, bits_for(b->tiles_per_view));
+    DG_TRY(sort_launch(ctx, tile_plan, b->keys->ptr, typed<uint32_t>(b->values), b->keys_alt->ptr,
+                       typed<uint32_t>(b->values_alt), typed<uint32_t>(b->scan_total), b->sort_scratch->ptr));
+    const bool odd = tile_plan.passes & 1;
+    const uint32_t* tile_keys = typed<uint32_t>(odd ? b->keys_alt : b->keys);
+    if (odd) pair_splats = typed<uint32_t>(b->values_alt);
+    DG_CUDA(cudaMemsetAsync(b->ranges->ptr, 0, (size_t)tiles * 8, ctx->stream));
+    DG_TRY(find_view_ranges_launch(ctx, tile_keys, typed<uint32_t>(b->scan_total), b->pair_capacity, shift,
+                                   b->tiles_per_view, tiles, typed<uint2>(b->ranges)));
+  }
   BlendForward f{};
   f.camera = typed<Camera>(b->cameras);
   f.raster_params = typed<float4>(b->raster_params);
@@ -185,6 +219,7 @@ dg_status launch_batch(dg_renderer* r, dg_view_batch* b, uchar4* targets, uint32
   f.counters = typed<uint32_t>(b->work);
   f.shape = b->shape;
   f.splat_cutoffs = true;  // preprocess_views_kernel's splats
+  f.planned = b->binned;
   DG_TRY(blend_forward(ctx, f));
   DG_CUDA(cudaMemcpyAsync(b->pinned_total, b->scan_total->ptr, 4, cudaMemcpyDeviceToHost, ctx->stream));
   return DG_OK;
@@ -196,9 +231,8 @@ dg_status render_batch(dg_renderer* r, dg_view_batch* b, const dg_camera* cams, 
                        uchar4* targets, uint32_t coop_min, BlendShape shape, bool use_graph) {
   dg_context* ctx = r->ctx;
   const uint32_t w = (uint32_t)cams[0].viewport[0], h = (uint32_t)cams[0].viewport[1];
-  const uint32_t tiles_per_view =
-      blend_tiles_along(ceil_div(w, TILE), shape.twl) * blend_tiles_along(ceil_div(h, TILE), shape.thl);
-  DG_TRY(prepare(b, count, r->count, tiles_per_view, w * h));
+  DG_TRY(prepare(b, count, r->count, blend_tiles_along(ceil_div(w, TILE), shape.twl),
+                 blend_tiles_along(ceil_div(h, TILE), shape.thl), w * h));
   b->shape = shape;
   std::vector<Camera> cameras(count);
   for (uint32_t k = 0; k < count; k++) {
@@ -214,7 +248,7 @@ dg_status render_batch(dg_renderer* r, dg_view_batch* b, const dg_camera* cams, 
   DG_TRY(write_async(ctx, b->raster_params->ptr, params, sizeof(params)));
   for (int attempt = 0; attempt < 2; attempt++) {
     const dg_view_batch::Key key{count, r->count, b->pair_capacity, coop_min, shape, r->gaussians->ptr, targets,
-                                 b->keys->ptr};
+                                 b->values->ptr};
     if (use_graph) {
       if (!b->graph || !(key == b->key)) {
         if (b->graph) cudaGraphExecDestroy(b->graph);
