@@ -4,28 +4,39 @@
 //
 // The reference finds the neighbours by brute force (src/shaders/nearestNeighbors.wgsl:13-44),
 // N² distances. Here the points are sorted along a Morton (Z-order) curve of 21
-// bits per axis, which makes every cell of the implicit octree over the points a
-// contiguous run of the sorted array. Each point then
-//   1. takes the third-smallest squared distance R² among its 2·WINDOW neighbours
-//      in curve order: its three nearest points lie within R;
-//   2. picks the finest octree level whose cells are at least R (plus a rounding
-//      margin) wide, so that every point within R lies in its own cell at that
-//      level or one of the 26 around it;
-//   3. scans those cells (a galloping binary search finds each one's run), skipping
-//      a cell once its nearest face is farther than the best third distance so far.
+// bits per axis, and each 32 consecutive ones (a leaf) get their bounding box, each
+// 32 leaves theirs, and so on up to at most 32 boxes. A warp then answers the 32
+// queries of one leaf together:
+//   1. every lane offers its point the leaf's other points and the two leaves beside
+//      it on the curve: a first bound on each third-smallest distance;
+//   2. the warp descends the tree, of a node's children (a lane each) the nearest to
+//      any of its points first, leaving out those no point is near enough to;
+//   3. a leaf it reaches is read once and offered to all 32 points (or, when few
+//      of them are near enough, to those).
+// One thread per point descending an octree by binary searches of the curve (27
+// cells a point) took 1,519 us for a clustered cloud of 180,000 points where this
+// takes 195: its threads waited for the warp's longest search and for one dependent
+// load after another; here 32 points share every box and every point that is read.
+// (The whole call: 1,448 -> 335 us.) What bounds
+// it: instructions at 1.1M points (16 a distance, 512 a leaf, about 28 leaves a
+// warp); at 180,000, whose warps all run at once, the longest walks.
+//
 // The search is exact: it finds the same three smallest squared distances, each
 // computed as the reference computes it (d = q - p, then d.x² + d.y² + d.z²
 // rounded in that order; this file is compiled without contraction), so every
-// result is the brute force's bit for bit. The visiting order does not matter:
+// result is the brute force's bit for bit. A box's distance is computed by the same
+// rounded operations from its nearest faces; each of them is monotone, so no point
+// in the box has a smaller computed distance, and a box at or past the third
+// distance so far cannot hold a smaller one. The visiting order does not matter:
 // the three smallest values of a set do not depend on the order they are met in.
 //
-// The octree spans the points' bounds trimmed to the mean ± 3 standard deviations
+// The curve spans the points' bounds trimmed to the mean ± 3 standard deviations
 // per axis (so that a few far outliers do not coarsen it); points outside are
-// clamped onto its border. Quantizing is monotone and non-expansive in each
-// coordinate, so the cell arguments above hold for clamped points too. Points
-// with a non-finite coordinate are no point's neighbours (their distances are
-// infinite or NaN, never below the starting 3.4e38) and get the reference's
-// result for a point without neighbours.
+// clamped onto its border. Points with a non-finite coordinate are no point's
+// neighbours (their distances are infinite or NaN, never below the starting 3.4e38),
+// so the boxes leave them out, and they get the reference's result for a point
+// without neighbours.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -36,77 +47,135 @@ namespace dg {
 namespace {
 
 constexpr uint32_t KNN_THREADS = 256;
-constexpr uint32_t BITS = 21;         // per axis: 63-bit Morton codes
-constexpr int32_t WINDOW = 8;         // curve neighbours on each side for the first bound
+constexpr uint32_t BITS = 21;  // per axis: 63-bit Morton codes
+constexpr uint32_t LEVELS = 6;  // of boxes: 32^6 points
+constexpr uint32_t QUERY_WARPS = 4;
+constexpr int FEW = 16;  // queries that a leaf is offered to one by one (10 and 22 measured the same)
 constexpr float FAR = 3.4e38f;        // nearestNeighbors.wgsl:19, the starting "distance"
 
 struct Octree {
   float lo[3];
   float scale;  // finest cells per unit length
-  float h0;     // finest cell width
-  float slack;  // margin for rounding in the quantizing and in the cell faces
 };
 
-// Order-preserving u32 image of a float, for atomicMin/atomicMax.
-__device__ __forceinline__ uint32_t ordered(float f) {
-  const uint32_t b = __float_as_uint(f);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
-inline float unordered(uint32_t o) {
-  const uint32_t b = (o & 0x80000000u) ? (o & 0x7fffffffu) : ~o;
-  float f;
-  std::memcpy(&f, &b, 4);
-  return f;
-}
-
+// The finite points' bounds and moments.
 struct Moments {
-  uint32_t lo[3], hi[3];  // ordered images
-  double sum[3], sum2[3];
-  uint32_t finite;        // points with three finite coordinates
+  float lo[3], hi[3];
+  double sum[3], sum2[3];  // of the coordinates less the first point's
+  uint32_t finite;         // points with three finite coordinates
 };
 
 __device__ __forceinline__ bool finite3(float4 p) { return isfinite(p.x) && isfinite(p.y) && isfinite(p.z); }
 
+__device__ __forceinline__ Moments no_moments() {
+  Moments m;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    m.lo[k] = INFINITY;
+    m.hi[k] = -INFINITY;
+    m.sum[k] = m.sum2[k] = 0.0;
+  }
+  m.finite = 0;
+  return m;
+}
+
+__device__ __forceinline__ void add_moments(Moments& m, const Moments& o) {
+  m.finite += o.finite;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    m.lo[k] = fminf(m.lo[k], o.lo[k]);
+    m.hi[k] = fmaxf(m.hi[k], o.hi[k]);
+    m.sum[k] += o.sum[k];
+    m.sum2[k] += o.sum2[k];
+  }
+}
+
+// Sums m over the CTA; thread 0 gets the whole.
+__device__ __forceinline__ void reduce_moments(Moments& m, Moments* s_warp) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    Moments o;
+    o.finite = __shfl_xor_sync(0xffffffffu, m.finite, off);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      o.lo[k] = __shfl_xor_sync(0xffffffffu, m.lo[k], off);
+      o.hi[k] = __shfl_xor_sync(0xffffffffu, m.hi[k], off);
+      o.sum[k] = __shfl_xor_sync(0xffffffffu, m.sum[k], off);
+      o.sum2[k] = __shfl_xor_sync(0xffffffffu, m.sum2[k], off);
+    }
+    add_moments(m, o);
+  }
+  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (uint32_t w = 1; w < KNN_THREADS / 32; w++) add_moments(m, s_warp[w]);
+}
+
+// Each CTA's share of the moments (4,900 warps adding to one global record took
+// 70 us at 180,000 points).
 __global__ void __launch_bounds__(KNN_THREADS) bounds_kernel(const float4* __restrict__ points, uint32_t n,
-                                                             Moments* __restrict__ out) {
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  double sum[3] = {0, 0, 0}, sum2[3] = {0, 0, 0};
-  uint32_t finite = 0;
+                                                             Moments* __restrict__ shares) {
+  __shared__ Moments s_warp[KNN_THREADS / 32];
+  Moments m = no_moments();
+  const float origin[3] = {finite3(points[0]) ? points[0].x : 0.0f, finite3(points[0]) ? points[0].y : 0.0f,
+                           finite3(points[0]) ? points[0].z : 0.0f};
+  // A thread's few points add up in float32: the moments only shape the curve, and
+  // FP64 runs at a fraction of its rate.
+  float sum[3] = {0.0f, 0.0f, 0.0f}, sum2[3] = {0.0f, 0.0f, 0.0f};
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 p = points[i];
     if (!finite3(p)) continue;
     const float c[3] = {p.x, p.y, p.z};
-    finite++;
+    m.finite++;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      lo[k] = fminf(lo[k], c[k]);
-      hi[k] = fmaxf(hi[k], c[k]);
-      sum[k] += c[k];
-      sum2[k] += (double)c[k] * c[k];
+      m.lo[k] = fminf(m.lo[k], c[k]);
+      m.hi[k] = fmaxf(m.hi[k], c[k]);
+      const float d = c[k] - origin[k];
+      sum[k] += d;
+      sum2[k] += d * d;
     }
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    finite += __shfl_xor_sync(0xffffffffu, finite, off);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], off));
-      hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], off));
-      sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], off);
-      sum2[k] += __shfl_xor_sync(0xffffffffu, sum2[k], off);
-    }
+  for (int k = 0; k < 3; k++) {
+    m.sum[k] = sum[k];
+    m.sum2[k] = sum2[k];
   }
-  if ((threadIdx.x & 31) == 0 && finite) {
-    atomicAdd(&out->finite, finite);
+  reduce_moments(m, s_warp);
+  if (threadIdx.x == 0) shares[blockIdx.x] = m;
+}
+
+// The octree for the shares' bounds and moments. One CTA.
+__global__ void __launch_bounds__(KNN_THREADS) octree_kernel(const float4* __restrict__ points,
+                                                             const Moments* __restrict__ shares, uint32_t count,
+                                                             Octree* __restrict__ out) {
+  __shared__ Moments s_warp[KNN_THREADS / 32];
+  Moments m = no_moments();
+  for (uint32_t k = threadIdx.x; k < count; k += KNN_THREADS) add_moments(m, shares[k]);
+  reduce_moments(m, s_warp);
+  if (threadIdx.x != 0) return;
+  Octree o;
+  const float origin[3] = {finite3(points[0]) ? points[0].x : 0.0f, finite3(points[0]) ? points[0].y : 0.0f,
+                           finite3(points[0]) ? points[0].z : 0.0f};
+  const double inv = 1.0 / (m.finite ? (double)m.finite : 1.0);
+  float extent = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      atomicMin(&out->lo[k], ordered(lo[k]));
-      atomicMax(&out->hi[k], ordered(hi[k]));
-      atomicAdd(&out->sum[k], sum[k]);
-      atomicAdd(&out->sum2[k], sum2[k]);
+  for (int k = 0; k < 3; k++) {
+    float lo = m.lo[k], hi = m.hi[k];
+    if (!(lo <= hi)) lo = hi = 0.0f;  // no finite points
+    const double mean = m.sum[k] * inv;
+    const float centre = origin[k] + (float)mean, reach = 3.0f * sqrtf((float)fmax(0.0, m.sum2[k] * inv - mean * mean));
+    if (isfinite(centre) && isfinite(reach)) {
+      lo = fmaxf(lo, centre - reach);
+      hi = fminf(hi, centre + reach);
+      if (!(lo <= hi)) lo = hi = centre;
     }
+    o.lo[k] = lo;
+    extent = fmaxf(extent, hi - lo);
   }
+  if (!(extent > 0.0f) || !isfinite(extent)) extent = 1.0f;
+  o.scale = (float)(1u << BITS) / extent;
+  *out = o;
 }
 
 // Finest-level cell coordinate of a position, clamped into the octree (NaN
@@ -136,10 +205,11 @@ __device__ __forceinline__ uint64_t morton(uint32_t x, uint32_t y, uint32_t z) {
 }
 
 // Each point's Morton code (the sort key, as (low, high) words) and index.
-__global__ void morton_kernel(const float4* __restrict__ points, uint32_t n, Octree o, uint2* __restrict__ keys,
-                              uint32_t* __restrict__ values) {
+__global__ void morton_kernel(const float4* __restrict__ points, uint32_t n, const Octree* __restrict__ octree,
+                              uint2* __restrict__ keys, uint32_t* __restrict__ values) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  const Octree o = *octree;
   const float4 p = points[i];
   uint32_t q[3];
   quantize(o, p.x, p.y, p.z, q);
@@ -148,34 +218,75 @@ __global__ void morton_kernel(const float4* __restrict__ points, uint32_t n, Oct
   values[i] = i;
 }
 
-// The points in curve order, each carrying its original index in w.
-__global__ void gather_points_kernel(const float4* __restrict__ points, uint32_t n, const uint32_t* __restrict__ order,
-                                     float4* __restrict__ sorted) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const uint32_t i = order[s];
-  const float4 p = points[i];
-  sorted[s] = make_float4(p.x, p.y, p.z, __uint_as_float(i));
+// A box of finite points (lo above hi when it holds none).
+struct Box {
+  float4 lo, hi;
+};
+
+// The union of the warp's 32 boxes, on every lane.
+__device__ __forceinline__ Box warp_box(Box b) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    b.lo.x = fminf(b.lo.x, __shfl_xor_sync(0xffffffffu, b.lo.x, off));
+    b.lo.y = fminf(b.lo.y, __shfl_xor_sync(0xffffffffu, b.lo.y, off));
+    b.lo.z = fminf(b.lo.z, __shfl_xor_sync(0xffffffffu, b.lo.z, off));
+    b.hi.x = fmaxf(b.hi.x, __shfl_xor_sync(0xffffffffu, b.hi.x, off));
+    b.hi.y = fmaxf(b.hi.y, __shfl_xor_sync(0xffffffffu, b.hi.y, off));
+    b.hi.z = fmaxf(b.hi.z, __shfl_xor_sync(0xffffffffu, b.hi.z, off));
+  }
+  return b;
 }
+
+__device__ __forceinline__ Box no_box() {
+  return Box{make_float4(INFINITY, INFINITY, INFINITY, 0.0f), make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f)};
+}
+
+// The points in curve order, each carrying its original index in w, and the box of
+// each 32.
+__global__ void __launch_bounds__(KNN_THREADS) gather_points_kernel(const float4* __restrict__ points, uint32_t n,
+                                                                    const uint32_t* __restrict__ order,
+                                                                    float4* __restrict__ sorted,
+                                                                    Box* __restrict__ leaves) {
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  Box b = no_box();
+  if (s < n) {
+    const uint32_t i = order[s];
+    const float4 p = points[i];
+    sorted[s] = make_float4(p.x, p.y, p.z, __uint_as_float(i));
+    if (finite3(p)) b = Box{p, p};
+  }
+  b = warp_box(b);
+  if ((s & 31u) == 0 && s < n) leaves[s >> 5] = b;
+}
+
+// The boxes of each 32 of `count` boxes.
+__global__ void __launch_bounds__(KNN_THREADS) parents_kernel(const Box* __restrict__ boxes, uint32_t count,
+                                                              Box* __restrict__ parents) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  Box b = no_box();
+  if (i < count) b = boxes[i];
+  b = warp_box(b);
+  if ((i & 31u) == 0 && i < count) parents[i >> 5] = b;
+}
+
+struct Tree {
+  const Box* boxes[LEVELS];  // level 0: the leaves
+  uint32_t count[LEVELS];
+  uint32_t top;  // the first level of at most 32 boxes
+};
 
 struct Best {
   float x = FAR, y = FAR, z = FAR;  // the three smallest squared distances, smallest first
 
-  // nearestNeighbors.wgsl:26-41
+  // nearestNeighbors.wgsl:26-41, without branches: a distance that is not below the
+  // third (or is NaN) is taken as FAR, which changes nothing.
   __device__ __forceinline__ void offer(float d2) {
-    if (d2 < z) {
-      if (d2 < y) {
-        z = y;
-        if (d2 < x) {
-          y = x;
-          x = d2;
-        } else {
-          y = d2;
-        }
-      } else {
-        z = d2;
-      }
-    }
+    const float d = d2 < z ? d2 : FAR;
+    const float a = fmaxf(x, d);
+    x = fminf(x, d);
+    const float b = fmaxf(y, a);
+    y = fminf(y, a);
+    z = fminf(z, b);
   }
 };
 
@@ -184,166 +295,130 @@ __device__ __forceinline__ float distance2(float4 q, float px, float py, float p
   return dx * dx + dy * dy + dz * dz;
 }
 
-__device__ __forceinline__ uint64_t key_at(const uint2* __restrict__ keys, int32_t i) {
-  const uint2 k = keys[i];
-  return (uint64_t)k.y << 32 | k.x;
+// No point of box b has a smaller distance2 from any point of [lo, hi] than this.
+__device__ __forceinline__ float gap2(const Box& b, float4 lo, float4 hi) {
+  const float dx = fmaxf(fmaxf(b.lo.x - hi.x, lo.x - b.hi.x), 0.0f);
+  const float dy = fmaxf(fmaxf(b.lo.y - hi.y, lo.y - b.hi.y), 0.0f);
+  const float dz = fmaxf(fmaxf(b.lo.z - hi.z, lo.z - b.hi.z), 0.0f);
+  return dx * dx + dy * dy + dz * dz;
 }
 
-// The first index whose key is >= target, searched outwards from `from`
-// (galloping, then binary): a few steps for a cell near the point's own.
-__device__ int32_t lower_bound_from(const uint2* __restrict__ keys, int32_t n, int32_t from, uint64_t target) {
-  int32_t lo, hi;  // keys[lo] < target <= keys[hi], with lo = -1 or hi = n at the ends
-  if (key_at(keys, from) < target) {
-    lo = from;
-    int32_t step = 1;
-    hi = from + 1;
-    while (hi < n && key_at(keys, hi) < target) {
-      lo = hi;
-      step <<= 1;
-      hi = from + step < n ? from + step : n;
-    }
-  } else {
-    hi = from;
-    int32_t step = 1;
-    lo = from - 1;
-    while (lo >= 0 && key_at(keys, lo) >= target) {
-      hi = lo;
-      step <<= 1;
-      lo = from - step >= 0 ? from - step : -1;
-    }
-  }
-  while (hi - lo > 1) {
-    const int32_t mid = lo + ((hi - lo) >> 1);
-    if (key_at(keys, mid) < target) lo = mid;
-    else hi = mid;
-  }
-  return hi;
-}
-
-// The first index in [lo, hi) whose key is >= target (hi if none).
-__device__ __forceinline__ int32_t lower_bound_in(const uint2* __restrict__ keys, int32_t lo, int32_t hi,
-                                                  uint64_t target) {
-  while (lo < hi) {
-    const int32_t mid = lo + ((hi - lo) >> 1);
-    if (key_at(keys, mid) < target) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// A lower bound on the squared distance from p to any point of cell c at
-// `level`, less the rounding margin per axis. The border cells' outer faces are
-// open: the points clamped onto the border lie beyond them.
-__device__ __forceinline__ float cell_gap2(const Octree& o, const float p[3], const uint32_t c[3], uint32_t level) {
-  const float h = ldexpf(o.h0, (int)level);
-  const uint32_t last = (1u << (BITS - level)) - 1u;
-  float g2 = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    float g = 0.0f;
-    if (c[k] > 0) g = fmaxf(g, (o.lo[k] + (float)c[k] * h) - p[k]);
-    if (c[k] < last) g = fmaxf(g, p[k] - (o.lo[k] + (float)(c[k] + 1) * h));
-    g = fmaxf(g - o.slack, 0.0f);
-    g2 += g * g;
-  }
-  return g2;
-}
-
-// A cell being searched: its coordinates at `level`, its run of the sorted
-// points, and the next of its 8 children to try.
-struct Frame {
-  uint32_t c[3];
-  int32_t begin, end;
-  uint32_t level, next;
-};
-
-constexpr int32_t LEAF = 32;  // cells with at most this many points are scanned whole
-
-// One thread per point, in curve order (a warp's points are neighbours and
-// search the same cells). A cell of more than LEAF points is searched through its
-// children, nearest first (the child on the point's side of each axis, then those
-// differing in one axis, two, three), each skipped once its box is farther than
-// the best third distance so far: a point beside a dense region visits only the
-// part of it that can hold a nearer point.
-__global__ void __launch_bounds__(KNN_THREADS) knn_query_kernel(const float4* __restrict__ sorted,
-                                                                const uint2* __restrict__ keys, uint32_t n, Octree o,
-                                                                float* __restrict__ distance2_out) {
-  const int32_t s = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (s >= (int32_t)n) return;
-  const float4 me = sorted[s];
-  const uint32_t self = __float_as_uint(me.w);
-  if (!finite3(me)) {
-    distance2_out[self] = (FAR + FAR + FAR) / 3.0f;  // no neighbours: nearestNeighbors.wgsl:43
-    return;
-  }
-  const int32_t count = (int32_t)n;
-  // 1. A first bound from the curve neighbours.
-  Best window;
-  for (int32_t j = max(s - WINDOW, 0); j <= min(s + WINDOW, count - 1); j++)
-    if (j != s) window.offer(distance2(sorted[j], me.x, me.y, me.z));
-  // Every point with a computed squared distance <= window.z is within `reach`
-  // (the factor covers the rounding of the computed distances).
-  const float reach = sqrtf(window.z) * 1.000001f + o.slack;
-  // 2. The finest level whose cells are at least `reach` wide (the root if none):
-  // every point within `reach` is in the point's cell or one of the 26 around it.
-  uint32_t level = 0;
-  while (level < BITS && ldexpf(o.h0, (int)level) < reach) level++;
-  uint32_t q[3];
-  quantize(o, me.x, me.y, me.z, q);
-  const int32_t cells = 1 << (BITS - level);
-  const int32_t c[3] = {(int32_t)(q[0] >> level), (int32_t)(q[1] >> level), (int32_t)(q[2] >> level)};
-  const float p[3] = {me.x, me.y, me.z};
-  // 3. The point's own cell, then the 26 around it, each searched down to leaves.
+// A warp per leaf. (Two or four lanes per query, so two or four warps per leaf, were
+// no faster from 10,000 points on, and half as fast at 1.1M.)
+__global__ void __launch_bounds__(QUERY_WARPS * 32) knn_query_kernel(const float4* __restrict__ sorted, uint32_t n,
+                                                                     const Tree tree,
+                                                                     float* __restrict__ distance2_out) {
+  __shared__ float4 s_points[QUERY_WARPS][32];
+  __shared__ Box s_boxes[QUERY_WARPS][32];
+  __shared__ uint32_t s_key[QUERY_WARPS][LEVELS][32];
+  __shared__ uint32_t s_base[QUERY_WARPS][LEVELS];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t leaf = blockIdx.x * QUERY_WARPS + warp;
+  if (leaf >= tree.count[0]) return;
+  const uint32_t s = leaf * 32 + lane;
+  const float4 me = s < n ? sorted[s] : make_float4(NAN, NAN, NAN, 0.0f);
+  const bool query = finite3(me);
+  const Box own = tree.boxes[0][leaf];
+  float4* points = s_points[warp];
+  Box* boxes = s_boxes[warp];
+  uint32_t(*keys)[32] = s_key[warp];
+  uint32_t* base = s_base[warp];
   Best best;
-  Frame stack[BITS + 1];
-  for (int32_t cell = 0; cell < 27 && best.z != 0.0f; cell++) {
-    const int32_t t = cell == 0 ? 13 : (cell <= 13 ? cell - 1 : cell);  // 13 is the centre
-    const int32_t cc[3] = {c[0] + t % 3 - 1, c[1] + (t / 3) % 3 - 1, c[2] + t / 9 - 1};
-    if (cc[0] < 0 || cc[1] < 0 || cc[2] < 0 || cc[0] >= cells || cc[1] >= cells || cc[2] >= cells) continue;
-    const uint32_t uc[3] = {(uint32_t)cc[0], (uint32_t)cc[1], (uint32_t)cc[2]};
-    if (cell_gap2(o, p, uc, level) > fminf(window.z, best.z) * 1.000002f) continue;
-    const uint64_t prefix = morton(uc[0], uc[1], uc[2]);
-    const int32_t begin = lower_bound_from(keys, count, s, prefix << (3 * level));
-    const int32_t end = lower_bound_from(keys, count, s, (prefix + 1) << (3 * level));
-    if (begin == end) continue;
-    int32_t top = 0;
-    stack[0] = Frame{{uc[0], uc[1], uc[2]}, begin, end, level, 0};
-    while (top >= 0 && best.z != 0.0f) {  // a zero third distance cannot improve
-      Frame& f = stack[top];
-      if (f.next == 0 && (f.end - f.begin <= LEAF || f.level == 0)) {
-        for (int32_t j = f.begin; j < f.end; j++)
-          if (j != s) best.offer(distance2(sorted[j], me.x, me.y, me.z));
-        top--;
-        continue;
-      }
-      if (f.next == 8) {
-        top--;
-        continue;
-      }
-      // Nearest child first: per axis, the half on the point's side.
-      const uint32_t cl = f.level - 1;
-      uint32_t near = 0;
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        const uint32_t pk = q[k] >> f.level;
-        const uint32_t side = pk == f.c[k] ? (q[k] >> cl) & 1u : (pk > f.c[k] ? 1u : 0u);
-        near |= side << k;
-      }
-      // Nibble i of `order` is the i-th child's offset from the nearest (XOR):
-      // 0, then 1, 2, 4 (one axis apart), 3, 5, 6 (two), 7 (the far corner).
-      constexpr uint32_t order = 0x76534210u;
-      const uint32_t k = ((order >> (4 * f.next)) & 0xfu) ^ near;
-      f.next++;
-      const uint32_t ch[3] = {2 * f.c[0] + (k & 1u), 2 * f.c[1] + ((k >> 1) & 1u), 2 * f.c[2] + (k >> 2)};
-      if (cell_gap2(o, p, ch, cl) > fminf(window.z, best.z) * 1.000002f) continue;
-      const uint64_t cp = morton(ch[0], ch[1], ch[2]);
-      const int32_t cb = lower_bound_in(keys, f.begin, f.end, cp << (3 * cl));
-      const int32_t ce = lower_bound_in(keys, cb, f.end, (cp + 1) << (3 * cl));
-      if (cb == ce) continue;
-      stack[++top] = Frame{{ch[0], ch[1], ch[2]}, cb, ce, cl, 0};
+  // The largest third distance of the queries (of non-negative floats the bits compare alike).
+  auto worst = [&]() { return __uint_as_float(__reduce_max_sync(0xffffffffu, query ? __float_as_uint(best.z) : 0u)); };
+  // Offers the 32 points of leaf f to every query (its own point is not its neighbour;
+  // past the end NaN).
+  auto offer_leaf = [&](uint32_t f, bool mine) {
+    __syncwarp();
+    points[lane] = f * 32 + lane < n ? sorted[f * 32 + lane] : make_float4(NAN, NAN, NAN, 0.0f);
+    __syncwarp();
+#pragma unroll 8
+    for (uint32_t j = 0; j < 32; j++) {
+      const float d = distance2(points[j], me.x, me.y, me.z);
+      best.offer(mine && j == lane ? FAR : d);
     }
+  };
+  offer_leaf(leaf, true);
+  if (leaf > 0) offer_leaf(leaf - 1, false);
+  if (leaf + 1 < tree.count[0]) offer_leaf(leaf + 1, false);
+  float bound = worst();
+  // A lane's child of the node at hand: the distance of the query nearest to it, with
+  // the lane in the low bits (rounded down: still a lower bound), or all ones when it
+  // is out of reach of all. The queries' own box sorts out most children at once; the
+  // rest are held against the queries one after another, independently. (Scattered
+  // outliers have a box that reaches everywhere, while they need about 30 leaves like
+  // the others.)
+  auto expand = [&](uint32_t level, uint32_t first) {
+    Box b = no_box();
+    if (first + lane < tree.count[level]) b = tree.boxes[level][first + lane];
+    __syncwarp();
+    boxes[lane] = b;
+    uint32_t left = __ballot_sync(0xffffffffu, gap2(b, own.lo, own.hi) < bound);
+    __syncwarp();
+    uint32_t key = ~0u;
+    while (left) {  // four at a time
+      uint32_t child[4], nearest[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++) {
+        child[u] = left ? __ffs(left) - 1 : child[0];
+        left &= left - 1;
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++) {
+        const float g = gap2(boxes[child[u]], me, me);
+        nearest[u] = __reduce_min_sync(0xffffffffu, query && g < best.z ? __float_as_uint(g) : ~0u);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++)
+        if (lane == child[u] && nearest[u] != ~0u) key = (nearest[u] & ~31u) | lane;
+    }
+    keys[level][lane] = key;
+    if (lane == 0) base[level] = first;
+    __syncwarp();
+  };
+  uint32_t level = tree.top;
+  expand(level, 0);
+  while (true) {
+    const uint32_t next = __reduce_min_sync(0xffffffffu, keys[level][lane]);
+    if (next == ~0u || __uint_as_float(next & ~31u) >= bound) {
+      if (level == tree.top) break;
+      level++;
+      continue;
+    }
+    const uint32_t child = next & 31u, node = base[level] + child;
+    __syncwarp();
+    if (lane == child) keys[level][lane] = ~0u;
+    __syncwarp();
+    if (level > 0) {
+      expand(--level, node * 32);
+      continue;
+    }
+    if (node + 1 >= leaf && node <= leaf + 1) continue;  // offered above
+    uint32_t near = __ballot_sync(0xffffffffu, query && gap2(tree.boxes[0][node], me, me) < best.z);
+    if (near == 0) continue;
+    if (__popc(near) > FEW) {
+      offer_leaf(node, false);
+    } else {
+      // For few queries, a lane per point of the leaf: each query's points below its
+      // third distance (mostly none) are offered to its lane.
+      const uint32_t at = node * 32 + lane;
+      const float4 p = at < n ? sorted[at] : make_float4(NAN, NAN, NAN, 0.0f);
+      for (; near; near &= near - 1) {
+        const int q = __ffs(near) - 1;
+        const float d = distance2(p, __shfl_sync(0xffffffffu, me.x, q), __shfl_sync(0xffffffffu, me.y, q),
+                                  __shfl_sync(0xffffffffu, me.z, q));
+        const float third = __shfl_sync(0xffffffffu, best.z, q);
+        for (uint32_t hits = __ballot_sync(0xffffffffu, d < third); hits; hits &= hits - 1) {
+          const float found = __shfl_sync(0xffffffffu, d, __ffs(hits) - 1);
+          if ((int)lane == q) best.offer(found);
+        }
+      }
+    }
+    bound = worst();
   }
-  distance2_out[self] = (best.x + best.y + best.z) / 3.0f;  // nearestNeighbors.wgsl:43
+  // nearestNeighbors.wgsl:43; a point that is not finite has no neighbours.
+  if (s < n)
+    distance2_out[__float_as_uint(me.w)] = query ? (best.x + best.y + best.z) / 3.0f : (FAR + FAR + FAR) / 3.0f;
 }
 
 __global__ void pad_points_kernel(const float* __restrict__ positions, uint32_t n, float4* __restrict__ points) {
@@ -396,69 +471,54 @@ struct Scratch {
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// The octree for these bounds and moments.
-Octree choose_octree(const Moments& m) {
-  Octree o{};
-  const double count = m.finite ? (double)m.finite : 1.0;
-  double extent = 0.0, maxabs = 0.0;
-  for (int k = 0; k < 3; k++) {
-    double lo = unordered(m.lo[k]), hi = unordered(m.hi[k]);
-    if (!(lo <= hi)) lo = hi = 0.0;  // no finite points
-    const double mean = m.sum[k] / count;
-    const double sd = std::sqrt(std::max(0.0, m.sum2[k] / count - mean * mean));
-    lo = std::max(lo, mean - 3.0 * sd);
-    hi = std::min(hi, mean + 3.0 * sd);
-    if (!(lo <= hi)) lo = hi = mean;
-    o.lo[k] = (float)lo;
-    extent = std::max(extent, hi - lo);
-    maxabs = std::max(maxabs, std::max(std::fabs(lo), std::fabs(hi)));
-  }
-  if (!(extent > 0.0) || !std::isfinite(extent)) extent = 1.0;
-  const double cells = (double)(1u << BITS);
-  o.scale = (float)(cells / extent);
-  o.h0 = (float)(extent / cells);
-  // Quantizing rounds (p - lo) and the product with scale, and the faces
-  // lo + c·h round too: a few finest cells plus a few ulps of the coordinates.
-  o.slack = (float)(4.0 * extent / cells + 8.0 * maxabs * 1.2e-7);
-  return o;
-}
-
 // Mean neighbour distances of n points (float4, xyz + padding) into distance2.
-// Blocks on one readback of the bounds.
 dg_status neighbor_distance2(dg_context* ctx, const float4* points, uint32_t n, float* distance2) {
   if (n == 0) return DG_OK;
   cudaStream_t st = ctx->stream;
-  Moments m{};
-  {
-    Scratch moments(st);
-    DG_CUDA(cudaMallocAsync(&moments.ptr, sizeof(Moments), st));
-    Moments init{};
-    for (int k = 0; k < 3; k++) init.lo[k] = 0xffffffffu;
-    DG_TRY(write_async(ctx, moments.ptr, &init, sizeof init));
-    const uint32_t blocks = std::min(ceil_div(n, KNN_THREADS), (uint32_t)ctx->sm_count * 4u);
-    DG_LAUNCH(ctx, "knn_bounds", bounds_kernel<<<blocks, KNN_THREADS, 0, st>>>(points, n, moments.at<Moments>(0)));
-    DG_CUDA(cudaMemcpyAsync(&m, moments.ptr, sizeof m, cudaMemcpyDeviceToHost, st));
-    DG_CUDA(cudaStreamSynchronize(st));
-  }
-  const Octree o = choose_octree(m);
   // 63-bit keys: all 32 low-word bits and 31 high-word bits, 8 even passes.
   const SortPlan plan = sort_plan_digits(n, 2, 3 * BITS - 32);
+  const uint32_t shares = std::min(ceil_div(n, KNN_THREADS), (uint32_t)ctx->sm_count * 2u);
+  Tree tree{};
+  size_t boxes = 0;
+  for (uint32_t count = ceil_div(n, 32);; count = ceil_div(count, 32)) {
+    tree.count[tree.top] = count;
+    boxes += count;
+    if (count <= 32) break;
+    tree.top++;
+  }
   const size_t off_values = align256((size_t)n * 8);
   const size_t off_keys_alt = align256(off_values + (size_t)n * 4);
   const size_t off_values_alt = align256(off_keys_alt + (size_t)n * 8);
   const size_t off_sort = align256(off_values_alt + (size_t)n * 4);
   const size_t off_sorted = align256(off_sort + sort_scratch_bytes(plan));
+  const size_t off_boxes = align256(off_sorted + (size_t)n * 16);
+  const size_t off_shares = align256(off_boxes + boxes * sizeof(Box));
+  const size_t off_octree = align256(off_shares + shares * sizeof(Moments));
   Scratch scratch(st);
-  DG_CUDA(cudaMallocAsync(&scratch.ptr, off_sorted + (size_t)n * 16, st));
+  DG_CUDA(cudaMallocAsync(&scratch.ptr, off_octree + sizeof(Octree), st));
   uint2* keys = scratch.at<uint2>(0);
   uint32_t* values = scratch.at<uint32_t>(off_values);
   float4* sorted = scratch.at<float4>(off_sorted);
+  Box* level = scratch.at<Box>(off_boxes);
+  Octree* octree = scratch.at<Octree>(off_octree);
+  DG_LAUNCH(ctx, "knn_bounds", bounds_kernel<<<shares, KNN_THREADS, 0, st>>>(points, n, scratch.at<Moments>(off_shares)));
+  DG_LAUNCH(ctx, "knn_octree", octree_kernel<<<1, KNN_THREADS, 0, st>>>(points, scratch.at<Moments>(off_shares), shares, octree));
   const uint32_t grid = ceil_div(n, KNN_THREADS);
-  DG_LAUNCH(ctx, "knn_morton", morton_kernel<<<grid, KNN_THREADS, 0, st>>>(points, n, o, keys, values));
+  DG_LAUNCH(ctx, "knn_morton", morton_kernel<<<grid, KNN_THREADS, 0, st>>>(points, n, octree, keys, values));
   DG_TRY(sort_launch(ctx, plan, keys, values, scratch.at<void>(off_keys_alt), scratch.at<uint32_t>(off_values_alt),
                      nullptr, scratch.at<void>(off_sort)));
-  DG_LAUNCH(ctx, "knn_gather", gather_points_kernel<<<grid, KNN_THREADS, 0, st>>>(points, n, values, sorted));
-  DG_LAUNCH(ctx, "knn_query", knn_query_kernel<<<grid, KNN_THREADS, 0, st>>>(sorted, keys, n, o, distance2));
+  DG_LAUNCH(ctx, "knn_gather", gather_points_kernel<<<grid, KNN_THREADS, 0, st>>>(points, n, values, sorted, level));
+  tree.boxes[0] = level;
+  for (uint32_t l = 1; l <= tree.top; l++) {
+    Box* parents = level + tree.count[l - 1];
+    DG_LAUNCH(ctx, "knn_parents",
+              parents_kernel<<<ceil_div(tree.count[l - 1], KNN_THREADS), KNN_THREADS, 0, st>>>(level, tree.count[l - 1],
+                                                                                               parents));
+    tree.boxes[l] = level = parents;
+  }
+  DG_LAUNCH(ctx, "knn_query",
+            knn_query_kernel<<<ceil_div(tree.count[0], QUERY_WARPS), QUERY_WARPS * 32, 0, st>>>(sorted, n, tree,
+                                                                                                distance2));
   return DG_OK;
 }
 

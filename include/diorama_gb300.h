@@ -465,12 +465,11 @@ dg_status dg_colmap_destroy(dg_colmap* r);
  * distance2[i] = the mean of the squared distances from point i to its 3 nearest
  * other points (duplicates count; with fewer than 4 points each missing neighbour
  * counts as 3.4e38, so 1 or 2 points give infinity). The same values as the
- * reference's brute force, found through a grid. positions: count × 3 f32 (host);
+ * reference's brute force, found through a tree of boxes. positions: count × 3 f32 (host);
  * distance2: count f32 (host). Blocks until done. */
 dg_status dg_mean_neighbor_distance2(dg_context* ctx, const float* positions, uint32_t count, float* distance2);
 /* The same on device buffers: points holds count × 4 f32 (xyz and padding, the
- * reference's points buffer), distance2 count f32. Blocks on one 64-byte readback
- * of the points' bounds; the rest is enqueued on the context's stream. */
+ * reference's points buffer), distance2 count f32. Enqueued on the context's stream. */
 dg_status dg_mean_neighbor_distance2_buffers(dg_context* ctx, dg_buffer* points, uint32_t count,
                                              dg_buffer* distance2);
 /* initialGaussians (src/loadDataset.ts:99-121): one raw Gaussian per point (params
