@@ -178,14 +178,25 @@ __device__ __forceinline__ void forward16(const uint32_t (&ax)[4], const __nv_bf
 }
 
 // ---- Inference on the fifth-generation tensor cores (tcgen05). A CTA of 128
-// threads scores 128 candidates: each layer is one 128 x N x K product, issued by
-// one thread as K / 16 tcgen05.mma instructions (BF16 operands in shared memory,
-// FP32 accumulators in tensor memory), completed on an mbarrier; thread t then
-// reads accumulator row t back (tcgen05.ld), adds the bias, applies GELU and
+// threads scores 128 candidates at a time: each layer is one 128 x N x K product,
+// issued by one thread as K / 16 tcgen05.mma instructions (BF16 operands in shared
+// memory, FP32 accumulators in tensor memory), completed on an mbarrier; thread t
+// then reads accumulator row t back (tcgen05.ld), adds the bias, applies GELU and
 // writes the row's BF16 activations for the next layer's product.
+//
+// The products are tiny and the tensor cores idle; what bounds it are the 128 GELUs
+// per candidate, an erff each (issue 73%). So nothing else is in their way: the CTAs
+// are persistent (weights and biases staged once, not per 128 candidates), their
+// accumulators share 64 tensor-memory columns, the next candidates' features load
+// during the products, and the GELU code is one loop body for both layers: inlined
+// 128 times (60 KB) it kept the warps waiting for instructions (59.6 us as 64, and
+// 62 with the weights staged per 128 candidates). 300,007 candidates: 62 -> 49 us;
+// 1.1M: 198 -> 154. (A cheaper erf, however exact, moves values across BF16's
+// rounding boundaries, and scores by up to 3e-3.)
 constexpr uint32_t TC_ROWS = 128;     // candidates per CTA: the products' M
 constexpr uint32_t TC_THREADS = 128;  // thread t owns row t (tensor-memory lane t)
-constexpr uint32_t TC_COLUMNS = 128;  // tensor-memory columns: layer 1 in [0, 64), 2 in [64, 128), 3 in [0, 16)
+constexpr uint32_t TC_COLUMNS = 64;   // tensor-memory columns, each layer's accumulators in turn
+constexpr uint32_t TC_PER_SM = 6;     // CTAs of an SM: 6 and 5 measured the same, 4, 3 and 2 slower
 constexpr uint32_t OUT_N = 16;        // layer 3's N, the smallest with M = 128 (outputs 0-1 real)
 
 // Element offset of (row r, column k) of a BF16 matrix with K columns kept as 8 x 8
@@ -260,44 +271,66 @@ __device__ __forceinline__ void stage_weights(__nv_bfloat16* dst, const __nv_bfl
   }
 }
 
-// Waits for the products committed to `bar` (phase `parity`); false on every
-// thread if any gave up (DEVICE_ERROR_MMA_WAIT is then set).
-__device__ __forceinline__ bool tc_layer_done(uint64_t* bar, uint32_t parity, uint32_t* __restrict__ error) {
-  const bool ok = mbar_wait_bounded(bar, parity);
-  const bool failed = __syncthreads_or(!ok);
-  if (failed && threadIdx.x == 0) atomicOr(error, DEVICE_ERROR_MMA_WAIT);
-  tc_fence_after();
-  return !failed;
-}
-
-// Bias, then GELU, of 16 accumulator columns [c0, c0 + 16) of layer `bias`, as
-// BF16 row t of the next layer's A (K = HID).
-__device__ __forceinline__ void tc_hidden(uint32_t taddr, const float* __restrict__ bias, uint32_t c0,
-                                          __nv_bfloat16* h, uint32_t t) {
-  float v[16];
-  tc_load16(taddr, v);
+// Bias, then GELU, of a layer's 64 accumulator columns, as BF16 row t of the next
+// layer's A (K = HID). Not unrolled: see above.
+__device__ __forceinline__ void tc_hidden(uint32_t taddr, const float* bias, __nv_bfloat16* h, uint32_t t) {
+#pragma unroll 1
+  for (uint32_t c0 = 0; c0 < HID; c0 += 16) {
+    float v[16];
+    tc_load16(taddr + c0, v);
 #pragma unroll
-  for (int e = 0; e < 16; e++) v[e] = gelu(v[e] + bias[c0 + e]);
-  store8(h + core_offset(t, c0, HID), v);
-  store8(h + core_offset(t, c0 + 8, HID), v + 8);
+    for (uint32_t e = 0; e < 16; e += 4) {
+      const float4 b = *reinterpret_cast<const float4*>(bias + c0 + e);
+      v[e] = gelu(v[e] + b.x);
+      v[e + 1] = gelu(v[e + 1] + b.y);
+      v[e + 2] = gelu(v[e + 2] + b.z);
+      v[e + 3] = gelu(v[e + 3] + b.w);
+    }
+    store8(h + core_offset(t, c0, HID), v);
+    store8(h + core_offset(t, c0 + 8, HID), v + 8);
+  }
 }
 
-// P(children survive) for each candidate: softmax of the two logits.
-__global__ void __launch_bounds__(TC_THREADS) mlp_predict_kernel(const float* __restrict__ features, uint32_t n,
-                                                                 const float* __restrict__ norm,
-                                                                 const __nv_bfloat16* __restrict__ packed,
-                                                                 const float* __restrict__ master,
-                                                                 float* __restrict__ survive,
-                                                                 uint32_t* __restrict__ error) {
+// A row's 12 features: three 16-byte loads where the array allows them.
+__device__ __forceinline__ void load_features(const float* __restrict__ features, uint32_t row, uint32_t n,
+                                              float (&f)[IN]) {
+#pragma unroll
+  for (uint32_t c = 0; c < IN; c++) f[c] = 0.0f;
+  if (row >= n) return;
+  const float* src = features + (size_t)row * IN;
+  if ((reinterpret_cast<uintptr_t>(features) & 15) == 0) {
+#pragma unroll
+    for (uint32_t q = 0; q < IN / 4; q++) {
+      const float4 v = reinterpret_cast<const float4*>(src)[q];
+      f[4 * q] = v.x;
+      f[4 * q + 1] = v.y;
+      f[4 * q + 2] = v.z;
+      f[4 * q + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (uint32_t c = 0; c < IN; c++) f[c] = src[c];
+  }
+}
+
+// P(children survive) for each candidate: softmax of the two logits. Persistent
+// CTAs over the 128s of candidates. A wait for a product that gives up
+// (DEVICE_ERROR_MMA_WAIT) ends the CTA's work: every thread learns of it at the
+// next barrier.
+__global__ void __launch_bounds__(TC_THREADS, TC_PER_SM)
+    mlp_predict_kernel(const float* __restrict__ features, uint32_t n, const float* __restrict__ norm,
+                       const __nv_bfloat16* __restrict__ packed, const float* __restrict__ master,
+                       float* __restrict__ survive, uint32_t* __restrict__ error) {
   __shared__ __align__(128) __nv_bfloat16 s_x[TC_ROWS * IN_PAD];
   __shared__ __align__(128) __nv_bfloat16 s_h[TC_ROWS * HID];  // layer 1's activations, then layer 2's
   __shared__ __align__(128) __nv_bfloat16 s_w1[HID * IN_PAD];
   __shared__ __align__(128) __nv_bfloat16 s_w2[HID * HID];
   __shared__ __align__(128) __nv_bfloat16 s_w3[OUT_N * HID];
+  __shared__ __align__(16) float s_bias[2 * HID];
+  __shared__ __align__(16) float s_norm[2 * IN];
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ uint32_t s_tmem;
   const uint32_t t = threadIdx.x, warp = t >> 5;
-  const uint32_t row = blockIdx.x * TC_ROWS + t;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_address(&s_tmem)),
                  "r"(TC_COLUMNS)
@@ -305,70 +338,72 @@ __global__ void __launch_bounds__(TC_THREADS) mlp_predict_kernel(const float* __
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   if (t == 0) mbar_init(&s_bar, 1);
-  {  // row t's normalized features (then zeros) as BF16
-    float x[IN_PAD];
-#pragma unroll
-    for (uint32_t c = 0; c < IN_PAD; c++)
-      x[c] = row < n && c < IN ? (features[(size_t)row * IN + c] - norm[c]) * norm[IN + c] : 0.0f;
-    store8(s_x + core_offset(t, 0, IN_PAD), x);
-    store8(s_x + core_offset(t, 8, IN_PAD), x + 8);
-  }
+  float f[IN];
+  load_features(features, blockIdx.x * TC_ROWS + t, n, f);
+  if (t < 2 * IN) s_norm[t] = norm[t];
+  s_bias[t] = master[(t < HID ? OFF_B1 : OFF_B2 - HID) + t];
+  const float b30 = master[OFF_B3], b31 = master[OFF_B3 + 1];
   stage_weights(s_w1, packed + P_W1T, HID, HID, IN_PAD);
   stage_weights(s_w2, packed + P_W2T, HID, HID, HID);
   stage_weights(s_w3, packed + P_W3T, OUT_N, OUT_PAD, HID);
-  async_proxy_fence();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s_tmem;
-  const uint32_t lanes = (warp * 32u) << 16;  // this warp's tensor-memory lanes
+  const uint32_t tmem = s_tmem, row_lanes = tmem + ((warp * 32u) << 16);  // this warp's tensor-memory lanes
   // Each 16-deep step takes the next two core matrices along K: 256 bytes on.
   constexpr uint32_t STEP = 128;  // elements
+  uint32_t phase = 0;
   bool ok = true;
-  if (t == 0) {
-    tc_mma(tmem, smem_descriptor(s_x, 128, 2 * 128), smem_descriptor(s_w1, 128, 2 * 128),
-           mma_descriptor(TC_ROWS, HID), false);
-    tc_commit(&s_bar);
-  }
-  ok = tc_layer_done(&s_bar, 0, error);
-  if (ok) {
-#pragma unroll
-    for (uint32_t c = 0; c < HID; c += 16) tc_hidden(tmem + lanes + c, master + OFF_B1, c, s_h, t);
+  // Issues a layer's product once every thread's row of A is written and its reads
+  // of the accumulators are done; false if a wait has given up.
+  auto product = [&](const __nv_bfloat16* a, const __nv_bfloat16* w, uint32_t k, uint32_t columns) {
     async_proxy_fence();
     tc_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) return false;
     tc_fence_after();
     if (t == 0) {
-#pragma unroll
-      for (uint32_t q = 0; q < HID / 16; q++)
-        tc_mma(tmem + HID, smem_descriptor(s_h + q * STEP, 128, 8 * 128), smem_descriptor(s_w2 + q * STEP, 128, 8 * 128),
-               mma_descriptor(TC_ROWS, HID), q > 0);
+      const uint32_t stride = (k / 8) * 128;
+      for (uint32_t q = 0; q < k / 16; q++)
+        tc_mma(tmem, smem_descriptor(a + q * STEP, 128, stride), smem_descriptor(w + q * STEP, 128, stride),
+               mma_descriptor(TC_ROWS, columns), q > 0);
       tc_commit(&s_bar);
     }
-    ok = tc_layer_done(&s_bar, 1, error);
-  }
-  if (ok) {
-#pragma unroll
-    for (uint32_t c = 0; c < HID; c += 16) tc_hidden(tmem + lanes + HID + c, master + OFF_B2, c, s_h, t);
-    async_proxy_fence();
-    tc_fence_before();
-    __syncthreads();
+    return true;
+  };
+  auto finish = [&]() {
+    ok = mbar_wait_bounded(&s_bar, phase & 1u);
+    phase++;
+    if (!ok) atomicOr(error, DEVICE_ERROR_MMA_WAIT);
     tc_fence_after();
-    if (t == 0) {
+  };
+  bool running = true;
+  for (uint32_t first = blockIdx.x * TC_ROWS; running && first < n; first += gridDim.x * TC_ROWS) {
+    const uint32_t row = first + t;
+    {  // row t's normalized features (then zeros) as BF16
+      float x[IN_PAD];
 #pragma unroll
-      for (uint32_t q = 0; q < HID / 16; q++)
-        tc_mma(tmem, smem_descriptor(s_h + q * STEP, 128, 8 * 128), smem_descriptor(s_w3 + q * STEP, 128, 8 * 128),
-               mma_descriptor(TC_ROWS, OUT_N), q > 0);
-      tc_commit(&s_bar);
+      for (uint32_t c = 0; c < IN_PAD; c++)
+        x[c] = row < n && c < IN ? (f[c] - s_norm[c]) * s_norm[IN + c] : 0.0f;
+      store8(s_x + core_offset(t, 0, IN_PAD), x);
+      store8(s_x + core_offset(t, 8, IN_PAD), x + 8);
     }
-    ok = tc_layer_done(&s_bar, 0, error);
-  }
-  if (ok) {
+    running = product(s_x, s_w1, IN_PAD, HID);
+    if (!running) break;
+    load_features(features, first + gridDim.x * TC_ROWS + t, n, f);  // the next candidates'
+#pragma unroll 1
+    for (uint32_t layer = 0; layer < 2 && running; layer++) {
+      finish();
+      tc_hidden(row_lanes, s_bias + layer * HID, s_h, t);
+      running = product(s_h, layer == 0 ? s_w2 : s_w3, HID, layer == 0 ? HID : OUT_N);
+    }
+    if (!running) break;
+    finish();
     float z[16];
-    tc_load16(tmem + lanes, z);
-    if (row < n) survive[row] = 1.0f / (1.0f + expf((z[0] + master[OFF_B3]) - (z[1] + master[OFF_B3 + 1])));
-  } else {
-    mbar_wait_bounded(&s_bar, 0);  // a product still in flight after a give-up: one more bounded wait
+    tc_load16(row_lanes, z);
+    if (ok && row < n) survive[row] = 1.0f / (1.0f + expf((z[0] + b30) - (z[1] + b31)));
+  }
+  if (!ok) {  // a product still in flight after a give-up: more bounded waits
+    mbar_wait_bounded(&s_bar, 0);
     mbar_wait_bounded(&s_bar, 1);
   }
   tc_fence_before();
@@ -663,9 +698,10 @@ namespace dg {
 dg_status mlp_predict_launch(dg_densify_mlp* m, const float* features, uint32_t n, float* survive) {
   if (n == 0) return DG_OK;
   DG_LAUNCH(m->ctx, "mlp_predict",
-            mlp_predict_kernel<<<ceil_div(n, TC_ROWS), TC_THREADS, 0, m->ctx->stream>>>(
-                features, n, typed<float>(m->norm), typed<__nv_bfloat16>(m->packed), typed<float>(m->master),
-                survive, m->ctx->device_error));
+            mlp_predict_kernel<<<std::min(ceil_div(n, TC_ROWS), TC_PER_SM * (uint32_t)m->ctx->sm_count), TC_THREADS,
+                                 0, m->ctx->stream>>>(features, n, typed<float>(m->norm),
+                                                      typed<__nv_bfloat16>(m->packed), typed<float>(m->master),
+                                                      survive, m->ctx->device_error));
   return DG_OK;
 }
 
