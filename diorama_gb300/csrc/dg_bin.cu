@@ -13,8 +13,7 @@
 //      (bin_scatter_kernel).
 // Before that, bin_count_kernel counts each chunk's splats per tile, bin_scan_kernel
 // turns the counts into the chunk's place within each tile's list, and
-// bin_plan_kernel scans the tiles and writes their ranges and the blend's work
-// plan. Within a tile the splats come out nearest first, ties by index: the order
+// bin_ranges_kernel scans the tiles and writes their ranges. Within a tile the splats come out nearest first, ties by index: the order
 // of the reference's stable sort of (tile, depth) keys.
 //
 // A stable two-pass radix sort of emitted pairs moves 16 bytes a pair and pass,
@@ -46,9 +45,7 @@ constexpr uint32_t SCATTER_ROOM = 6144;  // entries of one (chunk, bin) that go 
 constexpr uint32_t DENSE = 48;  // tiles of a bin that its splats cover on average, from which it is dense
 constexpr uint32_t ROUNDS = MAX_CHUNK / 1024;  // words of 32 splats a lane holds of a chunk at most
 constexpr uint32_t SCAN_THREADS = 1024, SCAN_ROWS = 24;
-constexpr uint32_t PLAN_THREADS = 1024;
-// Buckets of the plan: cooperative tiles by floor(log2(length)), then the others.
-constexpr uint32_t LIGHT = 32, BUCKETS = 33;
+constexpr uint32_t RANGE_THREADS = 1024;
 
 // Where a frame that needs more pairs than there is room for stops: the first
 // `kept` pairs of the splat `index` of chunk `chunk` are the last ones listed.
@@ -57,9 +54,6 @@ struct Limit {
 };
 struct State {
   Limit limit;
-  uint32_t bucket[BUCKETS];  // tiles per bucket
-  uint32_t multi, single;    // backward chunks of tiles with several, and tiles with one
-  uint32_t bucket_at[BUCKETS], multi_at, single_at;  // write cursors
 };
 
 struct Bins {
@@ -155,9 +149,6 @@ __global__ void __launch_bounds__(BIN_THREADS) bin_count_kernel(const Bins b, co
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
   const uint32_t chunk = blockIdx.x, view = blockIdx.y, row = view * b.chunks + chunk;
   const uint32_t width = b.s.grid_x, height = b.s.grid_y, pitch = count_pitch(width);
-  // The first CTA clears what the kernels after this one count into.
-  if (chunk == 0 && view == 0)
-    for (uint32_t k = t; k < sizeof(State) / 4; k += BIN_THREADS) reinterpret_cast<uint32_t*>(b.state)[k] = 0;
   for (uint32_t k = t; k < pitch * (height + 1); k += BIN_THREADS) smem[k] = 0;
   const uint32_t first = chunk * b.chunk, n = min(b.chunk, b.s.per_view - min(first, b.s.per_view));
   const size_t at0 = (size_t)view * b.s.per_view + first;
@@ -494,12 +485,12 @@ __device__ Limit find_limit(const Bins& b, uint32_t capacity) {
 }
 
 // Each tile's counts over the chunks become exclusive prefixes, its total goes to
-// totals, and the plan's buckets are tallied. A CTA takes 32 tiles, a lane each;
+// totals. A CTA takes 32 tiles, a lane each;
 // its 32 warps take consecutive runs of chunks, in registers up to SCAN_ROWS each
 // (1.5M splats a view), so the counts are read once and all at the same time.
 // (8 warps reading them twice took 55 us instead of 14 at 538 chunks x 8487 tiles.)
 // Grid: (tiles / 32, views).
-__global__ void __launch_bounds__(SCAN_THREADS) bin_scan_kernel(const Bins b, uint32_t capacity, uint32_t coop_min,
+__global__ void __launch_bounds__(SCAN_THREADS) bin_scan_kernel(const Bins b, uint32_t capacity,
                                                                 uint32_t* __restrict__ pair_total) {
   constexpr uint32_t WARPS = SCAN_THREADS / 32;
   __shared__ uint32_t s_sum[WARPS][32];
@@ -572,104 +563,43 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_scan_kernel(const Bins b, ui
       before += c;
     }
   }
-  if (warp != WARPS - 1) return;
   // The last warp has its tiles' lengths.
-  const uint32_t len = inside ? before : 0u;
-  if (inside) b.totals[(size_t)view * b.tiles + tile] = len;
-  const uint32_t bucket = !inside ? BUCKETS : len > coop_min ? 31u - __clz(len) : LIGHT;
-  const uint32_t peers = __match_any_sync(0xffffffffu, bucket);
-  if (bucket < BUCKETS && lane == (uint32_t)__ffs(peers) - 1) atomicAdd(&b.state->bucket[bucket], __popc(peers));
-  const uint32_t nb = (len + CHUNK - 1) / CHUNK;
-  const uint32_t multi = __reduce_add_sync(0xffffffffu, nb > 1 ? nb : 0u);
-  const uint32_t single = __popc(__ballot_sync(0xffffffffu, nb == 1));
-  if (lane == 0 && multi) atomicAdd(&b.state->multi, multi);
-  if (lane == 0 && single) atomicAdd(&b.state->single, single);
+  if (warp == WARPS - 1 && inside) b.totals[(size_t)view * b.tiles + tile] = before;
 }
 
-// Exclusive scan of one value per thread over a CTA of PLAN_THREADS; `total` gets the sum.
-__device__ __forceinline__ uint32_t plan_scan(uint32_t v, uint32_t* s_warp, uint32_t& total) {
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t incl = v;
+// A thread per tile: the tile's run of the pair list. Each CTA adds up the tiles
+// before its own (a few L2 reads a thread). The first clears what the blend's plan
+// counts into.
+__global__ void __launch_bounds__(RANGE_THREADS) bin_ranges_kernel(const Bins b, uint2* __restrict__ ranges,
+                                                                   uint32_t* __restrict__ plan,
+                                                                   uint32_t* __restrict__ work) {
+  constexpr uint32_t WARPS = RANGE_THREADS / 32;
+  static_assert(WARPS == 32, "a warp's lanes read one word per warp");
+  __shared__ uint32_t s_before[WARPS], s_sum[WARPS];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t tiles = b.s.views * b.tiles, t = blockIdx.x * RANGE_THREADS + tid;
+  if (blockIdx.x == 0) {
+    if (tid < PLAN_HEADER) plan[tid] = 0;
+    if (tid < 4) work[tid] = 0;
+  }
+  uint32_t before = 0;
+  for (uint32_t k = tid; k < blockIdx.x * RANGE_THREADS; k += RANGE_THREADS) before += b.totals[k];
+  const uint32_t len = t < tiles ? b.totals[t] : 0u;
+  uint32_t incl = len;
 #pragma unroll
   for (uint32_t d = 1; d < 32; d <<= 1) {
     const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
     if (lane >= d) incl += u;
   }
-  if (lane == 31) s_warp[warp] = incl;
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 31) {
+    s_before[warp] = before;
+    s_sum[warp] = incl;
+  }
   __syncthreads();
-  const uint32_t w = s_warp[lane];  // PLAN_THREADS / 32 == 32 warps
-  const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
-  total = __reduce_add_sync(0xffffffffu, w);
-  __syncthreads();
-  return before + incl - v;
-}
-
-// A thread per tile: the tile's run of the pair list, and its place in the blend's
-// work plan: tiles of more than coop_min entries first, longest first by powers of
-// two, then the rest, and the backward's (tile, chunk) pairs, those of tiles with
-// several chunks first. Each CTA adds up the tiles before its own (a few L2 reads
-// a thread). Order within a group follows atomics and does not change any result.
-__global__ void __launch_bounds__(PLAN_THREADS) bin_plan_kernel(const Bins b, uint32_t coop_min,
-                                                                uint2* __restrict__ ranges,
-                                                                uint32_t* __restrict__ plan,
-                                                                uint2* __restrict__ chunks,
-                                                                uint32_t* __restrict__ work) {
-  static_assert(PLAN_THREADS == 1024, "plan_scan reads one word per warp with one lane each");
-  __shared__ uint32_t s_warp[32];
-  __shared__ uint32_t s_bucket[BUCKETS], s_base[BUCKETS];
-  __shared__ uint32_t s_multi, s_single;
-  const uint32_t tid = threadIdx.x, lane = tid & 31u;
-  const uint32_t tiles = b.s.views * b.tiles, t = blockIdx.x * PLAN_THREADS + tid;
-  State& st = *b.state;
-  if (tid < BUCKETS) s_bucket[tid] = 0;
-  uint32_t part = 0;
-  for (uint32_t k = tid; k < blockIdx.x * PLAN_THREADS; k += PLAN_THREADS) part += b.totals[k];
-  const uint32_t len = t < tiles ? b.totals[t] : 0u;
-  uint32_t before, total;
-  plan_scan(part, s_warp, before);
-  const uint32_t start = before + plan_scan(len, s_warp, total);
+  const uint32_t start =
+      __reduce_add_sync(0xffffffffu, s_before[lane] + (lane < warp ? s_sum[lane] : 0u)) + incl - len;
   if (t < tiles) ranges[t] = len ? make_uint2(start, start + len) : make_uint2(0u, 0u);
-
-  // The tile's place among the CTA's of its bucket (warp, then CTA, then frame).
-  const uint32_t bucket = t >= tiles ? BUCKETS : len > coop_min ? 31u - __clz(len) : LIGHT;
-  const uint32_t peers = __match_any_sync(0xffffffffu, bucket);
-  const int leader = __ffs(peers) - 1;
-  uint32_t rank = 0;
-  if (bucket < BUCKETS && (int)lane == leader) rank = atomicAdd(&s_bucket[bucket], __popc(peers));
-  rank = __shfl_sync(0xffffffffu, rank, leader) + __popc(peers & ((1u << lane) - 1u));
-  const uint32_t nb = (len + CHUNK - 1) / CHUNK;
-  uint32_t multi, single;
-  const uint32_t multi_at = plan_scan(nb > 1 ? nb : 0u, s_warp, multi);
-  const uint32_t single_at = plan_scan(nb == 1 ? 1u : 0u, s_warp, single);
-  if (tid < BUCKETS) {
-    uint32_t base = 0;  // tiles of the buckets before this one
-    if (tid == LIGHT) {
-      for (uint32_t k = 0; k < LIGHT; k++) base += st.bucket[k];
-    } else {
-      for (uint32_t k = tid + 1; k < LIGHT; k++) base += st.bucket[k];
-    }
-    s_base[tid] = base + (s_bucket[tid] ? atomicAdd(&st.bucket_at[tid], s_bucket[tid]) : 0u);
-    if (tid == LIGHT && blockIdx.x == 0) {
-      plan[0] = base;
-      plan[1] = tiles;
-      plan[2] = st.multi + st.single;
-      plan[3] = 0;
-    }
-  } else if (tid == 64) {
-    s_multi = multi ? atomicAdd(&st.multi_at, multi) : 0u;
-    s_single = st.multi + (single ? atomicAdd(&st.single_at, single) : 0u);
-  } else if (tid >= 96 && tid < 100 && blockIdx.x == 0) {
-    work[tid - 96] = 0;
-  }
-  __syncthreads();
-  if (t >= tiles) return;
-  plan[PLAN_HEADER + s_base[bucket] + rank] = t;
-  if (!chunks) return;
-  if (nb > 1) {
-    for (uint32_t k = 0; k < nb; k++) chunks[s_multi + multi_at + k] = make_uint2(t, k);
-  } else if (nb == 1) {
-    chunks[s_single + single_at] = make_uint2(t, 0u);
-  }
 }
 
 // A warp per tile.
@@ -717,10 +647,10 @@ dg_status bin_launch(dg_context* ctx, const BinShape& s, const BinLaunch& l) {
                                                                                                     l.order));
   DG_LAUNCH(ctx, "bin_scan",
             bin_scan_kernel<<<dim3(ceil_div(b.tiles, 32), s.views), SCAN_THREADS, 0, ctx->stream>>>(
-                b, l.capacity, l.coop_min, l.pair_total));
-  DG_LAUNCH(ctx, "plan",
-            bin_plan_kernel<<<ceil_div((uint64_t)s.views * b.tiles, PLAN_THREADS), PLAN_THREADS, 0, ctx->stream>>>(
-                b, l.coop_min, l.ranges, l.plan, l.chunks, l.work));
+                b, l.capacity, l.pair_total));
+  DG_LAUNCH(ctx, "bin_ranges",
+            bin_ranges_kernel<<<ceil_div((uint64_t)s.views * b.tiles, RANGE_THREADS), RANGE_THREADS, 0, ctx->stream>>>(
+                b, l.ranges, l.plan, l.work));
   DG_LAUNCH(ctx, "bin_scatter",
             bin_scatter_kernel<<<dim3(b.bins, b.chunks, s.views), BIN_THREADS, scatter_bytes(b.chunk),
                                  ctx->stream>>>(b, l.order, l.ranges, l.values));

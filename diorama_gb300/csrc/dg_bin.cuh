@@ -20,16 +20,14 @@ struct BinLaunch {
   const uint32_t* rects;  // per splat, its rectangle of tiles (pack_rect)
   const uint32_t* order;  // splat numbers, view by view, nearest first
   uint32_t capacity;      // pairs that `values` holds
-  uint32_t coop_min;
   void* scratch;
   uint32_t* pair_total;  // element 0: the pairs the frame needs
   uint32_t* values;      // out: each tile's splats, nearest first, tile after tile
   uint2* ranges;         // out: each tile's run of values (0, 0 when it has none)
-  uint32_t* plan;        // out: the blend's work plan (PLAN_HEADER, dg_render_kernels.cuh)
-  uint2* chunks;         // out: the backward's (tile, chunk) list; may be NULL
+  uint32_t* plan;        // out: the blend's work plan, its header cleared (dg_render_kernels.cuh)
   uint32_t* work;        // out: the blend kernels' 4 item counters, cleared
 };
-// Lists every tile's splats and plans the blend. Of a frame that needs more than
+// Lists every tile's splats. Of a frame that needs more than
 // `capacity` pairs, the ones that come first in depth order (then row by row of
 // the splat's rectangle) are kept.
 dg_status bin_launch(dg_context* ctx, const BinShape& s, const BinLaunch& l);

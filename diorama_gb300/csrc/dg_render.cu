@@ -466,62 +466,94 @@ __device__ __forceinline__ unsigned char to_unorm8(float v) {
 }
 
 // ------------------------------------------------------------------ work plan
-// Orders the frame's blend work; one CTA. The forward pass takes tiles with more
-// than coop_min entries first, longest first by powers of two, then the rest; the
-// backward pass (when chunks is given) takes the (tile, chunk) pairs of tiles
-// with several chunks first. Order within a group follows atomics and does not
-// change any result.
-constexpr uint32_t PLAN_THREADS = 1024;
+// Orders the frame's blend work. A tile's work is the entries its pixels walk before
+// they are opaque, which is seldom its list's length (a captured scene's densest
+// tile lists 30,000 splats and walks a tenth). It is estimated from 32 entries
+// spread over the list: a splat's alpha integrates to 2 pi opacity / sqrt(det conic)
+// over the tiles that list it, and the tile is taken to be opaque where those
+// shares reach an optical depth of PLAN_DEPTH. The forward pass takes the tiles with
+// the most work first, by powers of two (half the list's length at least: a block of
+// the tile that little covers walks on); the backward pass (when chunks is given)
+// the (tile, chunk) pairs of tiles with several chunks first. Order within a group
+// follows atomics, and none of it changes a result. A warp estimates a tile; a CTA
+// places 32 of them together, one atomic per group.
+constexpr uint32_t PLAN_THREADS = 256, PLAN_CTA_TILES = 32, PLAN_SAMPLES = 32;
+constexpr float PLAN_DEPTH = 16.0f;
 
 __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(const uint2* __restrict__ ranges, uint32_t tiles,
-                                                            uint32_t coop_min, uint32_t* __restrict__ plan,
-                                                            uint2* __restrict__ chunks) {
-  __shared__ uint32_t s_bucket[32];  // cooperative tiles by floor(log2(length)); then write cursors
-  __shared__ uint32_t s_light, s_multi, s_single;
-  const uint32_t tid = threadIdx.x;
-  if (tid < 32) s_bucket[tid] = 0;
-  if (tid == 0) s_multi = 0;
-  __syncthreads();
-  for (uint32_t t = tid; t < tiles; t += PLAN_THREADS) {
-    const uint2 r = ranges[t];
-    const uint32_t len = r.y - r.x;
-    if (len > coop_min) atomicAdd(&s_bucket[31 - __clz(len)], 1u);
-    const uint32_t nb = (len + CHUNK - 1) / CHUNK;
-    if (nb > 1) atomicAdd(&s_multi, nb);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    uint32_t at = 0;
-    for (int k = 31; k >= 0; k--) {
-      const uint32_t c = s_bucket[k];
-      s_bucket[k] = at;
-      at += c;
+                                                            const uint32_t* __restrict__ pair_splats,
+                                                            const float* __restrict__ splats,
+                                                            uint32_t* __restrict__ plan, uint2* __restrict__ chunks,
+                                                            uint32_t chunk_room) {
+  __shared__ uint32_t s_work[PLAN_CTA_TILES], s_len[PLAN_CTA_TILES], s_rank[PLAN_CTA_TILES];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  for (uint32_t k = warp; k < PLAN_CTA_TILES; k += PLAN_THREADS / 32) {
+    const uint32_t t = blockIdx.x * PLAN_CTA_TILES + k;
+    const uint2 run = t < tiles ? ranges[t] : make_uint2(0u, 0u);
+    const uint32_t len = run.y - run.x;
+    uint32_t work = len;
+    if (len >= 2 * PLAN_SAMPLES) {
+      const uint32_t at = run.x + (uint32_t)((uint64_t)len * (2 * lane + 1) / (2 * PLAN_SAMPLES));
+      const float4* s = reinterpret_cast<const float4*>(splats + (size_t)pair_splats[at] * FLOATS_PER_SPLAT);
+      const float4 conic = s[1];
+      const float side = 2.0f * s[0].w / TILE + 1.0f;  // tiles, about
+      const float alpha = 6.2831853f * s[2].w * rsqrtf(conic.x * conic.z - conic.y * conic.y);
+      float depth = fminf(alpha / (side * side * TILE * TILE), 1.0f) * (float)len / PLAN_SAMPLES;
+      if (!(depth >= 0.0f)) depth = 0.0f;
+#pragma unroll
+      for (uint32_t d = 1; d < 32; d <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, depth, d);
+        if (lane >= d) depth += v;
+      }
+      const uint32_t opaque = __ballot_sync(0xffffffffu, depth >= PLAN_DEPTH);
+      if (opaque) work = (uint32_t)((uint64_t)len * __ffs(opaque) / PLAN_SAMPLES);
     }
-    plan[0] = at;
-    plan[1] = tiles;
-    s_light = at;
-    s_single = s_multi;
-    s_multi = 0;
-  }
-  __syncthreads();
-  uint32_t* order = plan + PLAN_HEADER;
-  for (uint32_t t = tid; t < tiles; t += PLAN_THREADS) {
-    const uint2 r = ranges[t];
-    const uint32_t len = r.y - r.x;
-    order[len > coop_min ? atomicAdd(&s_bucket[31 - __clz(len)], 1u) : atomicAdd(&s_light, 1u)] = t;
-    if (!chunks) continue;
-    const uint32_t nb = (len + CHUNK - 1) / CHUNK;
-    if (nb > 1) {
-      const uint32_t at = atomicAdd(&s_multi, nb);
-      for (uint32_t k = 0; k < nb; k++) chunks[at + k] = make_uint2(t, k);
-    } else if (nb == 1) {
-      chunks[atomicAdd(&s_single, 1u)] = make_uint2(t, 0u);
+    if (lane == 0) {
+      s_work[k] = work;
+      s_len[k] = len;
+      s_rank[k] = max(work, len / 2);
     }
   }
   __syncthreads();
-  if (tid == 0) {
-    plan[2] = s_single;
-    plan[3] = 0;
+  if (warp != 0) return;
+  const uint32_t t = blockIdx.x * PLAN_CTA_TILES + lane, work = s_work[lane], len = s_len[lane];
+  const uint32_t below = (1u << lane) - 1u;
+  const uint32_t bucket = t < tiles ? 31u - __clz(max(s_rank[lane], 1u)) : ~0u;
+  const uint32_t peers = __match_any_sync(0xffffffffu, bucket);
+  const int leader = __ffs(peers) - 1;
+  uint32_t at = 0;
+  if (t < tiles && (int)lane == leader) at = atomicAdd(&plan[bucket], __popc(peers));
+  at = __shfl_sync(0xffffffffu, at, leader) + __popc(peers & below);
+  if (t < tiles) plan[PLAN_HEADER + bucket * tiles + at] = t;
+  const uint32_t total = __reduce_add_sync(0xffffffffu, work), longest = __reduce_max_sync(0xffffffffu, len);
+  if (lane == 0) {
+    if (total) {
+      atomicAdd(&plan[PLAN_TOTAL], total);
+      atomicMax(&plan[PLAN_LONGEST], longest);
+    }
+    if (blockIdx.x == 0) {
+      plan[PLAN_TILES] = tiles;
+      plan[PLAN_CHUNKS] = chunk_room;
+    }
+  }
+  if (!chunks) return;
+  const uint32_t nb = (len + CHUNK - 1) / CHUNK;
+  uint32_t multi = nb > 1 ? nb : 0u;
+#pragma unroll
+  for (uint32_t d = 1; d < 32; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, multi, d);
+    if (lane >= d) multi += v;
+  }
+  const uint32_t single = __ballot_sync(0xffffffffu, nb == 1);
+  uint32_t multi_at = 0, single_at = 0;
+  if (lane == 31 && multi) multi_at = atomicAdd(&plan[PLAN_MULTI], multi);
+  if (lane == 31 && single) single_at = atomicAdd(&plan[PLAN_SINGLE], __popc(single));
+  multi_at = __shfl_sync(0xffffffffu, multi_at, 31) + multi - (nb > 1 ? nb : 0u);
+  single_at = __shfl_sync(0xffffffffu, single_at, 31) + __popc(single & below);
+  if (nb > 1) {
+    for (uint32_t k = 0; k < nb; k++) chunks[multi_at + k] = make_uint2(t, k);
+  } else if (nb == 1) {
+    chunks[chunk_room - 1 - single_at] = make_uint2(t, 0u);
   }
 }
 
@@ -678,8 +710,8 @@ __device__ __forceinline__ void write_pixel(const BlendItem& it, const PixelBlen
 // front to back exactly as the plain loop over every entry does, so results are
 // bit-identical to it; the split only decides who does the work:
 //
-// - Tiles with more entries than the plan's threshold (COOP_MIN unless tuned)
-//   come first, each block blended by a whole CTA. Three of its warps take
+// - Tiles with much more work than a warp gets on average come first, each block
+//   blended by a whole CTA. Three of its warps take
 //   consecutive 32-entry windows, keep the splats that can reach the block and
 //   compute their alphas at the block's pixels, queueing those some pixel blends;
 //   warp 0 applies the queues in list order one round behind, so the alphas of the
@@ -690,15 +722,27 @@ __device__ __forceinline__ void write_pixel(const BlendItem& it, const PixelBlen
 //   entries at a time.
 //
 // In both, a window's splat records are copied into shared memory while the
-// previous one blends, a splat rejected for the block has alpha below 1/255 at
+// previous one blends (two to four windows ahead were no faster), a splat rejected for the block has alpha below 1/255 at
 // all of its pixels, and a power under the splat's cutoff skips the exp: none of
 // these changes a result. The pixel state at each CHUNK boundary of the list is
 // saved for the backward pass, and which entries each block blended.
+// Cooperative blending costs about 1.4 times the instructions of a warp on its own and
+// its CTA's warps wait for each other every round, but a long walk takes a third of
+// the time. So it pays where a walk would outlast the rest of the frame: for tiles of
+// COOP_LOAD times the work a warp gets on average, and for all when the longest list
+// is COOP_CHAIN times that (some block of it may walk it to the end however opaque
+// the tile is, and shares its SM with fewer busy warps when all are cooperative).
+// Against blending every tile of more than 128 entries cooperatively: 1.1M splats at
+// 1960x1090 (at most 6,000 entries a tile, 75,000 a warp) 990 -> 494 us, 200,000 at
+// 1280x720 441 -> 244, 12 views of 300,000 948 -> 735; where chains bound it (1.1M at
+// 980x545, lists up to 30,000) 295 both ways. COOP_LOAD 0.5 and 2, COOP_CHAIN 8 and
+// PLAN_DEPTH 8, 32 and 64 were slower on one scene or another.
+constexpr float COOP_LOAD = 1.5f, COOP_CHAIN = 5.0f;
 template <uint32_t TWL, uint32_t THL>
 __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
     const Camera* __restrict__ camera, const float4* __restrict__ raster_params, const float* __restrict__ splats,
     const uint32_t* __restrict__ pair_splats, const uint2* __restrict__ ranges, const uint32_t* __restrict__ plan,
-    uint32_t tiles_per_view, uchar4* __restrict__ target, float4* __restrict__ pixel_color,
+    uint32_t tiles_per_view, uint32_t coop_min, uchar4* __restrict__ target, float4* __restrict__ pixel_color,
     uint32_t* __restrict__ pixel_last, float4* __restrict__ checkpoints, uint32_t* __restrict__ blend_mask,
     uint32_t* __restrict__ counters, bool cut_in_record) {
   __shared__ WarpStage stages[FWD_WARPS];
@@ -716,8 +760,27 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
   const uint32_t tiles_x = ((uint32_t)vpx + TILE - 1u) / TILE;
   const uint2 tiles16 = make_uint2(tiles_x, ((uint32_t)vpy + TILE - 1u) / TILE);
   const float4 bg = raster_params[0];
-  const uint32_t cooperative = plan[0], tiles = plan[1];
-  const uint32_t* order = plan + PLAN_HEADER;
+  // The plan's buckets, most work first (lane l: bucket 31 - l), and the tiles up to
+  // each; the first buckets are cooperative.
+  const uint32_t tiles = plan[PLAN_TILES];
+  const uint32_t in_bucket = plan[PLAN_BUCKETS - 1 - lane];
+  uint32_t up_to = in_bucket;
+#pragma unroll
+  for (uint32_t d = 1; d < 32; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, up_to, d);
+    if (lane >= d) up_to += v;
+  }
+  const float load = (float)plan[PLAN_TOTAL] * (float)(1u << BLOCK_SHIFT) / (float)(gridDim.x * FWD_WARPS);
+  const bool chain = (float)plan[PLAN_LONGEST] > COOP_CHAIN * load;
+  const float enough = chain ? (float)coop_min : fmaxf(COOP_LOAD * load, (float)coop_min);
+  const uint32_t coop_buckets = __popc(__ballot_sync(0xffffffffu, (float)(1u << (31u - lane)) >= enough));
+  const uint32_t cooperative = coop_buckets ? __shfl_sync(0xffffffffu, up_to, coop_buckets - 1) : 0u;
+  // The i-th tile of the plan; all lanes ask for the same.
+  auto tile_at = [&](uint32_t i) {
+    const uint32_t at = __popc(__ballot_sync(0xffffffffu, up_to <= i));
+    const uint32_t before = __shfl_sync(0xffffffffu, up_to - in_bucket, at);
+    return plan[PLAN_HEADER + (PLAN_BUCKETS - 1 - at) * tiles + i - before];
+  };
 
   // Cooperative items: one block of a long tile per CTA. Warps 1..PRODUCERS take
   // consecutive 32-entry windows of round r (window pw of the round is producer
@@ -737,18 +800,18 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
     const uint32_t item = s_item;
     if (item >= cooperative << BLOCK_SHIFT) break;
     const uint32_t block = item & BLOCK_MASK;
-    const BlendItem it(order[item >> BLOCK_SHIFT], block, lane, tiles_x, tiles_per_view, vpx, vpy, ranges, TWL, THL);
+    const BlendItem it(tile_at(item >> BLOCK_SHIFT), block, lane, tiles_x, tiles_per_view, vpx, vpy, ranges, TWL, THL);
     const TileMember tm{MEMBER, it.tx, it.ty, tiles16};
     const uint2 run = it.run;
     PixelBlend pb{(float)it.px + 0.5f, (float)it.py + 0.5f, 1.0f, 0.0f, 0.0f, 0.0f, 0u, !it.inside};
     uint32_t next_k = 1;  // the next checkpoint boundary (warp 0)
     const uint32_t pw = warp - 1u;  // producer index (warps >= 1)
-    // This producer lane's entry of the window in flight and of the one after it.
+    // This producer lane's entry of the window after the one in flight.
     uint32_t index = 0, next_index = 0;
     if (warp > 0) {
       const uint32_t k = run.x + 32u * pw + lane;
       if (k < run.y) index = pair_splats[k];
-      stage_issue(st, splats, index, k < run.y);
+      stage_issue(st.raw, splats, index, k < run.y);
       if (k + STRIDE < run.y) next_index = pair_splats[k + STRIDE];
     }
     const uint32_t rounds = (run.y - run.x + STRIDE - 1u) / STRIDE;
@@ -757,11 +820,11 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
       if (warp > 0) {
         const uint32_t start = run.x + r * STRIDE + 32u * pw;
         if (r < rounds && start < run.y) {
-          const uint32_t staged = stage_commit(st, run.x, start, run.y, index, it.x0, it.y0, cut_in_record, tm);
+          cp_async_wait_all();
+          const uint32_t staged = stage_commit(st, st.raw, run.x, start, run.y, it.x0, it.y0, cut_in_record, tm);
           {
             const uint32_t k = start + STRIDE + lane;
-            stage_issue(st, splats, next_index, k < run.y);
-            index = next_index;
+            stage_issue(st.raw, splats, next_index, k < run.y);
             next_index = k + STRIDE < run.y ? pair_splats[k + STRIDE] : 0u;
           }
           // Pixels warp 0 has stopped take no part (it publishes the mask after
@@ -839,17 +902,16 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= (tiles - cooperative) << BLOCK_SHIFT) break;
     const uint32_t block = item & BLOCK_MASK;
-    const BlendItem it(order[cooperative + (item >> BLOCK_SHIFT)], block, lane, tiles_x, tiles_per_view, vpx, vpy,
+    const BlendItem it(tile_at(cooperative + (item >> BLOCK_SHIFT)), block, lane, tiles_x, tiles_per_view, vpx, vpy,
                        ranges, TWL, THL);
     const TileMember tm{MEMBER, it.tx, it.ty, tiles16};
     const uint2 run = it.run;
     PixelBlend pb{(float)it.px + 0.5f, (float)it.py + 0.5f, 1.0f, 0.0f, 0.0f, 0.0f, 0u, !it.inside};
     uint32_t next_k = 1;
-    uint32_t index = 0, next_index = 0;
+    uint32_t next_index = 0;
     {
       const uint32_t k = run.x + lane;
-      if (k < run.y) index = pair_splats[k];
-      stage_issue(st, splats, index, k < run.y);
+      stage_issue(st.raw, splats, k < run.y ? pair_splats[k] : 0u, k < run.y);
       if (k + 32u < run.y) next_index = pair_splats[k + 32u];
     }
     for (uint32_t start = run.x; start < run.y; start += 32) {
@@ -858,11 +920,11 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
         save_checkpoints(checkpoints, run.x, next_k, next_k + 1, block, lane, pb.T, pb.r, pb.g, pb.b);
         next_k++;
       }
-      const uint32_t staged = stage_commit(st, run.x, start, run.y, index, it.x0, it.y0, cut_in_record, tm);
+      cp_async_wait_all();
+      const uint32_t staged = stage_commit(st, st.raw, run.x, start, run.y, it.x0, it.y0, cut_in_record, tm);
       {
         const uint32_t k = start + 32u + lane;
-        stage_issue(st, splats, next_index, k < run.y);
-        index = next_index;
+        stage_issue(st.raw, splats, next_index, k < run.y);
         next_index = k + 32u < run.y ? pair_splats[k + 32u] : 0u;
       }
       uint32_t blended = 0;
@@ -949,7 +1011,7 @@ dg_status rasterizer_create(dg_context* ctx, dg_buffer* camera, dg_buffer* splat
   uint32_t capacity = initial_pair_capacity ? initial_pair_capacity : std::max(1u << 16, count * 8u);
   tr->depth_first = depth_first;
   if (st == DG_OK) st = make_pairs(tr, capacity);
-  tr->coop_min = COOP_MIN;
+  tr->coop_min = COOP_FLOOR;
   if (st == DG_OK && depth_first) {
     const size_t n = std::max(count, 1u);
     tr->depth_plan = sort_plan_low_bits(std::max(count, 1u), 32);
@@ -1033,13 +1095,11 @@ dg_status rasterizer_launch(dg_tile_rasterizer* tr, dg_buffer* target, bool coun
     l.rects = typed<uint32_t>(tr->tile_offsets);
     l.order = order;
     l.capacity = tr->pair_capacity;
-    l.coop_min = tr->coop_min;
     l.scratch = tr->bin_scratch->ptr;
     l.pair_total = typed<uint32_t>(tr->scan_total);
     l.values = typed<uint32_t>(tr->values);
     l.ranges = typed<uint2>(tr->ranges);
     l.plan = typed<uint32_t>(tr->work_plan);
-    l.chunks = typed<uint2>(tr->chunks);
     l.work = typed<uint32_t>(tr->work);
     DG_TRY(bin_launch(ctx, BinShape{count, 1u, tr->tiles_x, tr->tiles_y}, l));
     tr->keys_in_ranges = true;
@@ -1113,6 +1173,7 @@ dg_status launch_rasterize(dg_tile_rasterizer* tr, dg_buffer* target) {
   f.coop_min = tr->coop_min;
   f.plan = typed<uint32_t>(tr->work_plan);
   f.chunks = typed<uint2>(tr->chunks);
+  f.chunk_room = (uint32_t)(tr->chunks->bytes / sizeof(uint2));
   f.target = target ? typed<uchar4>(target) : nullptr;
   f.pixel_color = typed<float4>(tr->pixel_color);
   f.pixel_last = typed<uint32_t>(tr->pixel_last);
@@ -1120,7 +1181,7 @@ dg_status launch_rasterize(dg_tile_rasterizer* tr, dg_buffer* target) {
   f.blend_mask = typed<uint32_t>(tr->blend_mask);
   f.counters = typed<uint32_t>(tr->work);
   f.splat_cutoffs = tr->splat_cutoffs;
-  f.planned = tr->keys_in_ranges;
+  f.cleared = tr->keys_in_ranges;
   return blend_forward(ctx, f);
 }
 
@@ -1130,7 +1191,7 @@ static dg_status launch_rasterize_kernel(dg_context* ctx, const BlendForward& f)
   const uint32_t items = f.tiles << (3u + TWL + THL);
   DG_LAUNCH(ctx, "rasterize",
             kernel<<<blend_grid(ctx, (const void*)kernel, FWD_THREADS, items), FWD_THREADS, 0, ctx->stream>>>(
-                f.camera, f.raster_params, f.splats, f.pair_splats, f.ranges, f.plan, f.tiles_per_view, f.target,
+                f.camera, f.raster_params, f.splats, f.pair_splats, f.ranges, f.plan, f.tiles_per_view, f.coop_min, f.target,
                 f.pixel_color, f.pixel_last, f.checkpoints, f.blend_mask, f.counters, f.splat_cutoffs));
   return DG_OK;
 }
@@ -1140,11 +1201,13 @@ dg_status blend_forward(dg_context* ctx, const BlendForward& f) {
   DG_REQUIRE(sh.twl <= MAX_BLEND_TILE_LOG2 && sh.thl <= MAX_BLEND_TILE_LOG2, "blend tiles of at most 2 x 2 tiles");
   DG_REQUIRE(sh.twl + sh.thl == 0 || (!f.checkpoints && !f.blend_mask && !f.chunks),
              "blend tiles larger than 16x16 have no backward pass");
-  if (!f.planned) {
+  if (!f.cleared) {
     DG_CUDA(cudaMemsetAsync(f.counters, 0, 16, ctx->stream));
-    DG_LAUNCH(ctx, "plan",
-              plan_kernel<<<1, PLAN_THREADS, 0, ctx->stream>>>(f.ranges, f.tiles, f.coop_min, f.plan, f.chunks));
+    DG_CUDA(cudaMemsetAsync(f.plan, 0, PLAN_HEADER * 4, ctx->stream));
   }
+  DG_LAUNCH(ctx, "plan",
+            plan_kernel<<<std::max(1u, ceil_div(f.tiles, PLAN_CTA_TILES)), PLAN_THREADS, 0, ctx->stream>>>(
+                f.ranges, f.tiles, f.pair_splats, f.splats, f.plan, f.chunks, f.chunk_room));
   if (sh.twl == 0 && sh.thl == 0) return launch_rasterize_kernel<0, 0>(ctx, f);
   if (sh.twl == 1 && sh.thl == 0) return launch_rasterize_kernel<1, 0>(ctx, f);
   if (sh.twl == 0 && sh.thl == 1) return launch_rasterize_kernel<0, 1>(ctx, f);
@@ -1201,7 +1264,7 @@ static dg_status ensure_plan(dg_tile_rasterizer* tr) {
   struct Need {
     dg_buffer** buf;
     size_t bytes;
-  } needs[] = {{&tr->work_plan, (PLAN_HEADER + tiles) * 4},
+  } needs[] = {{&tr->work_plan, plan_words(tiles) * 4},
                {&tr->chunks, (tiles + slots) * 8},
                {&tr->checkpoints, slots * 8 * 32 * 16},
                {&tr->blend_mask, ((size_t)tr->pair_capacity / 32 + 2) * 8 * 4}};

@@ -60,7 +60,7 @@ struct dg_tile_rasterizer {
   dg_buffer* chunks;
   dg_buffer* checkpoints;
   dg_buffer* blend_mask;  // which entries each 8x4 block blended (dg_render.cu, publish_blended)
-  uint32_t coop_min;      // tiles with more entries are blended by a whole CTA
+  uint32_t coop_min;      // the fewest entries of a tile that a whole CTA may blend
   bool splat_cutoffs;     // the splats come from this build's preprocess, cutoffs in slot 7
 };
 
@@ -105,6 +105,7 @@ struct BlendForward {
   uint32_t tiles, tiles_per_view, coop_min;
   uint32_t* plan;
   uint2* chunks;
+  uint32_t chunk_room;  // (tile, chunk) pairs that chunks holds
   uchar4* target;
   float4* pixel_color;
   uint32_t* pixel_last;
@@ -113,7 +114,7 @@ struct BlendForward {
   uint32_t* counters;  // 4 words, cleared here
   BlendShape shape;
   bool splat_cutoffs;  // the splats carry their blend cutoff (this build's preprocess wrote them)
-  bool planned;        // plan, chunks and counters are ready (bin_launch wrote them)
+  bool cleared;        // the plan's header and the counters are zero (bin_launch cleared them)
 };
 dg_status blend_forward(dg_context* ctx, const BlendForward& f);
 // The batched views' stages (dg_render.cu; used by dg_views.cu).

@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 6) rasterize_backward_kernel(
   WarpStage& st = stages[threadIdx.x >> 5];
   const float vpx = camera->viewport[0], vpy = camera->viewport[1];
   const uint32_t tiles_x = ((uint32_t)vpx + TILE - 1u) / TILE;
-  const uint32_t items = plan[2] * 8u;
+  const uint32_t multi = plan[PLAN_MULTI], items = (multi + plan[PLAN_SINGLE]) * 8u, room = plan[PLAN_CHUNKS];
   const float4 bg = raster_params[0];
   const int my_slot = reduce_slot<2 * SPLAT_GRADS>(lane);
   // Value my_slot belongs to the pair's first (further back) splat when below 9.
@@ -229,7 +229,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 6) rasterize_backward_kernel(
     if (lane == 0) item = atomicAdd(work_counter, 1u);
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= items) break;
-    const uint2 chunk = chunks[item >> 3];
+    const uint32_t which = item >> 3;
+    const uint2 chunk = chunks[which < multi ? which : room - 1u - (which - multi)];
     const uint32_t tile = chunk.x, block = item & 7u;
     const uint32_t bx = (tile % tiles_x) * TILE + (block & 1u) * 8u, by = (tile / tiles_x) * TILE + (block >> 1) * 4u;
     const uint32_t px = bx + (lane & 7u), py = by + (lane >> 3);
@@ -268,14 +269,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 6) rasterize_backward_kernel(
     uint32_t lo = window_start(end, chunk_lo);
     uint32_t bits = window_blended(words, chunk_lo, lo, end);
     uint32_t index = (bits >> lane) & 1u ? pair_splats[lo + lane] : 0u;
-    stage_issue(st, splats, index, (bits >> lane) & 1u);
+    stage_issue(st.raw, splats, index, (bits >> lane) & 1u);
     uint32_t next_lo = window_start(lo, chunk_lo);
     uint32_t next_bits = window_blended(words, chunk_lo, next_lo, lo);
     uint32_t next_index = (next_bits >> lane) & 1u ? pair_splats[next_lo + lane] : 0u;
     while (end > chunk_lo) {
       const uint32_t staged = stage_commit_blended(st, run.x, lo, index, bits, cut_in_record);
       {
-        stage_issue(st, splats, next_index, (next_bits >> lane) & 1u);
+        stage_issue(st.raw, splats, next_index, (next_bits >> lane) & 1u);
         end = lo;
         lo = next_lo;
         bits = next_bits;

@@ -261,15 +261,26 @@ constexpr uint32_t BWD_WARPS = BWD_THREADS / 32;
 // from the state the forward pass saved at the chunk's end (a checkpoint per
 // CHUNK entries). A multiple of the 32-entry window.
 constexpr uint32_t CHUNK = 512;
-// Tiles with more entries than this are blended by a whole CTA in the forward pass.
-#ifndef DG_COOP_MIN
-#define DG_COOP_MIN 128
-#endif
-constexpr uint32_t COOP_MIN = DG_COOP_MIN;
-// The frame's work plan (dg_render.cu, plan_kernel): a header of PLAN_HEADER
-// words (cooperative tiles, tiles, backward chunks, spare), the tiles in the
-// order the forward pass takes them, then the backward's (tile, chunk) pairs.
-constexpr uint32_t PLAN_HEADER = 4;
+// The fewest entries of a tile that the forward pass may blend with a whole CTA per
+// block: of a batch of views (the caller may change it), and of a frame.
+constexpr uint32_t COOP_MIN = 128, COOP_FLOOR = 64;
+// The frame's work plan (dg_render.cu, plan_kernel), in words:
+//   [0, 32)       tiles per bucket, a tile's bucket being floor(log2(entries that its
+//                 pixels are expected to walk))
+//   PLAN_TOTAL    those entries of all tiles
+//   PLAN_TILES    tiles
+//   PLAN_MULTI    backward chunks of tiles with several chunks: chunks[0..)
+//   PLAN_SINGLE   tiles with one chunk: chunks[PLAN_CHUNKS - 1] downwards
+//   PLAN_CHUNKS   the room in chunks
+//   PLAN_LONGEST  the longest tile's entries
+//   then for each bucket its tiles, in room for all tiles
+constexpr uint32_t PLAN_BUCKETS = 32, PLAN_TOTAL = 32, PLAN_TILES = 33, PLAN_MULTI = 34, PLAN_SINGLE = 35,
+                   PLAN_CHUNKS = 36, PLAN_LONGEST = 37, PLAN_HEADER = 40;
+constexpr size_t plan_words(size_t tiles) { return PLAN_HEADER + PLAN_BUCKETS * tiles; }
+
+// Splat records as they are copied in: lane l has the 48-byte record of its entry of
+// a window of 32.
+using RawWindow = float4[32][3];
 
 // A warp's own window of up to 32 list entries, staged in its slice of shared
 // memory: only the splats that can reach the warp's 8x4 pixel block, in list
@@ -281,8 +292,7 @@ struct WarpStage {
   float4 color[32];  // rgb, opacity
   uint32_t pos[32];  // position in the tile's list
   uint32_t index[32];
-  float4 raw[32][3];  // lane l: the 48-byte record of its entry of the window in flight
-  uint32_t live_count;  // cooperative blending: entries queued for warp 0
+  RawWindow raw;
 };
 
 // A pixel's state at the start of chunk boundary k of a tile (after every entry
@@ -357,14 +367,14 @@ __device__ __forceinline__ void stage_floats_async(float* dst, const float* __re
 }
 
 // Starts copying the splat record of this lane's entry of a window into `raw`.
-__device__ __forceinline__ void stage_issue(WarpStage& st, const float* __restrict__ splats, uint32_t index,
+__device__ __forceinline__ void stage_issue(RawWindow& raw, const float* __restrict__ splats, uint32_t index,
                                             bool valid) {
   if (valid) {
     const uint32_t lane = threadIdx.x & 31u;
     const float4* s = reinterpret_cast<const float4*>(splats + (size_t)index * FLOATS_PER_SPLAT);
-    cp_async16(&st.raw[lane][0], s);
-    cp_async16(&st.raw[lane][1], s + 1);
-    cp_async16(&st.raw[lane][2], s + 2);
+    cp_async16(&raw[lane][0], s);
+    cp_async16(&raw[lane][1], s + 1);
+    cp_async16(&raw[lane][2], s + 2);
   }
 }
 
@@ -379,26 +389,25 @@ struct TileMember {
   uint2 tiles;
 };
 
-// Waits for the window [lo, min(lo + 32, hi)) issued by stage_issue (lane l holds
-// entry lo + l, splat `index`) and keeps, in list order, the splats that can reach
-// the warp's block, whose pixel centers span [x0, x0 + 7] x [y0, y0 + 3] (and,
+// Takes the window [lo, min(lo + 32, hi)) whose records stage_issue has brought into
+// `raw` (lane l: entry lo + l; the caller has waited for the copies) and keeps, in
+// list order, the splats that can reach the warp's block, whose pixel centers span [x0, x0 + 7] x [y0, y0 + 3] (and,
 // with a TileMember, belong to its 16x16 tile's list). Returns how many were
 // kept. All 32 lanes must call it. Every value read from `raw` is consumed before
 // this returns, so the caller may issue the next window at once. cut_in_record:
 // the splats carry their blend cutoff in slot SPLAT_CUTOFF_SLOT (this build's
 // preprocess wrote them), else it is computed here.
-__device__ __forceinline__ uint32_t stage_commit(WarpStage& st, uint32_t run_x, uint32_t lo, uint32_t hi,
-                                                 uint32_t index, float x0, float y0, bool cut_in_record,
+__device__ __forceinline__ uint32_t stage_commit(WarpStage& st, const RawWindow& raw, uint32_t run_x, uint32_t lo,
+                                                 uint32_t hi, float x0, float y0, bool cut_in_record,
                                                  const TileMember& tm = TileMember{false, 0u, 0u, {0u, 0u}}) {
-  cp_async_wait_all();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t k = lo + lane;
   bool keep = false;
   float2 mean = make_float2(0.f, 0.f);
   float4 quad = make_float4(0.f, 0.f, 0.f, 0.f), color = quad;
   if (k < hi) {
-    const float4 s0 = st.raw[lane][0], s1 = st.raw[lane][1];
-    color = st.raw[lane][2];
+    const float4 s0 = raw[lane][0], s1 = raw[lane][1];
+    color = raw[lane][2];
     mean = make_float2(s0.x, s0.y);
     const float A = -0.5f * s1.x, b = s1.y, C = -0.5f * s1.z;
     const float cut = cut_in_record ? s1.w : blend_cutoff(color.w);
@@ -417,7 +426,6 @@ __device__ __forceinline__ uint32_t stage_commit(WarpStage& st, uint32_t run_x, 
     st.quad[at] = quad;
     st.color[at] = color;
     st.pos[at] = k - run_x;
-    st.index[at] = index;
   }
   __syncwarp();
   return __popc(kept);

@@ -140,7 +140,7 @@ dg_status prepare(dg_view_batch* b, uint32_t views, uint32_t count, uint32_t gri
   }
   DG_TRY(ensure(ctx, &b->scan_total, 16));
   DG_TRY(ensure(ctx, &b->ranges, (size_t)views * tiles_per_view * 8));
-  DG_TRY(ensure(ctx, &b->plan, (PLAN_HEADER + (size_t)views * tiles_per_view) * 4));
+  DG_TRY(ensure(ctx, &b->plan, plan_words((size_t)views * tiles_per_view) * 4));
   DG_TRY(ensure(ctx, &b->pixel_color, (size_t)views * pixels * 16));
   DG_TRY(ensure(ctx, &b->pixel_last, (size_t)views * pixels * 4));
   DG_TRY(ensure(ctx, &b->work, 16));
@@ -175,7 +175,6 @@ dg_status launch_batch(dg_renderer* r, dg_view_batch* b, uchar4* targets, uint32
     l.rects = typed<uint32_t>(b->tile_counts);
     l.order = order;
     l.capacity = b->pair_capacity;
-    l.coop_min = coop_min;
     l.scratch = b->bin_scratch->ptr;
     l.pair_total = typed<uint32_t>(b->scan_total);
     l.values = typed<uint32_t>(b->values);
@@ -219,7 +218,7 @@ dg_status launch_batch(dg_renderer* r, dg_view_batch* b, uchar4* targets, uint32
   f.counters = typed<uint32_t>(b->work);
   f.shape = b->shape;
   f.splat_cutoffs = true;  // preprocess_views_kernel's splats
-  f.planned = b->binned;
+  f.cleared = b->binned;
   DG_TRY(blend_forward(ctx, f));
   DG_CUDA(cudaMemcpyAsync(b->pinned_total, b->scan_total->ptr, 4, cudaMemcpyDeviceToHost, ctx->stream));
   return DG_OK;
