@@ -5,13 +5,28 @@
 //
 // The reference makes 7 dispatches over 5-map and 3-map vec4 buffers (moments,
 // blur h, blur v, ssim, blur h, blur v, gradient: ~900 B/pixel of traffic). Here
-// it is 2 kernels. Each CTA owns a 16x16 block of pixels, loads its 26x26 halo
-// once, and does the separable blurs in shared memory:
-//   ssim_kernel:     moments -> blur h -> blur v -> SSIM and its three partials
-//   gradient_kernel: partials -> blur h -> blur v -> dL/dpixel and the pixel loss
-// Sums run over the taps -5..5 in order, one fused multiply-add per tap (two
-// sums per packed FP32 instruction where they pair up); taps past the image add
-// exactly 0 (the halo holds zeros there), the same as the WGSL's skipping them.
+// it is 2 kernels:
+//   ssim_kernel:     moments -> blur h -> blur v -> SSIM, its three partials and the
+//                    pixel loss
+//   gradient_kernel: partials -> blur h -> blur v -> dL/dpixel
+// An ssim_kernel CTA owns a 16x16 block of pixels, loads its 26x26 halo once, and does
+// the separable blurs in shared memory. A gradient_kernel CTA walks down a strip of 32
+// columns instead: each row is staged and blurred along the row once, and the blur
+// down the columns stays in registers (the sums of the 11 output rows that a row
+// belongs to move up one place each as its tap is added, acc[k] = w[k] v + acc[k - 1]),
+// so no blurred row is stored or read back and a strip costs 10 extra rows, not a halo
+// around every 16x16 pixels.
+// Sums run over the taps -5..5 in order, one fused multiply-add per tap (in ssim_kernel
+// two sums per packed FP32 instruction where they pair up); taps past the image add
+// exactly 0 (zeros are staged there), the same as the WGSL's skipping them.
+//
+// Both are bound by instructions, not by memory (1957x1091: 132 bytes per pixel in
+// 170 us are 1.7 TB/s). Blocks against strips, in us, at 96x96 | 251x187 | 489x273 |
+// 980x545 | 1957x1091: gradient 8.3 | 10.1 | 14.2 | 33.0 | 127 with blocks, 10.2 | 10.6 |
+// 14.5 | 24.8 | 62 with strips. The SSIM pass has five maps to keep sums of, not three,
+// and spills: 12.2 | 13.2 | 17.4 | 36 | 110 with blocks, 22 | 22 | 25 | 45 | 132 with
+// strips (blocks of 16x32 pixels with two rows per thread: 15 | 17 | 17 | 35 | 109).
+// The partials lie in planes of their own, which a strip's warp reads in whole lines.
 //
 // The same ssim_kernel also measures held-out renders (PSNR and SSIM of the
 // 8-bit-quantized image, src/trainer.ts:371-386 and src/metrics.ts) on the GPU.
@@ -21,9 +36,17 @@
 namespace dg {
 namespace {
 
-constexpr int LT = 16;             // pixels per side of a CTA's block
 constexpr int HALO = 5;
+constexpr int TAPS = 2 * HALO + 1;
+// ssim_kernel: a CTA's block of pixels and its halo.
+constexpr int LT = 16;
 constexpr int LS = LT + 2 * HALO;  // 26
+// gradient_kernel: a strip's columns (a lane each) and its halo; a warp per channel.
+constexpr int COLS = 32;
+constexpr int SPAN = COLS + 2 * HALO;  // 42
+constexpr int STRIP_THREADS = 3 * 32;
+constexpr uint32_t STRIPS_PER_SM = 6;
+constexpr int MIN_ROWS = 6;
 constexpr float LAMBDA = 0.2f;
 constexpr float C1 = 0.0001f;
 constexpr float C2 = 0.0009f;
@@ -54,11 +77,14 @@ __device__ __forceinline__ float unorm8(uint32_t v, bool exact_quotient) {
   return exact_quotient ? __double2float_rn(v / 255.0) : (float)v / 255.0f;
 }
 
-// The 256 values of unorm8 in shared memory (thread t writes entry t of each
-// 256-thread CTA), so a pixel's three channels take three loads, not divisions.
-__device__ __forceinline__ void fill_unorm8(float* table, bool exact_quotient) {
-  table[threadIdx.x] = unorm8(threadIdx.x, exact_quotient);
+// The 256 values of unorm8 in shared memory, so a pixel's three channels take three
+// loads, not divisions.
+__device__ __forceinline__ void fill_unorm8(float* table, bool exact_quotient, uint32_t threads) {
+  for (uint32_t k = threadIdx.x; k < 256; k += threads) table[k] = unorm8(k, exact_quotient);
 }
+
+// The weight of tap k - 5.
+__device__ __forceinline__ int tap_weight(int k) { return k < HALO ? HALO - k : k - HALO; }
 
 __device__ __forceinline__ float3 load_y(const uchar4* target, int w, int h, int x, int y, const float* unorm) {
   if (x < 0 || y < 0 || x >= w || y >= h) return make_float3(0.f, 0.f, 0.f);
@@ -67,16 +93,17 @@ __device__ __forceinline__ float3 load_y(const uchar4* target, int w, int h, int
 }
 
 // Moments, both blurs and the SSIM partials for one 16x16 block. mode 0 (loss):
-// writes the three partials and S per channel to `partials` (12 floats per pixel,
-// laid out for the gradient pass's paired loads: (dS/dmu_x, dS/dE[x^2]) for r, g, b,
-// then dS/dE[xy] rgb, then S rgb). mode 1 (metrics): the render is quantized
-// first, and each CTA adds its Σ S and Σ squared error to `sums`.
+// writes each channel's partials, (dS/dmu_x, dS/dE[x^2]) and dS/dE[xy], in planes of
+// their own (`partials`: 3 planes of float2, then 3 of float, one value per pixel),
+// and the pixel loss. mode 1 (metrics): the render is quantized first, and each CTA
+// adds its Σ S and Σ squared error to `sums`.
 //
 // The x and y sums of each blur, and the x^2 and y^2 ones, run as pairs through
 // packed FP32 fused multiply-adds (F2): each lane is the scalar fmaf sum.
 __global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ rendered,
                                                    const uchar4* const* __restrict__ target_slot, int w, int h,
-                                                   Window win, float* __restrict__ partials, int mode,
+                                                   Window win, float* __restrict__ partials,
+                                                   float* __restrict__ pixel_loss, int mode,
                                                    double* __restrict__ sums) {
   __shared__ float2 s_xy[LS][LS][3];   // (x, y) per halo pixel and channel
   __shared__ float2 s_h01[LS][LT][3];  // horizontal blurs of x and y
@@ -87,7 +114,7 @@ __global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ re
   const uchar4* target = *target_slot;
   const int x0 = blockIdx.x * LT - HALO, y0 = blockIdx.y * LT - HALO;
   const bool metrics = mode == 1;
-  fill_unorm8(s_unorm, metrics);
+  fill_unorm8(s_unorm, metrics, 256);
   __syncthreads();
   for (int k = threadIdx.x; k < LS * LS; k += 256) {
     const int ly = k / LS, lx = k % LS;
@@ -138,43 +165,39 @@ __global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ re
   __syncthreads();
   const int lx = threadIdx.x % LT, ly = threadIdx.x / LT;
   const int gx = blockIdx.x * LT + lx, gy = blockIdx.y * LT + ly;
-  const bool inside = gx < w && gy < h;
   double s_sum = 0.0, se_sum = 0.0;
-  if (inside) {
-    float out[12];
+  if (gx < w && gy < h) {
+    const size_t pixels = (size_t)w * h, p = (size_t)gy * w + gx;
+    float lsum = 0.0f;
 #pragma unroll
     for (int ch = 0; ch < 3; ch++) {
       F2 m01 = f2(0.f, 0.f), m23 = f2(0.f, 0.f);
       float m4 = 0.f;
 #pragma unroll
-      for (int t = -HALO; t <= HALO; t++) {  // rows past the image were blurred to 0
-        const int at = t < 0 ? -t : t;
-        m01 = f2_fma(wp[at], f2_load(&s_h01[ly + HALO + t][lx][ch]), m01);
-        m23 = f2_fma(wp[at], f2_load(&s_h23[ly + HALO + t][lx][ch]), m23);
-        m4 = fmaf(win.w[at], s_h4[ly + HALO + t][lx][ch], m4);
+      for (int k = 0; k < TAPS; k++) {  // rows past the image were blurred to 0
+        const int at = tap_weight(k);
+        m01 = f2_fma(wp[at], f2_load(&s_h01[ly + k][lx][ch]), m01);
+        m23 = f2_fma(wp[at], f2_load(&s_h23[ly + k][lx][ch]), m23);
+        m4 = fmaf(win.w[at], s_h4[ly + k][lx][ch], m4);
       }
       const float mx = f2_lo(m01), my = f2_hi(m01);
       const float vx = f2_lo(m23) - mx * mx, vy = f2_hi(m23) - my * my, cxy = m4 - mx * my;
       const float a1 = 2.0f * mx * my + C1, a2 = 2.0f * cxy + C2;
       const float b1 = mx * mx + my * my + C1, b2 = vx + vy + C2;
       const float s = a1 * a2 / (b1 * b2);
-      out[2 * ch] = s * (2.0f * my / a1 - 2.0f * my / a2 - 2.0f * mx / b1 + 2.0f * mx / b2);
-      out[2 * ch + 1] = -s / b2;
-      out[6 + ch] = 2.0f * s / a2;
-      out[9 + ch] = s;
+      const float2 xy = s_xy[ly + HALO][lx + HALO][ch];
       if (metrics) {
         s_sum += (double)s;
-        const float2 xy = s_xy[ly + HALO][lx + HALO][ch];
         const double d = (double)xy.x - (double)xy.y;
         se_sum += d * d;
+      } else {
+        reinterpret_cast<float2*>(partials)[ch * pixels + p] =
+            make_float2(s * (2.0f * my / a1 - 2.0f * my / a2 - 2.0f * mx / b1 + 2.0f * mx / b2), -s / b2);
+        partials[(6 + ch) * pixels + p] = 2.0f * s / a2;
+        lsum = lsum + ((1.0f - LAMBDA) * fabsf(xy.x - xy.y) - LAMBDA * s);
       }
     }
-    if (!metrics) {
-      float4* dst = reinterpret_cast<float4*>(partials + ((size_t)gy * w + gx) * 12);
-      dst[0] = make_float4(out[0], out[1], out[2], out[3]);
-      dst[1] = make_float4(out[4], out[5], out[6], out[7]);
-      dst[2] = make_float4(out[8], out[9], out[10], out[11]);
-    }
+    if (!metrics) pixel_loss[p] = lsum * (1.0f / (float)(3u * (uint32_t)(w * h)));
   }
   if (metrics) {
 #pragma unroll
@@ -199,100 +222,115 @@ __global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ re
   }
 }
 
-// Blurs the three partials and forms dL/dpixel and the pixel loss
-// (src/shaders/loss.wgsl:108-121). The first two partials' blurs run as a pair
-// of packed FP32 sums.
-__global__ void __launch_bounds__(256) gradient_kernel(const float4* __restrict__ rendered,
-                                                       const uchar4* const* __restrict__ target_slot, int w, int h,
-                                                       Window win, const float* __restrict__ partials,
-                                                       float4* __restrict__ pixel_grads, float* __restrict__ pixel_loss) {
-  __shared__ float2 s_p01[LS][LS][3];
-  __shared__ float s_p2[LS][LS][3];
-  __shared__ float2 s_h01[LS][LT][3];
-  __shared__ float s_h2[LS][LT][3];
-  __shared__ float s_unorm[256];  // read after the barriers below
+// Blurs the three partials and forms dL/dpixel (src/shaders/loss.wgsl:108-121) for
+// one strip's rows [y_begin, y_end): a warp per channel, a lane per column.
+__global__ void __launch_bounds__(STRIP_THREADS, STRIPS_PER_SM) gradient_kernel(
+    const float4* __restrict__ rendered, const uchar4* const* __restrict__ target_slot, int w, int h, int rows,
+    Window win, const float* __restrict__ partials, float4* __restrict__ pixel_grads) {
+  __shared__ float2 s_p01[4][3][SPAN];
+  __shared__ float s_p2[4][3][SPAN];
+  __shared__ float s_grad[2][2][3][COLS];
+  __shared__ float s_unorm[256];
   const uchar4* target = *target_slot;
-  const int x0 = blockIdx.x * LT - HALO, y0 = blockIdx.y * LT - HALO;
-  fill_unorm8(s_unorm, false);
-  for (int k = threadIdx.x; k < LS * LS; k += 256) {
-    const int ly = k / LS, lx = k % LS;
-    const int gx = x0 + lx, gy = y0 + ly;
-    const bool in = gx >= 0 && gy >= 0 && gx < w && gy < h;
-    float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, q2 = q0;
-    if (in) {
-      const float4* src = reinterpret_cast<const float4*>(partials + ((size_t)gy * w + gx) * 12);
-      q0 = src[0];
-      q1 = src[1];
-      q2 = src[2];
-    }
-    s_p01[ly][lx][0] = make_float2(q0.x, q0.y);
-    s_p01[ly][lx][1] = make_float2(q0.z, q0.w);
-    s_p01[ly][lx][2] = make_float2(q1.x, q1.y);
-    s_p2[ly][lx][0] = q1.z;
-    s_p2[ly][lx][1] = q1.w;
-    s_p2[ly][lx][2] = q2.x;
-  }
-  F2 wp[6];
+  const int lane = threadIdx.x & 31, ch = threadIdx.x >> 5;
+  const int x0 = blockIdx.x * COLS - HALO, gx = blockIdx.x * COLS + lane;
+  const int y_begin = blockIdx.y * rows, y_end = min(y_begin + rows, h);
+  const size_t pixels = (size_t)w * h;
+  const float2* p01 = reinterpret_cast<const float2*>(partials) + ch * pixels;
+  const float* p2 = partials + (6 + ch) * pixels;
+  // The warp's channel of rows y and y + 1 (zeros past the image): lane l brings
+  // columns x0 + l and x0 + 32 + l (the first 10 lanes), loaded while the rows before
+  // are blurred.
+  float2 next01[2][2];
+  float next2[2][2];
+  auto fetch = [&](int y) {
 #pragma unroll
-  for (int k = 0; k < 6; k++) wp[k] = f2(win.w[k], win.w[k]);
-  __syncthreads();
-  // Two adjacent output columns per item, as in ssim_kernel.
-  for (int k = threadIdx.x; k < LS * (LT / 2) * 3; k += 256) {
-    const int ch = k % 3, col = 2 * ((k / 3) % (LT / 2)), row = k / (3 * (LT / 2));
-    F2 a01 = f2(0.f, 0.f), b01 = a01;
-    float a2 = 0.f, b2 = 0.f;
+    for (int r = 0; r < 2; r++)
 #pragma unroll
-    for (int t = -HALO; t <= HALO + 1; t++) {  // the halo holds zeros past the image
-      const F2 p01 = f2_load(&s_p01[row][col + HALO + t][ch]);
-      const float p2 = s_p2[row][col + HALO + t][ch];
-      if (t <= HALO) {  // column col, tap t
-        const int at = t < 0 ? -t : t;
-        a01 = f2_fma(wp[at], p01, a01);
-        a2 = fmaf(win.w[at], p2, a2);
+      for (int u = 0; u < 2; u++) {
+        const int c = 32 * u + lane, col = x0 + c;
+        const bool in = c < SPAN && col >= 0 && col < w && y + r >= 0 && y + r < h;
+        next01[r][u] = in ? p01[(size_t)(y + r) * w + col] : make_float2(0.f, 0.f);
+        next2[r][u] = in ? p2[(size_t)(y + r) * w + col] : 0.f;
       }
-      if (t > -HALO) {  // column col + 1, tap t - 1
-        const int at = t - 1 < 0 ? 1 - t : t - 1;
-        b01 = f2_fma(wp[at], p01, b01);
-        b2 = fmaf(win.w[at], p2, b2);
+  };
+  auto stage = [&](int y) {
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        if (32 * u + lane >= SPAN) continue;
+        s_p01[(y + r) & 3][ch][32 * u + lane] = next01[r][u];
+        s_p2[(y + r) & 3][ch][32 * u + lane] = next2[r][u];
       }
-    }
-    f2_store(&s_h01[row][col][ch], a01);
-    s_h2[row][col][ch] = a2;
-    f2_store(&s_h01[row][col + 1][ch], b01);
-    s_h2[row][col + 1][ch] = b2;
-  }
-  __syncthreads();
-  const int lx = threadIdx.x % LT, ly = threadIdx.x / LT;
-  const int gx = blockIdx.x * LT + lx, gy = blockIdx.y * LT + ly;
-  if (gx >= w || gy >= h) return;
-  const size_t p = (size_t)gy * w + gx;
+  };
+  // acc[m][k]: map m's sum over taps -5..k - 5 of the output row 5 - k rows below.
+  float acc[3][TAPS - 1];
+#pragma unroll
+  for (int m = 0; m < 3; m++)
+#pragma unroll
+    for (int k = 0; k < TAPS - 1; k++) acc[m][k] = 0.f;
   const float scale = 1.0f / (float)(3u * (uint32_t)(w * h));
-  const float4 xv4 = rendered[p];
-  const uchar4 t4 = target[p];
-  const float xs[3] = {xv4.x, xv4.y, xv4.z};
-  const float ys[3] = {s_unorm[t4.x], s_unorm[t4.y], s_unorm[t4.z]};
-  const float* own = partials + p * 12;
-  float grad[3];
-  float lsum = 0.0f;
+  fetch(y_begin - HALO);
+  fill_unorm8(s_unorm, false, STRIP_THREADS);
+  stage(y_begin - HALO);
+  fetch(y_begin - HALO + 2);
+  __syncthreads();
+  // Two rows at a time: twice the independent work per barrier.
+  for (int y = y_begin - HALO; y < y_end + HALO; y += 2) {
+    stage(y + 2);
+    fetch(y + 4);
+    // The output rows' own pixels.
+    float x[2];
+    uint32_t byte[2];
+    bool wanted[2];
 #pragma unroll
-  for (int ch = 0; ch < 3; ch++) {
-    F2 m01 = f2(0.f, 0.f);
-    float m2 = 0.f;
-#pragma unroll
-    for (int t = -HALO; t <= HALO; t++) {  // rows past the image were blurred to 0
-      const int at = t < 0 ? -t : t;
-      m01 = f2_fma(wp[at], f2_load(&s_h01[ly + HALO + t][lx][ch]), m01);
-      m2 = fmaf(win.w[at], s_h2[ly + HALO + t][lx][ch], m2);
+    for (int u = 0; u < 2; u++) {
+      const int out = y + u - HALO;
+      const size_t p = (size_t)out * w + gx;
+      wanted[u] = out >= y_begin && out < y_end && gx < w;
+      x[u] = wanted[u] ? reinterpret_cast<const float*>(rendered + p)[ch] : 0.f;
+      byte[u] = wanted[u] ? reinterpret_cast<const unsigned char*>(target + p)[ch] : 0u;
     }
-    const float x = xs[ch], y = ys[ch];
-    const float sg = f2_lo(m01) + 2.0f * x * f2_hi(m01) + y * m2;
-    const float diff = x - y;
-    const float sign = diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f);
-    grad[ch] = ((1.0f - LAMBDA) * sign - LAMBDA * sg) * scale;
-    lsum = lsum + ((1.0f - LAMBDA) * fabsf(diff) - LAMBDA * own[9 + ch]);
+    float b[2][3];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const float2* row01 = s_p01[(y + u) & 3][ch] + lane;
+      const float* row2 = s_p2[(y + u) & 3][ch] + lane;
+      b[u][0] = b[u][1] = b[u][2] = 0.f;
+#pragma unroll
+      for (int k = 0; k < TAPS; k++) {
+        const float2 v = row01[k];
+        const float wk = win.w[tap_weight(k)];
+        b[u][0] = fmaf(wk, v.x, b[u][0]);
+        b[u][1] = fmaf(wk, v.y, b[u][1]);
+        b[u][2] = fmaf(wk, row2[k], b[u][2]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      float sum[3];
+#pragma unroll
+      for (int m = 0; m < 3; m++) {
+        sum[m] = fmaf(win.w[HALO], b[u][m], acc[m][TAPS - 2]);
+#pragma unroll
+        for (int k = TAPS - 2; k > 0; k--) acc[m][k] = fmaf(win.w[tap_weight(k)], b[u][m], acc[m][k - 1]);
+        acc[m][0] = fmaf(win.w[HALO], b[u][m], 0.f);
+      }
+      if (wanted[u]) {
+        const float yv = s_unorm[byte[u]];
+        const float sg = sum[0] + 2.0f * x[u] * sum[1] + yv * sum[2];
+        const float diff = x[u] - yv;
+        const float sign = diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f);
+        s_grad[(y >> 1) & 1][u][ch][lane] = ((1.0f - LAMBDA) * sign - LAMBDA * sg) * scale;
+      }
+    }
+    __syncthreads();
+    if (ch < 2 && (ch == 0 ? wanted[0] : wanted[1])) {  // warps 0 and 1: a row each
+      const float(*g)[COLS] = s_grad[(y >> 1) & 1][ch];
+      pixel_grads[(size_t)(y + ch - HALO) * w + gx] = make_float4(g[0][lane], g[1][lane], g[2][lane], 0.0f);
+    }
   }
-  pixel_grads[p] = make_float4(grad[0], grad[1], grad[2], 0.0f);
-  pixel_loss[p] = lsum * scale;
 }
 
 // Σ pixel_loss in double, in a fixed order (per-CTA partial sums, then one CTA).
@@ -332,18 +370,30 @@ Window window_weights() {
 
 }  // namespace
 
+// Rows per strip of gradient_kernel (even): as few as still fit on the GPU at once, so
+// that no strip waits for another's end; each strip costs 10 rows more. Six strips per
+// SM: 5 take 65 us at 1957x1091, 6 take 62, 7 take 68, 8 take 60; at 489x273 14 us for 6,
+// 15 for 7 and 8. At least 6 rows: at 251x187 10.6 us, 8 rows 11.5, 12 rows 12.3, 4 rows
+// no faster and at 489x273 1 us slower.
+static int strip_rows(const dg_context* ctx, uint32_t width, uint32_t height) {
+  const uint32_t across = ceil_div(width, COLS), room = (uint32_t)ctx->sm_count * STRIPS_PER_SM;
+  const uint32_t down = std::max(1u, room / across);
+  return std::max(MIN_ROWS, (int)(ceil_div(ceil_div(height, down), 2) * 2));
+}
+
 dg_status loss_launch(dg_training_loss* l, dg_buffer* rendered) {
   dg_context* ctx = l->ctx;
   const Window win = window_weights();
-  dim3 grid(ceil_div(l->width, LT), ceil_div(l->height, LT));
+  const int w = (int)l->width, h = (int)l->height, rows = strip_rows(ctx, l->width, l->height);
+  const auto* target = typed<const uchar4* const>(l->target_slot);
   DG_LAUNCH(ctx, "loss_ssim",
-            ssim_kernel<<<grid, 256, 0, ctx->stream>>>(
-                typed<float4>(rendered), typed<const uchar4* const>(l->target_slot), (int)l->width, (int)l->height,
-                win, typed<float>(l->partials), 0, nullptr));
+            ssim_kernel<<<dim3(ceil_div(w, LT), ceil_div(h, LT)), 256, 0, ctx->stream>>>(
+                typed<float4>(rendered), target, w, h, win, typed<float>(l->partials), typed<float>(l->pixel_loss), 0,
+                nullptr));
   DG_LAUNCH(ctx, "loss_gradient",
-            gradient_kernel<<<grid, 256, 0, ctx->stream>>>(
-                typed<float4>(rendered), typed<const uchar4* const>(l->target_slot), (int)l->width, (int)l->height,
-                win, typed<float>(l->partials), typed<float4>(l->pixel_grads), typed<float>(l->pixel_loss)));
+            gradient_kernel<<<dim3(ceil_div(w, COLS), ceil_div(h, rows)), STRIP_THREADS, 0, ctx->stream>>>(
+                typed<float4>(rendered), target, w, h, rows, win, typed<float>(l->partials),
+                typed<float4>(l->pixel_grads)));
   return DG_OK;
 }
 
@@ -368,7 +418,7 @@ dg_status metrics_launch(dg_context* ctx, dg_buffer* rendered, dg_buffer* target
   DG_LAUNCH(ctx, "metrics_ssim",
             ssim_kernel<<<grid, 256, 0, ctx->stream>>>(typed<float4>(rendered),
                                                        typed<const uchar4* const>(target_slot), (int)width,
-                                                       (int)height, win, nullptr, 1, sums_device));
+                                                       (int)height, win, nullptr, nullptr, 1, sums_device));
   return DG_OK;
 }
 
@@ -389,7 +439,7 @@ dg_status dg_training_loss_create(dg_context* ctx, uint32_t width, uint32_t heig
   l->sum_blocks = std::max(1u, ceil_div(pixels, 4096));
   dg_status st = alloc_buffer(ctx, pixels * 16, &l->pixel_grads);
   if (st == DG_OK) st = alloc_buffer(ctx, pixels * 4, &l->pixel_loss);
-  if (st == DG_OK) st = alloc_buffer(ctx, pixels * 12 * 4, &l->partials);
+  if (st == DG_OK) st = alloc_buffer(ctx, pixels * 9 * 4, &l->partials);
   if (st == DG_OK) st = alloc_buffer(ctx, 8, &l->target_slot);
   if (st == DG_OK) st = alloc_buffer(ctx, (l->sum_blocks + 1) * 8, &l->sum_scratch);
   if (st != DG_OK) {

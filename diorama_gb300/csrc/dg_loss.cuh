@@ -7,7 +7,7 @@ struct dg_training_loss {
   uint32_t width, height;
   dg_buffer* pixel_grads;  // vec4 per pixel
   dg_buffer* pixel_loss;   // f32 per pixel
-  dg_buffer* partials;     // 12 floats per pixel: three SSIM partials and S, rgb each
+  dg_buffer* partials;     // 9 floats per pixel: three SSIM partials, rgb each (planes)
   dg_buffer* target_slot;  // device pointer to the photo (rgba8), read by the kernels
   dg_buffer* sum_scratch;  // per-block partial sums, then the total
   uint32_t sum_blocks;
