@@ -152,7 +152,7 @@ dg_status dg_context_create(int32_t device, dg_context** out) {
     return cuda_fail(err, "context allocation");
   }
   ctx->staging_bytes = STAGING_BYTES;
-  dg_status st = sort_init();
+  dg_status st = sort_init(ctx);
   if (st == DG_OK) st = bin_init();
   if (st != DG_OK) {
     dg_context_destroy(ctx);

@@ -35,7 +35,7 @@ SortPlan sort_plan_digits(uint32_t capacity, uint32_t key_words, uint32_t bits);
 // together) vary; its last pass then sorts a 4-bit digit when that covers them.
 void sort_plan_key_bits(SortPlan& p, uint32_t bits);
 // Per-device kernel attributes; called once when a context is created.
-dg_status sort_init();
+dg_status sort_init(dg_context* ctx);
 size_t sort_scratch_bytes(const SortPlan& plan);
 dg_status sort_launch(dg_context* ctx, const SortPlan& plan, void* keys, uint32_t* values, void* keys_alt,
                       uint32_t* values_alt, const uint32_t* count, void* scratch);

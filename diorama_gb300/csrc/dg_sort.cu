@@ -11,10 +11,11 @@
 // or more dispatches and four barriers per 256-key chunk). Here it is onesweep
 // (Adinets & Merrill 2022): one upfront kernel reads every key once and builds
 // the digit histograms of all passes, then each pass is ONE kernel. A CTA takes
-// the next tile of 3840 keys by ticket, ranks each key within its warp with
-// ballots (stable: warp-striped loads are ranked round by round), publishes its
+// the next tile of 3840 keys by ticket, ranks each key within its warp
+// (stable: warp-striped loads are ranked round by round), publishes its
 // per-digit counts, looks back over earlier tiles' counts (bounded waits), and
-// scatters through shared memory so each digit's run is written contiguously.
+// scatters through shared memory so each digit's run is written contiguously. Up to
+// 65,536 keys the passes run in one kernel instead (sort_cluster_kernel).
 #include "dg_common.cuh"
 #include "dg_scan.cuh"
 
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   uint32_t* s_block_start = s_whist + SORT_WARPS * RADIX;
   uint32_t* s_base = s_block_start + RADIX;
   uint32_t* s_tmp = s_base + RADIX;
+  uint32_t* s_match = reinterpret_cast<uint32_t*>(smem);  // [warp][2][digit], until the keys are placed
   __shared__ uint32_t s_tile;
 
   constexpr uint32_t DIGITS = 1u << DBITS, DMASK = DIGITS - 1u;
@@ -182,9 +184,11 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   if (blockIdx.x >= tiles) return;
   if (tid == 0) s_tile = atomicAdd(ticket, 1u);
   for (int i = tid; i < SORT_WARPS * RADIX; i += SORT_THREADS) s_whist[i] = 0;
+  for (int i = tid; i < SORT_WARPS * 2 * RADIX; i += SORT_THREADS) s_match[i] = 0;
   __syncthreads();
   const uint32_t tile = s_tile;
   if (tile >= tiles) return;
+  const uint32_t digit_total = tid < DIGITS ? pass_hist[tid] : 0u;  // on its way while the keys are ranked
 
   // Load, warp-striped: warp w owns keys [w*480, w*480+480) of the tile, round j
   // reads 32 consecutive ones, so order within the tile is (warp, round, lane).
@@ -201,25 +205,26 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   }
   const uint32_t lt_mask = (1u << lane) - 1u;
   uint32_t* my_hist = s_whist + warp * DIGITS;
+  // The lanes that hold the same digit, from a word per digit in which each lane sets
+  // its bit: two sets of words in turn, so that a round's bits need not wait for the
+  // round before to be cleared. Against eight ballots and their selects per round (the
+  // ALU pipe's, 45 cycles of an SM a round): 4.2M u64 keys 285 -> 261 us in six passes,
+  // 1.1M u32 keys 73 -> 65 in four, 100k 49 -> 44. __match_any_sync took 90 for 1.1M.
+  uint32_t* my_match = s_match + warp * 2 * DIGITS;
 #pragma unroll
   for (int j = 0; j < SORT_ITEMS; j++) {
-    bool valid = base + j * 32 < n;
-    uint32_t d = (uint32_t)(key[j] >> shift) & DMASK;
-    uint32_t peers = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-    for (int b = 0; b < DBITS; b++) {
-      uint32_t bit = (d >> b) & 1u;
-      uint32_t vote = __ballot_sync(0xffffffffu, bit);
-      peers &= bit ? vote : ~vote;
-    }
-    int leader = valid ? __ffs(peers) - 1 : lane;
-    uint32_t old = 0;
-    if (valid && lane == leader) {
-      old = my_hist[d];
+    const bool valid = base + j * 32 < n;
+    const uint32_t d = (uint32_t)(key[j] >> shift) & DMASK;
+    uint32_t* match = my_match + (j & 1) * DIGITS;
+    if (valid) atomicOr(&match[d], 1u << lane);
+    __syncwarp();
+    const uint32_t peers = match[d], old = my_hist[d], before = __popc(peers & lt_mask);
+    __syncwarp();
+    if (valid && before == 0) {  // the first of them counts them all
       my_hist[d] = old + __popc(peers);
+      match[d] = 0;
     }
-    old = __shfl_sync(0xffffffffu, old, leader);
-    rank[j] = old + __popc(peers & lt_mask);
+    rank[j] = old + before;
     __syncwarp();
   }
   __syncthreads();
@@ -240,7 +245,7 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   }
   const uint32_t tile_count = running;
   const uint32_t block_start = block_exclusive_256(tile_count, s_tmp);
-  const uint32_t global_start = block_exclusive_256(digit ? pass_hist[d] : 0u, s_tmp);
+  const uint32_t global_start = block_exclusive_256(digit_total, s_tmp);
   if (digit) s_block_start[d] = block_start;
 
   // Decoupled look-back over earlier tiles, for this thread's digit: the states
@@ -302,6 +307,270 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   }
 }
 
+// ---------------------------------------------------------------- one cluster
+// Few keys: the whole sort is one kernel on one cluster of 16 CTAs, which hold the
+// keys in their shared memory (CTA c has positions [c seg, (c + 1) seg)) from the
+// first pass to the last. A pass reads its keys into registers, ranks them within the
+// warp, exchanges the CTAs' digit counts over distributed shared memory, and stores
+// each key straight into its new place, in whichever CTA that lies: two cluster
+// barriers instead of a launch, a ticket, a look-back and a trip through L2 each.
+// What bounds it: at a few thousand keys the barriers (15 us for 300 keys), beyond that
+// 16 SMs' shared memory and ranking (0.3 us per 1,000 keys).
+// Passes (clear and histogram with them) against one cluster, in us, without the 3 us
+// that timing one kernel adds: u32 keys in four passes, 5,000 36 and 18; 16,000 36 and
+// 20; 50,000 38 and 28; 65,536 39 and 32; 100,000 40 and 42. u64 keys in six, 5,000 54
+// and 24; 32,000 54 and 44; 50,000 61 and 54; 65,536 64 and 68; 100,000 66 and 95.
+// 256 threads with the same room take as long, 1024 more (their bookkeeping); 8 CTAs 48
+// us where 16 take 38 (50,000 keys); putting a CTA's keys in digit order first, so that
+// its stores come in runs, changed nothing.
+constexpr uint32_t CLUSTER = 16;
+constexpr uint32_t CLUSTER_THREADS = 512, CLUSTER_WARPS = CLUSTER_THREADS / 32;
+constexpr uint32_t CLUSTER_PARTS = CLUSTER_THREADS / RADIX;  // 2 threads share a digit's sums
+constexpr int CLUSTER_ITEMS = 8;
+constexpr uint32_t CLUSTER_KEYS = CLUSTER * CLUSTER_THREADS * CLUSTER_ITEMS;  // 65,536
+
+template <int KW>
+struct ClusterShared {
+  static constexpr uint32_t ROOM = CLUSTER_THREADS * CLUSTER_ITEMS;
+  // u32 keys: a key and its value in one word, which one store brings to its place.
+  uint64_t keys[ROOM];
+  uint32_t vals[KW == 2 ? ROOM : 4];
+  alignas(16) uint16_t whist[CLUSTER_WARPS][RADIX];  // a warp's counts, then where its run of a digit begins in the CTA's
+  uint16_t counts[CLUSTER][RADIX];           // every CTA's counts
+  uint32_t match[CLUSTER_WARPS][2][RADIX];           // the lanes that have a digit; zero between rounds
+  uint32_t part[2][CLUSTER_PARTS][RADIX];
+  uint32_t base[RADIX];                      // the CTA's first place for a digit
+  uint32_t tmp[RADIX / 32];
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The address of this CTA's shared variable in CTA `cta` of the cluster.
+__device__ __forceinline__ uint32_t remote(const void* p, uint32_t cta) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
+  return a;
+}
+__device__ __forceinline__ void store_remote(uint32_t addr, uint16_t v) {
+  asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
+}
+__device__ __forceinline__ void store_remote(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void store_remote(uint32_t addr, uint64_t v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+
+template <int KW>
+__global__ void __launch_bounds__(CLUSTER_THREADS, 1)
+    sort_cluster_kernel(const typename KeyOf<KW>::type* keys_in, const uint32_t* vals_in,
+                        typename KeyOf<KW>::type* keys_out, uint32_t* vals_out, uint32_t capacity,
+                        const uint32_t* count, uint32_t passes, PassShifts shifts) {
+  using K = typename KeyOf<KW>::type;
+  extern __shared__ __align__(16) unsigned char smem[];
+  auto& s = *reinterpret_cast<ClusterShared<KW>*>(smem);
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = cluster_rank();
+  const uint32_t n = count ? min(*count, capacity) : capacity;
+  if (n == 0) return;  // in every CTA of the cluster
+  cluster_arrive();    // nothing is stored in a CTA that has not started
+  const uint32_t seg = ((n + CLUSTER - 1) / CLUSTER + 31) & ~31u;
+  // pos / seg = pos * magic >> 32: magic is off by less than seg <= 2^12 parts in 2^32,
+  // and pos < 2^16.
+  const uint32_t magic = 0xffffffffu / seg + 1u;
+  const uint32_t begin = cta * seg, mine = begin < n ? min(seg, n - begin) : 0u;
+  // Warp w has keys [w * rounds * 32, (w + 1) * rounds * 32) of the segment, round j
+  // reads 32 consecutive ones: order within the CTA is (warp, round, lane).
+  const uint32_t rounds = (seg + CLUSTER_THREADS - 1) / CLUSTER_THREADS;
+  const uint32_t first = warp * rounds * 32 + lane;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  const uint32_t digit = tid % RADIX, part = tid / RADIX;
+  uint16_t* my_hist = s.whist[warp];
+
+  for (uint32_t k = lane; k < 2 * RADIX; k += 32) s.match[warp][k / RADIX][k % RADIX] = 0;
+
+  for (uint32_t p = 0; p < passes; p++) {
+    const uint32_t shift = shifts.shift[p];
+    K key[CLUSTER_ITEMS];
+    uint32_t val[CLUSTER_ITEMS], rank[(CLUSTER_ITEMS + 1) / 2];
+    reinterpret_cast<uint4*>(my_hist)[lane] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < CLUSTER_ITEMS; j++) {
+      const uint32_t at = first + j * 32;
+      if (j < rounds && at < mine) {
+        if (p == 0) {
+          key[j] = keys_in[begin + at];
+          val[j] = vals_in[begin + at];
+        } else {
+          key[j] = (K)s.keys[at];
+          val[j] = KW == 1 ? (uint32_t)(s.keys[at] >> 32) : s.vals[at];
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < CLUSTER_ITEMS; j++) {
+      if (j >= rounds) break;
+      const bool valid = first + j * 32 < mine;
+      const uint32_t d = valid ? (uint32_t)(key[j] >> shift) & (RADIX - 1) : 0u;
+      uint32_t* m = s.match[warp][j & 1];
+      if (valid) atomicOr(&m[d], 1u << lane);
+      __syncwarp();
+      const uint32_t peers = m[d], old = my_hist[d], before = __popc(peers & lt_mask);
+      __syncwarp();
+      if (valid && before == 0) {
+        my_hist[d] = (uint16_t)(old + __popc(peers));
+        m[d] = 0;
+      }
+      rank[j / 2] = j & 1 ? rank[j / 2] | (old + before) << 16 : old + before;
+      __syncwarp();
+    }
+    __syncthreads();
+
+    // Where each warp's run of a digit begins; the CTA's counts, sent to every CTA.
+    // Thread (part, digit) has a share of the warps and of the CTAs.
+    constexpr uint32_t PARTS = CLUSTER_PARTS, WP = CLUSTER_WARPS / PARTS, CP = CLUSTER / PARTS;
+    uint32_t c[WP], sum = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < WP; w++) {
+      c[w] = s.whist[part * WP + w][digit];
+      sum += c[w];
+    }
+    s.part[0][part][digit] = sum;
+    __syncthreads();
+    uint32_t running = 0, total = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < PARTS; q++) {
+      const uint32_t v = s.part[0][q][digit];
+      running += q < part ? v : 0u;
+      total += v;
+    }
+#pragma unroll
+    for (uint32_t w = 0; w < WP; w++) {
+      s.whist[part * WP + w][digit] = (uint16_t)running;
+      running += c[w];
+    }
+    if (p == 0) cluster_wait();
+#pragma unroll
+    for (uint32_t k = 0; k < CP; k++)
+      store_remote(remote(&s.counts[cta][digit], part * CP + k), (uint16_t)total);
+    cluster_arrive();
+    cluster_wait();
+
+    // The first place of each digit of this CTA's: the keys of smaller digits, and
+    // those of the same digit in CTAs before.
+    uint32_t all = 0, before = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < CP; k++) {
+      const uint32_t v = s.counts[part * CP + k][digit];
+      all += v;
+      before += part * CP + k < cta ? v : 0u;
+    }
+    s.part[0][part][digit] = all;
+    s.part[1][part][digit] = before;
+    __syncthreads();
+    uint32_t incl = 0;
+    if (tid < RADIX) {
+#pragma unroll
+      for (uint32_t q = 1; q < PARTS; q++) {
+        all += s.part[0][q][digit];
+        before += s.part[1][q][digit];
+      }
+      incl = all;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+      }
+      if (lane == 31) s.tmp[warp] = incl;
+    }
+    __syncthreads();
+    if (tid < RADIX) {
+#pragma unroll
+      for (uint32_t w = 0; w < RADIX / 32; w++) before += w < warp ? s.tmp[w] : 0u;
+      s.base[digit] = incl - all + before;
+    }
+    __syncthreads();
+
+#pragma unroll
+    for (int j = 0; j < CLUSTER_ITEMS; j++) {
+      if (j >= rounds) break;
+      if (first + j * 32 < mine) {
+        const uint32_t d = (uint32_t)(key[j] >> shift) & (RADIX - 1);
+        const uint32_t r = j & 1 ? rank[j / 2] >> 16 : rank[j / 2] & 0xffffu;
+        const uint32_t pos = s.base[d] + my_hist[d] + r;
+        const uint32_t to = __umulhi(pos, magic), at = pos - to * seg;
+        if constexpr (KW == 1) {
+          store_remote(remote(&s.keys[at], to), (uint64_t)val[j] << 32 | key[j]);
+        } else {
+          store_remote(remote(&s.keys[at], to), key[j]);
+          store_remote(remote(&s.vals[at], to), val[j]);
+        }
+      }
+    }
+    cluster_arrive();
+    cluster_wait();
+  }
+  for (uint32_t k = tid; k < mine; k += CLUSTER_THREADS) {
+    keys_out[begin + k] = (K)s.keys[k];
+    vals_out[begin + k] = KW == 1 ? (uint32_t)(s.keys[k] >> 32) : s.vals[k];
+  }
+}
+
+template <int KW>
+cudaLaunchConfig_t cluster_config(cudaStream_t stream, cudaLaunchAttribute* cluster) {
+  *cluster = {};
+  cluster->id = cudaLaunchAttributeClusterDimension;
+  cluster->val.clusterDim.x = CLUSTER;
+  cluster->val.clusterDim.y = cluster->val.clusterDim.z = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = CLUSTER;
+  config.blockDim = CLUSTER_THREADS;
+  config.dynamicSmemBytes = sizeof(ClusterShared<KW>);
+  config.stream = stream;
+  config.attrs = cluster;
+  config.numAttrs = 1;
+  return config;
+}
+
+// Clears *fits where the device cannot run the cluster.
+template <int KW>
+void cluster_init(bool* fits) {
+  const auto kernel = sort_cluster_kernel<KW>;
+  cudaLaunchAttribute cluster;
+  const cudaLaunchConfig_t config = cluster_config<KW>(nullptr, &cluster);
+  int clusters = 0;
+  const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)config.dynamicSmemBytes) == cudaSuccess &&
+                  cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) == cudaSuccess && clusters > 0;
+  if (ok) return;
+  *fits = false;
+  cudaGetLastError();
+}
+
+template <int KW>
+dg_status cluster_launch(dg_context* ctx, const SortPlan& plan, void* keys, uint32_t* values, void* keys_alt,
+                         uint32_t* values_alt, const uint32_t* count) {
+  using K = typename KeyOf<KW>::type;
+  PassShifts shifts{};
+  for (uint32_t p = 0; p < plan.passes; p++) shifts.shift[p] = plan.shift[p];
+  const bool odd = plan.passes & 1;
+  cudaLaunchAttribute cluster;
+  const cudaLaunchConfig_t config = cluster_config<KW>(ctx->stream, &cluster);
+  cudaError_t err = cudaSuccess;
+  DG_LAUNCH(ctx, "sort_cluster",
+            err = cudaLaunchKernelEx(&config, sort_cluster_kernel<KW>, static_cast<const K*>(keys),
+                                     static_cast<const uint32_t*>(values), static_cast<K*>(odd ? keys_alt : keys),
+                                     odd ? values_alt : values, plan.capacity, count, plan.passes, shifts));
+  DG_CUDA(err);
+  return DG_OK;
+}
+
 template <int KW>
 size_t pass_smem_bytes() {
   return SORT_TILE * (sizeof(typename KeyOf<KW>::type) + 4) + (SORT_WARPS * RADIX + 2 * RADIX + 32) * 4;
@@ -326,6 +595,10 @@ template <int KW>
 dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32_t* values, void* keys_alt,
                        uint32_t* values_alt, const uint32_t* count, void* scratch) {
   using K = typename KeyOf<KW>::type;
+  // One cluster up to the sizes at which it still beats the passes (figures above
+  // sort_cluster_kernel).
+  if (ctx->cluster_sort && plan.capacity <= CLUSTER_KEYS)
+    return cluster_launch<KW>(ctx, plan, keys, values, keys_alt, values_alt, count);
   ScratchLayout l = layout_of(plan);
   char* s = static_cast<char*>(scratch);
   auto* tickets = reinterpret_cast<uint32_t*>(s + l.tickets);
@@ -359,7 +632,11 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
 
 }  // namespace
 
-dg_status sort_init() {
+dg_status sort_init(dg_context* ctx) {
+  // A device without 16 SMs in one GPC (a partition of one) sorts by passes.
+  ctx->cluster_sort = true;
+  cluster_init<1>(&ctx->cluster_sort);
+  cluster_init<2>(&ctx->cluster_sort);
   // The pass kernels use more than the default 48 KB of dynamic shared memory.
   DG_CUDA(cudaFuncSetAttribute(sort_pass_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)pass_smem_bytes<1>()));
