@@ -289,24 +289,28 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
-// exp_blend_core of two values at once: the polynomial's fused multiply-adds run
-// as packed pairs, each lane the same fmaf as exp_blend_core's, so both results
-// are exp_blend_core's bit for bit.
-__device__ __forceinline__ void exp_blend_core2(float x0, float x1, float& e0, float& e1) {
-  const float n0 = rintf(x0 * 1.44269504088896341f), n1 = rintf(x1 * 1.44269504088896341f);
-  const F2 n = f2(n0, n1);
-  F2 r = f2_fma(n, f2(-0.693145751953125f, -0.693145751953125f), f2(x0, x1));
-  r = f2_fma(n, f2(-1.428606820309417232e-6f, -1.428606820309417232e-6f), r);
-  F2 p = f2(1.98412698412698413e-4f, 1.98412698412698413e-4f);
+// exp_blend_core of -q for two values at once, each lane of the pair its result bit for
+// bit where it is defined: the sign of the argument goes into every other coefficient.
+// The fused multiply-adds run as packed pairs, and rintf is the addition of 1.5 * 2^23,
+// whose sum holds the rounded integer in its low bits (and in 2^n's exponent when
+// shifted up by 23), which takes two conversions per value off the special-function unit.
+__device__ __forceinline__ F2 exp_blend_negated(F2 q) {
+  constexpr float ROUND = 12582912.0f;  // 1.5 * 2^23: bits 0x4b400000
+  const float s0 = __fadd_rn(__fmul_rn(f2_lo(q), -1.44269504088896341f), ROUND);
+  const float s1 = __fadd_rn(__fmul_rn(f2_hi(q), -1.44269504088896341f), ROUND);
+  const F2 n = f2_add(f2(s0, s1), f2(-ROUND, -ROUND));
+  F2 r = f2_fma(n, f2(0.693145751953125f, 0.693145751953125f), q);
+  r = f2_fma(n, f2(1.428606820309417232e-6f, 1.428606820309417232e-6f), r);
+  F2 p = f2(-1.98412698412698413e-4f, -1.98412698412698413e-4f);
   p = f2_fma(p, r, f2(1.38888888888888889e-3f, 1.38888888888888889e-3f));
-  p = f2_fma(p, r, f2(8.33333333333333333e-3f, 8.33333333333333333e-3f));
+  p = f2_fma(p, r, f2(-8.33333333333333333e-3f, -8.33333333333333333e-3f));
   p = f2_fma(p, r, f2(4.16666666666666667e-2f, 4.16666666666666667e-2f));
-  p = f2_fma(p, r, f2(1.66666666666666667e-1f, 1.66666666666666667e-1f));
+  p = f2_fma(p, r, f2(-1.66666666666666667e-1f, -1.66666666666666667e-1f));
   p = f2_fma(p, r, f2(0.5f, 0.5f));
+  p = f2_fma(p, r, f2(-1.0f, -1.0f));
   p = f2_fma(p, r, f2(1.0f, 1.0f));
-  p = f2_fma(p, r, f2(1.0f, 1.0f));
-  e0 = f2_lo(p) * __int_as_float(((int32_t)n0 + 127) << 23);
-  e1 = f2_hi(p) * __int_as_float(((int32_t)n1 + 127) << 23);
+  return f2_mul(p, f2(__uint_as_float((__float_as_uint(s0) << 23) + 0x3f800000u),
+                      __uint_as_float((__float_as_uint(s1) << 23) + 0x3f800000u)));
 }
 #endif  // __CUDACC__
 

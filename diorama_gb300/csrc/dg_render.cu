@@ -570,97 +570,94 @@ __device__ __forceinline__ void save_checkpoints(float4* __restrict__ checkpoint
 struct PixelBlend {
   float cx, cy;
   float T, r, g, b;
-  uint32_t last;
   bool done;
 
-  // The alphas of up to 4 staged entries e[0..n) of `st` at this pixel, 0 where
-  // the pixel does not blend the splat (alpha under 1/255; a power under the
-  // splat's cutoff skips the exp with the same outcome). Computed together:
-  // independent work the SM can overlap. Returns false, with all alphas 0, when
-  // no lane reaches any of the 4 cutoffs.
-  __device__ __forceinline__ bool alphas4(const WarpStage& st, const uint32_t (&e)[4], uint32_t n, bool active,
-                                          float (&alpha)[4]) const {
-    float power[4], opacity[4];
-    bool need[4], any = false;
+  // The alphas of staged entries j..j + 3 of `st` at this pixel, and whether it blends
+  // them; an alpha is 0 where it does not (alpha under 1/255; a power under the splat's
+  // cutoff skips the exp with the same outcome). Two entries run as the lanes of packed
+  // instructions, on the negated power: each the scalar form's bits (blend_power,
+  // exp_blend_core). Returns false when no lane reaches any of the 4 cutoffs.
+  __device__ __forceinline__ bool alphas4(const BlendStage& st, uint32_t j, bool active, float (&alpha)[4],
+                                          bool (&has)[4]) const {
+    const F2 px = f2(cx, cx), py = f2(cy, cy);
+    F2 q[2];
 #pragma unroll
-    for (uint32_t u = 0; u < 4; u++) {
-      const float4 m = st.mean[e[u]];
-      const float4 q = st.quad[e[u]];
-      power[u] = blend_power(q.x, q.y, q.z, cx - m.x, cy - m.y);
-      opacity[u] = m.z;
-      need[u] = active && u < n && power[u] >= q.w && power[u] <= 0.0f;
-      any |= need[u];
+    for (uint32_t h = 0; h < 2; h++) {
+      const BlendPair& e = st.pair[j / 2 + h];
+      const ulonglong2 n = e.n, ab = e.ab, cl = e.cl;
+      const F2 dx = f2_add(px, F2{n.x}), dy = f2_add(py, F2{n.y});
+      const F2 s = f2_fma(F2{ab.x}, dx, f2_mul(F2{ab.y}, dy));
+      // + 0 makes a zero's sign positive: bits compare like values from 0 up.
+      q[h] = f2_add(f2_fma(s, dx, f2_mul(f2_mul(F2{cl.x}, dy), dy)), f2(0.0f, 0.0f));
+      const F2 limit{cl.y};
+      has[2 * h] = active && __float_as_uint(f2_lo(q[h])) < __float_as_uint(f2_lo(limit));
+      has[2 * h + 1] = active && __float_as_uint(f2_hi(q[h])) < __float_as_uint(f2_hi(limit));
     }
-    if (!__any_sync(0xffffffffu, any)) {
+    if (!__any_sync(0xffffffffu, has[0] || has[1] || has[2] || has[3])) return false;
 #pragma unroll
-      for (uint32_t u = 0; u < 4; u++) alpha[u] = 0.0f;
-      return false;
-    }
-    float G[4];
-    exp_blend_core2(need[0] ? power[0] : 0.0f, need[1] ? power[1] : 0.0f, G[0], G[1]);
-    exp_blend_core2(need[2] ? power[2] : 0.0f, need[3] ? power[3] : 0.0f, G[2], G[3]);
-#pragma unroll
-    for (uint32_t u = 0; u < 4; u++) {
-      const float a = fminf(0.99f, opacity[u] * G[u]);
-      alpha[u] = need[u] && a >= 1.0f / 255.0f ? a : 0.0f;
+    for (uint32_t h = 0; h < 2; h++) {
+      // Any value may come out where the limit was not kept.
+      const F2 a = f2_mul(F2{st.pair[j / 2 + h].opacity}, exp_blend_negated(q[h]));
+      const float a0 = fminf(0.99f, f2_lo(a)), a1 = fminf(0.99f, f2_hi(a));
+      has[2 * h] = has[2 * h] && a0 >= 1.0f / 255.0f;
+      has[2 * h + 1] = has[2 * h + 1] && a1 >= 1.0f / 255.0f;
+      alpha[2 * h] = has[2 * h] ? a0 : 0.0f;
+      alpha[2 * h + 1] = has[2 * h + 1] ? a1 : 0.0f;
     }
     return true;
   }
 
-  // Blends one splat of alpha `alpha` (0: not blended here) and colour c whose
-  // 1-based list position is pos1; stops before the splat that would take the
+  __device__ __forceinline__ void add(float4 c, float w) {
+    // color += c alpha T (src/shaders/rasterize.wgsl:88) as c (alpha T) + color,
+    // one fused multiply-add per channel (the oracle's same sequence).
+    r = __fmaf_rn(c.x, w, r);
+    g = __fmaf_rn(c.y, w, g);
+    b = __fmaf_rn(c.z, w, b);
+  }
+
+  // Blends one splat of alpha `alpha` (0: not blended here) and colour c, and sets
+  // `at` to `mark` if it did; stops before the splat that would take the
   // transmittance below 1e-4 (src/shaders/rasterize.wgsl:62-92). Without
   // branches: a splat the pixel does not take adds c * 0 (colours are
   // non-negative, so the sums do not change) and keeps T and last. While the pixel
   // runs T >= 1e-4, so alpha 0 (remaining = T) never stops it.
-  __device__ __forceinline__ void blend(float alpha, float4 c, uint32_t pos1) {
+  __device__ __forceinline__ void blend(float alpha, float4 c, uint32_t mark, uint32_t& at) {
     const float remaining = T * (1.0f - alpha);
     done = done || remaining < 0.0001f;
     const bool take = !done && alpha != 0.0f;
-    // color += c alpha T (src/shaders/rasterize.wgsl:88) as c (alpha T) + color,
-    // one fused multiply-add per channel (the oracle's same sequence).
-    const float w = take ? __fmul_rn(alpha, T) : 0.0f;
-    r = __fmaf_rn(c.x, w, r);
-    g = __fmaf_rn(c.y, w, g);
-    b = __fmaf_rn(c.z, w, b);
+    add(c, take ? __fmul_rn(alpha, T) : 0.0f);
     T = take ? remaining : T;
-    last = take ? pos1 : last;
+    at = take ? mark : at;
   }
 
-  // Applies up to 4 staged entries e[0..n) of `st` in list order. Sets bit
-  // (position - base) of `blended` for each entry with a nonzero alpha at some
-  // pixel of the warp that had not stopped: every entry a pixel blends, and at
-  // most a last one it stopped at.
-  __device__ __forceinline__ void apply4(const WarpStage& st, const uint32_t (&e)[4], uint32_t n, uint32_t base,
-                                         uint32_t& blended) {
-    float alpha[4];
-    if (!alphas4(st, e, n, !done, alpha)) return;
-    const uint32_t mine = (alpha[0] != 0.0f ? 1u : 0u) | (alpha[1] != 0.0f ? 2u : 0u) |
-                          (alpha[2] != 0.0f ? 4u : 0u) | (alpha[3] != 0.0f ? 8u : 0u);
-    const uint32_t any = __reduce_or_sync(0xffffffffu, mine);
+  // Blends 4 splats in order, those with `use` (the same on every lane), as blend()
+  // does one by one. The transmittance only falls, so when it ends at 1e-4 or more
+  // at every pixel, none stopped on the way and the tests and selects of each splat
+  // are not needed: a chain of four products, and as many as there are fused
+  // multiply-adds. A pixel that had stopped has alphas of 0 here.
+  template <class Color>
+  __device__ __forceinline__ void blend4(const float (&alpha)[4], const bool (&has)[4], const bool (&use)[4], Color color,
+                                         const uint32_t (&mark)[4], uint32_t& at) {
+    float before[4], t = T;
 #pragma unroll
     for (uint32_t u = 0; u < 4; u++) {
-      if ((any >> u) & 1u) {  // the same on every lane
-        const uint32_t pos = st.pos[e[u]];
-        blended |= 1u << (pos - base);
-        blend(alpha[u], st.color[e[u]], pos + 1);
-      }
+      before[u] = t;
+      t = t * (1.0f - alpha[u]);
     }
+    if (__any_sync(0xffffffffu, t < 0.0001f)) {
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++)
+        if (use[u]) blend(alpha[u], color(u), mark[u], at);
+      return;
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      if (use[u]) add(color(u), __fmul_rn(alpha[u], before[u]));
+      at = has[u] ? mark[u] : at;
+    }
+    T = t;
   }
 };
-
-// The blend mask: bit p % 32 of word (p / 32) * 8 + block is set when some pixel
-// of 8x4 block `block` of the tile holding pair p blended that pair's splat. The
-// forward pass sets the bits, the backward pass walks only those entries. Both
-// helpers take the 32 bits of positions [p0, p0 + 32) of the pair list.
-__device__ __forceinline__ void publish_blended(uint32_t* __restrict__ mask, uint32_t p0, uint32_t block,
-                                                uint32_t bits) {
-  if (bits == 0 || !mask) return;
-  const uint32_t w = p0 >> 5, shift = p0 & 31u;
-  const uint32_t lo = bits << shift, hi = shift ? bits >> (32u - shift) : 0u;
-  if (lo) atomicOr(&mask[(size_t)w * 8u + block], lo);
-  if (hi) atomicOr(&mask[(size_t)(w + 1) * 8u + block], hi);
-}
 
 // The geometry of a blend item: tile `tile` (of the view tile / tiles_per_view
 // when several views are blended together), 8x4 block `block`, this lane's pixel.
@@ -672,10 +669,12 @@ struct BlendItem {
   bool inside;
   float x0, y0;  // the block's first pixel center
   uint2 run;
+  uint32_t tile;
   uint32_t tx, ty;  // the block's 16x16 tile
   __device__ __forceinline__ BlendItem(uint32_t tile, uint32_t block, uint32_t lane, uint32_t tiles_x,
                                        uint32_t tiles_per_view, float vpx, float vpy, const uint2* __restrict__ ranges,
-                                       uint32_t twl = 0, uint32_t thl = 0) {
+                                       uint32_t twl = 0, uint32_t thl = 0)
+      : tile(tile) {
     const uint32_t view = tile / tiles_per_view, local = tile - view * tiles_per_view;
     const uint32_t blend_x = blend_tiles_along(tiles_x, twl), sub = block >> 3;
     tx = ((local % blend_x) << twl) + (sub & ((1u << twl) - 1u));
@@ -692,13 +691,13 @@ struct BlendItem {
   }
 };
 
-__device__ __forceinline__ void write_pixel(const BlendItem& it, const PixelBlend& pb, float4 bg,
+__device__ __forceinline__ void write_pixel(const BlendItem& it, const PixelBlend& pb, uint32_t last, float4 bg,
                                             uchar4* __restrict__ target, float4* __restrict__ pixel_color,
                                             uint32_t* __restrict__ pixel_last) {
   if (!it.inside) return;
   const float fr = pb.r + pb.T * bg.x, fg = pb.g + pb.T * bg.y, fb = pb.b + pb.T * bg.z;
   pixel_color[it.pixel] = make_float4(fr, fg, fb, pb.T);
-  pixel_last[it.pixel] = pb.last;
+  pixel_last[it.pixel] = last;
   if (target) target[it.pixel] = make_uchar4(to_unorm8(fr), to_unorm8(fg), to_unorm8(fb), 255);
 }
 
@@ -721,31 +720,44 @@ __device__ __forceinline__ void write_pixel(const BlendItem& it, const PixelBlen
 // - Every warp then takes the other blocks on its own, walking the list 32
 //   entries at a time.
 //
-// In both, a window's splat records are copied into shared memory while the
-// previous one blends (two to four windows ahead were no faster), a splat rejected for the block has alpha below 1/255 at
-// all of its pixels, and a power under the splat's cutoff skips the exp: none of
-// these changes a result. The pixel state at each CHUNK boundary of the list is
-// saved for the backward pass, and which entries each block blended.
+// In both, a window's splat records are loaded into registers while the previous one
+// blends, a splat rejected for the block has alpha below 1/255 at all of its pixels,
+// and a power under the splat's cutoff skips the exp: none of these changes a result.
+// The pixel state at each CHUNK boundary of the list is saved for the backward pass,
+// and which entries each block blended.
+//
+// Instructions bound it (74% of the issue slots of a frame, half of them the ALU
+// pipe's compares, selects and votes), where one long list does not. What each splat
+// costs was brought down by (1.1M splats at 1960x1090 | 1.1M at 980x545 | 201k at
+// 489x273 | 12 views of 300k, us): two entries per packed instruction and the stop test
+// once per 4 splats (496 | 294 | 130 | 721 -> 433 | 283 | 123 | 692), one integer
+// compare for the power's two limits, the rounding of the exp's argument by an addition
+// and two edges instead of four in the window's test (408 | 266 | 113 | 667), records in
+// registers instead of shared memory with room for 128 registers a thread (395 | 241 |
+// 105 | 517; 5 and 6 CTAs per SM 399 | 249 | 110 | 539 and 400 | 283 | 124 | 719), and no
+// vote per group on whether all pixels have stopped (380 | 242 | 104 | 500). Slower:
+// cooperative CTAs of 192 or 256 threads (294 and 398 us for 1.1M at 980x545), 8 entries
+// at a time in them (264), the next block's number fetched early (views 587).
 // Cooperative blending costs about 1.4 times the instructions of a warp on its own and
 // its CTA's warps wait for each other every round, but a long walk takes a third of
 // the time. So it pays where a walk would outlast the rest of the frame: for tiles of
 // COOP_LOAD times the work a warp gets on average, and for all when the longest list
 // is COOP_CHAIN times that (some block of it may walk it to the end however opaque
 // the tile is, and shares its SM with fewer busy warps when all are cooperative).
-// Against blending every tile of more than 128 entries cooperatively: 1.1M splats at
-// 1960x1090 (at most 6,000 entries a tile, 75,000 a warp) 990 -> 494 us, 200,000 at
-// 1280x720 441 -> 244, 12 views of 300,000 948 -> 735; where chains bound it (1.1M at
-// 980x545, lists up to 30,000) 295 both ways. COOP_LOAD 0.5 and 2, COOP_CHAIN 8 and
-// PLAN_DEPTH 8, 32 and 64 were slower on one scene or another.
+// Against blending every tile of more than 128 entries cooperatively, with the blend of
+// that time: 1.1M splats at 1960x1090 (at most 6,000 entries a tile, 75,000 a warp)
+// 990 -> 494 us, 200,000 at 1280x720 441 -> 244, 12 views of 300,000 948 -> 735; where
+// chains bound it (1.1M at 980x545, lists up to 30,000) 295 both ways. COOP_LOAD 1 and 4,
+// COOP_CHAIN 8 and 12 and PLAN_DEPTH 8, 32 and 64 were slower on one scene or another.
 constexpr float COOP_LOAD = 1.5f, COOP_CHAIN = 5.0f;
 template <uint32_t TWL, uint32_t THL>
-__global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
+__global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
     const Camera* __restrict__ camera, const float4* __restrict__ raster_params, const float* __restrict__ splats,
     const uint32_t* __restrict__ pair_splats, const uint2* __restrict__ ranges, const uint32_t* __restrict__ plan,
     uint32_t tiles_per_view, uint32_t coop_min, uchar4* __restrict__ target, float4* __restrict__ pixel_color,
     uint32_t* __restrict__ pixel_last, float4* __restrict__ checkpoints, uint32_t* __restrict__ blend_mask,
     uint32_t* __restrict__ counters, bool cut_in_record) {
-  __shared__ WarpStage stages[FWD_WARPS];
+  __shared__ BlendStage stages[FWD_WARPS];
   // Cooperative blending, double-buffered by round: each producer's queued entries
   // (alpha per pixel; colour with the 1-based list position's bits in w) and their count.
   __shared__ float s_alpha[2][PRODUCERS][32][32];
@@ -755,7 +767,7 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
   constexpr uint32_t BLOCK_SHIFT = 3u + TWL + THL, BLOCK_MASK = (1u << BLOCK_SHIFT) - 1u;
   constexpr bool MEMBER = TWL + THL > 0;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  WarpStage& st = stages[warp];
+  BlendStage& st = stages[warp];
   const float vpx = camera->viewport[0], vpy = camera->viewport[1];
   const uint32_t tiles_x = ((uint32_t)vpx + TILE - 1u) / TILE;
   const uint2 tiles16 = make_uint2(tiles_x, ((uint32_t)vpy + TILE - 1u) / TILE);
@@ -803,15 +815,16 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
     const BlendItem it(tile_at(item >> BLOCK_SHIFT), block, lane, tiles_x, tiles_per_view, vpx, vpy, ranges, TWL, THL);
     const TileMember tm{MEMBER, it.tx, it.ty, tiles16};
     const uint2 run = it.run;
-    PixelBlend pb{(float)it.px + 0.5f, (float)it.py + 0.5f, 1.0f, 0.0f, 0.0f, 0.0f, 0u, !it.inside};
+    PixelBlend pb{(float)it.px + 0.5f, (float)it.py + 0.5f, 1.0f, 0.0f, 0.0f, 0.0f, !it.inside};
+    uint32_t last = 0;
     uint32_t next_k = 1;  // the next checkpoint boundary (warp 0)
     const uint32_t pw = warp - 1u;  // producer index (warps >= 1)
     // This producer lane's entry of the window after the one in flight.
-    uint32_t index = 0, next_index = 0;
+    uint32_t next_index = 0;
+    SplatRecord raw;
     if (warp > 0) {
       const uint32_t k = run.x + 32u * pw + lane;
-      if (k < run.y) index = pair_splats[k];
-      stage_issue(st.raw, splats, index, k < run.y);
+      raw.load(splats, k < run.y ? pair_splats[k] : 0u, k < run.y);
       if (k + STRIDE < run.y) next_index = pair_splats[k + STRIDE];
     }
     const uint32_t rounds = (run.y - run.x + STRIDE - 1u) / STRIDE;
@@ -820,11 +833,10 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
       if (warp > 0) {
         const uint32_t start = run.x + r * STRIDE + 32u * pw;
         if (r < rounds && start < run.y) {
-          cp_async_wait_all();
-          const uint32_t staged = stage_commit(st, st.raw, run.x, start, run.y, it.x0, it.y0, cut_in_record, tm);
+          const uint32_t staged = stage_commit(st, raw, run.x, start, run.y, it.x0, it.y0, cut_in_record, tm);
           {
             const uint32_t k = start + STRIDE + lane;
-            stage_issue(st.raw, splats, next_index, k < run.y);
+            raw.load(splats, next_index, k < run.y);
             next_index = k + STRIDE < run.y ? pair_splats[k + STRIDE] : 0u;
           }
           // Pixels warp 0 has stopped take no part (it publishes the mask after
@@ -832,33 +844,31 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
           // keeps an entry that a fresh one would drop).
           uint32_t live = 0, blended = 0;
           for (uint32_t j = 0; j < staged; j += 4) {
-            const uint32_t e[4] = {j, min(j + 1, staged - 1), min(j + 2, staged - 1), min(j + 3, staged - 1)};
             const uint32_t done_mask = *reinterpret_cast<volatile uint32_t*>(&s_done);
             const bool active = it.inside && !((done_mask >> lane) & 1u);
             float alpha[4];
-            if (!pb.alphas4(st, e, staged - j, active, alpha)) continue;
-            // Entry u is queued when some pixel's alpha is nonzero (then u < the
-            // entries left, and e[u] = j + u). Lane u < 4 queues entry u's colour and
+            bool has[4];
+            if (!pb.alphas4(st, j, active, alpha, has)) continue;
+            // Entry u is queued when some pixel's alpha is nonzero (then j + u
+            // is staged). Lane u < 4 queues entry u's colour and
             // position and its blend-mask bit; every lane its alphas.
-            const uint32_t mine = (alpha[0] != 0.0f ? 1u : 0u) | (alpha[1] != 0.0f ? 2u : 0u) |
-                                  (alpha[2] != 0.0f ? 4u : 0u) | (alpha[3] != 0.0f ? 8u : 0u);
+            const uint32_t mine = (has[0] ? 1u : 0u) | (has[1] ? 2u : 0u) | (has[2] ? 4u : 0u) | (has[3] ? 8u : 0u);
             const uint32_t any = __reduce_or_sync(0xffffffffu, mine);
-            uint32_t bit = 0;
             if (lane < 4 && ((any >> lane) & 1u)) {
               const uint32_t slot = live + __popc(any & ((1u << lane) - 1u));
               const float4 c = st.color[j + lane];
               const uint32_t pos = st.pos[j + lane];
               s_qcolor[buf][pw][slot] = make_float4(c.x, c.y, c.z, __uint_as_float(pos + 1));
-              bit = 1u << (pos - (start - run.x));
+              blended |= 1u << (pos - (start - run.x));
             }
-            blended |= __reduce_or_sync(0xffffffffu, bit);
 #pragma unroll
             for (uint32_t u = 0; u < 4; u++)
               if ((any >> u) & 1u) s_alpha[buf][pw][live++][lane] = alpha[u];
           }
+          if (blend_mask) blended = __reduce_or_sync(0xffffffffu, blended);
           if (lane == 0) {
             s_qlive[buf][pw] = live;
-            publish_blended(blend_mask, start, block, blended);
+            if (blend_mask) blend_mask[mask_at(it.tile, tiles, run.x, (start - run.x) / 32u, block)] = blended;
           }
         } else if (lane == 0) {
           s_qlive[buf][pw] = 0;
@@ -877,7 +887,7 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
 #pragma unroll 4
           for (uint32_t m = 0; m < n; m++) {
             const float4 q = s_qcolor[prev][w][m];
-            pb.blend(s_alpha[prev][w][m][lane], q, __float_as_uint(q.w));
+            pb.blend(s_alpha[prev][w][m][lane], q, __float_as_uint(q.w), last);
           }
           const uint32_t done = __ballot_sync(0xffffffffu, pb.done);
           if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&s_done) = done;
@@ -887,11 +897,10 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
       __syncthreads();
       if (s_stop) break;
     }
-    cp_async_wait_all();
     if (warp == 0) {
       save_checkpoints(checkpoints, run.x, next_k, (run.y - run.x + CHUNK - 1) / CHUNK, block, lane, pb.T, pb.r, pb.g,
                        pb.b);
-      write_pixel(it, pb, bg, target, pixel_color, pixel_last);
+      write_pixel(it, pb, last, bg, target, pixel_color, pixel_last);
     }
   }
 
@@ -906,12 +915,14 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
                        ranges, TWL, THL);
     const TileMember tm{MEMBER, it.tx, it.ty, tiles16};
     const uint2 run = it.run;
-    PixelBlend pb{(float)it.px + 0.5f, (float)it.py + 0.5f, 1.0f, 0.0f, 0.0f, 0.0f, 0u, !it.inside};
+    PixelBlend pb{(float)it.px + 0.5f, (float)it.py + 0.5f, 1.0f, 0.0f, 0.0f, 0.0f, !it.inside};
+    uint32_t last = 0;
     uint32_t next_k = 1;
     uint32_t next_index = 0;
+    SplatRecord raw;
     {
       const uint32_t k = run.x + lane;
-      stage_issue(st.raw, splats, k < run.y ? pair_splats[k] : 0u, k < run.y);
+      raw.load(splats, k < run.y ? pair_splats[k] : 0u, k < run.y);
       if (k + 32u < run.y) next_index = pair_splats[k + 32u];
     }
     for (uint32_t start = run.x; start < run.y; start += 32) {
@@ -920,26 +931,38 @@ __global__ void __launch_bounds__(FWD_THREADS) rasterize_kernel(
         save_checkpoints(checkpoints, run.x, next_k, next_k + 1, block, lane, pb.T, pb.r, pb.g, pb.b);
         next_k++;
       }
-      cp_async_wait_all();
-      const uint32_t staged = stage_commit(st, st.raw, run.x, start, run.y, it.x0, it.y0, cut_in_record, tm);
+      const uint32_t staged = stage_commit(st, raw, run.x, start, run.y, it.x0, it.y0, cut_in_record, tm);
       {
         const uint32_t k = start + 32u + lane;
-        stage_issue(st.raw, splats, next_index, k < run.y);
+        raw.load(splats, next_index, k < run.y);
         next_index = k + 32u < run.y ? pair_splats[k + 32u] : 0u;
       }
-      uint32_t blended = 0;
+      // The staged entry this pixel blended last, and (bits) those some pixel did.
+      uint32_t slot = 32u, slots = 0;
       for (uint32_t j = 0; j < staged; j += 4) {
-        if (__all_sync(0xffffffffu, pb.done)) break;
-        const uint32_t e[4] = {j, min(j + 1, staged - 1), min(j + 2, staged - 1), min(j + 3, staged - 1)};
-        pb.apply4(st, e, staged - j, start - run.x, blended);
+        float alpha[4];
+        bool has[4];
+        if (!pb.alphas4(st, j, !pb.done, alpha, has)) continue;
+        const uint32_t mark[4] = {j, j + 1, j + 2, j + 3};
+        bool use[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+          use[u] = __any_sync(0xffffffffu, has[u]);
+          slots |= use[u] ? 1u << mark[u] : 0u;
+        }
+        pb.blend4(alpha, has, use, [&](uint32_t u) { return st.color[mark[u]]; }, mark, slot);
       }
-      if (lane == 0) publish_blended(blend_mask, start, block, blended);
+      if (slot < 32u) last = st.pos[slot] + 1;
+      if (blend_mask) {
+        const uint32_t bit = (slots >> lane) & 1u ? 1u << (st.pos[lane] - (start - run.x)) : 0u;
+        const uint32_t blended = __reduce_or_sync(0xffffffffu, bit);
+        if (lane == 0) blend_mask[mask_at(it.tile, tiles, run.x, (start - run.x) / 32u, block)] = blended;
+      }
       __syncwarp();
     }
-    cp_async_wait_all();  // a window may still be in flight after an early stop
     save_checkpoints(checkpoints, run.x, next_k, (run.y - run.x + CHUNK - 1) / CHUNK, block, lane, pb.T, pb.r, pb.g,
                      pb.b);
-    write_pixel(it, pb, bg, target, pixel_color, pixel_last);
+    write_pixel(it, pb, last, bg, target, pixel_color, pixel_last);
   }
 }
 
@@ -1162,7 +1185,6 @@ dg_status rasterizer_launch(dg_tile_rasterizer* tr, dg_buffer* target, bool coun
 
 dg_status launch_rasterize(dg_tile_rasterizer* tr, dg_buffer* target) {
   dg_context* ctx = tr->ctx;
-  DG_CUDA(cudaMemsetAsync(tr->blend_mask->ptr, 0, tr->blend_mask->bytes, ctx->stream));
   BlendForward f{};
   f.camera = typed<const Camera>(tr->camera);
   f.raster_params = typed<float4>(tr->raster_params);
@@ -1267,7 +1289,7 @@ static dg_status ensure_plan(dg_tile_rasterizer* tr) {
   } needs[] = {{&tr->work_plan, plan_words(tiles) * 4},
                {&tr->chunks, (tiles + slots) * 8},
                {&tr->checkpoints, slots * 8 * 32 * 16},
-               {&tr->blend_mask, ((size_t)tr->pair_capacity / 32 + 2) * 8 * 4}};
+               {&tr->blend_mask, (tiles + (size_t)tr->pair_capacity / 32 + 1) * 8 * 4}};
   for (const Need& n : needs) {
     if (*n.buf && (*n.buf)->bytes >= n.bytes) continue;
     free_buffer(*n.buf);

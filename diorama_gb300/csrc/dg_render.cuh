@@ -59,7 +59,7 @@ struct dg_tile_rasterizer {
   dg_buffer* work_plan;
   dg_buffer* chunks;
   dg_buffer* checkpoints;
-  dg_buffer* blend_mask;  // which entries each 8x4 block blended (dg_render.cu, publish_blended)
+  dg_buffer* blend_mask;  // which entries each 8x4 block blended (dg_render_kernels.cuh, mask_at)
   uint32_t coop_min;      // the fewest entries of a tile that a whole CTA may blend
   bool splat_cutoffs;     // the splats come from this build's preprocess, cutoffs in slot 7
 };

@@ -3,7 +3,7 @@
 //
 // Compiled with the default --fmad=true: gradients only need to agree to rounding
 // (their tile sums meet through float atomics anyway). The arithmetic that decides
-// which splats a pixel blended (blend_power, exp_blend_core, the alpha product and its
+// which splats a pixel blended (blend_power, exp_blend_negated, the alpha product and its
 // thresholds) is written with non-fusing intrinsics or explicit fmaf, so it makes
 // exactly the forward pass's decisions.
 #include "dg_adam.cuh"
@@ -100,7 +100,9 @@ __device__ __forceinline__ void blend_terms(const WarpStage& st, uint32_t e0, ui
   const float power1 = blend_power(q1.x, q1.y, q1.z, t1.dx, t1.dy);
   const bool need0 = eligible0 && power0 >= q0.w && power0 <= 0.0f;
   const bool need1 = eligible1 && power1 >= q1.w && power1 <= 0.0f;
-  exp_blend_core2(need0 ? power0 : 0.0f, need1 ? power1 : 0.0f, t0.G, t1.G);
+  const F2 G = exp_blend_negated(f2(-power0, -power1));  // any value where the power is not needed
+  t0.G = f2_lo(G);
+  t1.G = f2_hi(G);
   t0.alpha = fminf(0.99f, __fmul_rn(m0.z, t0.G));
   t1.alpha = fminf(0.99f, __fmul_rn(m1.z, t1.G));
   t0.blended = need0 && t0.alpha >= 1.0f / 255.0f;
@@ -170,19 +172,20 @@ __device__ __forceinline__ uint32_t window_start(uint32_t end, uint32_t floor) {
   return end - floor > 32u ? end - 32u : floor;
 }
 
-// The blend mask words of `block` covering a chunk's positions [lo, hi) (at most
-// CHUNK / 32 + 1 words): lane l holds word (lo / 32) + l, or 0 past them.
-__device__ __forceinline__ uint32_t chunk_mask_words(const uint32_t* __restrict__ mask, uint32_t lo, uint32_t hi,
-                                                     uint32_t block, uint32_t lane) {
-  static_assert(CHUNK / 32 + 1 <= 32, "a chunk's mask words fit in the warp's lanes");
-  const uint32_t w = (lo >> 5) + lane;
-  return w <= ((hi - 1u) >> 5) ? mask[(size_t)w * 8u + block] : 0u;
+// The blend mask words of `block` for a tile's windows [first, end) (at most CHUNK / 32):
+// lane l holds window first + l's, or 0 past them.
+__device__ __forceinline__ uint32_t chunk_mask_words(const uint32_t* __restrict__ mask, uint32_t tile, uint32_t tiles,
+                                                     uint32_t run_x, uint32_t first, uint32_t end, uint32_t block,
+                                                     uint32_t lane) {
+  static_assert(CHUNK / 32 <= 32, "a chunk's mask words fit in the warp's lanes");
+  const uint32_t k = first + lane;
+  return k < end ? mask[mask_at(tile, tiles, run_x, k, block)] : 0u;
 }
 
 // The blend mask bits of window [lo, hi) (none when it is empty) from the chunk's
 // words in the lanes (chunk_mask_words from position base). All lanes must call it.
 __device__ __forceinline__ uint32_t window_blended(uint32_t words, uint32_t base, uint32_t lo, uint32_t hi) {
-  const uint32_t at = (lo >> 5) - (base >> 5), shift = lo & 31u;
+  const uint32_t at = (lo - base) >> 5, shift = (lo - base) & 31u;
   const uint32_t a = __shfl_sync(0xffffffffu, words, at & 31u), b = __shfl_sync(0xffffffffu, words, (at + 1u) & 31u);
   if (hi <= lo) return 0u;
   const uint32_t bits = shift ? (a >> shift) | (b << (32u - shift)) : a;
@@ -264,7 +267,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 6) rasterize_backward_kernel(
     // Windows run back to front: [lo, end) with lo = max(chunk_lo, end - 32). Only
     // the entries some pixel of the block blended (the forward pass's mask) are
     // staged. This lane's entry of the window in flight and of the next one.
-    const uint32_t words = chunk_mask_words(blend_mask, chunk_lo, end_all, block, lane);
+    const uint32_t words = chunk_mask_words(blend_mask, tile, plan[PLAN_TILES], run.x, chunk.y * (CHUNK / 32u),
+                                            (end_all - run.x + 31u) / 32u, block, lane);
     uint32_t end = end_all;
     uint32_t lo = window_start(end, chunk_lo);
     uint32_t bits = window_blended(words, chunk_lo, lo, end);

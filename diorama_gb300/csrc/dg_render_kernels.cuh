@@ -223,36 +223,41 @@ __device__ __forceinline__ float blend_cutoff(float opacity) {
 }
 
 // Whether a splat can reach any pixel center of the rectangle
-// [dxl, dxh] x [dyl, dyh] (offsets pixel - mean): the maximum of the concave
-// quadratic q = A dx^2 - b dx dy + C dy^2 over the rectangle, compared with the
-// cutoff. The maximum is at the mean if the rectangle holds it, else on an edge,
-// where each 1D maximum is clamped to the edge. The margin covers the rounding
-// of both this maximum and the per-pixel power (a few ulps of the terms' sizes),
-// so a splat this rejects would have been skipped at every pixel anyway. The
-// quadratics are fused multiply-adds (one rounding each, inside that margin).
-__device__ __forceinline__ bool rect_reachable(float A, float b, float C, float kx, float ky, float cut, float dxl,
-                                               float dxh, float dyl, float dyh) {
-  if (dxl <= 0.0f && dxh >= 0.0f && dyl <= 0.0f && dyh >= 0.0f) return 0.0f >= cut;
+// [dxl, dxh] x [dyl, dyh] (offsets pixel - mean): whether the quadratic form
+// q = A dx^2 - b dx dy + C dy^2 comes up to the cutoff (below 0) on the edges that
+// face the mean, or on the axis through the mean where the rectangle straddles it.
+// They are enough: on the way from a pixel with q in [cutoff, 0] straight to the
+// mean, q shrinks towards 0 (by the square of the distance), and the way leaves the
+// rectangle through one of them or ends in it. On a line the maximum is at the
+// vertex, clamped to the rectangle; where the form opens upwards along an axis
+// (never for a splat of this renderer) the splat is kept. The margin covers the
+// rounding of both this maximum and the per-pixel power (a few ulps of the terms'
+// sizes), so a splat this rejects would have been skipped at every pixel anyway.
+// The quadratics are fused multiply-adds (one rounding each, inside that margin).
+// All four edges keep the same splats for twice the work.
+__device__ __forceinline__ bool rect_reachable(float A, float b, float C, float cut, float dxl, float dxh, float dyl,
+                                               float dyh) {
+  if (!(A < 0.0f && C < 0.0f)) return true;
   // (A dx - b dy) dx + C dy dy
   auto q = [&](float dx, float dy) {
     return __fmaf_rn(__fmaf_rn(A, dx, -__fmul_rn(b, dy)), dx, __fmul_rn(__fmul_rn(C, dy), dy));
   };
-  const float y1 = fminf(fmaxf(ky * dxl, dyl), dyh), y2 = fminf(fmaxf(ky * dxh, dyl), dyh);
-  const float x1 = fminf(fmaxf(kx * dyl, dxl), dxh), x2 = fminf(fmaxf(kx * dyh, dxl), dxh);
-  const float qmax = fmaxf(fmaxf(q(dxl, y1), q(dxh, y2)), fmaxf(q(x1, dyl), q(x2, dyh)));
+  const float xe = fminf(fmaxf(dxl, 0.0f), dxh), ye = fminf(fmaxf(dyl, 0.0f), dyh);  // the nearest to the mean
+  const float y1 = fminf(fmaxf(__fdividef(b, 2.0f * C) * xe, dyl), dyh);
+  const float x1 = fminf(fmaxf(__fdividef(b, 2.0f * A) * ye, dxl), dxh);
+  const float qmax = fmaxf(q(xe, y1), q(x1, ye));
   const float mx = fmaxf(fabsf(dxl), fabsf(dxh)), my = fmaxf(fabsf(dyl), fabsf(dyh));
   const float terms = __fmaf_rn(__fmaf_rn(fabsf(A), mx, fabsf(b) * my), mx, fabsf(C) * my * my);
   return __fmaf_rn(1e-6f, terms, qmax) + 1e-6f >= cut;
 }
 
 // CTA sizes of the blend kernels. The forward's 4 warps blend a block of a long
-// tile list together (3 computing alphas, 1 blending; 96 and 160 threads measured
-// slower: 331 and 363 us against 323 at 1.1M Gaussians); otherwise every warp
-// takes items of its own.
+// tile list together (3 computing alphas, 1 blending; more threads and fewer CTAs are
+// slower, see rasterize_kernel); otherwise every warp takes items of its own.
 #ifndef DG_FWD_THREADS
 #define DG_FWD_THREADS 128
 #endif
-constexpr uint32_t FWD_THREADS = DG_FWD_THREADS;  // 96 or 128 (measured 324 and 288 us at 1.1M)
+constexpr uint32_t FWD_THREADS = DG_FWD_THREADS;
 constexpr uint32_t FWD_WARPS = FWD_THREADS / 32;
 constexpr uint32_t PRODUCERS = FWD_WARPS - 1;  // cooperative blending: warps computing alphas for warp 0
 constexpr uint32_t BWD_THREADS = 128;
@@ -286,6 +291,22 @@ using RawWindow = float4[32][3];
 // memory: only the splats that can reach the warp's 8x4 pixel block, in list
 // order. `raw` receives the splat records of the next window by cp.async while
 // the current one blends.
+//
+// The forward pass's stage. Two entries share a BlendPair, each field's two values
+// side by side as packed instructions take them.
+struct BlendPair {
+  ulonglong2 n;   // -mean x, -mean y
+  ulonglong2 ab;  // 0.5 a, b
+  ulonglong2 cl;  // 0.5 c, and the bits that those of -power must be below for the
+                  // alpha to reach 1/255 (those of -cutoff, plus 1)
+  unsigned long long opacity, pad;
+};
+struct BlendStage {
+  BlendPair pair[16];
+  float4 color[32];  // rgb, opacity
+  uint32_t pos[32];  // position in the tile's list
+};
+// The backward pass's.
 struct WarpStage {
   float4 mean[32];   // mean x, y, opacity, 0
   float4 quad[32];   // A = -0.5 a, b, C = -0.5 c, cutoff
@@ -303,6 +324,17 @@ struct WarpStage {
 __device__ __forceinline__ size_t checkpoint_at(uint32_t run_x, uint32_t k, uint32_t block, uint32_t lane) {
   const size_t slot = (run_x + k * CHUNK) / CHUNK;
   return (slot * 8u + block) * 32u + lane;
+}
+
+// The blend mask: bit l of a word is set when some pixel of 8x4 block `block` of the
+// tile blended entry 32 k + l of the tile's list. The forward pass writes the word of
+// each window it walks, the backward pass reads those up to the last entry blended.
+// Window 0 of a tile has the tile's own place; the others follow by their position in
+// the pair list, 32 entries at least after the one before (so nothing is cleared, and
+// no two tiles share a word: with positions counted over all tiles, the clear and the
+// atomics they shared took 10 us of a frame of 29M pairs).
+__device__ __forceinline__ size_t mask_at(uint32_t tile, uint32_t tiles, uint32_t run_x, uint32_t k, uint32_t block) {
+  return (size_t)(k == 0 ? tile : tiles + (run_x + k * 32u) / 32u) * 8u + block;
 }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -389,31 +421,43 @@ struct TileMember {
   uint2 tiles;
 };
 
-// Takes the window [lo, min(lo + 32, hi)) whose records stage_issue has brought into
-// `raw` (lane l: entry lo + l; the caller has waited for the copies) and keeps, in
+// The record of this lane's entry of the forward pass's next window, in registers: on
+// its way while the window before is blended.
+struct SplatRecord {
+  float4 s0, s1, s2;
+  __device__ __forceinline__ void load(const float* __restrict__ splats, uint32_t index, bool valid) {
+    if (!valid) return;
+    const float4* s = reinterpret_cast<const float4*>(splats + (size_t)index * FLOATS_PER_SPLAT);
+    s0 = s[0];
+    s1 = s[1];
+    s2 = s[2];
+  }
+};
+
+// Takes the window [lo, min(lo + 32, hi)) whose records are in `raw` and keeps, in
 // list order, the splats that can reach the warp's block, whose pixel centers span [x0, x0 + 7] x [y0, y0 + 3] (and,
 // with a TileMember, belong to its 16x16 tile's list). Returns how many were
 // kept. All 32 lanes must call it. Every value read from `raw` is consumed before
 // this returns, so the caller may issue the next window at once. cut_in_record:
 // the splats carry their blend cutoff in slot SPLAT_CUTOFF_SLOT (this build's
 // preprocess wrote them), else it is computed here.
-__device__ __forceinline__ uint32_t stage_commit(WarpStage& st, const RawWindow& raw, uint32_t run_x, uint32_t lo,
+__device__ __forceinline__ uint32_t stage_commit(BlendStage& st, const SplatRecord& raw, uint32_t run_x, uint32_t lo,
                                                  uint32_t hi, float x0, float y0, bool cut_in_record,
                                                  const TileMember& tm = TileMember{false, 0u, 0u, {0u, 0u}}) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t k = lo + lane;
   bool keep = false;
-  float2 mean = make_float2(0.f, 0.f);
-  float4 quad = make_float4(0.f, 0.f, 0.f, 0.f), color = quad;
+  float2 mean = make_float2(0.f, 0.f), ab = mean, cl = mean;
+  float4 color = make_float4(0.f, 0.f, 0.f, 0.f);
   if (k < hi) {
-    const float4 s0 = raw[lane][0], s1 = raw[lane][1];
-    color = raw[lane][2];
+    const float4 s0 = raw.s0, s1 = raw.s1;
+    color = raw.s2;
     mean = make_float2(s0.x, s0.y);
     const float A = -0.5f * s1.x, b = s1.y, C = -0.5f * s1.z;
     const float cut = cut_in_record ? s1.w : blend_cutoff(color.w);
-    quad = make_float4(A, b, C, cut);
-    keep = cut < 0.0f && rect_reachable(A, b, C, __fdividef(b, 2.0f * A), __fdividef(b, 2.0f * C), cut,
-                                        x0 - mean.x, x0 + 7.0f - mean.x, y0 - mean.y, y0 + 3.0f - mean.y);
+    ab = make_float2(-A, b);
+    cl = make_float2(-C, cut);
+    keep = cut < 0.0f && rect_reachable(A, b, C, cut, x0 - mean.x, x0 + 7.0f - mean.x, y0 - mean.y, y0 + 3.0f - mean.y);
     if (tm.member && keep) {
       const uint4 rect = tile_rect(mean.x, mean.y, s0.w, tm.tiles);
       keep = tm.tx >= rect.x && tm.tx < rect.z && tm.ty >= rect.y && tm.ty < rect.w;
@@ -422,13 +466,22 @@ __device__ __forceinline__ uint32_t stage_commit(WarpStage& st, const RawWindow&
   const uint32_t kept = __ballot_sync(0xffffffffu, keep);
   if (keep) {
     const uint32_t at = __popc(kept & ((1u << lane) - 1u));
-    st.mean[at] = make_float4(mean.x, mean.y, color.w, 0.0f);
-    st.quad[at] = quad;
+    float* e = reinterpret_cast<float*>(&st.pair[at / 2]) + (at & 1u);
+    e[0] = -mean.x;
+    e[2] = -mean.y;
+    e[4] = ab.x;
+    e[6] = ab.y;
+    e[8] = cl.x;
+    e[10] = __uint_as_float(__float_as_uint(-cl.y) + 1u);
+    e[12] = color.w;
     st.color[at] = color;
     st.pos[at] = k - run_x;
   }
+  // Entries past the last are taken in groups of 4 with it: nothing is below theirs.
+  const uint32_t staged = __popc(kept), past = staged + lane;
+  if (lane < 3u && past < 32u) reinterpret_cast<uint32_t*>(&st.pair[past / 2].cl.y)[past & 1u] = 0u;
   __syncwarp();
-  return __popc(kept);
+  return staged;
 }
 
 
