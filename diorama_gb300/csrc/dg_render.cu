@@ -473,18 +473,16 @@ __device__ __forceinline__ unsigned char to_unorm8(float v) {
 // over the tiles that list it, and the tile is taken to be opaque where those
 // shares reach an optical depth of PLAN_DEPTH. The forward pass takes the tiles with
 // the most work first, by powers of two (half the list's length at least: a block of
-// the tile that little covers walks on); the backward pass (when chunks is given)
-// the (tile, chunk) pairs of tiles with several chunks first. Order within a group
-// follows atomics, and none of it changes a result. A warp estimates a tile; a CTA
-// places 32 of them together, one atomic per group.
+// the tile that little covers walks on). Order within a group follows atomics, and
+// none of it changes a result. A warp estimates a tile; a CTA places 32 of them
+// together, one atomic per group.
 constexpr uint32_t PLAN_THREADS = 256, PLAN_CTA_TILES = 32, PLAN_SAMPLES = 32;
 constexpr float PLAN_DEPTH = 16.0f;
 
 __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(const uint2* __restrict__ ranges, uint32_t tiles,
                                                             const uint32_t* __restrict__ pair_splats,
                                                             const float* __restrict__ splats,
-                                                            uint32_t* __restrict__ plan, uint2* __restrict__ chunks,
-                                                            uint32_t chunk_room) {
+                                                            uint32_t* __restrict__ plan) {
   __shared__ uint32_t s_work[PLAN_CTA_TILES], s_len[PLAN_CTA_TILES], s_rank[PLAN_CTA_TILES];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   for (uint32_t k = warp; k < PLAN_CTA_TILES; k += PLAN_THREADS / 32) {
@@ -531,38 +529,8 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(const uint2* __restr
       atomicAdd(&plan[PLAN_TOTAL], total);
       atomicMax(&plan[PLAN_LONGEST], longest);
     }
-    if (blockIdx.x == 0) {
-      plan[PLAN_TILES] = tiles;
-      plan[PLAN_CHUNKS] = chunk_room;
-    }
+    if (blockIdx.x == 0) plan[PLAN_TILES] = tiles;
   }
-  if (!chunks) return;
-  const uint32_t nb = (len + CHUNK - 1) / CHUNK;
-  uint32_t multi = nb > 1 ? nb : 0u;
-#pragma unroll
-  for (uint32_t d = 1; d < 32; d <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, multi, d);
-    if (lane >= d) multi += v;
-  }
-  const uint32_t single = __ballot_sync(0xffffffffu, nb == 1);
-  uint32_t multi_at = 0, single_at = 0;
-  if (lane == 31 && multi) multi_at = atomicAdd(&plan[PLAN_MULTI], multi);
-  if (lane == 31 && single) single_at = atomicAdd(&plan[PLAN_SINGLE], __popc(single));
-  multi_at = __shfl_sync(0xffffffffu, multi_at, 31) + multi - (nb > 1 ? nb : 0u);
-  single_at = __shfl_sync(0xffffffffu, single_at, 31) + __popc(single & below);
-  if (nb > 1) {
-    for (uint32_t k = 0; k < nb; k++) chunks[multi_at + k] = make_uint2(t, k);
-  } else if (nb == 1) {
-    chunks[chunk_room - 1 - single_at] = make_uint2(t, 0u);
-  }
-}
-
-// Writes the checkpoints of boundaries [k_from, k_to) of a tile with one pixel state.
-__device__ __forceinline__ void save_checkpoints(float4* __restrict__ checkpoints, uint32_t run_x, uint32_t k_from,
-                                                 uint32_t k_to, uint32_t block, uint32_t lane, float T, float r,
-                                                 float g, float b) {
-  if (!checkpoints) return;
-  for (uint32_t k = k_from; k < k_to; k++) checkpoints[checkpoint_at(run_x, k, block, lane)] = make_float4(T, r, g, b);
 }
 
 // One pixel's front-to-back blend (src/shaders/rasterize.wgsl:62-92), the lane's
@@ -575,21 +543,15 @@ struct PixelBlend {
   // The alphas of staged entries j..j + 3 of `st` at this pixel, and whether it blends
   // them; an alpha is 0 where it does not (alpha under 1/255; a power under the splat's
   // cutoff skips the exp with the same outcome). Two entries run as the lanes of packed
-  // instructions, on the negated power: each the scalar form's bits (blend_power,
-  // exp_blend_core). Returns false when no lane reaches any of the 4 cutoffs.
+  // instructions (blend_power_negated, exp_blend_negated). Returns false when no lane reaches any of the 4 cutoffs.
   __device__ __forceinline__ bool alphas4(const BlendStage& st, uint32_t j, bool active, float (&alpha)[4],
                                           bool (&has)[4]) const {
     const F2 px = f2(cx, cx), py = f2(cy, cy);
     F2 q[2];
 #pragma unroll
     for (uint32_t h = 0; h < 2; h++) {
-      const BlendPair& e = st.pair[j / 2 + h];
-      const ulonglong2 n = e.n, ab = e.ab, cl = e.cl;
-      const F2 dx = f2_add(px, F2{n.x}), dy = f2_add(py, F2{n.y});
-      const F2 s = f2_fma(F2{ab.x}, dx, f2_mul(F2{ab.y}, dy));
-      // + 0 makes a zero's sign positive: bits compare like values from 0 up.
-      q[h] = f2_add(f2_fma(s, dx, f2_mul(f2_mul(F2{cl.x}, dy), dy)), f2(0.0f, 0.0f));
-      const F2 limit{cl.y};
+      F2 limit;
+      q[h] = blend_power_negated(st.pair[j / 2 + h], px, py, limit);
       has[2 * h] = active && __float_as_uint(f2_lo(q[h])) < __float_as_uint(f2_lo(limit));
       has[2 * h + 1] = active && __float_as_uint(f2_hi(q[h])) < __float_as_uint(f2_hi(limit));
     }
@@ -659,6 +621,13 @@ struct PixelBlend {
   }
 };
 
+// Writes the checkpoint of chunk boundary k. Boundaries that the walk does not reach
+// have none: no pixel blends a splat behind them.
+__device__ __forceinline__ void save_checkpoint(float4* __restrict__ checkpoints, uint32_t run_x, uint32_t k,
+                                                uint32_t block, uint32_t lane, const PixelBlend& pb) {
+  if (checkpoints) checkpoints[checkpoint_at(run_x, k, block, lane)] = make_float4(pb.T, pb.r, pb.g, pb.b);
+}
+
 // The geometry of a blend item: tile `tile` (of the view tile / tiles_per_view
 // when several views are blended together), 8x4 block `block`, this lane's pixel.
 // A blend tile of 2^twl x 2^thl 16x16 tiles has 8 blocks per 16x16 tile, those
@@ -699,6 +668,25 @@ __device__ __forceinline__ void write_pixel(const BlendItem& it, const PixelBlen
   pixel_color[it.pixel] = make_float4(fr, fg, fb, pb.T);
   pixel_last[it.pixel] = last;
   if (target) target[it.pixel] = make_uchar4(to_unorm8(fr), to_unorm8(fg), to_unorm8(fb), 255);
+}
+
+// The backward pass's items of a block whose pixels have ended: the chunks of its list
+// up to the last entry that one of them blended.
+__device__ __forceinline__ void list_items(uint2* __restrict__ items, uint32_t* __restrict__ item_count,
+                                           uint32_t item_room, uint32_t tile, uint32_t block, uint32_t lane,
+                                           uint32_t last) {
+  if (!items) return;
+  const uint32_t most = __reduce_max_sync(0xffffffffu, last);
+  // Whole chunks are in the first class, the rest of the list in its own.
+  const uint32_t whole = most / CHUNK, rest = most % CHUNK;
+  uint32_t at = 0;
+  if (lane == 0 && whole) at = atomicAdd(item_count, whole);
+  if (lane == 1 && rest) at = atomicAdd(item_count + item_class(rest), 1u);
+  if (lane == 1 && rest && at < item_room)
+    items[(size_t)item_class(rest) * item_room + at] = make_uint2(tile * 8u + block, whole);
+  at = __shfl_sync(0xffffffffu, at, 0);
+  for (uint32_t k = lane; k < whole; k += 32u)
+    if (at + k < item_room) items[at + k] = make_uint2(tile * 8u + block, k);
 }
 
 // src/shaders/rasterize.wgsl:32-100. The work is split into items, one per (tile,
@@ -756,7 +744,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
     const uint32_t* __restrict__ pair_splats, const uint2* __restrict__ ranges, const uint32_t* __restrict__ plan,
     uint32_t tiles_per_view, uint32_t coop_min, uchar4* __restrict__ target, float4* __restrict__ pixel_color,
     uint32_t* __restrict__ pixel_last, float4* __restrict__ checkpoints, uint32_t* __restrict__ blend_mask,
-    uint32_t* __restrict__ counters, bool cut_in_record) {
+    uint2* __restrict__ items, uint32_t* __restrict__ item_count, uint32_t item_room, uint32_t* __restrict__ counters,
+    bool cut_in_record) {
   __shared__ BlendStage stages[FWD_WARPS];
   // Cooperative blending, double-buffered by round: each producer's queued entries
   // (alpha per pixel; colour with the 1-based list position's bits in w) and their count.
@@ -880,7 +869,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
           const uint32_t ws = run.x + (r - 1u) * STRIDE + 32u * w;
           if (ws >= run.y) break;
           if (ws - run.x == next_k * CHUNK) {
-            save_checkpoints(checkpoints, run.x, next_k, next_k + 1, block, lane, pb.T, pb.r, pb.g, pb.b);
+            save_checkpoint(checkpoints, run.x, next_k, block, lane, pb);
             next_k++;
           }
           const uint32_t n = s_qlive[prev][w];
@@ -898,9 +887,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
       if (s_stop) break;
     }
     if (warp == 0) {
-      save_checkpoints(checkpoints, run.x, next_k, (run.y - run.x + CHUNK - 1) / CHUNK, block, lane, pb.T, pb.r, pb.g,
-                       pb.b);
       write_pixel(it, pb, last, bg, target, pixel_color, pixel_last);
+      list_items(items, item_count, item_room, it.tile, block, lane, last);
     }
   }
 
@@ -928,7 +916,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
     for (uint32_t start = run.x; start < run.y; start += 32) {
       if (__all_sync(0xffffffffu, pb.done)) break;
       if (start - run.x == next_k * CHUNK) {
-        save_checkpoints(checkpoints, run.x, next_k, next_k + 1, block, lane, pb.T, pb.r, pb.g, pb.b);
+        save_checkpoint(checkpoints, run.x, next_k, block, lane, pb);
         next_k++;
       }
       const uint32_t staged = stage_commit(st, raw, run.x, start, run.y, it.x0, it.y0, cut_in_record, tm);
@@ -960,9 +948,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
       }
       __syncwarp();
     }
-    save_checkpoints(checkpoints, run.x, next_k, (run.y - run.x + CHUNK - 1) / CHUNK, block, lane, pb.T, pb.r, pb.g,
-                     pb.b);
     write_pixel(it, pb, last, bg, target, pixel_color, pixel_last);
+    list_items(items, item_count, item_room, it.tile, block, lane, last);
   }
 }
 
@@ -1194,8 +1181,8 @@ dg_status launch_rasterize(dg_tile_rasterizer* tr, dg_buffer* target) {
   f.tiles = f.tiles_per_view = tr->tiles_x * tr->tiles_y;
   f.coop_min = tr->coop_min;
   f.plan = typed<uint32_t>(tr->work_plan);
-  f.chunks = typed<uint2>(tr->chunks);
-  f.chunk_room = (uint32_t)(tr->chunks->bytes / sizeof(uint2));
+  f.items = typed<uint2>(tr->items);
+  f.item_room = (uint32_t)(tr->items->bytes / sizeof(uint2) / ITEM_CLASSES);
   f.target = target ? typed<uchar4>(target) : nullptr;
   f.pixel_color = typed<float4>(tr->pixel_color);
   f.pixel_last = typed<uint32_t>(tr->pixel_last);
@@ -1214,14 +1201,15 @@ static dg_status launch_rasterize_kernel(dg_context* ctx, const BlendForward& f)
   DG_LAUNCH(ctx, "rasterize",
             kernel<<<blend_grid(ctx, (const void*)kernel, FWD_THREADS, items), FWD_THREADS, 0, ctx->stream>>>(
                 f.camera, f.raster_params, f.splats, f.pair_splats, f.ranges, f.plan, f.tiles_per_view, f.coop_min, f.target,
-                f.pixel_color, f.pixel_last, f.checkpoints, f.blend_mask, f.counters, f.splat_cutoffs));
+                f.pixel_color, f.pixel_last, f.checkpoints, f.blend_mask, f.items, f.plan + PLAN_ITEMS, f.item_room,
+                f.counters, f.splat_cutoffs));
   return DG_OK;
 }
 
 dg_status blend_forward(dg_context* ctx, const BlendForward& f) {
   const BlendShape sh = f.shape;
   DG_REQUIRE(sh.twl <= MAX_BLEND_TILE_LOG2 && sh.thl <= MAX_BLEND_TILE_LOG2, "blend tiles of at most 2 x 2 tiles");
-  DG_REQUIRE(sh.twl + sh.thl == 0 || (!f.checkpoints && !f.blend_mask && !f.chunks),
+  DG_REQUIRE(sh.twl + sh.thl == 0 || (!f.checkpoints && !f.blend_mask && !f.items),
              "blend tiles larger than 16x16 have no backward pass");
   if (!f.cleared) {
     DG_CUDA(cudaMemsetAsync(f.counters, 0, 16, ctx->stream));
@@ -1229,7 +1217,7 @@ dg_status blend_forward(dg_context* ctx, const BlendForward& f) {
   }
   DG_LAUNCH(ctx, "plan",
             plan_kernel<<<std::max(1u, ceil_div(f.tiles, PLAN_CTA_TILES)), PLAN_THREADS, 0, ctx->stream>>>(
-                f.ranges, f.tiles, f.pair_splats, f.splats, f.plan, f.chunks, f.chunk_room));
+                f.ranges, f.tiles, f.pair_splats, f.splats, f.plan));
   if (sh.twl == 0 && sh.thl == 0) return launch_rasterize_kernel<0, 0>(ctx, f);
   if (sh.twl == 1 && sh.thl == 0) return launch_rasterize_kernel<1, 0>(ctx, f);
   if (sh.twl == 0 && sh.thl == 1) return launch_rasterize_kernel<0, 1>(ctx, f);
@@ -1287,7 +1275,7 @@ static dg_status ensure_plan(dg_tile_rasterizer* tr) {
     dg_buffer** buf;
     size_t bytes;
   } needs[] = {{&tr->work_plan, plan_words(tiles) * 4},
-               {&tr->chunks, (tiles + slots) * 8},
+               {&tr->items, (tiles + slots) * 8 * ITEM_CLASSES * sizeof(uint2)},
                {&tr->checkpoints, slots * 8 * 32 * 16},
                {&tr->blend_mask, (tiles + (size_t)tr->pair_capacity / 32 + 1) * 8 * 4}};
   for (const Need& n : needs) {
@@ -1499,7 +1487,7 @@ dg_status dg_tile_rasterizer_destroy(dg_tile_rasterizer* tr) {
   for (dg_buffer* b : {tr->tile_offsets, tr->scan_total, tr->scan_scratch, tr->raster_params, tr->keys, tr->values,
                        tr->keys_alt, tr->values_alt, tr->sort_scratch, tr->ranges, tr->pixel_color, tr->pixel_last,
                        tr->depth_keys, tr->depth_values, tr->depth_keys_alt, tr->depth_values_alt, tr->depth_scratch,
-                       tr->counts_sorted, tr->bin_scratch, tr->keys64, tr->work, tr->work_plan, tr->chunks, tr->checkpoints,
+                       tr->counts_sorted, tr->bin_scratch, tr->keys64, tr->work, tr->work_plan, tr->items, tr->checkpoints,
                        tr->blend_mask})
     free_buffer(b);
   for (cudaEvent_t e : tr->readback_events)

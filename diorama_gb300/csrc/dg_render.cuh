@@ -54,12 +54,10 @@ struct dg_tile_rasterizer {
   dg_buffer* counts_sorted;  // tile counts in depth order, then their scan
   dg_buffer* keys64;         // the reference's 64-bit sorted keys, rebuilt on request
   dg_buffer* work;           // item counters of the blend kernels
-  // The blend kernels' work plan (plan_kernel, dg_render.cu): tile order, the
-  // backward's (tile, chunk) pairs and the forward's per-chunk pixel states.
-  dg_buffer* work_plan;
-  dg_buffer* chunks;
-  dg_buffer* checkpoints;
-  dg_buffer* blend_mask;  // which entries each 8x4 block blended (dg_render_kernels.cuh, mask_at)
+  dg_buffer* work_plan;    // tile order and counts (plan_kernel, dg_render.cu)
+  dg_buffer* items;        // the backward pass's (tile, block) and chunk, listed by the forward pass
+  dg_buffer* checkpoints;  // the forward's per-chunk pixel states
+  dg_buffer* blend_mask;   // which entries each 8x4 block blended (dg_render_kernels.cuh, mask_at)
   uint32_t coop_min;      // the fewest entries of a tile that a whole CTA may blend
   bool splat_cutoffs;     // the splats come from this build's preprocess, cutoffs in slot 7
 };
@@ -94,7 +92,7 @@ struct BlendShape {
 constexpr uint32_t MAX_BLEND_TILE_LOG2 = 1;  // blend tiles of up to 2 x 2 16x16 tiles
 
 // The forward blend (plan + rasterize kernels) over `tiles` tiles of
-// tiles_per_view each; checkpoints, blend_mask and chunks may be NULL when no
+// tiles_per_view each; checkpoints, blend_mask and items may be NULL when no
 // backward pass follows, and must be with blend tiles larger than 16x16.
 struct BlendForward {
   const Camera* camera;
@@ -104,8 +102,8 @@ struct BlendForward {
   const uint2* ranges;
   uint32_t tiles, tiles_per_view, coop_min;
   uint32_t* plan;
-  uint2* chunks;
-  uint32_t chunk_room;  // (tile, chunk) pairs that chunks holds
+  uint2* items;
+  uint32_t item_room;  // that items holds
   uchar4* target;
   float4* pixel_color;
   uint32_t* pixel_last;

@@ -3,7 +3,7 @@
 //
 // Compiled with the default --fmad=true: gradients only need to agree to rounding
 // (their tile sums meet through float atomics anyway). The arithmetic that decides
-// which splats a pixel blended (blend_power, exp_blend_negated, the alpha product and its
+// which splats a pixel blended (blend_power_negated, exp_blend_negated, the alpha product and its
 // thresholds) is written with non-fusing intrinsics or explicit fmaf, so it makes
 // exactly the forward pass's decisions.
 #include "dg_adam.cuh"
@@ -17,96 +17,6 @@ __device__ __forceinline__ void load_camera(Camera& dst, const Camera* src) {
   const float* s = reinterpret_cast<const float*>(src);
   float* d = reinterpret_cast<float*>(&dst);
   for (int k = threadIdx.x; k < 36; k += blockDim.x) d[k] = s[k];
-}
-
-// One halving step of a reduce-scatter over the warp: a lane holding M partial
-// sums keeps the lower or the upper half of them (by bit D of its lane index) and
-// adds its partner's copy of that half. With M == 1 both lanes keep the sum.
-template <int M, int D>
-__device__ __forceinline__ void reduce_half(float* v, uint32_t lane) {
-  if constexpr (M == 1) {
-    v[0] = v[0] + __shfl_xor_sync(0xffffffffu, v[0], D);
-  } else {
-    constexpr int H = (M + 1) / 2;
-    const bool upper = lane & D;
-#pragma unroll
-    for (int k = 0; k < H; k++) {
-      const float lo = v[k], hi = H + k < M ? v[H + k] : 0.0f;
-      const float got = __shfl_xor_sync(0xffffffffu, upper ? lo : hi, D);
-      v[k] = (upper ? hi : lo) + got;
-    }
-  }
-}
-
-// Sums N <= 32 values over the warp's 32 lanes with about N shuffles (N = 18:
-// 20 shuffles in 5 dependent steps, against 5 N in 5 N steps for N separate
-// butterflies). Afterwards lane l holds the total of value reduce_slot<N>(l), or
-// a copy or padding where that is -1. Clobbers v.
-template <int N>
-__device__ __forceinline__ float warp_reduce_scatter(float (&v)[N], uint32_t lane) {
-  static_assert(N <= 32, "one value per lane at most");
-  constexpr int M2 = (N + 1) / 2, M3 = (M2 + 1) / 2, M4 = (M3 + 1) / 2, M5 = (M4 + 1) / 2;
-  static_assert(M5 == 1 || (M5 == 2 && N > 16), "the last step leaves one value per lane");
-  reduce_half<N, 16>(v, lane);
-  reduce_half<M2, 8>(v, lane);
-  reduce_half<M3, 4>(v, lane);
-  reduce_half<M4, 2>(v, lane);
-  reduce_half<M5, 1>(v, lane);
-  return v[0];
-}
-
-// Which of the N values lane `lane` holds after warp_reduce_scatter<N>: the index
-// ranges each step keeps, followed for this lane's bits; -1 for padding or for the
-// upper lane of a pair that holds the same sum.
-template <int N>
-__device__ __forceinline__ int reduce_slot(uint32_t lane) {
-  int base = 0, real = N, m = N;
-#pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) {
-    if (m == 1) {
-      if (lane & d) real = 0;
-      continue;
-    }
-    const int h = (m + 1) / 2;
-    if (lane & d) {
-      base += h;
-      real = real > h ? real - h : 0;
-    } else {
-      real = real < h ? real : h;
-    }
-    m = h;
-  }
-  return real > 0 ? base : -1;
-}
-
-// The exponent, Gaussian and alpha of a splat at this lane's pixel, and whether
-// the forward pass blended it there (the same decisions, made with the same
-// non-fusing arithmetic).
-struct BlendTerm {
-  float dx, dy, G, alpha;
-  bool blended;
-};
-
-// The terms of two entries at once (their exps as one packed pair).
-__device__ __forceinline__ void blend_terms(const WarpStage& st, uint32_t e0, uint32_t e1, bool eligible0,
-                                            bool eligible1, float cx, float cy, BlendTerm& t0, BlendTerm& t1) {
-  const float4 m0 = st.mean[e0], m1 = st.mean[e1];  // .z: opacity
-  const float4 q0 = st.quad[e0], q1 = st.quad[e1];
-  t0.dx = cx - m0.x;
-  t0.dy = cy - m0.y;
-  t1.dx = cx - m1.x;
-  t1.dy = cy - m1.y;
-  const float power0 = blend_power(q0.x, q0.y, q0.z, t0.dx, t0.dy);
-  const float power1 = blend_power(q1.x, q1.y, q1.z, t1.dx, t1.dy);
-  const bool need0 = eligible0 && power0 >= q0.w && power0 <= 0.0f;
-  const bool need1 = eligible1 && power1 >= q1.w && power1 <= 0.0f;
-  const F2 G = exp_blend_negated(f2(-power0, -power1));  // any value where the power is not needed
-  t0.G = f2_lo(G);
-  t1.G = f2_hi(G);
-  t0.alpha = fminf(0.99f, __fmul_rn(m0.z, t0.G));
-  t1.alpha = fminf(0.99f, __fmul_rn(m1.z, t1.G));
-  t0.blended = need0 && t0.alpha >= 1.0f / 255.0f;
-  t1.blended = need1 && t1.alpha >= 1.0f / 255.0f;
 }
 
 // A pixel's state on its back-to-front walk: the transmittance in front of the
@@ -131,9 +41,9 @@ struct PixelBackward {
     na = ncx = ncy = ncz = 0.0f;
   }
 
-  // Steps in front of a splat this pixel blended and writes its 9 gradient shares.
-  __device__ __forceinline__ void shares(const BlendTerm& t, float4 q, float4 c, float* w) {
-    const float alpha = t.alpha, G = t.G, dx = t.dx, dy = t.dy;
+  // Steps in front of a splat of this alpha and colour (alpha 0: one that the pixel did
+  // not blend, which changes nothing) and returns the gradient of its alpha.
+  __device__ __forceinline__ float step(float alpha, float4 c) {
     // 1 / (1 - alpha), used twice; the approximate reciprocal (~1 ulp) is plenty:
     // a chunk's chain of divisions is at most CHUNK entries long.
     float inv;
@@ -148,100 +58,144 @@ struct PixelBackward {
     ncy = c.y;
     ncz = c.z;
     const float dotv = (c.x - bhx) * pgx + (c.y - bhy) * pgy + (c.z - bhz) * pgz;
-    const float alpha_grad = T * dotv - inv * tf_bg;
-    const float power_grad = alpha_grad * c.w * G;
-    // The conic is (a, b, c) = (-2A, b, -2C): the power's gradient is
-    // -(a dx + b dy, b dx + c dy) for the mean and (-dx^2 / 2, -dx dy, -dy^2 / 2)
-    // for the conic, here as multiples of (power_grad dx, power_grad dy).
-    const float pdx = power_grad * dx, pdy = power_grad * dy;
-    w[0] = -2.0f * q.x * pdx + q.y * pdy;
-    w[1] = q.y * pdx - 2.0f * q.z * pdy;
-    w[2] = -0.5f * pdx * dx;
-    w[3] = -pdx * dy;
-    w[4] = -0.5f * pdy * dy;
-    w[5] = alpha_grad * G;
-    const float wt = alpha * T;
-    w[6] = wt * pgx;
-    w[7] = wt * pgy;
-    w[8] = wt * pgz;
+    return T * dotv - inv * tf_bg;
   }
 };
 
-// The start of the back-to-front window that ends at `end`: max(floor, end - 32).
-__device__ __forceinline__ uint32_t window_start(uint32_t end, uint32_t floor) {
-  return end - floor > 32u ? end - 32u : floor;
-}
+// Per-warp shared memory of the backward blend.
+constexpr uint32_t BATCH = 32, HALF_BATCH = BATCH / 2;
+constexpr uint32_t SHARE_ROW = 34;  // 32 pixels, and rows that begin two banks apart
+struct BackStage {
+  BlendPair pair[BATCH / 2];
+  float4 color[BATCH];
+  uint32_t pos[BATCH];    // position in the tile's list
+  uint32_t index[BATCH];  // splat
+  // Per pixel (pixel p at place 2 (p % 16) + p / 16: p and p + 16 side by side, as
+  // packed instructions take them): its gradients, and half a batch's shares: the
+  // gradients of the powers and of the opacities, and alpha T.
+  float grad[3][32];
+  float share[3][HALF_BATCH][SHARE_ROW];
+  uint16_t list[CHUNK];  // the chunk's entries some pixel of the block blended, back to front
+};
 
-// The blend mask words of `block` for a tile's windows [first, end) (at most CHUNK / 32):
-// lane l holds window first + l's, or 0 past them.
-__device__ __forceinline__ uint32_t chunk_mask_words(const uint32_t* __restrict__ mask, uint32_t tile, uint32_t tiles,
-                                                     uint32_t run_x, uint32_t first, uint32_t end, uint32_t block,
-                                                     uint32_t lane) {
-  static_assert(CHUNK / 32 <= 32, "a chunk's mask words fit in the warp's lanes");
-  const uint32_t k = first + lane;
-  return k < end ? mask[mask_at(tile, tiles, run_x, k, block)] : 0u;
-}
-
-// The blend mask bits of window [lo, hi) (none when it is empty) from the chunk's
-// words in the lanes (chunk_mask_words from position base). All lanes must call it.
-__device__ __forceinline__ uint32_t window_blended(uint32_t words, uint32_t base, uint32_t lo, uint32_t hi) {
-  const uint32_t at = (lo - base) >> 5, shift = (lo - base) & 31u;
-  const uint32_t a = __shfl_sync(0xffffffffu, words, at & 31u), b = __shfl_sync(0xffffffffu, words, (at + 1u) & 31u);
-  if (hi <= lo) return 0u;
-  const uint32_t bits = shift ? (a >> shift) | (b << (32u - shift)) : a;
-  return hi - lo >= 32u ? bits : bits & ((1u << (hi - lo)) - 1u);
+// The 9 gradients of half a batch's splats from the shares: lane l sums splat l % 16
+// over the pixels p with p % 2 = l / 16, both lanes' sums meet, and they go to the
+// splat's global gradients, one atomic add each. The sums run in the order of a
+// butterfly over the block's pixels (p + 16 first, p + 1 last). Pixel p is at
+// (corner_x + p % 8, corner_y + p / 8).
+__device__ __forceinline__ void add_gradients(const BackStage& st, uint32_t first, uint32_t n, uint32_t lane,
+                                              float corner_x, float corner_y, float* __restrict__ splat_grads) {
+  const uint32_t s = lane & 15u, h = lane >> 4, e = first + s;
+  const float* f = reinterpret_cast<const float*>(&st.pair[e / 2]) + (e & 1u);
+  const float nx = f[0], ny = f[2], a = 2.0f * f[4], b = f[6], c = 2.0f * f[8];  // conic (a, b, c)
+  const F2 a2 = f2(a, a), b2 = f2(b, b), c2 = f2(c, c);
+  constexpr int N = SPLAT_GRADS;
+  // Pixels p = 2 k + h and p + 16.
+  auto leaf = [&](uint32_t k, float (&out)[N]) {
+    const uint32_t at = 2u * (2u * k + h);
+    auto two = [&](const float* row) { return f2_load(reinterpret_cast<const float2*>(row + at)); };
+    const F2 pg = two(st.share[0][s]), og = two(st.share[1][s]), wt = two(st.share[2][s]);
+    const float dx = (corner_x + (float)(2u * k % 8u + h)) + nx, y = corner_y + (float)(2u * k / 8u);
+    const F2 dx2 = f2(dx, dx), dy2 = f2(y + ny, (y + 2.0f) + ny);
+    const F2 pdx = f2_mul(pg, dx2), pdy = f2_mul(pg, dy2);
+    // The power's gradient is -(a dx + b dy, b dx + c dy) for the pixel's offset and
+    // (-dx^2 / 2, -dx dy, -dy^2 / 2) for the conic (factors without a rounding later).
+    const F2 v[N] = {f2_fma(b2, pdy, f2_mul(a2, pdx)),
+                     f2_fma(b2, pdx, f2_mul(c2, pdy)),
+                     f2_mul(pdx, dx2),
+                     f2_mul(pdx, dy2),
+                     f2_mul(pdy, dy2),
+                     og,
+                     f2_mul(wt, two(st.grad[0])),
+                     f2_mul(wt, two(st.grad[1])),
+                     f2_mul(wt, two(st.grad[2]))};
+#pragma unroll
+    for (int i = 0; i < N; i++) out[i] = __fadd_rn(f2_lo(v[i]), f2_hi(v[i]));
+  };
+  auto add = [](float (&x)[N], const float (&y)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i++) x[i] = __fadd_rn(x[i], y[i]);
+  };
+  float sum[N], odd[N], l[N], m[N];
+  leaf(0, sum), leaf(4, l), add(sum, l);
+  leaf(2, m), leaf(6, l), add(m, l), add(sum, m);
+  leaf(1, odd), leaf(5, l), add(odd, l);
+  leaf(3, m), leaf(7, l), add(m, l), add(odd, m);
+  add(sum, odd);
+#pragma unroll
+  for (int i = 0; i < N; i++) sum[i] = __fadd_rn(sum[i], __shfl_xor_sync(0xffffffffu, sum[i], 16));
+  if (s >= n) return;
+  sum[2] *= -0.5f;
+  sum[3] = -sum[3];
+  sum[4] *= -0.5f;
+  float* out = splat_grads + (size_t)st.index[e] * SPLAT_GRADS;
+#pragma unroll
+  for (int i = 0; i < N; i++)
+    if ((i < 5) == (h == 0) && sum[i] != 0.0f) atomicAdd(out + i, sum[i]);
 }
 
 // src/shaders/rasterizeBackward.wgsl:50-163. The work is split into independent
 // items, one per (tile, CHUNK-entry chunk of its list, 8x4 pixel block), taken by
 // persistent warps from a counter in the plan's order, so no warp waits for
-// another and a long list is spread over many warps. For an item, the warp walks
-// its chunk back to front from the largest `last` among its pixels, keeping in its
-// own slice of shared memory, 32 entries at a time, only the splats some pixel of
-// its block blended in the forward pass (the forward's blend mask; the records of
-// the next window are copied in meanwhile). Each pixel
+// another and a long list is spread over many warps. For an item, the warp lists the
+// chunk's entries that some pixel of its block blended in the forward pass (the
+// forward's blend mask), back to front, and takes 32 of them at a time; the records of
+// the next 32 are loaded meanwhile. Each pixel
 // starts from its state behind the chunk: the transmittance the forward pass saved
 // at the chunk's end, and the colour behind it, (final colour - colour saved) /
 // that transmittance; behind its last splat (the whole list for most tiles) these
-// are the final transmittance and nothing. Splats are then taken two at a time:
-// their alphas are computed together, then each pixel recovers the transmittance
-// in front of each splat by dividing by (1 - alpha), in list order. The 18
-// gradient shares of the pair are summed over the warp's 32 pixels in one
-// reduce-scatter and added to the splats' global gradients, one atomic add per
-// nonzero total.
-__global__ void __launch_bounds__(BWD_THREADS, 6) rasterize_backward_kernel(
+// are the final transmittance and nothing. The alphas of four splats are computed
+// together, then each pixel recovers the transmittance in front of each splat by
+// dividing by (1 - alpha), in list order, and leaves three numbers per splat in shared
+// memory; after 16 splats the lanes change over from pixels to splats and sum them
+// (add_gradients).
+//
+// What bounds it: on large frames instructions and shared memory, on small ones the
+// longest items (512 entries, 20 us and more for one warp) and an item's first loads (a
+// chain of eight, 3 us). Summing 9 shares over the pixels took most of it: with a
+// reduce-scatter over the warp per two splats (18 shares, 20 shuffles and as many
+// selects and adds) 280 us for 1.1M splats at 980x545, 147 for 100k, 122 for 201k at
+// 489x273, 38 for 5k at 251x187; this way, in the same order of additions, 179 | 92 |
+// 65 | 21. Items only for what the forward pass walked, and the longest first: 152 | 80 |
+// 61 | 22. 5 and 6 CTAs per SM 155 | 83 | 65 and 167 | 88 | 66; the groups of 4 unrolled
+// 2 or 4 times the same. Chunks of 256 entries 140 | 75 | 45 | 18, and the shares' sums
+// as moments about the block's center 20% less, but both round otherwise, and a first
+// step of Adam turns a gradient's last bits into the sign of a whole step where it is 0
+// but for rounding.
+__global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
     const Camera* __restrict__ camera, const float4* __restrict__ raster_params, const float* __restrict__ splats,
     const uint32_t* __restrict__ pair_splats, const uint2* __restrict__ ranges, const uint32_t* __restrict__ plan,
-    const uint2* __restrict__ chunks, const float4* __restrict__ pixel_color, const uint32_t* __restrict__ pixel_last,
+    const uint2* __restrict__ item_list, uint32_t item_room, const float4* __restrict__ pixel_color, const uint32_t* __restrict__ pixel_last,
     const float4* __restrict__ checkpoints, const uint32_t* __restrict__ blend_mask,
     const float4* __restrict__ pixel_grads, float* __restrict__ splat_grads, uint32_t* __restrict__ work_counter,
     bool cut_in_record) {
-  __shared__ WarpStage stages[BWD_WARPS];
+  __shared__ BackStage stages[BWD_WARPS];
   const uint32_t lane = threadIdx.x & 31u;
-  WarpStage& st = stages[threadIdx.x >> 5];
+  BackStage& st = stages[threadIdx.x >> 5];
   const float vpx = camera->viewport[0], vpy = camera->viewport[1];
   const uint32_t tiles_x = ((uint32_t)vpx + TILE - 1u) / TILE;
-  const uint32_t multi = plan[PLAN_MULTI], items = (multi + plan[PLAN_SINGLE]) * 8u, room = plan[PLAN_CHUNKS];
+  const uint32_t tiles = plan[PLAN_TILES];
+  uint32_t up_to[ITEM_CLASSES], items = 0;  // the items up to each class
+#pragma unroll
+  for (uint32_t k = 0; k < ITEM_CLASSES; k++) up_to[k] = items += min(plan[PLAN_ITEMS + k], item_room);
   const float4 bg = raster_params[0];
-  const int my_slot = reduce_slot<2 * SPLAT_GRADS>(lane);
-  // Value my_slot belongs to the pair's first (further back) splat when below 9.
-  const uint32_t my_entry = my_slot >= (int)SPLAT_GRADS ? 1u : 0u;
-  const uint32_t my_grad = my_slot >= 0 ? (uint32_t)my_slot - my_entry * SPLAT_GRADS : 0u;
   while (true) {
     uint32_t item = 0;
     if (lane == 0) item = atomicAdd(work_counter, 1u);
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= items) break;
-    const uint32_t which = item >> 3;
-    const uint2 chunk = chunks[which < multi ? which : room - 1u - (which - multi)];
-    const uint32_t tile = chunk.x, block = item & 7u;
+    size_t at = item;
+#pragma unroll
+    for (uint32_t k = 1; k < ITEM_CLASSES; k++)
+      if (item >= up_to[k - 1]) at = (size_t)k * item_room + item - up_to[k - 1];
+    const uint2 it = item_list[at];
+    const uint32_t tile = it.x >> 3, block = it.x & 7u, chunk = it.y;
     const uint32_t bx = (tile % tiles_x) * TILE + (block & 1u) * 8u, by = (tile / tiles_x) * TILE + (block >> 1) * 4u;
     const uint32_t px = bx + (lane & 7u), py = by + (lane >> 3);
     const bool inside = (float)px < vpx && (float)py < vpy;
-    const float cx = (float)px + 0.5f, cy = (float)py + 0.5f;
     const uint2 run = ranges[tile];
-    const uint32_t chunk_lo = run.x + chunk.y * CHUNK, chunk_hi = min(chunk_lo + CHUNK, run.y);
-    const uint32_t boundary = (chunk.y + 1u) * CHUNK;  // the chunk's end, relative to run.x
+    const uint32_t chunk_lo = run.x + chunk * CHUNK, chunk_hi = min(chunk_lo + CHUNK, run.y);
+    const uint32_t boundary = (chunk + 1u) * CHUNK;  // the chunk's end, relative to run.x
     float4 color = make_float4(0.f, 0.f, 0.f, 0.f), pg = color;
     uint32_t last = 0;
     if (inside) {
@@ -253,63 +207,107 @@ __global__ void __launch_bounds__(BWD_THREADS, 6) rasterize_backward_kernel(
     // Splats at or past the warp's largest `last` contribute nothing to it.
     const uint32_t end_all = min(chunk_hi, run.x + __reduce_max_sync(0xffffffffu, last));
     if (end_all <= chunk_lo) continue;
+    // The chunk's blended entries: lane k has the mask word of window k (at most
+    // CHUNK / 32), and the entries in the windows behind it.
+    static_assert(CHUNK / 32 <= 32, "a chunk's mask words fit in the warp's lanes");
+    const uint32_t windows = (end_all - chunk_lo + 31u) / 32u;
+    uint32_t word = 0;
+    if (lane < windows) {
+      word = blend_mask[mask_at(tile, tiles, run.x, chunk * (CHUNK / 32u) + lane, block)];
+      const uint32_t left = end_all - chunk_lo - lane * 32u;
+      if (left < 32u) word &= (1u << left) - 1u;
+    }
+    uint32_t behind_it = __popc(word);
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t v = __shfl_down_sync(0xffffffffu, behind_it, d);
+      if (lane + d < 32u) behind_it += v;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, behind_it, 0);
+    if (total == 0) continue;
+    behind_it -= __popc(word);
+    for (uint32_t k = 0; k < windows; k++) {
+      const uint32_t bits = __shfl_sync(0xffffffffu, word, k), at = __shfl_sync(0xffffffffu, behind_it, k);
+      if ((bits >> lane) & 1u) st.list[at + __popc(bits >> lane) - 1u] = (uint16_t)(k * 32u + lane);
+    }
+    const uint32_t place = 2u * (lane & 15u) + (lane >> 4);
+    st.grad[0][place] = pg.x;
+    st.grad[1][place] = pg.y;
+    st.grad[2][place] = pg.z;
+    __syncwarp();
     float T0 = color.w;
     float3 behind = make_float3(0.f, 0.f, 0.f);
     if (last > boundary) {  // the pixel blends splats behind this chunk
-      const float4 ck = checkpoints[checkpoint_at(run.x, chunk.y + 1u, block, lane)];
+      const float4 ck = checkpoints[checkpoint_at(run.x, chunk + 1u, block, lane)];
       const float inv = 1.0f / ck.x;
       T0 = ck.x;
       behind = make_float3((color.x - color.w * bg.x - ck.y) * inv, (color.y - color.w * bg.y - ck.z) * inv,
                            (color.z - color.w * bg.z - ck.w) * inv);
     }
-    PixelBackward px_state;
-    px_state.begin(color.w, T0, behind, pg.x, pg.y, pg.z, bg);
-    // Windows run back to front: [lo, end) with lo = max(chunk_lo, end - 32). Only
-    // the entries some pixel of the block blended (the forward pass's mask) are
-    // staged. This lane's entry of the window in flight and of the next one.
-    const uint32_t words = chunk_mask_words(blend_mask, tile, plan[PLAN_TILES], run.x, chunk.y * (CHUNK / 32u),
-                                            (end_all - run.x + 31u) / 32u, block, lane);
-    uint32_t end = end_all;
-    uint32_t lo = window_start(end, chunk_lo);
-    uint32_t bits = window_blended(words, chunk_lo, lo, end);
-    uint32_t index = (bits >> lane) & 1u ? pair_splats[lo + lane] : 0u;
-    stage_issue(st.raw, splats, index, (bits >> lane) & 1u);
-    uint32_t next_lo = window_start(lo, chunk_lo);
-    uint32_t next_bits = window_blended(words, chunk_lo, next_lo, lo);
-    uint32_t next_index = (next_bits >> lane) & 1u ? pair_splats[next_lo + lane] : 0u;
-    while (end > chunk_lo) {
-      const uint32_t staged = stage_commit_blended(st, run.x, lo, index, bits, cut_in_record);
-      {
-        stage_issue(st.raw, splats, next_index, (next_bits >> lane) & 1u);
-        end = lo;
-        lo = next_lo;
-        bits = next_bits;
-        index = next_index;
-        next_lo = window_start(lo, chunk_lo);
-        next_bits = window_blended(words, chunk_lo, next_lo, lo);
-        next_index = (next_bits >> lane) & 1u ? pair_splats[next_lo + lane] : 0u;
-      }
-      for (uint32_t slot = staged; slot > 0;) {
-        // Entries j0 (further back, taken first) and j1 = j0 - 1 when there is one.
-        const uint32_t j0 = slot - 1, j1 = slot >= 2 ? slot - 2 : j0;
-        const bool pair = slot >= 2;
-        slot = pair ? slot - 2 : 0;
-        BlendTerm t0, t1;
-        blend_terms(st, j0, j1, inside && st.pos[j0] < last, pair && inside && st.pos[j1] < last, cx, cy, t0, t1);
-        if (!__any_sync(0xffffffffu, t0.blended || t1.blended)) continue;
-        float v[2 * SPLAT_GRADS];
-#pragma unroll
-        for (int q = 0; q < 2 * (int)SPLAT_GRADS; q++) v[q] = 0.0f;
-        // Back to front: j0, then j1.
-        if (t0.blended) px_state.shares(t0, st.quad[j0], st.color[j0], v);
-        if (t1.blended) px_state.shares(t1, st.quad[j1], st.color[j1], v + SPLAT_GRADS);
-        const float total = warp_reduce_scatter(v, lane);
-        if (my_slot >= 0 && total != 0.0f && (my_entry == 0 || pair))
-          atomicAdd(&splat_grads[(size_t)st.index[my_entry ? j1 : j0] * SPLAT_GRADS + my_grad], total);
+    PixelBackward pb;
+    pb.begin(color.w, T0, behind, pg.x, pg.y, pg.z, bg);
+    const F2 cx = f2((float)px + 0.5f, (float)px + 0.5f), cy = f2((float)py + 0.5f, (float)py + 0.5f);
+    // This lane's entry of the next batch, and the splat of the one after.
+    auto entry = [&](uint32_t k) { return k < total ? (uint32_t)st.list[k] : 0u; };
+    SplatRecord raw;
+    uint32_t index = lane < total ? pair_splats[chunk_lo + entry(lane)] : 0u;
+    raw.load(splats, index, lane < total);
+    uint32_t next_index = BATCH + lane < total ? pair_splats[chunk_lo + entry(BATCH + lane)] : 0u;
+    for (uint32_t first = 0; first < total; first += BATCH) {
+      const uint32_t staged = min(BATCH, total - first);
+      float* e = reinterpret_cast<float*>(&st.pair[lane / 2]) + (lane & 1u);
+      if (lane < staged) {
+        stage_entry(e, raw, cut_in_record ? raw.s1.w : blend_cutoff(raw.s2.w));
+        st.color[lane] = raw.s2;
+        st.pos[lane] = chunk * CHUNK + entry(first + lane);
+        st.index[lane] = index;
+      } else {
+        e[10] = 0.0f;  // nothing is below it
       }
       __syncwarp();
+      index = next_index;
+      raw.load(splats, index, first + BATCH + lane < total);
+      const uint32_t ahead = first + 2 * BATCH + lane;
+      next_index = ahead < total ? pair_splats[chunk_lo + entry(ahead)] : 0u;
+#pragma unroll 1
+      for (uint32_t half = 0; half < staged; half += HALF_BATCH) {
+        const uint32_t n = min(HALF_BATCH, staged - half);
+#pragma unroll 1
+        for (uint32_t j = 0; j < n; j += 4) {
+          const uint4 pos = *reinterpret_cast<const uint4*>(&st.pos[half + j]);
+          bool has[4] = {pos.x < last, pos.y < last, pos.z < last, pos.w < last};
+          float alpha[4], G[4];
+#pragma unroll
+          for (uint32_t h = 0; h < 2; h++) {
+            const BlendPair& pr = st.pair[(half + j) / 2 + h];
+            F2 limit;
+            const F2 q = blend_power_negated(pr, cx, cy, limit);
+            has[2 * h] = has[2 * h] && __float_as_uint(f2_lo(q)) < __float_as_uint(f2_lo(limit));
+            has[2 * h + 1] = has[2 * h + 1] && __float_as_uint(f2_hi(q)) < __float_as_uint(f2_hi(limit));
+            // Any value may come out where the limit was not kept.
+            const F2 ex = exp_blend_negated(q), al = f2_mul(F2{pr.opacity}, ex);
+            G[2 * h] = f2_lo(ex);
+            G[2 * h + 1] = f2_hi(ex);
+            alpha[2 * h] = fminf(0.99f, f2_lo(al));
+            alpha[2 * h + 1] = fminf(0.99f, f2_hi(al));
+          }
+#pragma unroll
+          for (uint32_t u = 0; u < 4; u++) {
+            has[u] = has[u] && alpha[u] >= 1.0f / 255.0f;
+            const float al = has[u] ? alpha[u] : 0.0f;
+            const float4 c = st.color[half + j + u];
+            const float alpha_grad = pb.step(al, c);
+            st.share[0][j + u][place] = has[u] ? alpha_grad * c.w * G[u] : 0.0f;
+            st.share[1][j + u][place] = has[u] ? alpha_grad * G[u] : 0.0f;
+            st.share[2][j + u][place] = al * pb.T;
+          }
+        }
+        __syncwarp();
+        add_gradients(st, half, n, lane, (float)bx + 0.5f, (float)by + 0.5f, splat_grads);
+        __syncwarp();
+      }
     }
-    cp_async_wait_all();
+    __syncwarp();
   }
 }
 
@@ -771,7 +769,7 @@ dg_status launch_rasterize_backward(dg_tile_rasterizer* tr, dg_buffer* pixel_gra
                                         BWD_THREADS, 0, ctx->stream>>>(
                 typed<const Camera>(tr->camera), typed<float4>(tr->raster_params), typed<float>(tr->splats),
                 typed<uint32_t>(tr->values), typed<uint2>(tr->ranges), typed<uint32_t>(tr->work_plan),
-                typed<uint2>(tr->chunks), typed<float4>(tr->pixel_color), typed<uint32_t>(tr->pixel_last),
+                typed<uint2>(tr->items), (uint32_t)(tr->items->bytes / sizeof(uint2) / ITEM_CLASSES), typed<float4>(tr->pixel_color), typed<uint32_t>(tr->pixel_last),
                 typed<float4>(tr->checkpoints), typed<uint32_t>(tr->blend_mask), typed<float4>(pixel_grads),
                 typed<float>(splat_grads), counter, tr->splat_cutoffs));
   return DG_OK;

@@ -204,16 +204,12 @@ __device__ __forceinline__ void sh_basis_gradient(const float d[3], float g[15][
 // ------------------------------------------------------------------ blending
 // The exponent of a splat at a pixel, `power = -0.5 (a dx^2 + c dy^2) - b dx dy`
 // (src/shaders/rasterize.wgsl:68), from A = -0.5 a and C = -0.5 c (exact
-// scalings), evaluated as dx (A dx - b dy) + (C dy) dy: three products and two
+// scalings), is evaluated as dx (A dx - b dy) + (C dy) dy: three products and two
 // fused multiply-adds instead of five products and three sums (WGSL leaves
-// contraction to the implementation; the oracle evaluates this same sequence).
-// Written with round-to-nearest intrinsics, which the compiler neither fuses
-// further nor splits, so the forward and backward passes compute identical powers
-// whatever their --fmad setting.
-__device__ __forceinline__ float blend_power(float A, float b, float C, float dx, float dy) {
-  const float t = __fmaf_rn(A, dx, -__fmul_rn(b, dy));
-  return __fmaf_rn(t, dx, __fmul_rn(__fmul_rn(C, dy), dy));
-}
+// contraction to the implementation; the oracle evaluates this same sequence), on the
+// negated values (blend_power_negated). Written with explicit instructions, which the
+// compiler neither fuses further nor splits, so the forward and backward passes compute
+// identical powers whatever their --fmad setting.
 
 // A power below which alpha = opacity * exp(power) is certainly under 1/255, so
 // the exp can be skipped with the same outcome: ln(1 / (255 opacity)), lowered by
@@ -274,26 +270,22 @@ constexpr uint32_t COOP_MIN = 128, COOP_FLOOR = 64;
 //                 pixels are expected to walk))
 //   PLAN_TOTAL    those entries of all tiles
 //   PLAN_TILES    tiles
-//   PLAN_MULTI    backward chunks of tiles with several chunks: chunks[0..)
-//   PLAN_SINGLE   tiles with one chunk: chunks[PLAN_CHUNKS - 1] downwards
-//   PLAN_CHUNKS   the room in chunks
+//   PLAN_ITEMS    the backward pass's items per class, listed by the forward pass
 //   PLAN_LONGEST  the longest tile's entries
 //   then for each bucket its tiles, in room for all tiles
-constexpr uint32_t PLAN_BUCKETS = 32, PLAN_TOTAL = 32, PLAN_TILES = 33, PLAN_MULTI = 34, PLAN_SINGLE = 35,
-                   PLAN_CHUNKS = 36, PLAN_LONGEST = 37, PLAN_HEADER = 40;
+constexpr uint32_t PLAN_BUCKETS = 32, PLAN_TOTAL = 32, PLAN_TILES = 33, PLAN_LONGEST = 34, PLAN_ITEMS = 35,
+                   ITEM_CLASSES = 4, PLAN_HEADER = PLAN_ITEMS + ITEM_CLASSES;
+// The class of a backward item of so many entries, the longest first: warps that take a
+// long item last keep the GPU waiting.
+__device__ __forceinline__ uint32_t item_class(uint32_t entries) {
+  return ITEM_CLASSES - 1u - (entries - 1u) * ITEM_CLASSES / CHUNK;
+}
 constexpr size_t plan_words(size_t tiles) { return PLAN_HEADER + PLAN_BUCKETS * tiles; }
 
-// Splat records as they are copied in: lane l has the 48-byte record of its entry of
-// a window of 32.
-using RawWindow = float4[32][3];
-
-// A warp's own window of up to 32 list entries, staged in its slice of shared
-// memory: only the splats that can reach the warp's 8x4 pixel block, in list
-// order. `raw` receives the splat records of the next window by cp.async while
-// the current one blends.
-//
-// The forward pass's stage. Two entries share a BlendPair, each field's two values
-// side by side as packed instructions take them.
+// The forward pass's stage: a warp's own window of up to 32 list entries, in its slice
+// of shared memory: only the splats that can reach the warp's 8x4 pixel block, in list
+// order. Two entries share a BlendPair, each field's two values side by side as packed
+// instructions take them.
 struct BlendPair {
   ulonglong2 n;   // -mean x, -mean y
   ulonglong2 ab;  // 0.5 a, b
@@ -306,16 +298,6 @@ struct BlendStage {
   float4 color[32];  // rgb, opacity
   uint32_t pos[32];  // position in the tile's list
 };
-// The backward pass's.
-struct WarpStage {
-  float4 mean[32];   // mean x, y, opacity, 0
-  float4 quad[32];   // A = -0.5 a, b, C = -0.5 c, cutoff
-  float4 color[32];  // rgb, opacity
-  uint32_t pos[32];  // position in the tile's list
-  uint32_t index[32];
-  RawWindow raw;
-};
-
 // A pixel's state at the start of chunk boundary k of a tile (after every entry
 // before position k * CHUNK): transmittance and the colour blended so far. One
 // slot of 8 blocks x 32 pixels per CHUNK entries of the pair list; boundary k of
@@ -398,18 +380,6 @@ __device__ __forceinline__ void stage_floats_async(float* dst, const float* __re
   }
 }
 
-// Starts copying the splat record of this lane's entry of a window into `raw`.
-__device__ __forceinline__ void stage_issue(RawWindow& raw, const float* __restrict__ splats, uint32_t index,
-                                            bool valid) {
-  if (valid) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const float4* s = reinterpret_cast<const float4*>(splats + (size_t)index * FLOATS_PER_SPLAT);
-    cp_async16(&raw[lane][0], s);
-    cp_async16(&raw[lane][1], s + 1);
-    cp_async16(&raw[lane][2], s + 2);
-  }
-}
-
 __device__ __forceinline__ uint4 tile_rect(float mx, float my, float radius, uint2 tiles);
 
 // The 16x16 tile a blend item's block lies in, for blend tiles of several 16x16
@@ -434,6 +404,30 @@ struct SplatRecord {
   }
 };
 
+// Writes a record's half of its BlendPair (e: the pair as floats, plus 1 for the upper
+// half).
+__device__ __forceinline__ void stage_entry(float* e, const SplatRecord& raw, float cut) {
+  e[0] = -raw.s0.x;
+  e[2] = -raw.s0.y;
+  e[4] = 0.5f * raw.s1.x;
+  e[6] = raw.s1.y;
+  e[8] = 0.5f * raw.s1.z;
+  e[10] = __uint_as_float(__float_as_uint(-cut) + 1u);
+  e[12] = raw.s2.w;
+}
+
+// -power of a pair of staged entries at pixel (px, py), two lanes of packed
+// instructions; its bits are below those of `limit`'s where the splat's alpha may
+// reach 1/255.
+__device__ __forceinline__ F2 blend_power_negated(const BlendPair& e, F2 px, F2 py, F2& limit) {
+  const ulonglong2 n = e.n, ab = e.ab, cl = e.cl;
+  const F2 dx = f2_add(px, F2{n.x}), dy = f2_add(py, F2{n.y});
+  const F2 s = f2_fma(F2{ab.x}, dx, f2_mul(F2{ab.y}, dy));
+  limit = F2{cl.y};
+  // + 0 makes a zero's sign positive: bits compare like values from 0 up.
+  return f2_add(f2_fma(s, dx, f2_mul(f2_mul(F2{cl.x}, dy), dy)), f2(0.0f, 0.0f));
+}
+
 // Takes the window [lo, min(lo + 32, hi)) whose records are in `raw` and keeps, in
 // list order, the splats that can reach the warp's block, whose pixel centers span [x0, x0 + 7] x [y0, y0 + 3] (and,
 // with a TileMember, belong to its 16x16 tile's list). Returns how many were
@@ -447,34 +441,22 @@ __device__ __forceinline__ uint32_t stage_commit(BlendStage& st, const SplatReco
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t k = lo + lane;
   bool keep = false;
-  float2 mean = make_float2(0.f, 0.f), ab = mean, cl = mean;
-  float4 color = make_float4(0.f, 0.f, 0.f, 0.f);
+  float cut = 0.0f;
   if (k < hi) {
-    const float4 s0 = raw.s0, s1 = raw.s1;
-    color = raw.s2;
-    mean = make_float2(s0.x, s0.y);
-    const float A = -0.5f * s1.x, b = s1.y, C = -0.5f * s1.z;
-    const float cut = cut_in_record ? s1.w : blend_cutoff(color.w);
-    ab = make_float2(-A, b);
-    cl = make_float2(-C, cut);
+    const float2 mean = make_float2(raw.s0.x, raw.s0.y);
+    const float A = -0.5f * raw.s1.x, b = raw.s1.y, C = -0.5f * raw.s1.z;
+    cut = cut_in_record ? raw.s1.w : blend_cutoff(raw.s2.w);
     keep = cut < 0.0f && rect_reachable(A, b, C, cut, x0 - mean.x, x0 + 7.0f - mean.x, y0 - mean.y, y0 + 3.0f - mean.y);
     if (tm.member && keep) {
-      const uint4 rect = tile_rect(mean.x, mean.y, s0.w, tm.tiles);
+      const uint4 rect = tile_rect(mean.x, mean.y, raw.s0.w, tm.tiles);
       keep = tm.tx >= rect.x && tm.tx < rect.z && tm.ty >= rect.y && tm.ty < rect.w;
     }
   }
   const uint32_t kept = __ballot_sync(0xffffffffu, keep);
   if (keep) {
     const uint32_t at = __popc(kept & ((1u << lane) - 1u));
-    float* e = reinterpret_cast<float*>(&st.pair[at / 2]) + (at & 1u);
-    e[0] = -mean.x;
-    e[2] = -mean.y;
-    e[4] = ab.x;
-    e[6] = ab.y;
-    e[8] = cl.x;
-    e[10] = __uint_as_float(__float_as_uint(-cl.y) + 1u);
-    e[12] = color.w;
-    st.color[at] = color;
+    stage_entry(reinterpret_cast<float*>(&st.pair[at / 2]) + (at & 1u), raw, cut);
+    st.color[at] = raw.s2;
     st.pos[at] = k - run_x;
   }
   // Entries past the last are taken in groups of 4 with it: nothing is below theirs.
@@ -484,27 +466,6 @@ __device__ __forceinline__ uint32_t stage_commit(BlendStage& st, const SplatReco
   return staged;
 }
 
-
-// Like stage_commit for a window whose entries the block blended are known:
-// lane l keeps entry lo + l when bit l of `blended` is set (lanes past hi must
-// have it clear), with no rectangle test.
-__device__ __forceinline__ uint32_t stage_commit_blended(WarpStage& st, uint32_t run_x, uint32_t lo, uint32_t index,
-                                                         uint32_t blended, bool cut_in_record) {
-  cp_async_wait_all();
-  const uint32_t lane = threadIdx.x & 31u;
-  const bool keep = (blended >> lane) & 1u;
-  if (keep) {
-    const uint32_t at = __popc(blended & ((1u << lane) - 1u));
-    const float4 s0 = st.raw[lane][0], s1 = st.raw[lane][1], color = st.raw[lane][2];
-    st.mean[at] = make_float4(s0.x, s0.y, color.w, 0.0f);
-    st.quad[at] = make_float4(-0.5f * s1.x, s1.y, -0.5f * s1.z, cut_in_record ? s1.w : blend_cutoff(color.w));
-    st.color[at] = color;
-    st.pos[at] = lo + lane - run_x;
-    st.index[at] = index;
-  }
-  __syncwarp();
-  return __popc(blended);
-}
 
 // tile_count / tile_rect (src/shaders/common.wgsl:31-42).
 __device__ __forceinline__ uint2 tile_grid(const Camera& cam) {
