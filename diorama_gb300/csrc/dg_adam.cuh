@@ -61,9 +61,9 @@ __device__ __forceinline__ float adam_param_slot(const AdamParams& ap, uint32_t 
 // radius go into stats; aux (the learned densification's extra statistics) gets
 // the squared length and the count of steps seen over the Gaussian's life.
 // The same from the values: the splat's radius and its mean's two gradients.
-__device__ __forceinline__ void accumulate_stats_values(const float* __restrict__ viewport, float radius,
+__device__ __forceinline__ void accumulate_stats_values(const float* viewport, float radius,
                                                         float mean_grad_x, float mean_grad_y,
-                                                        float4* __restrict__ stats, float2* __restrict__ aux,
+                                                        float4* stats, float2* aux,
                                                         uint32_t i) {
   if (radius == 0.0f) return;
   const float gx = mean_grad_x * viewport[0] * 0.5f;
@@ -75,10 +75,10 @@ __device__ __forceinline__ void accumulate_stats_values(const float* __restrict_
   aux[i] = make_float2(a.x + len * len, a.y + 1.0f);
 }
 
-__device__ __forceinline__ void accumulate_stats_one(const float* __restrict__ viewport,
-                                                     const float* __restrict__ splats,
-                                                     const float* __restrict__ splat_grads, float4* __restrict__ stats,
-                                                     float2* __restrict__ aux, uint32_t i) {
+__device__ __forceinline__ void accumulate_stats_one(const float* viewport,
+                                                     const float* splats,
+                                                     const float* splat_grads, float4* stats,
+                                                     float2* aux, uint32_t i) {
   accumulate_stats_values(viewport, splats[(size_t)i * FLOATS_PER_SPLAT + 3], splat_grads[(size_t)i * SPLAT_GRADS],
                           splat_grads[(size_t)i * SPLAT_GRADS + 1], stats, aux, i);
 }

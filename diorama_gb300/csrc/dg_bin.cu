@@ -142,8 +142,9 @@ __device__ __forceinline__ uint64_t rect_bins(uint32_t r, uint32_t bins_x) {
 // the counts: four shared-memory additions a splat whatever it covers. (Counting
 // bits of the bins' words like the scatter took 52 us instead of 15 at 1.1M
 // splats and 8487 tiles.) Grid: (chunks, views).
-__global__ void __launch_bounds__(BIN_THREADS) bin_count_kernel(const Bins b, const uint32_t* __restrict__ rects,
-                                                                const uint32_t* __restrict__ order) {
+__global__ void __launch_bounds__(BIN_THREADS) bin_count_kernel(const Bins b, const uint32_t* rects,
+                                                                const uint32_t* order) {
+  chain_begin();
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_sum[BIN_WARPS];
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
@@ -274,9 +275,10 @@ __device__ __forceinline__ uint32_t bin_exclusive(uint32_t v, uint32_t* s_warp, 
 //   costs a 32-byte sector.
 // Grid: (bins, chunks, views): the nearest chunks, which cover the most tiles, first.
 __global__ void __launch_bounds__(BIN_THREADS) bin_scatter_kernel(const Bins b,
-                                                                  const uint32_t* __restrict__ order,
-                                                                  const uint2* __restrict__ ranges,
-                                                                  uint32_t* __restrict__ values) {
+                                                                  const uint32_t* order,
+                                                                  const uint2* ranges,
+                                                                  uint32_t* values) {
+  chain_begin();
   extern __shared__ uint32_t smem[];
   constexpr uint32_t TILES = BIN_SIDE * BIN_SIDE;
   static_assert(TILES == BIN_THREADS, "a thread per tile of the bin");
@@ -491,7 +493,8 @@ __device__ Limit find_limit(const Bins& b, uint32_t capacity) {
 // (8 warps reading them twice took 55 us instead of 14 at 538 chunks x 8487 tiles.)
 // Grid: (tiles / 32, views).
 __global__ void __launch_bounds__(SCAN_THREADS) bin_scan_kernel(const Bins b, uint32_t capacity,
-                                                                uint32_t* __restrict__ pair_total) {
+                                                                uint32_t* pair_total) {
+  chain_begin();
   constexpr uint32_t WARPS = SCAN_THREADS / 32;
   __shared__ uint32_t s_sum[WARPS][32];
   __shared__ unsigned long long s_pairs[WARPS];
@@ -570,9 +573,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_scan_kernel(const Bins b, ui
 // A thread per tile: the tile's run of the pair list. Each CTA adds up the tiles
 // before its own (a few L2 reads a thread). The first clears what the blend's plan
 // counts into.
-__global__ void __launch_bounds__(RANGE_THREADS) bin_ranges_kernel(const Bins b, uint2* __restrict__ ranges,
-                                                                   uint32_t* __restrict__ plan,
-                                                                   uint32_t* __restrict__ work) {
+__global__ void __launch_bounds__(RANGE_THREADS) bin_ranges_kernel(const Bins b, uint2* ranges,
+                                                                   uint32_t* plan,
+                                                                   uint32_t* work) {
+  chain_begin();
   constexpr uint32_t WARPS = RANGE_THREADS / 32;
   static_assert(WARPS == 32, "a warp's lanes read one word per warp");
   __shared__ uint32_t s_before[WARPS], s_sum[WARPS];
@@ -642,18 +646,14 @@ dg_status bin_init() {
 
 dg_status bin_launch(dg_context* ctx, const BinShape& s, const BinLaunch& l) {
   const Bins b = bins_of(s, l.scratch);
-  DG_LAUNCH(ctx, "bin_count",
-            bin_count_kernel<<<dim3(b.chunks, s.views), BIN_THREADS, count_bytes(b), ctx->stream>>>(b, l.rects,
-                                                                                                    l.order));
-  DG_LAUNCH(ctx, "bin_scan",
-            bin_scan_kernel<<<dim3(ceil_div(b.tiles, 32), s.views), SCAN_THREADS, 0, ctx->stream>>>(
-                b, l.capacity, l.pair_total));
-  DG_LAUNCH(ctx, "bin_ranges",
-            bin_ranges_kernel<<<ceil_div((uint64_t)s.views * b.tiles, RANGE_THREADS), RANGE_THREADS, 0, ctx->stream>>>(
-                b, l.ranges, l.plan, l.work));
-  DG_LAUNCH(ctx, "bin_scatter",
-            bin_scatter_kernel<<<dim3(b.bins, b.chunks, s.views), BIN_THREADS, scatter_bytes(b.chunk),
-                                 ctx->stream>>>(b, l.order, l.ranges, l.values));
+  DG_CHAIN(ctx, "bin_count", (bin_count_kernel), dim3(b.chunks, s.views), BIN_THREADS, count_bytes(b),
+           b, l.rects, l.order);
+  DG_CHAIN(ctx, "bin_scan", (bin_scan_kernel), dim3(ceil_div(b.tiles, 32), s.views), SCAN_THREADS, 0,
+           b, l.capacity, l.pair_total);
+  DG_CHAIN(ctx, "bin_ranges", (bin_ranges_kernel), ceil_div((uint64_t)s.views * b.tiles, RANGE_THREADS), RANGE_THREADS, 0,
+           b, l.ranges, l.plan, l.work);
+  DG_CHAIN(ctx, "bin_scatter", (bin_scatter_kernel), dim3(b.bins, b.chunks, s.views), BIN_THREADS, scatter_bytes(b.chunk),
+           b, l.order, l.ranges, l.values);
   return DG_OK;
 }
 

@@ -130,16 +130,17 @@ __device__ __forceinline__ void load_gaussian(const float* __restrict__ gaussian
 // half of s_sh (cp.async) and its Gaussian records loading into registers, so
 // the loads of one block wait behind the arithmetic of the previous one instead
 // of in front of it.
-__global__ void __launch_bounds__(PRE_THREADS) preprocess_kernel(const Camera* __restrict__ camera,
-                                                                 const float* __restrict__ gaussians,
-                                                                 const float* __restrict__ sh, uint32_t count,
-                                                                 const uint32_t* __restrict__ scene_params,
-                                                                 float* __restrict__ splats,
-                                                                 uint32_t* __restrict__ tile_counts,
-                                                                 uint32_t* __restrict__ rects,
-                                                                 uint32_t* __restrict__ depth_keys,
-                                                                 uint32_t* __restrict__ depth_order,
-                                                                 float* __restrict__ radii) {
+__global__ void __launch_bounds__(PRE_THREADS) preprocess_kernel(const Camera* camera,
+                                                                 const float* gaussians,
+                                                                 const float* sh, uint32_t count,
+                                                                 const uint32_t* scene_params,
+                                                                 float* splats,
+                                                                 uint32_t* tile_counts,
+                                                                 uint32_t* rects,
+                                                                 uint32_t* depth_keys,
+                                                                 uint32_t* depth_order,
+                                                                 float* radii) {
+  chain_begin();
   __shared__ Camera s_cam;
   __shared__ __align__(16) float s_sh[2][PRE_THREADS * SH_REST_FLOATS];
   load_camera(s_cam, camera);
@@ -199,10 +200,11 @@ uint32_t preprocess_grid(const dg_context* ctx, uint32_t count) {
 // Splat (view v, Gaussian i) is number v * count + i; its depth-sort key puts
 // the view above the depth's bits, so one sort orders every view by depth.
 __global__ void __launch_bounds__(PRE_THREADS) preprocess_views_kernel(
-    const Camera* __restrict__ cameras, uint32_t views, const float* __restrict__ gaussians,
-    const float* __restrict__ sh, uint32_t count, const uint32_t* __restrict__ scene_params,
-    float* __restrict__ splats, uint32_t* __restrict__ tile_counts, uint32_t* __restrict__ rects,
-    uint2* __restrict__ depth_keys, uint32_t* __restrict__ depth_order, uint32_t twl, uint32_t thl) {
+    const Camera* cameras, uint32_t views, const float* gaussians,
+    const float* sh, uint32_t count, const uint32_t* scene_params,
+    float* splats, uint32_t* tile_counts, uint32_t* rects,
+    uint2* depth_keys, uint32_t* depth_order, uint32_t twl, uint32_t thl) {
+  chain_begin();
   __shared__ float s_sh[PRE_THREADS * SH_REST_FLOATS];
   const uint32_t degree = scene_params[0];
   const uint32_t basis_count = (degree + 1u) * (degree + 1u) - 1u;
@@ -1239,10 +1241,9 @@ dg_status views_preprocess_launch(dg_context* ctx, const Camera* cameras, uint32
                                   const float* sh, uint32_t count, const uint32_t* scene_params, float* splats,
                                   uint32_t* tile_counts, uint32_t* rects, uint2* depth_keys, uint32_t* order,
                                   BlendShape shape) {
-  DG_LAUNCH(ctx, "preprocess",
-            preprocess_views_kernel<<<ceil_div(count, PRE_THREADS), PRE_THREADS, 0, ctx->stream>>>(
-                cameras, views, gaussians, sh, count, scene_params, splats, tile_counts, rects, depth_keys, order,
-                shape.twl, shape.thl));
+  DG_CHAIN(ctx, "preprocess", (preprocess_views_kernel), ceil_div(count, PRE_THREADS), PRE_THREADS, 0,
+           cameras, views, gaussians, sh, count, scene_params, splats, tile_counts, rects, depth_keys, order,
+           shape.twl, shape.thl);
   return DG_OK;
 }
 
@@ -1405,14 +1406,12 @@ dg_status renderer_prepare(dg_renderer* r, const dg_camera* camera, const float 
 dg_status renderer_launch_forward(dg_renderer* r, dg_buffer* target) {
   dg_context* ctx = r->ctx;
   if (r->count > 0) {
-    DG_LAUNCH(ctx, "preprocess",
-              preprocess_kernel<<<preprocess_grid(ctx, r->count), PRE_THREADS, 0, ctx->stream>>>(
-                  typed<const Camera>(r->camera), typed<float>(r->gaussians), typed<float>(r->sh), r->count,
-                  typed<uint32_t>(r->scene_params), typed<float>(r->splats),
-                  typed<uint32_t>(r->rasterizer->tile_offsets),
-                  r->rasterizer->binned ? typed<uint32_t>(r->rasterizer->tile_offsets) : nullptr,
-                  typed<uint32_t>(r->rasterizer->depth_keys),
-                  typed<uint32_t>(r->rasterizer->depth_values), typed<float>(r->radii)));
+    DG_CHAIN(ctx, "preprocess", (preprocess_kernel), preprocess_grid(ctx, r->count), PRE_THREADS, 0,
+             typed<const Camera>(r->camera), typed<float>(r->gaussians), typed<float>(r->sh), r->count,
+             typed<uint32_t>(r->scene_params), typed<float>(r->splats), typed<uint32_t>(r->rasterizer->tile_offsets),
+             r->rasterizer->binned ? typed<uint32_t>(r->rasterizer->tile_offsets) : nullptr,
+             typed<uint32_t>(r->rasterizer->depth_keys), typed<uint32_t>(r->rasterizer->depth_values),
+             typed<float>(r->radii));
   }
   return rasterizer_launch(r->rasterizer, target, true);
 }

@@ -163,12 +163,13 @@ __device__ __forceinline__ void add_gradients(const BackStage& st, uint32_t firs
 // step of Adam turns a gradient's last bits into the sign of a whole step where it is 0
 // but for rounding.
 __global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
-    const Camera* __restrict__ camera, const float4* __restrict__ raster_params, const float* __restrict__ splats,
-    const uint32_t* __restrict__ pair_splats, const uint2* __restrict__ ranges, const uint32_t* __restrict__ plan,
-    const uint2* __restrict__ item_list, uint32_t item_room, const float4* __restrict__ pixel_color, const uint32_t* __restrict__ pixel_last,
-    const float4* __restrict__ checkpoints, const uint32_t* __restrict__ blend_mask,
-    const float4* __restrict__ pixel_grads, float* __restrict__ splat_grads, uint32_t* __restrict__ work_counter,
+    const Camera* camera, const float4* raster_params, const float* splats,
+    const uint32_t* pair_splats, const uint2* ranges, const uint32_t* plan,
+    const uint2* item_list, uint32_t item_room, const float4* pixel_color, const uint32_t* pixel_last,
+    const float4* checkpoints, const uint32_t* blend_mask,
+    const float4* pixel_grads, float* splat_grads, uint32_t* work_counter,
     bool cut_in_record) {
+  chain_begin();
   __shared__ BackStage stages[BWD_WARPS];
   const uint32_t lane = threadIdx.x & 31u;
   BackStage& st = stages[threadIdx.x >> 5];
@@ -544,9 +545,10 @@ __device__ __forceinline__ void store16(float* __restrict__ dst, const float (&v
 // and its SH gradients written back from there, both as contiguous copies (a
 // thread's own 45 floats would otherwise be 180 bytes apart from its neighbour's).
 __global__ void __launch_bounds__(PBWD_THREADS) preprocess_backward_kernel(
-    const Camera* __restrict__ camera, const float* __restrict__ gaussians, const float* __restrict__ sh,
-    uint32_t count, const uint32_t* __restrict__ scene_params, const float* __restrict__ splats,
-    const float* __restrict__ splat_grads, float* __restrict__ gaussian_grads, float* __restrict__ sh_grads) {
+    const Camera* camera, const float* gaussians, const float* sh,
+    uint32_t count, const uint32_t* scene_params, const float* splats,
+    const float* splat_grads, float* gaussian_grads, float* sh_grads) {
+  chain_begin();
   __shared__ Camera s_cam;
   __shared__ __align__(16) float s_sh[PBWD_THREADS * SH_REST_FLOATS];
   load_camera(s_cam, camera);
@@ -610,11 +612,12 @@ __device__ __forceinline__ float4 f4_load(const float* p) { return *reinterpret_
 // that every buffer starts 16-byte aligned. A copy that does not complete within
 // the wait limit sets DEVICE_ERROR_COPY_WAIT and the CTA returns.
 __global__ void DG_PBWD_BOUNDS preprocess_backward_adam_kernel(
-    const Camera* __restrict__ camera, float* __restrict__ gaussians, float* __restrict__ sh, uint32_t count,
-    const uint32_t* __restrict__ scene_params, const float* __restrict__ radii, const float* __restrict__ splat_grads,
-    const AdamParams* __restrict__ adam, float* __restrict__ params, float2* __restrict__ moments,
-    float4* __restrict__ stats, float2* __restrict__ aux, float* __restrict__ gaussian_grads,
-    float* __restrict__ sh_grads, uint32_t* __restrict__ error) {
+    const Camera* camera, float* gaussians, float* sh, uint32_t count,
+    const uint32_t* scene_params, const float* radii, const float* splat_grads,
+    const AdamParams* adam, float* params, float2* moments,
+    float4* stats, float2* aux, float* gaussian_grads,
+    float* sh_grads, uint32_t* error) {
+  chain_begin();
   constexpr uint32_t GP = FLOATS_PER_GAUSSIAN + 1;  // a row pitch prime to 32
   __shared__ Camera s_cam;
   __shared__ __align__(16) float s_sh[PBWD_THREADS * SH_REST_FLOATS];  // coefficients, then their gradients
@@ -781,21 +784,19 @@ dg_status launch_preprocess_backward_adam(dg_renderer* r, const AdamParams* adam
   const void* starts[] = {params, moments, ptr_of(r->gaussians), ptr_of(r->sh)};
   for (const void* p : starts)
     DG_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15) == 0, "the training buffers must start 16-byte aligned");
-  DG_LAUNCH(r->ctx, "preprocess_backward_adam",
-            preprocess_backward_adam_kernel<<<ceil_div(r->count, PBWD_THREADS), PBWD_THREADS, 0, r->ctx->stream>>>(
-                typed<const Camera>(r->camera), typed<float>(r->gaussians), typed<float>(r->sh), r->count,
-                typed<uint32_t>(r->scene_params), typed<float>(r->radii), typed<float>(r->grad_splats), adam, params,
-                moments, stats, aux, keep_gradients ? typed<float>(r->grad_gaussians) : nullptr,
-                keep_gradients ? typed<float>(r->grad_sh) : nullptr, r->ctx->device_error));
+  DG_CHAIN(r->ctx, "preprocess_backward_adam", (preprocess_backward_adam_kernel), ceil_div(r->count, PBWD_THREADS), PBWD_THREADS, 0,
+           typed<const Camera>(r->camera), typed<float>(r->gaussians), typed<float>(r->sh), r->count,
+           typed<uint32_t>(r->scene_params), typed<float>(r->radii), typed<float>(r->grad_splats), adam, params,
+           moments, stats, aux, keep_gradients ? typed<float>(r->grad_gaussians) : nullptr,
+           keep_gradients ? typed<float>(r->grad_sh) : nullptr, r->ctx->device_error);
   return DG_OK;
 }
 
 dg_status launch_preprocess_backward(dg_renderer* r) {
-  DG_LAUNCH(r->ctx, "preprocess_backward",
-            preprocess_backward_kernel<<<ceil_div(r->count, PBWD_THREADS), PBWD_THREADS, 0, r->ctx->stream>>>(
-                typed<const Camera>(r->camera), typed<float>(r->gaussians), typed<float>(r->sh), r->count,
-                typed<uint32_t>(r->scene_params), typed<float>(r->splats), typed<float>(r->grad_splats),
-                typed<float>(r->grad_gaussians), typed<float>(r->grad_sh)));
+  DG_CHAIN(r->ctx, "preprocess_backward", (preprocess_backward_kernel), ceil_div(r->count, PBWD_THREADS), PBWD_THREADS, 0,
+           typed<const Camera>(r->camera), typed<float>(r->gaussians), typed<float>(r->sh), r->count,
+           typed<uint32_t>(r->scene_params), typed<float>(r->splats), typed<float>(r->grad_splats),
+           typed<float>(r->grad_gaussians), typed<float>(r->grad_sh));
   return DG_OK;
 }
 

@@ -370,7 +370,7 @@ __device__ __forceinline__ void st_hinted(void* p, float4 v, uint64_t policy) {
 // threads: every 16-byte chunk is issued at once (cp.async), instead of each
 // thread waiting for one load before issuing the next. The caller waits
 // (cp_async_wait_all) and synchronizes the CTA before reading dst.
-__device__ __forceinline__ void stage_floats_async(float* dst, const float* __restrict__ src, uint32_t n) {
+__device__ __forceinline__ void stage_floats_async(float* dst, const float* src, uint32_t n) {
   if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
     const uint32_t vecs = n / 4;
     for (uint32_t k = threadIdx.x; k < vecs; k += blockDim.x) cp_async16(dst + 4 * k, src + 4 * k);
@@ -395,7 +395,7 @@ struct TileMember {
 // its way while the window before is blended.
 struct SplatRecord {
   float4 s0, s1, s2;
-  __device__ __forceinline__ void load(const float* __restrict__ splats, uint32_t index, bool valid) {
+  __device__ __forceinline__ void load(const float* splats, uint32_t index, bool valid) {
     if (!valid) return;
     const float4* s = reinterpret_cast<const float4*>(splats + (size_t)index * FLOATS_PER_SPLAT);
     s0 = s[0];

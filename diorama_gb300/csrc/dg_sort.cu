@@ -88,10 +88,11 @@ constexpr uint32_t HIST_ITEMS = 8;
 #endif
 
 template <int KW>
-__global__ void __launch_bounds__(HIST_THREADS) sort_histogram_kernel(const typename KeyOf<KW>::type* __restrict__ keys,
-                                                                      uint32_t capacity, const uint32_t* __restrict__ count,
+__global__ void __launch_bounds__(HIST_THREADS) sort_histogram_kernel(const typename KeyOf<KW>::type* keys,
+                                                                      uint32_t capacity, const uint32_t* count,
                                                                       uint32_t passes, PassShifts shifts,
-                                                                      uint32_t* __restrict__ hist) {
+                                                                      uint32_t* hist) {
+  chain_begin();
   using K = typename KeyOf<KW>::type;
   __shared__ uint32_t s_hist[MAX_PASSES][RADIX];
   for (uint32_t i = threadIdx.x; i < passes * RADIX; i += HIST_THREADS) s_hist[i / RADIX][i % RADIX] = 0;
@@ -159,11 +160,12 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t* s_
 // prefix work and look-back run on 16 threads instead of 256.
 template <int KW, int DBITS>
 __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
-    sort_pass_kernel(const typename KeyOf<KW>::type* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-                     typename KeyOf<KW>::type* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-                     uint32_t capacity, const uint32_t* __restrict__ count, uint32_t shift,
-                     const uint32_t* __restrict__ pass_hist, uint32_t* __restrict__ status,
-                     uint32_t* __restrict__ ticket, uint32_t* __restrict__ error) {
+    sort_pass_kernel(const typename KeyOf<KW>::type* keys_in, const uint32_t* vals_in,
+                     typename KeyOf<KW>::type* keys_out, uint32_t* vals_out,
+                     uint32_t capacity, const uint32_t* count, uint32_t shift,
+                     const uint32_t* pass_hist, uint32_t* status,
+                     uint32_t* ticket, uint32_t* error) {
+  chain_begin();
   using K = typename KeyOf<KW>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   K* s_keys = reinterpret_cast<K*>(smem);
@@ -371,6 +373,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1)
     sort_cluster_kernel(const typename KeyOf<KW>::type* keys_in, const uint32_t* vals_in,
                         typename KeyOf<KW>::type* keys_out, uint32_t* vals_out, uint32_t capacity,
                         const uint32_t* count, uint32_t passes, PassShifts shifts) {
+  chain_begin();
   using K = typename KeyOf<KW>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   auto& s = *reinterpret_cast<ClusterShared<KW>*>(smem);
@@ -522,18 +525,20 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1)
 }
 
 template <int KW>
-cudaLaunchConfig_t cluster_config(cudaStream_t stream, cudaLaunchAttribute* cluster) {
-  *cluster = {};
-  cluster->id = cudaLaunchAttributeClusterDimension;
-  cluster->val.clusterDim.x = CLUSTER;
-  cluster->val.clusterDim.y = cluster->val.clusterDim.z = 1;
+cudaLaunchConfig_t cluster_config(cudaStream_t stream, cudaLaunchAttribute (&attrs)[2]) {
+  attrs[0] = attrs[1] = {};
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = CLUSTER;
+  attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as DG_CHAIN's
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t config{};
   config.gridDim = CLUSTER;
   config.blockDim = CLUSTER_THREADS;
   config.dynamicSmemBytes = sizeof(ClusterShared<KW>);
   config.stream = stream;
-  config.attrs = cluster;
-  config.numAttrs = 1;
+  config.attrs = attrs;
+  config.numAttrs = 2;
   return config;
 }
 
@@ -541,8 +546,8 @@ cudaLaunchConfig_t cluster_config(cudaStream_t stream, cudaLaunchAttribute* clus
 template <int KW>
 void cluster_init(bool* fits) {
   const auto kernel = sort_cluster_kernel<KW>;
-  cudaLaunchAttribute cluster;
-  const cudaLaunchConfig_t config = cluster_config<KW>(nullptr, &cluster);
+  cudaLaunchAttribute attrs[2];
+  const cudaLaunchConfig_t config = cluster_config<KW>(nullptr, attrs);
   int clusters = 0;
   const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)config.dynamicSmemBytes) == cudaSuccess &&
@@ -560,8 +565,8 @@ dg_status cluster_launch(dg_context* ctx, const SortPlan& plan, void* keys, uint
   PassShifts shifts{};
   for (uint32_t p = 0; p < plan.passes; p++) shifts.shift[p] = plan.shift[p];
   const bool odd = plan.passes & 1;
-  cudaLaunchAttribute cluster;
-  const cudaLaunchConfig_t config = cluster_config<KW>(ctx->stream, &cluster);
+  cudaLaunchAttribute attrs[2];
+  const cudaLaunchConfig_t config = cluster_config<KW>(ctx->stream, attrs);
   cudaError_t err = cudaSuccess;
   DG_LAUNCH(ctx, "sort_cluster",
             err = cudaLaunchKernelEx(&config, sort_cluster_kernel<KW>, static_cast<const K*>(keys),
@@ -610,9 +615,8 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
   uint32_t hist_blocks =
       std::min<uint32_t>(ceil_div(plan.capacity, HIST_THREADS * HIST_ITEMS * DG_HIST_ROUNDS), (uint32_t)ctx->sm_count * 8);
   hist_blocks = std::max(1u, hist_blocks);
-  DG_LAUNCH(ctx, "sort_histogram",
-            sort_histogram_kernel<KW><<<hist_blocks, HIST_THREADS, 0, ctx->stream>>>(
-                static_cast<const K*>(keys), plan.capacity, count, plan.passes, shifts, hist));
+  DG_CHAIN(ctx, "sort_histogram", (sort_histogram_kernel<KW>), hist_blocks, HIST_THREADS, 0,
+           static_cast<const K*>(keys), plan.capacity, count, plan.passes, shifts, hist);
   size_t smem = pass_smem_bytes<KW>();
   K* in_k = static_cast<K*>(keys);
   uint32_t* in_v = values;
@@ -620,10 +624,9 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
   uint32_t* out_v = values_alt;
   for (uint32_t p = 0; p < plan.passes; p++) {
     const auto kernel = plan.narrow_last && p + 1 == plan.passes ? sort_pass_kernel<KW, 4> : sort_pass_kernel<KW, 8>;
-    DG_LAUNCH(ctx, "sort_pass",
-              kernel<<<l.max_tiles, SORT_THREADS, smem, ctx->stream>>>(
-                  in_k, in_v, out_k, out_v, plan.capacity, count, shifts.shift[p], hist + p * RADIX,
-                  status + (size_t)p * l.max_tiles * RADIX, tickets + p, ctx->device_error));
+    DG_CHAIN(ctx, "sort_pass", (kernel), l.max_tiles, SORT_THREADS, smem,
+             in_k, in_v, out_k, out_v, plan.capacity, count, shifts.shift[p], hist + p * RADIX,
+             status + (size_t)p * l.max_tiles * RADIX, tickets + p, ctx->device_error);
     std::swap(in_k, out_k);
     std::swap(in_v, out_v);
   }
