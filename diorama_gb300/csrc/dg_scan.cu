@@ -3,12 +3,14 @@
 // buffer, writing the grand total to `total[0]`.
 //
 // The reference runs a 512-value Blelloch scan per workgroup, recursively, with
-// 2·levels + 1 dispatches. Here it is ONE launch: a single-pass scan with
-// decoupled look-back (Merrill & Garland 2016). Each CTA takes the next tile of
-// 4096 values by an atomic ticket (so the tiles before it are already running),
-// scans it with warp shuffles, publishes its aggregate, and looks back over its
-// predecessors' published values a warp at a time. Every wait is bounded: after
-// SPIN_LIMIT polls it sets DEVICE_ERROR_SCAN_WAIT and stops waiting.
+// 2·levels + 1 dispatches. Here it is two launches (one up to 4096 values): the sums
+// of tiles of 4096 values, then each tile's scan from the sums before it.
+// Where the values are gathered, and for callers that cannot allocate, it is ONE
+// launch: a single-pass scan with decoupled look-back (Merrill & Garland 2016). Each
+// CTA takes the next tile of 4096 values by an atomic ticket (so the tiles before it
+// are already running), scans it with warp shuffles, publishes its aggregate, and looks
+// back over its predecessors' published values a warp at a time. Every wait is bounded:
+// after SPIN_LIMIT polls it sets DEVICE_ERROR_SCAN_WAIT and stops waiting.
 #include "dg_common.cuh"
 #include "dg_scan.cuh"
 
@@ -175,7 +177,7 @@ __device__ __forceinline__ void st_u4_hinted(uint4* p, uint4 v, uint64_t policy)
 // Loads a thread's SCAN_ITEMS consecutive values of tile `tile` (zeros past n),
 // with L2 eviction policy `policy` (l2_policy_*). `full`: all of them are in
 // range and 16-byte aligned.
-__device__ __forceinline__ void load_items(const uint32_t* __restrict__ data, uint32_t n, uint32_t tile,
+__device__ __forceinline__ void load_items(const uint32_t* data, uint32_t n, uint32_t tile,
                                            uint32_t (&v)[SCAN_ITEMS], bool& full, uint64_t& base, uint64_t policy) {
   base = (uint64_t)tile * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
   full = base + SCAN_ITEMS <= n && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
@@ -192,19 +194,22 @@ __device__ __forceinline__ void load_items(const uint32_t* __restrict__ data, ui
   }
 }
 
-// Large scans without a gather: reduce, then re-scan each tile from its prefix, the
+// Without a gather: reduce, then re-scan each tile from its prefix, the
 // sum of the tile sums before it, which each CTA adds up itself from L2 (up to
-// FOLD_MAX_TILES tiles; past that a single-pass scan of the tile sums runs in
-// between). A second read of the values, but no look-back: in one wave of
+// FOLD_MAX_TILES tiles; past that the tile sums are scanned in between, the same way).
+// A second read of the values, but no look-back: in one wave of
 // single-pass CTAs, a tile early in the wave waits on a chain of look-backs about
-// as long as its place in the wave (at 12M values the single-pass scan ran at
-// ~0.3 of the copy rate). The reduce reads the values with an L2 evict-last
+// as long as its place in the wave, and its tickets and states have to be cleared
+// first. Single pass (with the clear) against two levels, in us per scan of many: 6.2 and
+// 3.6 for 5,000 values, 8.4 and 5.0 for 200,000, 14.3 and 9.4 for 1.1M, 17.5 and 8.5 for
+// 2M, 49 and 26 for 12M. The reduce reads the values with an L2 evict-last
 // policy (48 MB at 12M values, well inside L2), so the re-scan reads them from
 // L2, with evict-first loads and stores as their last use.
-__global__ void __launch_bounds__(SCAN_THREADS) scan_reduce_kernel(const uint32_t* __restrict__ data, uint32_t capacity,
-                                                                   const uint32_t* __restrict__ count,
-                                                                   uint32_t* __restrict__ tile_sums) {
+__global__ void __launch_bounds__(SCAN_THREADS) scan_reduce_kernel(const uint32_t* data, uint32_t capacity,
+                                                                   const uint32_t* count,
+                                                                   uint32_t* tile_sums) {
   __shared__ uint32_t s_warp[SCAN_THREADS / 32];
+  chain_begin();
   const uint32_t n = count ? min(*count, capacity) : capacity;
   uint32_t v[SCAN_ITEMS];
   bool full;
@@ -228,12 +233,13 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_reduce_kernel(const uint32_
 // fold: tile_sums holds each tile's sum, and each CTA adds up those before its
 // own; the last tile's CTA writes the grand total. Otherwise tile_sums holds the
 // scanned tile sums (each tile's exclusive prefix) and `total` is not touched.
-__global__ void __launch_bounds__(SCAN_THREADS) scan_tiles_kernel(uint32_t* __restrict__ data, uint32_t capacity,
-                                                                  const uint32_t* __restrict__ count,
-                                                                  const uint32_t* __restrict__ tile_sums, bool fold,
-                                                                  uint32_t* __restrict__ total) {
+__global__ void __launch_bounds__(SCAN_THREADS) scan_tiles_kernel(uint32_t* data, uint32_t capacity,
+                                                                  const uint32_t* count,
+                                                                  const uint32_t* tile_sums, bool fold,
+                                                                  uint32_t* total) {
   __shared__ uint32_t s_warp[SCAN_THREADS / 32];
   __shared__ uint32_t s_part[SCAN_THREADS / 32];
+  chain_begin();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t n = count ? min(*count, capacity) : capacity;
   const uint32_t tiles = (uint32_t)(((uint64_t)n + SCAN_TILE - 1) / SCAN_TILE);  // tiles holding values
@@ -288,10 +294,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_tiles_kernel(uint32_t* __re
   }
 }
 
-// From this many values (and without a gather) the two-level scan runs: at 1.1M
-// values the single pass is faster (16 us against 21), at 12M the two-level one
-// (37 us against 49).
-constexpr uint32_t TWO_LEVEL_MIN = 1u << 21;
 // Up to this many tiles (16.7M values) each re-scanning CTA adds up the tile sums
 // before it itself (at most 16 L2 reads a thread).
 constexpr uint32_t FOLD_MAX_TILES = 4096;
@@ -305,8 +307,7 @@ size_t single_pass_scratch_bytes(uint32_t capacity) {
 
 size_t scan_scratch_bytes(uint32_t capacity) {
   const size_t single = single_pass_scratch_bytes(capacity);
-  if (capacity < TWO_LEVEL_MIN) return single;
-  // Two-level: the tile sums, then the single-pass scan's scratch for scanning them.
+  // Two-level: the tile sums, then the scratch for scanning those.
   const uint32_t tiles = std::max(1u, ceil_div(capacity, SCAN_TILE));
   const size_t sums = ((size_t)tiles * 4 + 255) & ~(size_t)255;
   return std::max(single, sums + single_pass_scratch_bytes(tiles));
@@ -315,15 +316,14 @@ size_t scan_scratch_bytes(uint32_t capacity) {
 dg_status scan_launch(dg_context* ctx, uint32_t* data, uint32_t capacity, const uint32_t* count, uint32_t* total,
                       void* scratch, const uint32_t* gather, const uint32_t* source) {
   uint32_t tiles = std::max(1u, ceil_div(capacity, SCAN_TILE));
-  if (!gather && capacity >= TWO_LEVEL_MIN) {
+  if (!gather) {
     auto* sums = static_cast<uint32_t*>(scratch);
     void* inner = static_cast<char*>(scratch) + (((size_t)tiles * 4 + 255) & ~(size_t)255);
-    DG_LAUNCH(ctx, "scan_reduce",
-              scan_reduce_kernel<<<tiles, SCAN_THREADS, 0, ctx->stream>>>(data, capacity, count, sums));
     const bool fold = tiles <= FOLD_MAX_TILES;
-    if (!fold) DG_TRY(scan_launch(ctx, sums, tiles, nullptr, total, inner));  // tiles < TWO_LEVEL_MIN: single pass
-    DG_LAUNCH(ctx, "scan",
-              scan_tiles_kernel<<<tiles, SCAN_THREADS, 0, ctx->stream>>>(data, capacity, count, sums, fold, total));
+    if (tiles > 1)
+      DG_CHAIN(ctx, "scan_reduce", (scan_reduce_kernel), tiles, SCAN_THREADS, 0, data, capacity, count, sums);
+    if (!fold) DG_TRY(scan_launch(ctx, sums, tiles, nullptr, total, inner));
+    DG_CHAIN(ctx, "scan", (scan_tiles_kernel), tiles, SCAN_THREADS, 0, data, capacity, count, sums, fold, total);
     return DG_OK;
   }
   auto* ticket = static_cast<uint32_t*>(scratch);
