@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(PRE_THREADS) preprocess_views_kernel(
     const Camera* cameras, uint32_t views, const float* gaussians,
     const float* sh, uint32_t count, const uint32_t* scene_params,
     float* splats, uint32_t* tile_counts, uint32_t* rects,
-    uint2* depth_keys, uint32_t* depth_order, uint32_t twl, uint32_t thl) {
+    uint32_t* depth_keys, uint32_t* depth_order, uint32_t twl, uint32_t thl) {
   chain_begin();
   __shared__ float s_sh[PRE_THREADS * SH_REST_FLOATS];
   const uint32_t degree = scene_params[0];
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(PRE_THREADS) preprocess_views_kernel(
       rects[at] = pack_rect(pr.rect);
     else
       tile_counts[at] = pr.tiles();
-    depth_keys[at] = make_uint2(pr.depth_bits, v);
+    depth_keys[at] = pr.depth_bits;
     depth_order[at] = (uint32_t)at;
   }
 }
@@ -1239,7 +1239,7 @@ uint32_t blend_grid(dg_context* ctx, const void* kernel, uint32_t threads, uint3
 
 dg_status views_preprocess_launch(dg_context* ctx, const Camera* cameras, uint32_t views, const float* gaussians,
                                   const float* sh, uint32_t count, const uint32_t* scene_params, float* splats,
-                                  uint32_t* tile_counts, uint32_t* rects, uint2* depth_keys, uint32_t* order,
+                                  uint32_t* tile_counts, uint32_t* rects, uint32_t* depth_keys, uint32_t* order,
                                   BlendShape shape) {
   DG_CHAIN(ctx, "preprocess", (preprocess_views_kernel), ceil_div(count, PRE_THREADS), PRE_THREADS, 0,
            cameras, views, gaussians, sh, count, scene_params, splats, tile_counts, rects, depth_keys, order,

@@ -118,7 +118,7 @@ dg_status blend_forward(dg_context* ctx, const BlendForward& f);
 // The batched views' stages (dg_render.cu; used by dg_views.cu).
 dg_status views_preprocess_launch(dg_context* ctx, const Camera* cameras, uint32_t views, const float* gaussians,
                                   const float* sh, uint32_t count, const uint32_t* scene_params, float* splats,
-                                  uint32_t* tile_counts, uint32_t* rects, uint2* depth_keys, uint32_t* order,
+                                  uint32_t* tile_counts, uint32_t* rects, uint32_t* depth_keys, uint32_t* order,
                                   BlendShape shape);
 dg_status duplicate_sorted_launch(dg_context* ctx, const Camera* camera, const float* splats, const uint32_t* order,
                                   const uint32_t* offsets, uint32_t count, uint32_t per_view, uint32_t view_shift,

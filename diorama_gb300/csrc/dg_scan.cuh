@@ -23,6 +23,7 @@ struct SortPlan {
   uint32_t passes;     // even in the reference's plans, so the result lands back in keys/values
   uint32_t shift[8];   // bit offset of each pass's 8-bit digit within the key
   bool narrow_last;    // the key's bits above the last pass's low 4 are all zero: a 4-bit last pass
+  uint32_t segments = 1;  // runs of `capacity` keys each, back to back, sorted on their own (then without a count)
 };
 SortPlan sort_plan(uint32_t capacity, uint32_t high_bits);
 // u32 keys of which only the low `bits` bits vary (bits a multiple of 16).

@@ -74,6 +74,10 @@ __device__ __forceinline__ void store_status(uint32_t* p, uint32_t v) {
 struct PassShifts {
   uint32_t shift[MAX_PASSES];
 };
+// Words from one segment's digit histograms, and states, to the next one's.
+struct SegmentStates {
+  uint32_t hist, status;
+};
 
 // Digit histograms of every pass from one read of the keys. Each thread takes
 // HIST_ITEMS consecutive keys and counts runs of equal digits in a register,
@@ -95,6 +99,8 @@ __global__ void __launch_bounds__(HIST_THREADS) sort_histogram_kernel(const type
   chain_begin();
   using K = typename KeyOf<KW>::type;
   __shared__ uint32_t s_hist[MAX_PASSES][RADIX];
+  keys += (size_t)blockIdx.y * capacity;  // the segment's
+  hist += (size_t)blockIdx.y * passes * RADIX;
   for (uint32_t i = threadIdx.x; i < passes * RADIX; i += HIST_THREADS) s_hist[i / RADIX][i % RADIX] = 0;
   __syncthreads();
   const uint32_t n = count ? min(*count, capacity) : capacity;
@@ -164,7 +170,7 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
                      typename KeyOf<KW>::type* keys_out, uint32_t* vals_out,
                      uint32_t capacity, const uint32_t* count, uint32_t shift,
                      const uint32_t* pass_hist, uint32_t* status,
-                     uint32_t* ticket, uint32_t* error) {
+                     uint32_t* ticket, SegmentStates states, uint32_t* error) {
   chain_begin();
   using K = typename KeyOf<KW>::type;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -176,6 +182,16 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   uint32_t* s_tmp = s_base + RADIX;
   uint32_t* s_match = reinterpret_cast<uint32_t*>(smem);  // [warp][2][digit], until the keys are placed
   __shared__ uint32_t s_tile;
+
+  // The segment's keys and states.
+  const size_t segment = (size_t)blockIdx.y * capacity;
+  keys_in += segment;
+  vals_in += segment;
+  keys_out += segment;
+  vals_out += segment;
+  pass_hist += (size_t)blockIdx.y * states.hist;
+  status += (size_t)blockIdx.y * states.status;
+  ticket += blockIdx.y * MAX_PASSES;
 
   constexpr uint32_t DIGITS = 1u << DBITS, DMASK = DIGITS - 1u;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -380,6 +396,11 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1)
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = cluster_rank();
   const uint32_t n = count ? min(*count, capacity) : capacity;
   if (n == 0) return;  // in every CTA of the cluster
+  const size_t segment = (size_t)(blockIdx.x / CLUSTER) * capacity;  // the cluster's
+  keys_in += segment;
+  vals_in += segment;
+  keys_out += segment;
+  vals_out += segment;
   cluster_arrive();    // nothing is stored in a CTA that has not started
   const uint32_t seg = ((n + CLUSTER - 1) / CLUSTER + 31) & ~31u;
   // pos / seg = pos * magic >> 32: magic is off by less than seg <= 2^12 parts in 2^32,
@@ -525,7 +546,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1)
 }
 
 template <int KW>
-cudaLaunchConfig_t cluster_config(cudaStream_t stream, cudaLaunchAttribute (&attrs)[2]) {
+cudaLaunchConfig_t cluster_config(uint32_t clusters, cudaStream_t stream, cudaLaunchAttribute (&attrs)[2]) {
   attrs[0] = attrs[1] = {};
   attrs[0].id = cudaLaunchAttributeClusterDimension;
   attrs[0].val.clusterDim.x = CLUSTER;
@@ -533,7 +554,7 @@ cudaLaunchConfig_t cluster_config(cudaStream_t stream, cudaLaunchAttribute (&att
   attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as DG_CHAIN's
   attrs[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t config{};
-  config.gridDim = CLUSTER;
+  config.gridDim = CLUSTER * clusters;
   config.blockDim = CLUSTER_THREADS;
   config.dynamicSmemBytes = sizeof(ClusterShared<KW>);
   config.stream = stream;
@@ -542,20 +563,20 @@ cudaLaunchConfig_t cluster_config(cudaStream_t stream, cudaLaunchAttribute (&att
   return config;
 }
 
-// Clears *fits where the device cannot run the cluster.
+// The clusters that the device runs at once; 0 where it cannot run one.
 template <int KW>
-void cluster_init(bool* fits) {
+int cluster_init() {
   const auto kernel = sort_cluster_kernel<KW>;
   cudaLaunchAttribute attrs[2];
-  const cudaLaunchConfig_t config = cluster_config<KW>(nullptr, attrs);
+  const cudaLaunchConfig_t config = cluster_config<KW>(1, nullptr, attrs);
   int clusters = 0;
   const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)config.dynamicSmemBytes) == cudaSuccess &&
                   cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                  cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) == cudaSuccess && clusters > 0;
-  if (ok) return;
-  *fits = false;
+                  cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) == cudaSuccess;
+  if (ok) return clusters;
   cudaGetLastError();
+  return 0;
 }
 
 template <int KW>
@@ -566,7 +587,7 @@ dg_status cluster_launch(dg_context* ctx, const SortPlan& plan, void* keys, uint
   for (uint32_t p = 0; p < plan.passes; p++) shifts.shift[p] = plan.shift[p];
   const bool odd = plan.passes & 1;
   cudaLaunchAttribute attrs[2];
-  const cudaLaunchConfig_t config = cluster_config<KW>(ctx->stream, attrs);
+  const cudaLaunchConfig_t config = cluster_config<KW>(plan.segments, ctx->stream, attrs);
   cudaError_t err = cudaSuccess;
   DG_LAUNCH(ctx, "sort_cluster",
             err = cudaLaunchKernelEx(&config, sort_cluster_kernel<KW>, static_cast<const K*>(keys),
@@ -590,9 +611,9 @@ ScratchLayout layout_of(const SortPlan& plan) {
   ScratchLayout l;
   l.max_tiles = std::max(1u, ceil_div(plan.capacity, SORT_TILE));
   l.tickets = 0;
-  l.hist = 256;
-  l.status = l.hist + (size_t)plan.passes * RADIX * 4;
-  l.total = l.status + (size_t)plan.passes * l.max_tiles * RADIX * 4;
+  l.hist = ((size_t)plan.segments * MAX_PASSES * 4 + 255) & ~(size_t)255;
+  l.status = l.hist + (size_t)plan.segments * plan.passes * RADIX * 4;
+  l.total = l.status + (size_t)plan.segments * plan.passes * l.max_tiles * RADIX * 4;
   return l;
 }
 
@@ -602,7 +623,7 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
   using K = typename KeyOf<KW>::type;
   // One cluster up to the sizes at which it still beats the passes (figures above
   // sort_cluster_kernel).
-  if (ctx->cluster_sort && plan.capacity <= CLUSTER_KEYS)
+  if (plan.segments <= (uint32_t)ctx->sort_clusters && plan.capacity <= CLUSTER_KEYS)
     return cluster_launch<KW>(ctx, plan, keys, values, keys_alt, values_alt, count);
   ScratchLayout l = layout_of(plan);
   char* s = static_cast<char*>(scratch);
@@ -614,8 +635,9 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
   for (uint32_t p = 0; p < plan.passes; p++) shifts.shift[p] = plan.shift[p];
   uint32_t hist_blocks =
       std::min<uint32_t>(ceil_div(plan.capacity, HIST_THREADS * HIST_ITEMS * DG_HIST_ROUNDS), (uint32_t)ctx->sm_count * 8);
-  hist_blocks = std::max(1u, hist_blocks);
-  DG_CHAIN(ctx, "sort_histogram", (sort_histogram_kernel<KW>), hist_blocks, HIST_THREADS, 0,
+  hist_blocks = std::max(1u, std::min(hist_blocks, ceil_div((uint32_t)ctx->sm_count * 8, plan.segments)));
+  const SegmentStates states{plan.passes * RADIX, plan.passes * l.max_tiles * RADIX};
+  DG_CHAIN(ctx, "sort_histogram", (sort_histogram_kernel<KW>), dim3(hist_blocks, plan.segments), HIST_THREADS, 0,
            static_cast<const K*>(keys), plan.capacity, count, plan.passes, shifts, hist);
   size_t smem = pass_smem_bytes<KW>();
   K* in_k = static_cast<K*>(keys);
@@ -624,9 +646,9 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
   uint32_t* out_v = values_alt;
   for (uint32_t p = 0; p < plan.passes; p++) {
     const auto kernel = plan.narrow_last && p + 1 == plan.passes ? sort_pass_kernel<KW, 4> : sort_pass_kernel<KW, 8>;
-    DG_CHAIN(ctx, "sort_pass", (kernel), l.max_tiles, SORT_THREADS, smem,
+    DG_CHAIN(ctx, "sort_pass", (kernel), dim3(l.max_tiles, plan.segments), SORT_THREADS, smem,
              in_k, in_v, out_k, out_v, plan.capacity, count, shifts.shift[p], hist + p * RADIX,
-             status + (size_t)p * l.max_tiles * RADIX, tickets + p, ctx->device_error);
+             status + (size_t)p * l.max_tiles * RADIX, tickets + p, states, ctx->device_error);
     std::swap(in_k, out_k);
     std::swap(in_v, out_v);
   }
@@ -637,9 +659,7 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
 
 dg_status sort_init(dg_context* ctx) {
   // A device without 16 SMs in one GPC (a partition of one) sorts by passes.
-  ctx->cluster_sort = true;
-  cluster_init<1>(&ctx->cluster_sort);
-  cluster_init<2>(&ctx->cluster_sort);
+  ctx->sort_clusters = std::min(cluster_init<1>(), cluster_init<2>());
   // The pass kernels use more than the default 48 KB of dynamic shared memory.
   DG_CUDA(cudaFuncSetAttribute(sort_pass_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)pass_smem_bytes<1>()));

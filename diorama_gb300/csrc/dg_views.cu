@@ -88,6 +88,15 @@ void view_batch_destroy(dg_view_batch* b) {
 
 namespace {
 
+// Each view's splats by depth, on their own: all views in the same launches. (As one
+// sort of (view, depth) keys, 12 views of 300,000 took 190 us in five passes over 64-bit
+// keys, this way 135.)
+SortPlan depth_sort(uint32_t views, uint32_t count) {
+  SortPlan plan = sort_plan_low_bits(count, 32);
+  plan.segments = views;
+  return plan;
+}
+
 dg_status grow_pairs(dg_view_batch* b, uint32_t capacity) {
   dg_context* ctx = b->ctx;
   DG_TRY(ensure(ctx, &b->values, (size_t)capacity * 4));
@@ -122,13 +131,13 @@ dg_status prepare(dg_view_batch* b, uint32_t views, uint32_t count, uint32_t gri
   b->count = count;
   b->tiles_per_view = tiles_per_view;
   b->pixels = pixels;
-  const SortPlan depth_plan = sort_plan_digits((uint32_t)n, 2, bits_for(views));
+  const SortPlan depth_plan = depth_sort(views, count);
   DG_TRY(ensure(ctx, &b->cameras, (size_t)views * sizeof(Camera)));
   DG_TRY(ensure(ctx, &b->raster_params, 16));
   DG_TRY(ensure(ctx, &b->splats, n * FLOATS_PER_SPLAT * 4));
   DG_TRY(ensure(ctx, &b->tile_counts, n * 4));
-  DG_TRY(ensure(ctx, &b->depth_keys, n * 8));
-  DG_TRY(ensure(ctx, &b->depth_keys_alt, n * 8));
+  DG_TRY(ensure(ctx, &b->depth_keys, n * 4));
+  DG_TRY(ensure(ctx, &b->depth_keys_alt, n * 4));
   DG_TRY(ensure(ctx, &b->order, n * 4));
   DG_TRY(ensure(ctx, &b->order_alt, n * 4));
   DG_TRY(ensure(ctx, &b->depth_scratch, sort_scratch_bytes(depth_plan)));
@@ -162,13 +171,12 @@ dg_status launch_batch(dg_renderer* r, dg_view_batch* b, uchar4* targets, uint32
   DG_TRY(views_preprocess_launch(ctx, typed<Camera>(b->cameras), b->views, typed<float>(r->gaussians),
                                  typed<float>(r->sh), b->count, typed<uint32_t>(r->scene_params),
                                  typed<float>(b->splats), typed<uint32_t>(b->tile_counts),
-                                 b->binned ? typed<uint32_t>(b->tile_counts) : nullptr, typed<uint2>(b->depth_keys),
+                                 b->binned ? typed<uint32_t>(b->tile_counts) : nullptr, typed<uint32_t>(b->depth_keys),
                                  typed<uint32_t>(b->order), b->shape));
-  // (view, depth) keys: 4 passes over the depth bits and one per 8 bits of view.
-  const SortPlan depth_plan = sort_plan_digits(n, 2, bits_for(b->views));
+  const SortPlan depth_plan = depth_sort(b->views, b->count);
   DG_TRY(sort_launch(ctx, depth_plan, b->depth_keys->ptr, typed<uint32_t>(b->order), b->depth_keys_alt->ptr,
                      typed<uint32_t>(b->order_alt), nullptr, b->depth_scratch->ptr));
-  uint32_t* order = depth_plan.passes & 1 ? typed<uint32_t>(b->order_alt) : typed<uint32_t>(b->order);
+  uint32_t* order = typed<uint32_t>(b->order);
   const uint32_t* pair_splats = typed<uint32_t>(b->values);
   if (b->binned) {
     BinLaunch l{};
