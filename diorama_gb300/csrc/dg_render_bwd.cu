@@ -310,6 +310,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
     }
     __syncwarp();
   }
+  // The last warp leaves the counters as it found them, for the next pass.
+  if (lane == 0 && atomicAdd(work_counter + 1, 1u) == gridDim.x * BWD_WARPS - 1u) {
+    work_counter[0] = 0;
+    work_counter[1] = 0;
+  }
 }
 
 #ifndef DG_PBWD_THREADS
@@ -765,7 +770,6 @@ __global__ void DG_PBWD_BOUNDS preprocess_backward_adam_kernel(
 dg_status launch_rasterize_backward(dg_tile_rasterizer* tr, dg_buffer* pixel_grads, dg_buffer* splat_grads) {
   dg_context* ctx = tr->ctx;
   uint32_t* counter = typed<uint32_t>(tr->work) + 2;
-  DG_CUDA(cudaMemsetAsync(counter, 0, sizeof(uint32_t), ctx->stream));
   DG_LAUNCH(ctx, "rasterize_backward",
             rasterize_backward_kernel<<<blend_grid(ctx, (const void*)rasterize_backward_kernel, BWD_THREADS,
                                                     tr->tiles_x * tr->tiles_y * 8u),
