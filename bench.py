@@ -210,13 +210,12 @@ def algorithmic_bytes(name: str, n: int, pairs: int, pixels: int, tiles: int, pa
         "preprocess_backward_adam": 1576.0 * n + 48.0 * drawn,
         "preprocess": 300.0 * n,  # read Gaussian 64 + SH 180, write splat 48 + tile count 4 + radius 4
         "preprocess_backward": (64 + 180 + 48 + 36 + 64 + 180) * float(n),
-        "sort_pass": 24.0 * pairs,  # per pass: read and write 8 B key + 4 B value
-        "sort_histogram": 8.0 * pairs,
-        "scan": 8.0 * n,
-        "duplicate": 20.0 * n + 12.0 * pairs,
-        "find_ranges": 8.0 * pairs + 8.0 * tiles,
-        "loss_ssim": 20.0 * pixels + 48.0 * pixels,
-        "loss_gradient": 20.0 * pixels + 48.0 * pixels + 20.0 * pixels,
+        "sort_pass": 16.0 * n,  # the depths, per pass: read and write 4 B key + 4 B value
+        "sort_histogram": 4.0 * n,
+        "bin_count": 12.0 * n,  # read order and tile rectangle, write the rectangle in order
+        "bin_scatter": 8.0 * n + 4.0 * pairs,
+        "loss_ssim": 20.0 * pixels + 36.0 * pixels + 4.0 * pixels,
+        "loss_gradient": 20.0 * pixels + 36.0 * pixels + 16.0 * pixels,
         "stats": (4 + 8 + 16 + 16) * float(n),
     }.get(name)
 
@@ -642,7 +641,7 @@ def run_sort_stress(args, rank, local):
         "metric": "sort/scan/ranges keys/s", "workload": "1.1M random Gaussians in [-3,3]^3 at 1960x1090, "
         "16x16 tiles, reference-structured tile stage", "keys": keys, "gaussians": n, "tiles": tiles,
         "steps": args.steps, "peak_hbm_gbs": hbm,
-        "sort": frac(sort_bytes, sort_us), "scan": frac(scan_bytes, per.get("scan", 0.0)),
+        "sort": frac(sort_bytes, sort_us), "scan": frac(scan_bytes, per.get("scan_reduce", 0.0) + per.get("scan", 0.0)),
         "scan_12M": frac(8.0 * big, scan12_us),
         "find_ranges": frac(ranges_bytes, per.get("find_ranges", 0.0)),
         "kernels": {k: {"avg_us": round(v, 2), "launches_per_frame": launches[k]} for k, v in per.items()},
