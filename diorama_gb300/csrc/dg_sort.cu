@@ -11,7 +11,7 @@
 // or more dispatches and four barriers per 256-key chunk). Here it is onesweep
 // (Adinets & Merrill 2022): one upfront kernel reads every key once and builds
 // the digit histograms of all passes, then each pass is ONE kernel. A CTA takes
-// the next tile of 3840 keys by ticket, ranks each key within its warp
+// the next tile of 3840 keys (2816 while they are few) by ticket, ranks each key within its warp
 // (stable: warp-striped loads are ranked round by round), publishes its
 // per-digit counts, looks back over earlier tiles' counts (bounded waits), and
 // scatters through shared memory so each digit's run is written contiguously. Up to
@@ -27,18 +27,20 @@ namespace {
 
 constexpr int SORT_THREADS = 256;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
-#ifndef DG_SORT_ITEMS
-#define DG_SORT_ITEMS 15
-#endif
 #ifndef DG_SORT_MIN_BLOCKS
 #define DG_SORT_MIN_BLOCKS 3  // resident CTAs per SM the pass kernel's registers allow
 #endif
-// Keys per thread: 15 at 3 CTAs per SM measured fastest (per in-step pass 29.0 us,
-// 26M keys 1,319 us) against 8 and 11 (36.0, 30.8 us: smaller tiles, longer
-// look-backs) and 19 and 23 at 2 CTAs per SM (31.5, 30.7 us).
-constexpr int SORT_ITEMS = DG_SORT_ITEMS;
-constexpr uint32_t WARP_ITEMS = 32 * SORT_ITEMS;             // 480
-constexpr uint32_t SORT_TILE = SORT_THREADS * SORT_ITEMS;    // 3840
+// Keys per thread: 15 at 3 CTAs per SM measured fastest for many keys (26M keys 1,319
+// us) against 8 and 11 (smaller tiles, longer look-backs) and 19 and 23 at 2 CTAs per
+// SM. While the tiles are few, a pass is one tile's chain of 15 rounds, and 11 are
+// faster: four passes over 100,000 u32 keys 46.8 and 40.9 us, 201,000 48.5 and 40.7,
+// 400,000 48.5 and 48.4, 700,000 62.6 and 56.8, 1.1M 65.0 and 71.8; six over 201,000 u64
+// keys 73.7 and 63.6, 700,000 97.7 and 88.7, 1.1M 109.6 and 111.8 (8 keys: as 11 up to
+// 201,000, slower beyond).
+constexpr int SORT_ITEMS = 15, SORT_ITEMS_FEW = 11;
+constexpr uint32_t FEW_KEYS = 800'000;
+template <int ITEMS>
+constexpr uint32_t SORT_TILE = SORT_THREADS * ITEMS;  // 3840 and 2816
 constexpr uint32_t RADIX = 256;
 constexpr uint32_t FLAG_AGGREGATE = 1u << 30;
 constexpr uint32_t FLAG_PREFIX = 2u << 30;
@@ -164,7 +166,7 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t* s_
 // One pass over digits of DBITS bits (8, or 4 for a last pass whose key bits
 // above it are all zero): fewer ballots per key, and with 16 digits the per-tile
 // prefix work and look-back run on 16 threads instead of 256.
-template <int KW, int DBITS>
+template <int KW, int DBITS, int ITEMS>
 __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
     sort_pass_kernel(const typename KeyOf<KW>::type* keys_in, const uint32_t* vals_in,
                      typename KeyOf<KW>::type* keys_out, uint32_t* vals_out,
@@ -173,10 +175,12 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
                      uint32_t* ticket, SegmentStates states, uint32_t* error) {
   chain_begin();
   using K = typename KeyOf<KW>::type;
+  constexpr uint32_t TILE = SORT_TILE<ITEMS>;
+  static_assert(TILE * 8 >= SORT_WARPS * 2 * RADIX * 4, "the bits lie where the keys and values are placed");
   extern __shared__ __align__(16) unsigned char smem[];
   K* s_keys = reinterpret_cast<K*>(smem);
-  uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + SORT_TILE);
-  uint32_t* s_whist = s_vals + SORT_TILE;          // [warp][digit]
+  uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + TILE);
+  uint32_t* s_whist = s_vals + TILE;          // [warp][digit]
   uint32_t* s_block_start = s_whist + SORT_WARPS * RADIX;
   uint32_t* s_base = s_block_start + RADIX;
   uint32_t* s_tmp = s_base + RADIX;
@@ -196,7 +200,7 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   constexpr uint32_t DIGITS = 1u << DBITS, DMASK = DIGITS - 1u;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t n = count ? min(*count, capacity) : capacity;
-  const uint32_t tiles = (n + SORT_TILE - 1) / SORT_TILE;
+  const uint32_t tiles = (n + TILE - 1) / TILE;
   // The grid covers the capacity; CTAs past the tiles of this call's keys leave at
   // once. The first `tiles` CTAs take the tickets 0..tiles-1, in arrival order.
   if (blockIdx.x >= tiles) return;
@@ -208,14 +212,14 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   if (tile >= tiles) return;
   const uint32_t digit_total = tid < DIGITS ? pass_hist[tid] : 0u;  // on its way while the keys are ranked
 
-  // Load, warp-striped: warp w owns keys [w*480, w*480+480) of the tile, round j
+  // Load, warp-striped: warp w owns 32 * ITEMS consecutive keys of the tile, round j
   // reads 32 consecutive ones, so order within the tile is (warp, round, lane).
-  const uint32_t base = tile * SORT_TILE + warp * WARP_ITEMS + lane;
-  K key[SORT_ITEMS];
-  uint32_t val[SORT_ITEMS];
-  uint32_t rank[SORT_ITEMS];
+  const uint32_t base = tile * TILE + warp * 32 * ITEMS + lane;
+  K key[ITEMS];
+  uint32_t val[ITEMS];
+  uint32_t rank[ITEMS];
 #pragma unroll
-  for (int j = 0; j < SORT_ITEMS; j++) {
+  for (int j = 0; j < ITEMS; j++) {
     uint32_t idx = base + j * 32;
     bool valid = idx < n;
     key[j] = valid ? keys_in[idx] : K(0);
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
   // 1.1M u32 keys 73 -> 65 in four, 100k 49 -> 44. __match_any_sync took 90 for 1.1M.
   uint32_t* my_match = s_match + warp * 2 * DIGITS;
 #pragma unroll
-  for (int j = 0; j < SORT_ITEMS; j++) {
+  for (int j = 0; j < ITEMS; j++) {
     const bool valid = base + j * 32 < n;
     const uint32_t d = (uint32_t)(key[j] >> shift) & DMASK;
     uint32_t* match = my_match + (j & 1) * DIGITS;
@@ -303,7 +307,7 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
 
   // Place each key at its rank within the tile, grouped by digit.
 #pragma unroll
-  for (int j = 0; j < SORT_ITEMS; j++) {
+  for (int j = 0; j < ITEMS; j++) {
     if (base + j * 32 < n) {
       uint32_t dj = (uint32_t)(key[j] >> shift) & DMASK;
       uint32_t pos = s_block_start[dj] + s_whist[warp * DIGITS + dj] + rank[j];
@@ -312,7 +316,7 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
     }
   }
   __syncthreads();
-  const uint32_t here = min(SORT_TILE, n - tile * SORT_TILE);
+  const uint32_t here = min(TILE, n - tile * TILE);
   for (uint32_t k = tid; k < here; k += SORT_THREADS) {
     K kk = s_keys[k];
     uint32_t dk = (uint32_t)(kk >> shift) & DMASK;
@@ -597,19 +601,30 @@ dg_status cluster_launch(dg_context* ctx, const SortPlan& plan, void* keys, uint
   return DG_OK;
 }
 
-template <int KW>
+template <int KW, int ITEMS>
 size_t pass_smem_bytes() {
-  return SORT_TILE * (sizeof(typename KeyOf<KW>::type) + 4) + (SORT_WARPS * RADIX + 2 * RADIX + 32) * 4;
+  return SORT_TILE<ITEMS> * (sizeof(typename KeyOf<KW>::type) + 4) + (SORT_WARPS * RADIX + 2 * RADIX + 32) * 4;
+}
+
+template <int KW, int ITEMS>
+dg_status pass_init() {
+  DG_CUDA(cudaFuncSetAttribute(sort_pass_kernel<KW, 8, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)pass_smem_bytes<KW, ITEMS>()));
+  DG_CUDA(cudaFuncSetAttribute(sort_pass_kernel<KW, 4, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)pass_smem_bytes<KW, ITEMS>()));
+  return DG_OK;
 }
 
 struct ScratchLayout {
   size_t tickets, hist, status, total;
-  uint32_t max_tiles;
+  uint32_t tile, max_tiles;  // keys per tile, tiles per segment
 };
 
 ScratchLayout layout_of(const SortPlan& plan) {
   ScratchLayout l;
-  l.max_tiles = std::max(1u, ceil_div(plan.capacity, SORT_TILE));
+  const bool few = (uint64_t)plan.capacity * plan.segments <= FEW_KEYS;
+  l.tile = few ? SORT_TILE<SORT_ITEMS_FEW> : SORT_TILE<SORT_ITEMS>;
+  l.max_tiles = std::max(1u, ceil_div(plan.capacity, l.tile));
   l.tickets = 0;
   l.hist = ((size_t)plan.segments * MAX_PASSES * 4 + 255) & ~(size_t)255;
   l.status = l.hist + (size_t)plan.segments * plan.passes * RADIX * 4;
@@ -639,13 +654,16 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
   const SegmentStates states{plan.passes * RADIX, plan.passes * l.max_tiles * RADIX};
   DG_CHAIN(ctx, "sort_histogram", (sort_histogram_kernel<KW>), dim3(hist_blocks, plan.segments), HIST_THREADS, 0,
            static_cast<const K*>(keys), plan.capacity, count, plan.passes, shifts, hist);
-  size_t smem = pass_smem_bytes<KW>();
+  const bool few = l.tile == SORT_TILE<SORT_ITEMS_FEW>;
+  const size_t smem = few ? pass_smem_bytes<KW, SORT_ITEMS_FEW>() : pass_smem_bytes<KW, SORT_ITEMS>();
   K* in_k = static_cast<K*>(keys);
   uint32_t* in_v = values;
   K* out_k = static_cast<K*>(keys_alt);
   uint32_t* out_v = values_alt;
   for (uint32_t p = 0; p < plan.passes; p++) {
-    const auto kernel = plan.narrow_last && p + 1 == plan.passes ? sort_pass_kernel<KW, 4> : sort_pass_kernel<KW, 8>;
+    const bool narrow = plan.narrow_last && p + 1 == plan.passes;
+    const auto kernel = few ? (narrow ? sort_pass_kernel<KW, 4, SORT_ITEMS_FEW> : sort_pass_kernel<KW, 8, SORT_ITEMS_FEW>)
+                            : (narrow ? sort_pass_kernel<KW, 4, SORT_ITEMS> : sort_pass_kernel<KW, 8, SORT_ITEMS>);
     DG_CHAIN(ctx, "sort_pass", (kernel), dim3(l.max_tiles, plan.segments), SORT_THREADS, smem,
              in_k, in_v, out_k, out_v, plan.capacity, count, shifts.shift[p], hist + p * RADIX,
              status + (size_t)p * l.max_tiles * RADIX, tickets + p, states, ctx->device_error);
@@ -661,14 +679,10 @@ dg_status sort_init(dg_context* ctx) {
   // A device without 16 SMs in one GPC (a partition of one) sorts by passes.
   ctx->sort_clusters = std::min(cluster_init<1>(), cluster_init<2>());
   // The pass kernels use more than the default 48 KB of dynamic shared memory.
-  DG_CUDA(cudaFuncSetAttribute(sort_pass_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)pass_smem_bytes<1>()));
-  DG_CUDA(cudaFuncSetAttribute(sort_pass_kernel<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)pass_smem_bytes<1>()));
-  DG_CUDA(cudaFuncSetAttribute(sort_pass_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)pass_smem_bytes<2>()));
-  DG_CUDA(cudaFuncSetAttribute(sort_pass_kernel<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)pass_smem_bytes<2>()));
+  DG_TRY((pass_init<1, SORT_ITEMS>()));
+  DG_TRY((pass_init<2, SORT_ITEMS>()));
+  DG_TRY((pass_init<1, SORT_ITEMS_FEW>()));
+  DG_TRY((pass_init<2, SORT_ITEMS_FEW>()));
   return DG_OK;
 }
 
