@@ -21,11 +21,14 @@
 // exactly 0 (zeros are staged there), the same as the WGSL's skipping them.
 //
 // Both are bound by instructions, not by memory (1957x1091: 132 bytes per pixel in
-// 170 us are 1.7 TB/s). Blocks against strips, in us, at 96x96 | 251x187 | 489x273 |
+// 167 us are 1.7 TB/s). Blocks against strips, in us, at 96x96 | 251x187 | 489x273 |
 // 980x545 | 1957x1091: gradient 8.3 | 10.1 | 14.2 | 33.0 | 127 with blocks, 10.2 | 10.6 |
 // 14.5 | 24.8 | 62 with strips. The SSIM pass has five maps to keep sums of, not three,
 // and spills: 12.2 | 13.2 | 17.4 | 36 | 110 with blocks, 22 | 22 | 25 | 45 | 132 with
-// strips (blocks of 16x32 pixels with two rows per thread: 15 | 17 | 17 | 35 | 109).
+// strips (blocks of 16x32 pixels with two rows per thread: 15 | 17 | 17 | 35 | 109; of
+// 16x16 with two rows and half the threads 13.5 | 17 | 18 | 34 | 119). Without bank
+// conflicts in its horizontal pass, and the halo's loads ahead of the table of bytes, it
+// takes 11 | 13 | 17.4 | 34 | 105.
 // The partials lie in planes of their own, which a strip's warp reads in whole lines.
 //
 // The same ssim_kernel also measures held-out renders (PSNR and SSIM of the
@@ -41,6 +44,7 @@ constexpr int TAPS = 2 * HALO + 1;
 // ssim_kernel: a CTA's block of pixels and its halo.
 constexpr int LT = 16;
 constexpr int LS = LT + 2 * HALO;  // 26
+constexpr int SSIM_THREADS = LT * LT;
 // gradient_kernel: a strip's columns (a lane each) and its halo; a warp per channel.
 constexpr int COLS = 32;
 constexpr int SPAN = COLS + 2 * HALO;  // 42
@@ -55,19 +59,14 @@ struct Window {
   float w[6];
 };
 
-__device__ __forceinline__ float3 load_x(const float4* rendered, int w, int h, int x, int y, bool quantize) {
-  if (x < 0 || y < 0 || x >= w || y >= h) return make_float3(0.f, 0.f, 0.f);
-  float4 v = rendered[(size_t)y * w + x];
-  if (quantize) {
-    // src/trainer.ts:381: round(min(1, max(0, v)) * 255) / 255, in double as the
-    // TypeScript does, then stored as float32.
-    auto q = [](float c) {
-      double d = rint((double)fminf(1.0f, fmaxf(0.0f, c)) * 255.0);
-      return __double2float_rn(d / 255.0);
-    };
-    return make_float3(q(v.x), q(v.y), q(v.z));
-  }
-  return make_float3(v.x, v.y, v.z);
+// src/trainer.ts:381: round(min(1, max(0, v)) * 255) / 255, in double as the
+// TypeScript does, then stored as float32.
+__device__ __forceinline__ float3 quantized(float4 v) {
+  auto q = [](float c) {
+    double d = rint((double)fminf(1.0f, fmaxf(0.0f, c)) * 255.0);
+    return __double2float_rn(d / 255.0);
+  };
+  return make_float3(q(v.x), q(v.y), q(v.z));
 }
 
 // A byte's value as float, v / 255: the loss's float quotient, or for metrics
@@ -86,12 +85,6 @@ __device__ __forceinline__ void fill_unorm8(float* table, bool exact_quotient, u
 // The weight of tap k - 5.
 __device__ __forceinline__ int tap_weight(int k) { return k < HALO ? HALO - k : k - HALO; }
 
-__device__ __forceinline__ float3 load_y(const uchar4* target, int w, int h, int x, int y, const float* unorm) {
-  if (x < 0 || y < 0 || x >= w || y >= h) return make_float3(0.f, 0.f, 0.f);
-  uchar4 t = target[(size_t)y * w + x];
-  return make_float3(unorm[t.x], unorm[t.y], unorm[t.z]);
-}
-
 // Moments, both blurs and the SSIM partials for one 16x16 block. mode 0 (loss):
 // writes each channel's partials, (dS/dmu_x, dS/dE[x^2]) and dS/dE[xy], in planes of
 // their own (`partials`: 3 planes of float2, then 3 of float, one value per pixel),
@@ -100,29 +93,45 @@ __device__ __forceinline__ float3 load_y(const uchar4* target, int w, int h, int
 //
 // The x and y sums of each blur, and the x^2 and y^2 ones, run as pairs through
 // packed FP32 fused multiply-adds (F2): each lane is the scalar fmaf sum.
-__global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ rendered,
+__global__ void __launch_bounds__(SSIM_THREADS, 5) ssim_kernel(const float4* __restrict__ rendered,
                                                    const uchar4* const* __restrict__ target_slot, int w, int h,
                                                    Window win, float* __restrict__ partials,
                                                    float* __restrict__ pixel_loss, int mode,
                                                    double* __restrict__ sums) {
-  __shared__ float2 s_xy[LS][LS][3];   // (x, y) per halo pixel and channel
-  __shared__ float2 s_h01[LS][LT][3];  // horizontal blurs of x and y
-  __shared__ float2 s_h23[LS][LT][3];  // of x^2 and y^2
-  __shared__ float s_h4[LS][LT][3];    // of xy
-  __shared__ double s_red[2][8];
+  // Rows of odd length: the lanes of the horizontal pass read and write two rows or
+  // channels at once, eight pairs of columns each, without bank conflicts.
+  __shared__ float2 s_xy[LS][LS * 3 + 1];   // (x, y) per halo pixel and channel
+  __shared__ float2 s_h01[LS][LT * 3 + 1];  // horizontal blurs of x and y
+  __shared__ float2 s_h23[LS][LT * 3 + 1];  // of x^2 and y^2
+  __shared__ float s_h4[LS][LT * 3 + 1];    // of xy
+  __shared__ double s_red[2][SSIM_THREADS / 32];
   __shared__ float s_unorm[256];
   const uchar4* target = *target_slot;
   const int x0 = blockIdx.x * LT - HALO, y0 = blockIdx.y * LT - HALO;
   const bool metrics = mode == 1;
-  fill_unorm8(s_unorm, metrics, 256);
+  // The halo's pixels are on their way while the table is filled.
+  constexpr int EACH = (LS * LS + SSIM_THREADS - 1) / SSIM_THREADS;
+  float4 px[EACH];
+  uchar4 py[EACH];
+#pragma unroll
+  for (int u = 0; u < EACH; u++) {
+    const int k = threadIdx.x + u * SSIM_THREADS, x = x0 + k % LS, y = y0 + k / LS;
+    const bool in = k < LS * LS && x >= 0 && y >= 0 && x < w && y < h;
+    px[u] = in ? rendered[(size_t)y * w + x] : make_float4(0.f, 0.f, 0.f, 0.f);
+    py[u] = in ? target[(size_t)y * w + x] : make_uchar4(0, 0, 0, 0);
+  }
+  fill_unorm8(s_unorm, metrics, SSIM_THREADS);
   __syncthreads();
-  for (int k = threadIdx.x; k < LS * LS; k += 256) {
-    const int ly = k / LS, lx = k % LS;
-    float3 xv = load_x(rendered, w, h, x0 + lx, y0 + ly, metrics);
-    float3 yv = load_y(target, w, h, x0 + lx, y0 + ly, s_unorm);
-    s_xy[ly][lx][0] = make_float2(xv.x, yv.x);
-    s_xy[ly][lx][1] = make_float2(xv.y, yv.y);
-    s_xy[ly][lx][2] = make_float2(xv.z, yv.z);
+#pragma unroll
+  for (int u = 0; u < EACH; u++) {
+    const int k = threadIdx.x + u * SSIM_THREADS;
+    if (k >= LS * LS) break;
+    // Past the image both are 0, as the table's entry for 0 is.
+    const float3 xv = metrics ? quantized(px[u]) : make_float3(px[u].x, px[u].y, px[u].z);
+    float2* to = &s_xy[k / LS][3 * (k % LS)];
+    to[0] = make_float2(xv.x, s_unorm[py[u].x]);
+    to[1] = make_float2(xv.y, s_unorm[py[u].y]);
+    to[2] = make_float2(xv.z, s_unorm[py[u].z]);
   }
   F2 wp[6];
 #pragma unroll
@@ -131,15 +140,15 @@ __global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ re
   // Horizontal pass over every halo row, for the 16 output columns, two adjacent
   // columns per item: their 11-tap windows share 10 halo values, read (and
   // squared) once. Each column's sums still run over its taps -5..5 in order.
-  for (int k = threadIdx.x; k < LS * (LT / 2) * 3; k += 256) {
-    const int ch = k % 3, col = 2 * ((k / 3) % (LT / 2)), row = k / (3 * (LT / 2));
+  for (int k = threadIdx.x; k < LS * (LT / 2) * 3; k += SSIM_THREADS) {
+    const int col = 2 * (k % (LT / 2)), ch = k / (LT / 2) % 3, row = k / (3 * (LT / 2));
     F2 a01 = f2(0.f, 0.f), a23 = f2(0.f, 0.f), b01 = a01, b23 = a01;
     float a4 = 0.f, b4 = 0.f;
     // Taps past the image read the halo's zeros and add exactly 0: the same sums
     // as skipping them, without a branch per tap.
 #pragma unroll
     for (int t = -HALO; t <= HALO + 1; t++) {  // halo column col + HALO + t
-      const F2 xy = f2_load(&s_xy[row][col + HALO + t][ch]);
+      const F2 xy = f2_load(&s_xy[row][3 * (col + HALO + t) + ch]);
       const F2 sq = f2_mul(xy, xy);
       const float pr = f2_lo(xy) * f2_hi(xy);
       if (t <= HALO) {  // column col, tap t
@@ -155,12 +164,12 @@ __global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ re
         b4 = fmaf(win.w[at], pr, b4);
       }
     }
-    f2_store(&s_h01[row][col][ch], a01);
-    f2_store(&s_h23[row][col][ch], a23);
-    s_h4[row][col][ch] = a4;
-    f2_store(&s_h01[row][col + 1][ch], b01);
-    f2_store(&s_h23[row][col + 1][ch], b23);
-    s_h4[row][col + 1][ch] = b4;
+    f2_store(&s_h01[row][3 * col + ch], a01);
+    f2_store(&s_h23[row][3 * col + ch], a23);
+    s_h4[row][3 * col + ch] = a4;
+    f2_store(&s_h01[row][3 * col + 3 + ch], b01);
+    f2_store(&s_h23[row][3 * col + 3 + ch], b23);
+    s_h4[row][3 * col + 3 + ch] = b4;
   }
   __syncthreads();
   const int lx = threadIdx.x % LT, ly = threadIdx.x / LT;
@@ -176,16 +185,16 @@ __global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ re
 #pragma unroll
       for (int k = 0; k < TAPS; k++) {  // rows past the image were blurred to 0
         const int at = tap_weight(k);
-        m01 = f2_fma(wp[at], f2_load(&s_h01[ly + k][lx][ch]), m01);
-        m23 = f2_fma(wp[at], f2_load(&s_h23[ly + k][lx][ch]), m23);
-        m4 = fmaf(win.w[at], s_h4[ly + k][lx][ch], m4);
+        m01 = f2_fma(wp[at], f2_load(&s_h01[ly + k][3 * lx + ch]), m01);
+        m23 = f2_fma(wp[at], f2_load(&s_h23[ly + k][3 * lx + ch]), m23);
+        m4 = fmaf(win.w[at], s_h4[ly + k][3 * lx + ch], m4);
       }
       const float mx = f2_lo(m01), my = f2_hi(m01);
       const float vx = f2_lo(m23) - mx * mx, vy = f2_hi(m23) - my * my, cxy = m4 - mx * my;
       const float a1 = 2.0f * mx * my + C1, a2 = 2.0f * cxy + C2;
       const float b1 = mx * mx + my * my + C1, b2 = vx + vy + C2;
       const float s = a1 * a2 / (b1 * b2);
-      const float2 xy = s_xy[ly + HALO][lx + HALO][ch];
+      const float2 xy = s_xy[ly + HALO][3 * (lx + HALO) + ch];
       if (metrics) {
         s_sum += (double)s;
         const double d = (double)xy.x - (double)xy.y;
@@ -212,7 +221,7 @@ __global__ void __launch_bounds__(256) ssim_kernel(const float4* __restrict__ re
     __syncthreads();
     if (threadIdx.x == 0) {
       double a = 0, b = 0;
-      for (int k = 0; k < 8; k++) {
+      for (int k = 0; k < SSIM_THREADS / 32; k++) {
         a += s_red[0][k];
         b += s_red[1][k];
       }
@@ -387,7 +396,7 @@ dg_status loss_launch(dg_training_loss* l, dg_buffer* rendered) {
   const int w = (int)l->width, h = (int)l->height, rows = strip_rows(ctx, l->width, l->height);
   const auto* target = typed<const uchar4* const>(l->target_slot);
   DG_LAUNCH(ctx, "loss_ssim",
-            ssim_kernel<<<dim3(ceil_div(w, LT), ceil_div(h, LT)), 256, 0, ctx->stream>>>(
+            ssim_kernel<<<dim3(ceil_div(w, LT), ceil_div(h, LT)), SSIM_THREADS, 0, ctx->stream>>>(
                 typed<float4>(rendered), target, w, h, win, typed<float>(l->partials), typed<float>(l->pixel_loss), 0,
                 nullptr));
   DG_LAUNCH(ctx, "loss_gradient",
@@ -416,7 +425,7 @@ dg_status metrics_launch(dg_context* ctx, dg_buffer* rendered, dg_buffer* target
   const Window win = window_weights();
   dim3 grid(ceil_div(width, LT), ceil_div(height, LT));
   DG_LAUNCH(ctx, "metrics_ssim",
-            ssim_kernel<<<grid, 256, 0, ctx->stream>>>(typed<float4>(rendered),
+            ssim_kernel<<<grid, SSIM_THREADS, 0, ctx->stream>>>(typed<float4>(rendered),
                                                        typed<const uchar4* const>(target_slot), (int)width,
                                                        (int)height, win, nullptr, nullptr, 1, sums_device));
   return DG_OK;
