@@ -197,6 +197,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
     const uint2 run = ranges[tile];
     const uint32_t chunk_lo = run.x + chunk * CHUNK, chunk_hi = min(chunk_lo + CHUNK, run.y);
     const uint32_t boundary = (chunk + 1u) * CHUNK;  // the chunk's end, relative to run.x
+    // Lane k's mask word, of window k of the chunk; those past the walk hold anything.
+    static_assert(CHUNK / 32 <= 32, "a chunk's mask words fit in the warp's lanes");
+    uint32_t word = 0;
+    if (chunk_lo + lane * 32u < chunk_hi)
+      word = blend_mask[mask_at(tile, tiles, run.x, chunk * (CHUNK / 32u) + lane, block)];
     float4 color = make_float4(0.f, 0.f, 0.f, 0.f), pg = color;
     uint32_t last = 0;
     if (inside) {
@@ -208,16 +213,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
     // Splats at or past the warp's largest `last` contribute nothing to it.
     const uint32_t end_all = min(chunk_hi, run.x + __reduce_max_sync(0xffffffffu, last));
     if (end_all <= chunk_lo) continue;
-    // The chunk's blended entries: lane k has the mask word of window k (at most
-    // CHUNK / 32), and the entries in the windows behind it.
-    static_assert(CHUNK / 32 <= 32, "a chunk's mask words fit in the warp's lanes");
+    // The chunk's blended entries: lane k has those of window k, and counts those behind it.
     const uint32_t windows = (end_all - chunk_lo + 31u) / 32u;
-    uint32_t word = 0;
-    if (lane < windows) {
-      word = blend_mask[mask_at(tile, tiles, run.x, chunk * (CHUNK / 32u) + lane, block)];
-      const uint32_t left = end_all - chunk_lo - lane * 32u;
-      if (left < 32u) word &= (1u << left) - 1u;
-    }
+    if (lane >= windows) word = 0;
+    const uint32_t left = end_all - chunk_lo - lane * 32u;
+    if (lane < windows && left < 32u) word &= (1u << left) - 1u;
     uint32_t behind_it = __popc(word);
 #pragma unroll
     for (uint32_t d = 1; d < 32; d <<= 1) {

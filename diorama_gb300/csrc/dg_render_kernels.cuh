@@ -291,7 +291,7 @@ struct BlendPair {
   ulonglong2 ab;  // 0.5 a, b
   ulonglong2 cl;  // 0.5 c, and the bits that those of -power must be below for the
                   // alpha to reach 1/255 (those of -cutoff, plus 1)
-  unsigned long long opacity, pad;
+  unsigned long long opacity, pad[3];  // 80 bytes: 16 pairs lie in all banks
 };
 struct BlendStage {
   BlendPair pair[16];
