@@ -760,6 +760,9 @@ __device__ __forceinline__ void list_items(uint2* __restrict__ items, uint32_t* 
 // chains bound it (1.1M at 980x545, lists up to 30,000) 295 both ways. COOP_LOAD 1 and 4,
 // COOP_CHAIN 8 and 12 and PLAN_DEPTH 8, 32 and 64 were slower on one scene or another.
 constexpr float COOP_LOAD = 1.5f, COOP_CHAIN = 5.0f;
+// Warp 0's word that all pixels have stopped, by round: a warp reads round r's after the
+// round's barrier, while warp 0 may be at the end of round r + 1 already, and in none later.
+constexpr uint32_t STOP_WORDS = 2;
 template <uint32_t TWL, uint32_t THL>
 __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
     const Camera* __restrict__ camera, const float4* __restrict__ raster_params, const float* __restrict__ splats,
@@ -774,7 +777,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
   __shared__ float s_alpha[2][PRODUCERS][32][32];
   __shared__ float4 s_qcolor[2][PRODUCERS][32];
   __shared__ uint32_t s_qlive[2][PRODUCERS];
-  __shared__ uint32_t s_item, s_stop, s_done;  // s_done: warp 0's pixels that have stopped
+  __shared__ uint32_t s_item, s_stop[STOP_WORDS], s_done;  // s_done: warp 0's pixels that have stopped
   constexpr uint32_t BLOCK_SHIFT = 3u + TWL + THL, BLOCK_MASK = (1u << BLOCK_SHIFT) - 1u;
   constexpr bool MEMBER = TWL + THL > 0;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -817,7 +820,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
     if (threadIdx.x == 0) {
       s_item = atomicAdd(&counters[0], 1u);
       s_done = 0;
-      s_stop = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < STOP_WORDS; k++) s_stop[k] = 0;
     }
     __syncthreads();
     const uint32_t item = s_item;
@@ -903,10 +907,10 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
           const uint32_t done = __ballot_sync(0xffffffffu, pb.done);
           if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&s_done) = done;
         }
-        if (lane == 0) s_stop = s_done == 0xffffffffu;
+        if (lane == 0) s_stop[r % STOP_WORDS] = s_done == 0xffffffffu;
       }
       __syncthreads();
-      if (s_stop) break;
+      if (s_stop[r % STOP_WORDS]) break;
     }
     if (warp == 0) {
       write_pixel(it, pb, last, bg, target, pixel_color, pixel_last);
