@@ -692,23 +692,13 @@ __device__ __forceinline__ void write_pixel(const BlendItem& it, const PixelBlen
   if (target) target[it.pixel] = make_uchar4(to_unorm8(fr), to_unorm8(fg), to_unorm8(fb), 255);
 }
 
-// The backward pass's items of a block whose pixels have ended: the chunks of its list
-// up to the last entry that one of them blended.
-__device__ __forceinline__ void list_items(uint2* __restrict__ items, uint32_t* __restrict__ item_count,
-                                           uint32_t item_room, uint32_t tile, uint32_t block, uint32_t lane,
-                                           uint32_t last) {
-  if (!items) return;
+// For the backward pass: how many entries of a block's list its walk has to take, up to
+// the last one that a pixel of it blended.
+__device__ __forceinline__ void save_walked(uint32_t* __restrict__ walked, uint32_t tile, uint32_t block, uint32_t lane,
+                                            uint32_t last) {
+  if (!walked) return;
   const uint32_t most = __reduce_max_sync(0xffffffffu, last);
-  // Whole chunks are in the first class, the rest of the list in its own.
-  const uint32_t whole = most / CHUNK, rest = most % CHUNK;
-  uint32_t at = 0;
-  if (lane == 0 && whole) at = atomicAdd(item_count, whole);
-  if (lane == 1 && rest) at = atomicAdd(item_count + item_class(rest), 1u);
-  if (lane == 1 && rest && at < item_room)
-    items[(size_t)item_class(rest) * item_room + at] = make_uint2(tile * 8u + block, whole);
-  at = __shfl_sync(0xffffffffu, at, 0);
-  for (uint32_t k = lane; k < whole; k += 32u)
-    if (at + k < item_room) items[at + k] = make_uint2(tile * 8u + block, k);
+  if (lane == 0) walked[tile * 8u + block] = most;
 }
 
 // src/shaders/rasterize.wgsl:32-100. The work is split into items, one per (tile,
@@ -769,7 +759,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
     const uint32_t* __restrict__ pair_splats, const uint2* __restrict__ ranges, const uint32_t* __restrict__ plan,
     uint32_t tiles_per_view, uint32_t coop_min, uchar4* __restrict__ target, float4* __restrict__ pixel_color,
     uint32_t* __restrict__ pixel_last, float4* __restrict__ checkpoints, uint32_t* __restrict__ blend_mask,
-    uint2* __restrict__ items, uint32_t* __restrict__ item_count, uint32_t item_room, uint32_t* __restrict__ counters,
+    uint32_t* __restrict__ walked, uint32_t* __restrict__ counters,
     bool cut_in_record) {
   __shared__ BlendStage stages[FWD_WARPS];
   // Cooperative blending, double-buffered by round: each producer's queued entries
@@ -914,7 +904,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
     }
     if (warp == 0) {
       write_pixel(it, pb, last, bg, target, pixel_color, pixel_last);
-      list_items(items, item_count, item_room, it.tile, block, lane, last);
+      save_walked(walked, it.tile, block, lane, last);
     }
   }
 
@@ -975,7 +965,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 4) rasterize_kernel(
       __syncwarp();
     }
     write_pixel(it, pb, last, bg, target, pixel_color, pixel_last);
-    list_items(items, item_count, item_room, it.tile, block, lane, last);
+    save_walked(walked, it.tile, block, lane, last);
   }
 }
 
@@ -1207,8 +1197,7 @@ dg_status launch_rasterize(dg_tile_rasterizer* tr, dg_buffer* target) {
   f.tiles = f.tiles_per_view = tr->tiles_x * tr->tiles_y;
   f.coop_min = tr->coop_min;
   f.plan = typed<uint32_t>(tr->work_plan);
-  f.items = typed<uint2>(tr->items);
-  f.item_room = (uint32_t)(tr->items->bytes / sizeof(uint2) / ITEM_CLASSES);
+  f.walked = typed<uint32_t>(tr->walked);
   f.target = target ? typed<uchar4>(target) : nullptr;
   f.pixel_color = typed<float4>(tr->pixel_color);
   f.pixel_last = typed<uint32_t>(tr->pixel_last);
@@ -1227,15 +1216,14 @@ static dg_status launch_rasterize_kernel(dg_context* ctx, const BlendForward& f)
   DG_LAUNCH(ctx, "rasterize",
             kernel<<<blend_grid(ctx, (const void*)kernel, FWD_THREADS, items), FWD_THREADS, 0, ctx->stream>>>(
                 f.camera, f.raster_params, f.splats, f.pair_splats, f.ranges, f.plan, f.tiles_per_view, f.coop_min, f.target,
-                f.pixel_color, f.pixel_last, f.checkpoints, f.blend_mask, f.items, f.plan + PLAN_ITEMS, f.item_room,
-                f.counters, f.splat_cutoffs));
+                f.pixel_color, f.pixel_last, f.checkpoints, f.blend_mask, f.walked, f.counters, f.splat_cutoffs));
   return DG_OK;
 }
 
 dg_status blend_forward(dg_context* ctx, const BlendForward& f) {
   const BlendShape sh = f.shape;
   DG_REQUIRE(sh.twl <= MAX_BLEND_TILE_LOG2 && sh.thl <= MAX_BLEND_TILE_LOG2, "blend tiles of at most 2 x 2 tiles");
-  DG_REQUIRE(sh.twl + sh.thl == 0 || (!f.checkpoints && !f.blend_mask && !f.items),
+  DG_REQUIRE(sh.twl + sh.thl == 0 || (!f.checkpoints && !f.blend_mask && !f.walked),
              "blend tiles larger than 16x16 have no backward pass");
   if (!f.cleared) {
     DG_CUDA(cudaMemsetAsync(f.counters, 0, 16, ctx->stream));
@@ -1300,6 +1288,7 @@ static dg_status ensure_plan(dg_tile_rasterizer* tr) {
     dg_buffer** buf;
     size_t bytes;
   } needs[] = {{&tr->work_plan, plan_words(tiles) * 4},
+               {&tr->walked, tiles * 8 * 4},
                {&tr->items, (tiles + slots) * 8 * ITEM_CLASSES * sizeof(uint2)},
                {&tr->checkpoints, slots * 8 * 32 * 16},
                {&tr->blend_mask, (tiles + (size_t)tr->pair_capacity / 32 + 1) * 8 * 4}};
@@ -1368,12 +1357,6 @@ dg_status rasterizer_queue_readback(dg_tile_rasterizer* tr) {
   DG_CUDA(cudaEventRecord(tr->readback_events[slot], tr->ctx->stream));
   tr->readback_head++;
   return DG_OK;
-}
-
-dg_status rasterizer_launch_backward(dg_tile_rasterizer* tr, dg_buffer* pixel_grads, dg_buffer* splat_grads) {
-  dg_context* ctx = tr->ctx;
-  DG_CUDA(cudaMemsetAsync(splat_grads->ptr, 0, (size_t)tr->count * SPLAT_GRADS * 4, ctx->stream));
-  return launch_rasterize_backward(tr, pixel_grads, splat_grads);
 }
 
 // ------------------------------------------------------------ GaussianRenderer
@@ -1449,7 +1432,7 @@ dg_status renderer_ensure_gradients(dg_renderer* r) {
 }
 
 dg_status renderer_launch_backward(dg_renderer* r, dg_buffer* pixel_grads, bool write_gaussian_grads) {
-  DG_TRY(rasterizer_launch_backward(r->rasterizer, pixel_grads, r->grad_splats));
+  DG_TRY(launch_rasterize_backward(r->rasterizer, pixel_grads, r->grad_splats));
   if (!write_gaussian_grads || r->count == 0) return DG_OK;
   return launch_preprocess_backward(r);
 }
@@ -1487,7 +1470,7 @@ dg_status dg_tile_rasterizer_encode_backward(dg_tile_rasterizer* tr, const float
   if (!tr->pixel_color || !tr->ranges) return fail(DG_ERROR_STATE, "Encode a frame before its backward pass.");
   DG_REQUIRE(splat_grads->bytes >= (uint64_t)tr->count * SPLAT_GRADS * 4, "splat gradient buffer too small");
   DG_REQUIRE(pixel_grads->bytes >= (uint64_t)tr->pixel_count * 16, "pixel gradient buffer too small");
-  return rasterizer_launch_backward(tr, pixel_grads, splat_grads);
+  return launch_rasterize_backward(tr, pixel_grads, splat_grads);
 }
 
 dg_status dg_tile_rasterizer_after_submit(dg_tile_rasterizer* tr, int32_t wait) {
@@ -1510,7 +1493,8 @@ dg_status dg_tile_rasterizer_destroy(dg_tile_rasterizer* tr) {
   for (dg_buffer* b : {tr->tile_offsets, tr->scan_total, tr->scan_scratch, tr->raster_params, tr->keys, tr->values,
                        tr->keys_alt, tr->values_alt, tr->sort_scratch, tr->ranges, tr->pixel_color, tr->pixel_last,
                        tr->depth_keys, tr->depth_values, tr->depth_keys_alt, tr->depth_values_alt, tr->depth_scratch,
-                       tr->counts_sorted, tr->bin_scratch, tr->keys64, tr->work, tr->work_plan, tr->items, tr->checkpoints,
+                       tr->counts_sorted, tr->bin_scratch, tr->keys64, tr->work, tr->work_plan, tr->walked, tr->items,
+                       tr->checkpoints,
                        tr->blend_mask})
     free_buffer(b);
   for (cudaEvent_t e : tr->readback_events)

@@ -55,7 +55,8 @@ struct dg_tile_rasterizer {
   dg_buffer* keys64;         // the reference's 64-bit sorted keys, rebuilt on request
   dg_buffer* work;           // item counters of the blend kernels
   dg_buffer* work_plan;    // tile order and counts (plan_kernel, dg_render.cu)
-  dg_buffer* items;        // the backward pass's (tile, block) and chunk, listed by the forward pass
+  dg_buffer* walked;       // entries that the backward pass walks of each (tile, block)'s list
+  dg_buffer* items;        // the backward pass's (tile, block) and chunk
   dg_buffer* checkpoints;  // the forward's per-chunk pixel states
   dg_buffer* blend_mask;   // which entries each 8x4 block blended (dg_render_kernels.cuh, mask_at)
   uint32_t coop_min;      // the fewest entries of a tile that a whole CTA may blend
@@ -73,7 +74,6 @@ dg_status rasterizer_launch(dg_tile_rasterizer* tr, dg_buffer* target, bool coun
 dg_status rasterizer_queue_readback(dg_tile_rasterizer* tr);
 // Grows the pair buffers to 2^ceil(log2(1.25 * pairs)) if pairs exceed them.
 dg_status rasterizer_reserve_pairs(dg_tile_rasterizer* tr, uint64_t pairs);
-dg_status rasterizer_launch_backward(dg_tile_rasterizer* tr, dg_buffer* pixel_grads, dg_buffer* splat_grads);
 // own_splats: `splats` is written by this build's preprocess (blend cutoffs in slot 7).
 dg_status rasterizer_create(dg_context* ctx, dg_buffer* camera, dg_buffer* splats, uint32_t count,
                             uint32_t initial_pair_capacity, bool depth_first, bool own_splats,
@@ -92,7 +92,7 @@ struct BlendShape {
 constexpr uint32_t MAX_BLEND_TILE_LOG2 = 1;  // blend tiles of up to 2 x 2 16x16 tiles
 
 // The forward blend (plan + rasterize kernels) over `tiles` tiles of
-// tiles_per_view each; checkpoints, blend_mask and items may be NULL when no
+// tiles_per_view each; checkpoints, blend_mask and walked may be NULL when no
 // backward pass follows, and must be with blend tiles larger than 16x16.
 struct BlendForward {
   const Camera* camera;
@@ -102,8 +102,7 @@ struct BlendForward {
   const uint2* ranges;
   uint32_t tiles, tiles_per_view, coop_min;
   uint32_t* plan;
-  uint2* items;
-  uint32_t item_room;  // that items holds
+  uint32_t* walked;
   uchar4* target;
   float4* pixel_color;
   uint32_t* pixel_last;

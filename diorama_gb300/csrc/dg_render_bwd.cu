@@ -10,6 +10,8 @@
 #include "dg_render.cuh"
 #include "dg_render_kernels.cuh"
 
+#include <algorithm>
+
 namespace dg {
 namespace {
 
@@ -134,9 +136,72 @@ __device__ __forceinline__ void add_gradients(const BackStage& st, uint32_t firs
     if ((i < 5) == (h == 0) && sum[i] != 0.0f) atomicAdd(out + i, sum[i]);
 }
 
+// The items of rasterize_backward_kernel, and the splats' gradients cleared for it: for
+// each tile the chunks that some block of it walked, chunk by chunk with the blocks of one
+// beside each other, tiles of several chunks before those of one. The order decides nothing
+// but in which one the blocks' sums of a splat meet, and so the last bits of its gradients;
+// the blocks of a chunk run together. (With the chunks listed block by block as the forward
+// pass ended, the longest first, the blend took 149 us for 1.1M splats at 980x545 and 79
+// for 100k, this way 159 and 84. But where a gradient is 0 but for rounding, a first step
+// of Adam turns its sign into a whole step, and the sums that met in another order changed
+// more of those: of 1.6M gradients of a step of 100k splats 57 differ by over a thousandth
+// between a run of that order and one of this, 50 between two runs of this.) A warp per
+// tile, one atomic per CTA and class.
+constexpr uint32_t LIST_THREADS = 256, LIST_WARPS = LIST_THREADS / 32;
+
+__global__ void __launch_bounds__(LIST_THREADS) list_items_kernel(const uint2* ranges, const uint32_t* walked,
+                                                                  uint32_t* plan, uint2* items, uint32_t item_room,
+                                                                  float* splat_grads, size_t floats) {
+  chain_begin();
+  const size_t i = (size_t)blockIdx.x * LIST_THREADS + threadIdx.x, step = (size_t)gridDim.x * LIST_THREADS;
+  const size_t vecs = (reinterpret_cast<uintptr_t>(splat_grads) & 15) == 0 ? floats / 4 : 0;
+  for (size_t k = i; k < vecs; k += step) reinterpret_cast<float4*>(splat_grads)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (size_t k = 4 * vecs + i; k < floats; k += step) splat_grads[k] = 0.0f;
+  const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u, block = lane & 7u;
+  const uint32_t tiles = plan[PLAN_TILES];
+  __shared__ uint32_t s_total[LIST_WARPS], s_at[LIST_WARPS];
+  const uint32_t warp = threadIdx.x >> 5;
+  for (uint32_t first = blockIdx.x * LIST_WARPS; first < tiles; first += gridDim.x * LIST_WARPS) {
+    const uint32_t tile = first + warp;
+    uint32_t chunks = 0, total = 0, several = 0;
+    if (tile < tiles) {
+      const uint2 run = ranges[tile];
+      chunks = (walked[tile * 8u + block] + CHUNK - 1u) / CHUNK;
+      total = __reduce_add_sync(0xffffffffu, lane < 8u ? chunks : 0u);
+      several = run.y - run.x > CHUNK;
+    }
+    // One atomic per class for the CTA's tiles.
+    if (lane == 0) s_total[warp] = total << 1 | several;
+    __syncthreads();
+    if (warp < ITEM_CLASSES) {
+      const uint32_t has = lane < LIST_WARPS ? s_total[lane] : 0u, n = (has & 1u) != warp ? has >> 1 : 0u;
+      uint32_t incl = n;
+#pragma unroll
+      for (uint32_t d = 1; d < LIST_WARPS; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+      }
+      uint32_t base = 0;
+      if (lane == LIST_WARPS - 1u && incl) base = atomicAdd(plan + PLAN_ITEMS + warp, incl);
+      base = __shfl_sync(0xffffffffu, base, LIST_WARPS - 1);
+      if (n) s_at[lane] = base + incl - n;
+    }
+    __syncthreads();
+    uint32_t at = s_at[warp];
+    uint2* out = items + (several ? 0 : (size_t)item_room);
+    const uint32_t most = __reduce_max_sync(0xffffffffu, chunks);
+    for (uint32_t k0 = 0; k0 < most; k0 += 4u) {  // lane (k, block): chunk k0 + k
+      const uint32_t k = k0 + (lane >> 3);
+      const uint32_t listed = __ballot_sync(0xffffffffu, k < chunks), to = at + __popc(listed & below);
+      if (k < chunks && to < item_room) out[to] = make_uint2(tile * 8u + block, k);
+      at += __popc(listed);
+    }
+  }
+}
+
 // src/shaders/rasterizeBackward.wgsl:50-163. The work is split into independent
 // items, one per (tile, CHUNK-entry chunk of its list, 8x4 pixel block), taken by
-// persistent warps from a counter in the plan's order, so no warp waits for
+// persistent warps from a counter in list_items_kernel's order, so no warp waits for
 // another and a long list is spread over many warps. For an item, the warp lists the
 // chunk's entries that some pixel of its block blended in the forward pass (the
 // forward's blend mask), back to front, and takes 32 of them at a time; the records of
@@ -156,15 +221,16 @@ __device__ __forceinline__ void add_gradients(const BackStage& st, uint32_t firs
 // reduce-scatter over the warp per two splats (18 shares, 20 shuffles and as many
 // selects and adds) 280 us for 1.1M splats at 980x545, 147 for 100k, 122 for 201k at
 // 489x273, 38 for 5k at 251x187; this way, in the same order of additions, 179 | 92 |
-// 65 | 21. Items only for what the forward pass walked, and the longest first: 152 | 80 |
-// 61 | 22. 5 and 6 CTAs per SM 155 | 83 | 65 and 167 | 88 | 66; the groups of 4 unrolled
+// 65 | 21. Items only for what the forward pass walked: 159 | 84 | 62 | 21.5. With the
+// longest items first, 5 and 6 CTAs per SM took 155 | 83 | 65 and 167 | 88 | 66 against
+// 152 | 80 | 61 with 4; the groups of 4 unrolled
 // 2 or 4 times the same. Chunks of 256 entries 140 | 75 | 45 | 18, and the shares' sums
 // as moments about the block's center 20% less, but both round otherwise, and a first
 // step of Adam turns a gradient's last bits into the sign of a whole step where it is 0
 // but for rounding.
 __global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
     const Camera* camera, const float4* raster_params, const float* splats,
-    const uint32_t* pair_splats, const uint2* ranges, const uint32_t* plan,
+    const uint32_t* pair_splats, const uint2* ranges, uint32_t* plan,
     const uint2* item_list, uint32_t item_room, const float4* pixel_color, const uint32_t* pixel_last,
     const float4* checkpoints, const uint32_t* blend_mask,
     const float4* pixel_grads, float* splat_grads, uint32_t* work_counter,
@@ -314,6 +380,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
   if (lane == 0 && atomicAdd(work_counter + 1, 1u) == gridDim.x * BWD_WARPS - 1u) {
     work_counter[0] = 0;
     work_counter[1] = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < ITEM_CLASSES; k++) plan[PLAN_ITEMS + k] = 0;
   }
 }
 
@@ -770,13 +838,21 @@ __global__ void DG_PBWD_BOUNDS preprocess_backward_adam_kernel(
 dg_status launch_rasterize_backward(dg_tile_rasterizer* tr, dg_buffer* pixel_grads, dg_buffer* splat_grads) {
   dg_context* ctx = tr->ctx;
   uint32_t* counter = typed<uint32_t>(tr->work) + 2;
+  const uint32_t item_room = (uint32_t)(tr->items->bytes / sizeof(uint2) / ITEM_CLASSES);
+  const size_t floats = (size_t)tr->count * SPLAT_GRADS;
+  const uint32_t tiles = tr->tiles_x * tr->tiles_y;
+  const uint64_t ctas = std::max<uint64_t>(ceil_div(tiles, LIST_WARPS), ceil_div(floats, 4 * LIST_THREADS));
+  DG_CHAIN(ctx, "list_items", (list_items_kernel),
+           (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(ctas, (uint64_t)ctx->sm_count * 8)), LIST_THREADS, 0,
+           typed<uint2>(tr->ranges), typed<uint32_t>(tr->walked), typed<uint32_t>(tr->work_plan),
+           typed<uint2>(tr->items), item_room, typed<float>(splat_grads), floats);
   DG_LAUNCH(ctx, "rasterize_backward",
             rasterize_backward_kernel<<<blend_grid(ctx, (const void*)rasterize_backward_kernel, BWD_THREADS,
                                                     tr->tiles_x * tr->tiles_y * 8u),
                                         BWD_THREADS, 0, ctx->stream>>>(
                 typed<const Camera>(tr->camera), typed<float4>(tr->raster_params), typed<float>(tr->splats),
                 typed<uint32_t>(tr->values), typed<uint2>(tr->ranges), typed<uint32_t>(tr->work_plan),
-                typed<uint2>(tr->items), (uint32_t)(tr->items->bytes / sizeof(uint2) / ITEM_CLASSES), typed<float4>(tr->pixel_color), typed<uint32_t>(tr->pixel_last),
+                typed<uint2>(tr->items), item_room, typed<float4>(tr->pixel_color), typed<uint32_t>(tr->pixel_last),
                 typed<float4>(tr->checkpoints), typed<uint32_t>(tr->blend_mask), typed<float4>(pixel_grads),
                 typed<float>(splat_grads), counter, tr->splat_cutoffs));
   return DG_OK;

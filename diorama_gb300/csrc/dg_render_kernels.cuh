@@ -270,16 +270,11 @@ constexpr uint32_t COOP_MIN = 128, COOP_FLOOR = 64;
 //                 pixels are expected to walk))
 //   PLAN_TOTAL    those entries of all tiles
 //   PLAN_TILES    tiles
-//   PLAN_ITEMS    the backward pass's items per class, listed by the forward pass
+//   PLAN_ITEMS    the backward pass's items per class (dg_render_bwd.cu)
 //   PLAN_LONGEST  the longest tile's entries
 //   then for each bucket its tiles, in room for all tiles
 constexpr uint32_t PLAN_BUCKETS = 32, PLAN_TOTAL = 32, PLAN_TILES = 33, PLAN_LONGEST = 34, PLAN_ITEMS = 35,
-                   ITEM_CLASSES = 4, PLAN_HEADER = PLAN_ITEMS + ITEM_CLASSES;
-// The class of a backward item of so many entries, the longest first: warps that take a
-// long item last keep the GPU waiting.
-__device__ __forceinline__ uint32_t item_class(uint32_t entries) {
-  return ITEM_CLASSES - 1u - (entries - 1u) * ITEM_CLASSES / CHUNK;
-}
+                   ITEM_CLASSES = 2, PLAN_HEADER = PLAN_ITEMS + ITEM_CLASSES;
 constexpr size_t plan_words(size_t tiles) { return PLAN_HEADER + PLAN_BUCKETS * tiles; }
 
 // The forward pass's stage: a warp's own window of up to 32 list entries, in its slice
