@@ -30,13 +30,6 @@ uint32_t bits_for(uint32_t n) {
 // fewer than 2^24 tiles, so the view always fits above them.
 uint32_t view_shift_for(uint32_t tiles_per_view) { return (bits_for(tiles_per_view) + 7) / 8 * 8; }
 
-dg_status ensure(dg_context* ctx, dg_buffer** buf, size_t bytes) {
-  if (*buf && (*buf)->bytes >= bytes) return DG_OK;
-  free_buffer(*buf);
-  *buf = nullptr;
-  return alloc_buffer(ctx, std::max<size_t>(bytes, 16), buf);
-}
-
 }  // namespace
 }  // namespace dg
 
@@ -57,15 +50,20 @@ struct dg_view_batch {
   dg_buffer* bin_scratch = nullptr;
   dg_buffer *ranges = nullptr, *plan = nullptr, *pixel_color = nullptr, *pixel_last = nullptr, *work = nullptr;
   uint32_t* pinned_total = nullptr;
-  // The captured batch (valid while its key matches).
+  uint64_t allocations = 0;  // of the buffers above, up to now
+  // The captured batch, valid while its key matches: everything that its launches carry
+  // by value (the sizes, the grid of tiles) and every pointer in them, those of the
+  // buffers above by their allocations.
   cudaGraphExec_t graph = nullptr;
   struct Key {
-    uint32_t views, count, capacity, coop_min;
+    uint32_t views, count, width, height, capacity, coop_min;
     BlendShape shape;
-    const void *gaussians, *targets, *values;
+    uint64_t allocations;
+    const void *gaussians, *sh, *scene_params, *targets;
     bool operator==(const Key& o) const {
-      return views == o.views && count == o.count && capacity == o.capacity && coop_min == o.coop_min &&
-             shape == o.shape && gaussians == o.gaussians && targets == o.targets && values == o.values;
+      return views == o.views && count == o.count && width == o.width && height == o.height &&
+             capacity == o.capacity && coop_min == o.coop_min && shape == o.shape && allocations == o.allocations &&
+             gaussians == o.gaussians && sh == o.sh && scene_params == o.scene_params && targets == o.targets;
     }
   } key{};
   uint32_t last_total = 0;
@@ -88,6 +86,14 @@ void view_batch_destroy(dg_view_batch* b) {
 
 namespace {
 
+dg_status ensure(dg_view_batch* b, dg_buffer** buf, size_t bytes) {
+  if (*buf && (*buf)->bytes >= bytes) return DG_OK;
+  b->allocations++;
+  free_buffer(*buf);
+  *buf = nullptr;
+  return alloc_buffer(b->ctx, std::max<size_t>(bytes, 16), buf);
+}
+
 // Each view's splats by depth, on their own: all views in the same launches. (As one
 // sort of (view, depth) keys, 12 views of 300,000 took 190 us in five passes over 64-bit
 // keys, this way 135.)
@@ -98,14 +104,13 @@ SortPlan depth_sort(uint32_t views, uint32_t count) {
 }
 
 dg_status grow_pairs(dg_view_batch* b, uint32_t capacity) {
-  dg_context* ctx = b->ctx;
-  DG_TRY(ensure(ctx, &b->values, (size_t)capacity * 4));
+  DG_TRY(ensure(b, &b->values, (size_t)capacity * 4));
   if (!b->binned) {
     const SortPlan tile_plan = sort_plan_digits(capacity, 1, bits_for(b->tiles_per_view));
-    DG_TRY(ensure(ctx, &b->keys, (size_t)capacity * 4));
-    DG_TRY(ensure(ctx, &b->keys_alt, (size_t)capacity * 4));
-    DG_TRY(ensure(ctx, &b->values_alt, (size_t)capacity * 4));
-    DG_TRY(ensure(ctx, &b->sort_scratch, sort_scratch_bytes(tile_plan)));
+    DG_TRY(ensure(b, &b->keys, (size_t)capacity * 4));
+    DG_TRY(ensure(b, &b->keys_alt, (size_t)capacity * 4));
+    DG_TRY(ensure(b, &b->values_alt, (size_t)capacity * 4));
+    DG_TRY(ensure(b, &b->sort_scratch, sort_scratch_bytes(tile_plan)));
   }
   b->pair_capacity = capacity;
   return DG_OK;
@@ -115,7 +120,6 @@ dg_status grow_pairs(dg_view_batch* b, uint32_t capacity) {
 // grid_x x grid_y blend tiles each.
 dg_status prepare(dg_view_batch* b, uint32_t views, uint32_t count, uint32_t grid_x, uint32_t grid_y,
                   uint32_t pixels) {
-  dg_context* ctx = b->ctx;
   const uint32_t tiles_per_view = grid_x * grid_y;
   const size_t n = (size_t)views * count;
   if (n >= (1ull << 31)) return fail(DG_ERROR_INVALID_ARGUMENT, "too many view x Gaussian pairs in one batch");
@@ -132,27 +136,27 @@ dg_status prepare(dg_view_batch* b, uint32_t views, uint32_t count, uint32_t gri
   b->tiles_per_view = tiles_per_view;
   b->pixels = pixels;
   const SortPlan depth_plan = depth_sort(views, count);
-  DG_TRY(ensure(ctx, &b->cameras, (size_t)views * sizeof(Camera)));
-  DG_TRY(ensure(ctx, &b->raster_params, 16));
-  DG_TRY(ensure(ctx, &b->splats, n * FLOATS_PER_SPLAT * 4));
-  DG_TRY(ensure(ctx, &b->tile_counts, n * 4));
-  DG_TRY(ensure(ctx, &b->depth_keys, n * 4));
-  DG_TRY(ensure(ctx, &b->depth_keys_alt, n * 4));
-  DG_TRY(ensure(ctx, &b->order, n * 4));
-  DG_TRY(ensure(ctx, &b->order_alt, n * 4));
-  DG_TRY(ensure(ctx, &b->depth_scratch, sort_scratch_bytes(depth_plan)));
+  DG_TRY(ensure(b, &b->cameras, (size_t)views * sizeof(Camera)));
+  DG_TRY(ensure(b, &b->raster_params, 16));
+  DG_TRY(ensure(b, &b->splats, n * FLOATS_PER_SPLAT * 4));
+  DG_TRY(ensure(b, &b->tile_counts, n * 4));
+  DG_TRY(ensure(b, &b->depth_keys, n * 4));
+  DG_TRY(ensure(b, &b->depth_keys_alt, n * 4));
+  DG_TRY(ensure(b, &b->order, n * 4));
+  DG_TRY(ensure(b, &b->order_alt, n * 4));
+  DG_TRY(ensure(b, &b->depth_scratch, sort_scratch_bytes(depth_plan)));
   if (binned) {
-    DG_TRY(ensure(ctx, &b->bin_scratch, bin_scratch_bytes(BinShape{count, views, grid_x, grid_y})));
+    DG_TRY(ensure(b, &b->bin_scratch, bin_scratch_bytes(BinShape{count, views, grid_x, grid_y})));
   } else {
-    DG_TRY(ensure(ctx, &b->counts_sorted, n * 4));
-    DG_TRY(ensure(ctx, &b->scan_scratch, scan_scratch_bytes((uint32_t)n)));
+    DG_TRY(ensure(b, &b->counts_sorted, n * 4));
+    DG_TRY(ensure(b, &b->scan_scratch, scan_scratch_bytes((uint32_t)n)));
   }
-  DG_TRY(ensure(ctx, &b->scan_total, 16));
-  DG_TRY(ensure(ctx, &b->ranges, (size_t)views * tiles_per_view * 8));
-  DG_TRY(ensure(ctx, &b->plan, plan_words((size_t)views * tiles_per_view) * 4));
-  DG_TRY(ensure(ctx, &b->pixel_color, (size_t)views * pixels * 16));
-  DG_TRY(ensure(ctx, &b->pixel_last, (size_t)views * pixels * 4));
-  DG_TRY(ensure(ctx, &b->work, 16));
+  DG_TRY(ensure(b, &b->scan_total, 16));
+  DG_TRY(ensure(b, &b->ranges, (size_t)views * tiles_per_view * 8));
+  DG_TRY(ensure(b, &b->plan, plan_words((size_t)views * tiles_per_view) * 4));
+  DG_TRY(ensure(b, &b->pixel_color, (size_t)views * pixels * 16));
+  DG_TRY(ensure(b, &b->pixel_last, (size_t)views * pixels * 4));
+  DG_TRY(ensure(b, &b->work, 16));
   if (!b->pinned_total && cudaMallocHost(&b->pinned_total, 4) != cudaSuccess)
     return fail(DG_ERROR_OUT_OF_MEMORY, "pinned");
   if (reshaped || b->pair_capacity == 0) {
@@ -254,8 +258,8 @@ dg_status render_batch(dg_renderer* r, dg_view_batch* b, const dg_camera* cams, 
   const float params[4] = {bg[0], bg[1], bg[2], 1.0f};
   DG_TRY(write_async(ctx, b->raster_params->ptr, params, sizeof(params)));
   for (int attempt = 0; attempt < 2; attempt++) {
-    const dg_view_batch::Key key{count, r->count, b->pair_capacity, coop_min, shape, r->gaussians->ptr, targets,
-                                 b->values->ptr};
+    const dg_view_batch::Key key{count,    r->count,       w, h, b->pair_capacity, coop_min, shape, b->allocations,
+                                 r->gaussians->ptr, r->sh->ptr, r->scene_params->ptr, targets};
     if (use_graph) {
       if (!b->graph || !(key == b->key)) {
         if (b->graph) cudaGraphExecDestroy(b->graph);
