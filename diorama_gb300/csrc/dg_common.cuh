@@ -112,6 +112,7 @@ struct dg_context {
   cudaStream_t stream = nullptr;
   uint32_t* device_error = nullptr;  // set by bounded waits
   int sm_count = 0;
+  uint64_t generations = 0;  // of its rasterizers' buffers (dg_render.cuh), up to now
   int sort_clusters = 0;  // clusters of 16 CTAs that sort at once (dg_sort.cu)
   // Pinned staging ring for queue.writeBuffer: each write is copied here at call
   // time, so the caller's memory is free on return, as with WebGPU.

@@ -982,8 +982,13 @@ __global__ void clear_target_kernel(uchar4* __restrict__ target, uint32_t pixels
 static dg_status ensure_plan(dg_tile_rasterizer* tr);
 static dg_status ensure_pair_sort(dg_tile_rasterizer* tr);
 
+// A buffer that the frame's kernels use: a graph that was captured before does not know it.
+static dg_status new_buffer(dg_tile_rasterizer* tr, uint64_t bytes, dg_buffer** out) {
+  tr->generation = ++tr->ctx->generations;
+  return alloc_buffer(tr->ctx, bytes, out);
+}
+
 static dg_status make_pairs(dg_tile_rasterizer* tr, uint32_t capacity) {
-  dg_context* ctx = tr->ctx;
   free_buffer(tr->keys);
   free_buffer(tr->values);
   free_buffer(tr->keys_alt);
@@ -993,7 +998,7 @@ static dg_status make_pairs(dg_tile_rasterizer* tr, uint32_t capacity) {
   tr->plan = sort_plan(capacity, TILE_INDEX_BITS);
   tr->tile_plan = sort_plan_low_bits(capacity, TILE_INDEX_BITS);
   tr->pair_capacity = capacity;
-  DG_TRY(alloc_buffer(ctx, (size_t)capacity * 4, &tr->values));
+  DG_TRY(new_buffer(tr, (size_t)capacity * 4, &tr->values));
   if (!tr->depth_first) DG_TRY(ensure_pair_sort(tr));
   return ensure_plan(tr);
 }
@@ -1001,16 +1006,15 @@ static dg_status make_pairs(dg_tile_rasterizer* tr, uint32_t capacity) {
 // The buffers of frames whose pairs are sorted; binned frames need none of them.
 static dg_status ensure_pair_sort(dg_tile_rasterizer* tr) {
   if (tr->sort_scratch) return DG_OK;
-  dg_context* ctx = tr->ctx;
   const size_t capacity = tr->pair_capacity;
   for (dg_buffer** b : {&tr->keys, &tr->keys_alt, &tr->values_alt}) {
     free_buffer(*b);
     *b = nullptr;
   }
-  DG_TRY(alloc_buffer(ctx, capacity * 8, &tr->keys));
-  DG_TRY(alloc_buffer(ctx, capacity * 8, &tr->keys_alt));
-  DG_TRY(alloc_buffer(ctx, capacity * 4, &tr->values_alt));
-  return alloc_buffer(ctx, std::max(sort_scratch_bytes(tr->plan), sort_scratch_bytes(tr->tile_plan)),
+  DG_TRY(new_buffer(tr, capacity * 8, &tr->keys));
+  DG_TRY(new_buffer(tr, capacity * 8, &tr->keys_alt));
+  DG_TRY(new_buffer(tr, capacity * 4, &tr->values_alt));
+  return new_buffer(tr, std::max(sort_scratch_bytes(tr->plan), sort_scratch_bytes(tr->tile_plan)),
                       &tr->sort_scratch);
 }
 
@@ -1024,11 +1028,11 @@ dg_status rasterizer_create(dg_context* ctx, dg_buffer* camera, dg_buffer* splat
   tr->camera = camera;
   tr->splats = splats;
   tr->count = count;
-  dg_status st = alloc_buffer(ctx, (size_t)std::max(count, 1u) * 4, &tr->tile_offsets);
-  if (st == DG_OK) st = alloc_buffer(ctx, 4, &tr->scan_total);
-  if (st == DG_OK) st = alloc_buffer(ctx, scan_scratch_bytes(std::max(count, 1u)), &tr->scan_scratch);
-  if (st == DG_OK) st = alloc_buffer(ctx, 16, &tr->raster_params);
-  if (st == DG_OK) st = alloc_buffer(ctx, 16, &tr->work);
+  dg_status st = new_buffer(tr, (size_t)std::max(count, 1u) * 4, &tr->tile_offsets);
+  if (st == DG_OK) st = new_buffer(tr, 4, &tr->scan_total);
+  if (st == DG_OK) st = new_buffer(tr, scan_scratch_bytes(std::max(count, 1u)), &tr->scan_scratch);
+  if (st == DG_OK) st = new_buffer(tr, 16, &tr->raster_params);
+  if (st == DG_OK) st = new_buffer(tr, 16, &tr->work);
   if (st == DG_OK && cudaMallocHost(&tr->pinned_totals, 4 * dg_tile_rasterizer::READBACKS) != cudaSuccess)
     st = fail(DG_ERROR_OUT_OF_MEMORY, "pinned");
   for (uint32_t k = 0; k < dg_tile_rasterizer::READBACKS && st == DG_OK; k++)
@@ -1041,12 +1045,12 @@ dg_status rasterizer_create(dg_context* ctx, dg_buffer* camera, dg_buffer* splat
   if (st == DG_OK && depth_first) {
     const size_t n = std::max(count, 1u);
     tr->depth_plan = sort_plan_low_bits(std::max(count, 1u), 32);
-    st = alloc_buffer(ctx, n * 4, &tr->depth_keys);
-    if (st == DG_OK) st = alloc_buffer(ctx, n * 4, &tr->depth_values);
-    if (st == DG_OK) st = alloc_buffer(ctx, n * 4, &tr->depth_keys_alt);
-    if (st == DG_OK) st = alloc_buffer(ctx, n * 4, &tr->depth_values_alt);
-    if (st == DG_OK) st = alloc_buffer(ctx, sort_scratch_bytes(tr->depth_plan), &tr->depth_scratch);
-    if (st == DG_OK) st = alloc_buffer(ctx, n * 4, &tr->counts_sorted);
+    st = new_buffer(tr, n * 4, &tr->depth_keys);
+    if (st == DG_OK) st = new_buffer(tr, n * 4, &tr->depth_values);
+    if (st == DG_OK) st = new_buffer(tr, n * 4, &tr->depth_keys_alt);
+    if (st == DG_OK) st = new_buffer(tr, n * 4, &tr->depth_values_alt);
+    if (st == DG_OK) st = new_buffer(tr, sort_scratch_bytes(tr->depth_plan), &tr->depth_scratch);
+    if (st == DG_OK) st = new_buffer(tr, n * 4, &tr->counts_sorted);
   }
   if (st != DG_OK) {
     dg_tile_rasterizer_destroy(tr);
@@ -1078,7 +1082,7 @@ dg_status rasterizer_prepare(dg_tile_rasterizer* tr, const float viewport[2], co
     if (!tr->bin_scratch || tr->bin_scratch->bytes < bytes) {
       free_buffer(tr->bin_scratch);
       tr->bin_scratch = nullptr;
-      DG_TRY(alloc_buffer(tr->ctx, bytes, &tr->bin_scratch));
+      DG_TRY(new_buffer(tr, bytes, &tr->bin_scratch));
     }
   } else {
     DG_TRY(ensure_pair_sort(tr));
@@ -1086,7 +1090,7 @@ dg_status rasterizer_prepare(dg_tile_rasterizer* tr, const float viewport[2], co
   if (!tr->ranges || tr->ranges_tiles < tiles) {
     free_buffer(tr->ranges);
     tr->ranges = nullptr;
-    DG_TRY(alloc_buffer(tr->ctx, (size_t)std::max(tiles, 1u) * 8, &tr->ranges));
+    DG_TRY(new_buffer(tr, (size_t)std::max(tiles, 1u) * 8, &tr->ranges));
     tr->ranges_tiles = tiles;
     DG_TRY(ensure_plan(tr));
   }
@@ -1095,8 +1099,8 @@ dg_status rasterizer_prepare(dg_tile_rasterizer* tr, const float viewport[2], co
     free_buffer(tr->pixel_color);
     free_buffer(tr->pixel_last);
     tr->pixel_color = tr->pixel_last = nullptr;
-    DG_TRY(alloc_buffer(tr->ctx, (size_t)std::max(pixels, 1u) * 16, &tr->pixel_color));
-    DG_TRY(alloc_buffer(tr->ctx, (size_t)std::max(pixels, 1u) * 4, &tr->pixel_last));
+    DG_TRY(new_buffer(tr, (size_t)std::max(pixels, 1u) * 16, &tr->pixel_color));
+    DG_TRY(new_buffer(tr, (size_t)std::max(pixels, 1u) * 4, &tr->pixel_last));
     tr->pixel_count = pixels;
   }
   const float params[4] = {background[0], background[1], background[2], 1.0f};
@@ -1296,7 +1300,7 @@ static dg_status ensure_plan(dg_tile_rasterizer* tr) {
     if (*n.buf && (*n.buf)->bytes >= n.bytes) continue;
     free_buffer(*n.buf);
     *n.buf = nullptr;
-    DG_TRY(alloc_buffer(tr->ctx, n.bytes, n.buf));
+    DG_TRY(new_buffer(tr, n.bytes, n.buf));
   }
   return DG_OK;
 }

@@ -60,6 +60,7 @@ struct dg_tile_rasterizer {
   dg_buffer* checkpoints;  // the forward's per-chunk pixel states
   dg_buffer* blend_mask;   // which entries each 8x4 block blended (dg_render_kernels.cuh, mask_at)
   uint32_t coop_min;      // the fewest entries of a tile that a whole CTA may blend
+  uint64_t generation;    // of the buffers above: another one, never seen before, after each allocation
   bool splat_cutoffs;     // the splats come from this build's preprocess, cutoffs in slot 7
 };
 

@@ -443,14 +443,11 @@ struct dg_trainer {
   uint32_t prefetch_slot = 0, slot_used = 1;
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_launches = 0;
-  struct Key {
-    uint32_t count, capacity;
-    void *gaussians, *pairs, *pixel_grads;
-    bool operator==(const Key& o) const {
-      return count == o.count && capacity == o.capacity && gaussians == o.gaussians && pairs == o.pairs &&
-             pixel_grads == o.pixel_grads;
-    }
-  } graph_key{};
+  // The buffers that the graph was captured for: the rasterizer's, of the scene that it
+  // came with (a frame of another size on the trainer's renderer allocates them anew, and
+  // a densification makes another rasterizer). What else a step uses, densify and the
+  // setters drop the graph for.
+  uint64_t graph_generation = 0;
   // Learned densification. Every Gaussian has an identity (children get fresh
   // ones) and aux statistics (float2: squared gradient norms since the last
   // densification, steps seen over its life).
@@ -558,10 +555,8 @@ static void drop_graph(dg_trainer* t) {
 }
 
 static dg_status run_graph_step(dg_trainer* t) {
-  dg_renderer* r = t->renderer;
-  dg_trainer::Key key{t->count, r->rasterizer->pair_capacity, r->gaussians->ptr, r->rasterizer->values->ptr,
-                      t->loss->pixel_grads->ptr};
-  if (!t->graph_exec || !(key == t->graph_key)) {
+  const uint64_t generation = t->renderer->rasterizer->generation;
+  if (!t->graph_exec || generation != t->graph_generation) {
     drop_graph(t);
     cudaGraph_t graph;
     const uint64_t before = t->ctx->launches;
@@ -578,7 +573,7 @@ static dg_status run_graph_step(dg_trainer* t) {
     cudaError_t inst = cudaGraphInstantiate(&t->graph_exec, graph, 0);
     cudaGraphDestroy(graph);
     DG_CUDA(inst);
-    t->graph_key = key;
+    t->graph_generation = generation;
     t->graph_launches = t->ctx->launches - before;
     t->ctx->launches = before;
   }
