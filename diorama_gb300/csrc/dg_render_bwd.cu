@@ -11,6 +11,7 @@
 #include "dg_render_kernels.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace dg {
 namespace {
@@ -43,8 +44,8 @@ struct PixelBackward {
     na = ncx = ncy = ncz = 0.0f;
   }
 
-  // Steps in front of a splat of this alpha and colour (alpha 0: one that the pixel did
-  // not blend, which changes nothing) and returns the gradient of its alpha.
+  // Steps in front of a splat of this alpha and colour (alpha 0 and a finite colour: one
+  // that the pixel did not blend, which changes nothing) and returns the gradient of its alpha.
   __device__ __forceinline__ float step(float alpha, float4 c) {
     // 1 / (1 - alpha), used twice; the approximate reciprocal (~1 ulp) is plenty:
     // a chunk's chain of divisions is at most CHUNK entries long.
@@ -331,6 +332,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
       } else {
         e[10] = 0.0f;  // nothing is below it
       }
+      // A colour that is not finite must not reach a pixel that does not blend its splat,
+      // where step() would multiply it by 0. Batches with one have a loop of their own (1%
+      // of the pass; as a select in the one loop 2.4%).
+      const bool endless = __any_sync(
+          0xffffffffu, lane < staged && !(fabsf(raw.s2.x) + fabsf(raw.s2.y) + fabsf(raw.s2.z) < INFINITY));
       __syncwarp();
       index = next_index;
       raw.load(splats, index, first + BATCH + lane < total);
@@ -339,36 +345,44 @@ __global__ void __launch_bounds__(BWD_THREADS, 4) rasterize_backward_kernel(
 #pragma unroll 1
       for (uint32_t half = 0; half < staged; half += HALF_BATCH) {
         const uint32_t n = min(HALF_BATCH, staged - half);
+        auto walk = [&](auto endless_batch) {
+          constexpr bool ENDLESS = decltype(endless_batch)::value;
 #pragma unroll 1
-        for (uint32_t j = 0; j < n; j += 4) {
-          const uint4 pos = *reinterpret_cast<const uint4*>(&st.pos[half + j]);
-          bool has[4] = {pos.x < last, pos.y < last, pos.z < last, pos.w < last};
-          float alpha[4], G[4];
+          for (uint32_t j = 0; j < n; j += 4) {
+            const uint4 pos = *reinterpret_cast<const uint4*>(&st.pos[half + j]);
+            bool has[4] = {pos.x < last, pos.y < last, pos.z < last, pos.w < last};
+            float alpha[4], G[4];
 #pragma unroll
-          for (uint32_t h = 0; h < 2; h++) {
-            const BlendPair& pr = st.pair[(half + j) / 2 + h];
-            F2 limit;
-            const F2 q = blend_power_negated(pr, cx, cy, limit);
-            has[2 * h] = has[2 * h] && __float_as_uint(f2_lo(q)) < __float_as_uint(f2_lo(limit));
-            has[2 * h + 1] = has[2 * h + 1] && __float_as_uint(f2_hi(q)) < __float_as_uint(f2_hi(limit));
-            // Any value may come out where the limit was not kept.
-            const F2 ex = exp_blend_negated(q), al = f2_mul(F2{pr.opacity}, ex);
-            G[2 * h] = f2_lo(ex);
-            G[2 * h + 1] = f2_hi(ex);
-            alpha[2 * h] = fminf(0.99f, f2_lo(al));
-            alpha[2 * h + 1] = fminf(0.99f, f2_hi(al));
-          }
+            for (uint32_t h = 0; h < 2; h++) {
+              const BlendPair& pr = st.pair[(half + j) / 2 + h];
+              F2 limit;
+              const F2 q = blend_power_negated(pr, cx, cy, limit);
+              has[2 * h] = has[2 * h] && __float_as_uint(f2_lo(q)) < __float_as_uint(f2_lo(limit));
+              has[2 * h + 1] = has[2 * h + 1] && __float_as_uint(f2_hi(q)) < __float_as_uint(f2_hi(limit));
+              // Any value may come out where the limit was not kept.
+              const F2 ex = exp_blend_negated(q), al = f2_mul(F2{pr.opacity}, ex);
+              G[2 * h] = f2_lo(ex);
+              G[2 * h + 1] = f2_hi(ex);
+              alpha[2 * h] = fminf(0.99f, f2_lo(al));
+              alpha[2 * h + 1] = fminf(0.99f, f2_hi(al));
+            }
 #pragma unroll
-          for (uint32_t u = 0; u < 4; u++) {
-            has[u] = has[u] && alpha[u] >= 1.0f / 255.0f;
-            const float al = has[u] ? alpha[u] : 0.0f;
-            const float4 c = st.color[half + j + u];
-            const float alpha_grad = pb.step(al, c);
-            st.share[0][j + u][place] = has[u] ? alpha_grad * c.w * G[u] : 0.0f;
-            st.share[1][j + u][place] = has[u] ? alpha_grad * G[u] : 0.0f;
-            st.share[2][j + u][place] = al * pb.T;
+            for (uint32_t u = 0; u < 4; u++) {
+              has[u] = has[u] && alpha[u] >= 1.0f / 255.0f;
+              const float al = has[u] ? alpha[u] : 0.0f;
+              float4 c = st.color[half + j + u];
+              if (ENDLESS && !has[u]) c.x = c.y = c.z = 0.0f;
+              const float alpha_grad = pb.step(al, c);
+              st.share[0][j + u][place] = has[u] ? alpha_grad * c.w * G[u] : 0.0f;
+              st.share[1][j + u][place] = has[u] ? alpha_grad * G[u] : 0.0f;
+              st.share[2][j + u][place] = al * pb.T;
+            }
           }
-        }
+        };
+        if (endless)
+          walk(std::true_type{});
+        else
+          walk(std::false_type{});
         __syncwarp();
         add_gradients(st, half, n, lane, (float)bx + 0.5f, (float)by + 0.5f, splat_grads);
         __syncwarp();
