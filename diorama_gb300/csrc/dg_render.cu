@@ -117,9 +117,9 @@ __device__ __forceinline__ void load_gaussian(const float* __restrict__ gaussian
   }
 }
 
-// One thread per Gaussian, one view. The tiles each splat touches are written too,
-// as a packed rectangle when rects is given (dg_bin.cu's input), else as their
-// number in tile_counts (src/shaders/tiles.wgsl:24-35, fused); when depth_keys is
+// One thread per Gaussian, one view. The tiles each splat touches are written too, their
+// number in tile_counts (src/shaders/tiles.wgsl:24-35, fused) and, when rects is given,
+// their packed rectangle (dg_bin.cu's input); when depth_keys is
 // given, the depth's bits (all ones when culled) and the splat's index,
 // the input of the depth sort; when radii is given, each splat's radius densely
 // (the training step's fused backward reads it there, not from the 48-byte
@@ -168,10 +168,8 @@ __global__ void __launch_bounds__(PRE_THREADS) preprocess_kernel(const Camera* c
     if (i < count) {
       const Projected pr = preprocess_one(s_cam, g, s_sh[step & 1] + threadIdx.x * SH_REST_FLOATS, basis_count,
                                           reinterpret_cast<float4*>(splats + (size_t)i * FLOATS_PER_SPLAT));
-      if (rects)
-        rects[i] = pack_rect(pr.rect);
-      else
-        tile_counts[i] = pr.tiles();
+      tile_counts[i] = pr.tiles();
+      if (rects) rects[i] = pack_rect(pr.rect);
       if (depth_keys) depth_keys[i] = pr.depth_bits;
       if (depth_order) depth_order[i] = i;
       if (radii) radii[i] = pr.radius;
@@ -1051,6 +1049,7 @@ dg_status rasterizer_create(dg_context* ctx, dg_buffer* camera, dg_buffer* splat
     if (st == DG_OK) st = new_buffer(tr, n * 4, &tr->depth_values_alt);
     if (st == DG_OK) st = new_buffer(tr, sort_scratch_bytes(tr->depth_plan), &tr->depth_scratch);
     if (st == DG_OK) st = new_buffer(tr, n * 4, &tr->counts_sorted);
+    if (st == DG_OK) st = new_buffer(tr, n * 4, &tr->rects);
   }
   if (st != DG_OK) {
     dg_tile_rasterizer_destroy(tr);
@@ -1114,15 +1113,15 @@ dg_status rasterizer_launch(dg_tile_rasterizer* tr, dg_buffer* target, bool coun
   const auto* cam = typed<const Camera>(tr->camera);
   tr->keys_in_ranges = false;
   if (tr->binned && counts_ready) {
-    // tile_offsets holds each splat's rectangle of tiles; depth_keys/depth_values its
-    // depth bits and index (both written by the renderer's preprocess).
+    // rects holds each splat's rectangle of tiles; depth_keys/depth_values its depth bits
+    // and index (all written by the renderer's preprocess).
     uint32_t* order = typed<uint32_t>(tr->depth_values);
     if (count > 0) {
       DG_TRY(sort_launch(ctx, tr->depth_plan, tr->depth_keys->ptr, order, tr->depth_keys_alt->ptr,
                          typed<uint32_t>(tr->depth_values_alt), nullptr, tr->depth_scratch->ptr));
     }
     BinLaunch l{};
-    l.rects = typed<uint32_t>(tr->tile_offsets);
+    l.rects = typed<uint32_t>(tr->rects);
     l.order = order;
     l.capacity = tr->pair_capacity;
     l.scratch = tr->bin_scratch->ptr;
@@ -1420,7 +1419,7 @@ dg_status renderer_launch_forward(dg_renderer* r, dg_buffer* target) {
     DG_CHAIN(ctx, "preprocess", (preprocess_kernel), preprocess_grid(ctx, r->count), PRE_THREADS, 0,
              typed<const Camera>(r->camera), typed<float>(r->gaussians), typed<float>(r->sh), r->count,
              typed<uint32_t>(r->scene_params), typed<float>(r->splats), typed<uint32_t>(r->rasterizer->tile_offsets),
-             r->rasterizer->binned ? typed<uint32_t>(r->rasterizer->tile_offsets) : nullptr,
+             r->rasterizer->binned ? typed<uint32_t>(r->rasterizer->rects) : nullptr,
              typed<uint32_t>(r->rasterizer->depth_keys), typed<uint32_t>(r->rasterizer->depth_values),
              typed<float>(r->radii));
   }
@@ -1497,7 +1496,7 @@ dg_status dg_tile_rasterizer_destroy(dg_tile_rasterizer* tr) {
   for (dg_buffer* b : {tr->tile_offsets, tr->scan_total, tr->scan_scratch, tr->raster_params, tr->keys, tr->values,
                        tr->keys_alt, tr->values_alt, tr->sort_scratch, tr->ranges, tr->pixel_color, tr->pixel_last,
                        tr->depth_keys, tr->depth_values, tr->depth_keys_alt, tr->depth_values_alt, tr->depth_scratch,
-                       tr->counts_sorted, tr->bin_scratch, tr->keys64, tr->work, tr->work_plan, tr->walked, tr->items,
+                       tr->counts_sorted, tr->rects, tr->bin_scratch, tr->keys64, tr->work, tr->work_plan, tr->walked, tr->items,
                        tr->checkpoints,
                        tr->blend_mask})
     free_buffer(b);

@@ -10,7 +10,7 @@ struct dg_tile_rasterizer {
   dg_buffer* camera;  // borrowed: the 144-byte Camera uniform
   dg_buffer* splats;  // borrowed
   uint32_t count;
-  dg_buffer* tile_offsets;   // per splat: tiles touched, then its first pair slot
+  dg_buffer* tile_offsets;   // per splat: tiles touched; then its first pair slot, where they are scanned in place
   dg_buffer* scan_total;     // PrefixSum.total: pairs this frame needs
   dg_buffer* scan_scratch;
   dg_buffer* raster_params;  // background (rgb, 1)
@@ -44,6 +44,7 @@ struct dg_tile_rasterizer {
   bool binned;          // the prepared frame's tile stage
   bool keys_are_tiles;  // the last frame left u32 tile indices in `keys`
   bool keys_in_ranges;  // the last frame was binned: it has no keys, only ranges
+  dg_buffer* rects;  // per splat: its rectangle of tiles (a binned frame's)
   dg_buffer* bin_scratch;
   dg::SortPlan depth_plan, tile_plan;
   dg_buffer* depth_keys;

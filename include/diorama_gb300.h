@@ -173,7 +173,8 @@ dg_buffer* dg_tile_rasterizer_ranges(dg_tile_rasterizer* tr);      /* debugBuffe
 dg_buffer* dg_tile_rasterizer_pair_keys(dg_tile_rasterizer* tr);   /* sorted (depth, tile) keys */
 dg_buffer* dg_tile_rasterizer_pixel_color(dg_tile_rasterizer* tr); /* .pixelColor, vec4 per pixel */
 dg_buffer* dg_tile_rasterizer_pixel_last(dg_tile_rasterizer* tr);  /* .pixelLast, u32 per pixel */
-dg_buffer* dg_tile_rasterizer_tile_offsets(dg_tile_rasterizer* tr);/* scanned per-splat first pair slots */
+/* Per splat, its first pair slot; of a renderer's rasterizer, which sorts by depth first, the tiles it touches. */
+dg_buffer* dg_tile_rasterizer_tile_offsets(dg_tile_rasterizer* tr);
 dg_buffer* dg_tile_rasterizer_pair_total(dg_tile_rasterizer* tr);  /* element 0: pairs the last frame needed */
 dg_status dg_tile_rasterizer_destroy(dg_tile_rasterizer* tr);
 
