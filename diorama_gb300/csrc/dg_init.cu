@@ -17,7 +17,7 @@
 // cells a point) took 1,519 us for a clustered cloud of 180,000 points where this
 // takes 195: its threads waited for the warp's longest search and for one dependent
 // load after another; here 32 points share every box and every point that is read.
-// (The whole call: 1,448 -> 335 us.) What bounds
+// (The whole call: 1,448 -> 315 us.) What bounds
 // it: instructions at 1.1M points (16 a distance, 512 a leaf, about 28 leaves a
 // warp); at 180,000, whose warps all run at once, the longest walks.
 //
@@ -61,7 +61,7 @@ struct Octree {
 // The finite points' bounds and moments.
 struct Moments {
   float lo[3], hi[3];
-  double sum[3], sum2[3];  // of the coordinates less the first point's
+  double sum[3], sum2[3];  // in 64 bits: squares of float32 coordinates may exceed float32
   uint32_t finite;         // points with three finite coordinates
 };
 
@@ -90,10 +90,9 @@ __device__ __forceinline__ void add_moments(Moments& m, const Moments& o) {
   }
 }
 
-// Sums m over the CTA; thread 0 gets the whole.
-__device__ __forceinline__ void reduce_moments(Moments& m, Moments* s_warp) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
+// Sums m over `lanes` lanes of the warp, lane ^ 1 last.
+__device__ __forceinline__ void reduce_lanes(Moments& m, int lanes) {
+  for (int off = lanes / 2; off > 0; off >>= 1) {
     Moments o;
     o.finite = __shfl_xor_sync(0xffffffffu, m.finite, off);
 #pragma unroll
@@ -105,23 +104,28 @@ __device__ __forceinline__ void reduce_moments(Moments& m, Moments* s_warp) {
     }
     add_moments(m, o);
   }
-  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = m;
+}
+
+// Sums m over the CTA; the first warp's first 8 lanes get the whole.
+__device__ __forceinline__ void reduce_moments(Moments& m, Moments* s_warp) {
+  constexpr uint32_t WARPS = KNN_THREADS / 32;
+  const uint32_t lane = threadIdx.x & 31u;
+  reduce_lanes(m, 32);
+  if (lane == 0) s_warp[threadIdx.x >> 5] = m;
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (uint32_t w = 1; w < KNN_THREADS / 32; w++) add_moments(m, s_warp[w]);
+  if (threadIdx.x >= 32) return;
+  m = s_warp[lane % WARPS];
+  reduce_lanes(m, WARPS);
 }
 
 // Each CTA's share of the moments (4,900 warps adding to one global record took
-// 70 us at 180,000 points).
+// 70 us at 180,000 points). Bound by the FP64 sums: with a thread's points summed in
+// float32 12.3 us instead of 15.4 at 180,000 points and 16 instead of 37 at 1.1M, but
+// coordinates past 2^64 then gave no trimmed span and took 14 times as long to search.
 __global__ void __launch_bounds__(KNN_THREADS) bounds_kernel(const float4* __restrict__ points, uint32_t n,
                                                              Moments* __restrict__ shares) {
   __shared__ Moments s_warp[KNN_THREADS / 32];
   Moments m = no_moments();
-  const float origin[3] = {finite3(points[0]) ? points[0].x : 0.0f, finite3(points[0]) ? points[0].y : 0.0f,
-                           finite3(points[0]) ? points[0].z : 0.0f};
-  // A thread's few points add up in float32: the moments only shape the curve, and
-  // FP64 runs at a fraction of its rate.
-  float sum[3] = {0.0f, 0.0f, 0.0f}, sum2[3] = {0.0f, 0.0f, 0.0f};
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 p = points[i];
     if (!finite3(p)) continue;
@@ -131,51 +135,38 @@ __global__ void __launch_bounds__(KNN_THREADS) bounds_kernel(const float4* __res
     for (int k = 0; k < 3; k++) {
       m.lo[k] = fminf(m.lo[k], c[k]);
       m.hi[k] = fmaxf(m.hi[k], c[k]);
-      const float d = c[k] - origin[k];
-      sum[k] += d;
-      sum2[k] += d * d;
+      m.sum[k] += (double)c[k];
+      m.sum2[k] += (double)c[k] * (double)c[k];
     }
-  }
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    m.sum[k] = sum[k];
-    m.sum2[k] = sum2[k];
   }
   reduce_moments(m, s_warp);
   if (threadIdx.x == 0) shares[blockIdx.x] = m;
 }
 
 // The octree for the shares' bounds and moments. One CTA.
-__global__ void __launch_bounds__(KNN_THREADS) octree_kernel(const float4* __restrict__ points,
-                                                             const Moments* __restrict__ shares, uint32_t count,
+__global__ void __launch_bounds__(KNN_THREADS) octree_kernel(const Moments* __restrict__ shares, uint32_t count,
                                                              Octree* __restrict__ out) {
   __shared__ Moments s_warp[KNN_THREADS / 32];
   Moments m = no_moments();
   for (uint32_t k = threadIdx.x; k < count; k += KNN_THREADS) add_moments(m, shares[k]);
   reduce_moments(m, s_warp);
-  if (threadIdx.x != 0) return;
-  Octree o;
-  const float origin[3] = {finite3(points[0]) ? points[0].x : 0.0f, finite3(points[0]) ? points[0].y : 0.0f,
-                           finite3(points[0]) ? points[0].z : 0.0f};
-  const double inv = 1.0 / (m.finite ? (double)m.finite : 1.0);
-  float extent = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    float lo = m.lo[k], hi = m.hi[k];
-    if (!(lo <= hi)) lo = hi = 0.0f;  // no finite points
-    const double mean = m.sum[k] * inv;
-    const float centre = origin[k] + (float)mean, reach = 3.0f * sqrtf((float)fmax(0.0, m.sum2[k] * inv - mean * mean));
-    if (isfinite(centre) && isfinite(reach)) {
-      lo = fmaxf(lo, centre - reach);
-      hi = fminf(hi, centre + reach);
-      if (!(lo <= hi)) lo = hi = centre;
-    }
-    o.lo[k] = lo;
-    extent = fmaxf(extent, hi - lo);
-  }
-  if (!(extent > 0.0f) || !isfinite(extent)) extent = 1.0f;
-  o.scale = (float)(1u << BITS) / extent;
-  *out = o;
+  if (threadIdx.x >= 32) return;
+  // Lane k: axis k.
+  const uint32_t k = threadIdx.x % 3;
+  const double finite = m.finite ? (double)m.finite : 1.0;
+  auto axis = [&](const auto (&v)[3]) { return k == 0 ? v[0] : k == 1 ? v[1] : v[2]; };
+  double lo = axis(m.lo), hi = axis(m.hi);
+  if (!(lo <= hi)) lo = hi = 0.0;  // no finite points
+  const double mean = axis(m.sum) / finite;
+  const double reach = 3.0 * sqrt(fmax(0.0, axis(m.sum2) / finite - mean * mean));
+  lo = fmax(lo, mean - reach);
+  hi = fmin(hi, mean + reach);
+  if (!(lo <= hi)) lo = hi = mean;
+  if (threadIdx.x < 3) out->lo[k] = (float)lo;
+  double extent = hi - lo;
+  for (int other = 1; other < 3; other++) extent = fmax(extent, __shfl_sync(0xffffffffu, hi - lo, (k + other) % 3));
+  if (!(extent > 0.0) || !isfinite(extent)) extent = 1.0;
+  if (threadIdx.x == 0) out->scale = (float)((double)(1u << BITS) / extent);
 }
 
 // Finest-level cell coordinate of a position, clamped into the octree (NaN
@@ -502,7 +493,7 @@ dg_status neighbor_distance2(dg_context* ctx, const float4* points, uint32_t n, 
   Box* level = scratch.at<Box>(off_boxes);
   Octree* octree = scratch.at<Octree>(off_octree);
   DG_LAUNCH(ctx, "knn_bounds", bounds_kernel<<<shares, KNN_THREADS, 0, st>>>(points, n, scratch.at<Moments>(off_shares)));
-  DG_LAUNCH(ctx, "knn_octree", octree_kernel<<<1, KNN_THREADS, 0, st>>>(points, scratch.at<Moments>(off_shares), shares, octree));
+  DG_LAUNCH(ctx, "knn_octree", octree_kernel<<<1, KNN_THREADS, 0, st>>>(scratch.at<Moments>(off_shares), shares, octree));
   const uint32_t grid = ceil_div(n, KNN_THREADS);
   DG_LAUNCH(ctx, "knn_morton", morton_kernel<<<grid, KNN_THREADS, 0, st>>>(points, n, octree, keys, values));
   DG_TRY(sort_launch(ctx, plan, keys, values, scratch.at<void>(off_keys_alt), scratch.at<uint32_t>(off_values_alt),
