@@ -273,7 +273,7 @@ __device__ __forceinline__ uint32_t bin_exclusive(uint32_t v, uint32_t* s_warp, 
 //   The entries go through shared memory when they fit there, grouped by tile, so
 //   that a tile's run is written together; a 4-byte store into a list of its own
 //   costs a 32-byte sector.
-// Grid: (bins, chunks, views): the nearest chunks, which cover the most tiles, first.
+// Grid: (bins x chunks, views): the nearest chunks, which cover the most tiles, first.
 __global__ void __launch_bounds__(BIN_THREADS) bin_scatter_kernel(const Bins b,
                                                                   const uint32_t* order,
                                                                   const uint2* ranges,
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(BIN_THREADS) bin_scatter_kernel(const Bins b,
   __shared__ uint32_t s_excl[BIN_WARPS][32];   // of a warp's 32 splats: the pairs before each,
   __shared__ uint2 s_hit[BIN_WARPS][32];       // and its rectangle
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, below = (1u << lane) - 1u;
-  const uint32_t bin = blockIdx.x, chunk = blockIdx.y, view = blockIdx.z, row = view * b.chunks + chunk;
+  const uint32_t bin = blockIdx.x % b.bins, chunk = blockIdx.x / b.bins, view = blockIdx.y, row = view * b.chunks + chunk;
   const uint32_t rounds = b.chunk / 32;  // 32 splats each
   const ChunkStage st{smem, reinterpret_cast<uint16_t*>(smem + b.chunk)};
   uint16_t* const buffer = st.list + b.chunk;                                      // [SCATTER_ROOM]
@@ -652,7 +652,7 @@ dg_status bin_launch(dg_context* ctx, const BinShape& s, const BinLaunch& l) {
            b, l.capacity, l.pair_total);
   DG_CHAIN(ctx, "bin_ranges", (bin_ranges_kernel), ceil_div((uint64_t)s.views * b.tiles, RANGE_THREADS), RANGE_THREADS, 0,
            b, l.ranges, l.plan, l.work);
-  DG_CHAIN(ctx, "bin_scatter", (bin_scatter_kernel), dim3(b.bins, b.chunks, s.views), BIN_THREADS, scatter_bytes(b.chunk),
+  DG_CHAIN(ctx, "bin_scatter", (bin_scatter_kernel), dim3(b.bins * b.chunks, s.views), BIN_THREADS, scatter_bytes(b.chunk),
            b, l.order, l.ranges, l.values);
   return DG_OK;
 }

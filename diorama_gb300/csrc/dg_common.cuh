@@ -189,7 +189,9 @@ cudaError_t launch_chained(cudaStream_t stream, void (*kernel)(Params...), dim3 
   config.stream = stream;
   config.attrs = &chained;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+  const cudaError_t err = cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+  if (err != cudaSuccess) cudaGetLastError();  // told here: not to be found by the next launch
+  return err;
 }
 }  // namespace dg
 #define DG_CHAIN(ctx, name, kernel, grid, block, shared, ...)                                                \

@@ -94,6 +94,10 @@ dg_status ensure(dg_view_batch* b, dg_buffer** buf, size_t bytes) {
   return alloc_buffer(b->ctx, std::max<size_t>(bytes, 16), buf);
 }
 
+// Views of one batch at most: the launches that have a row of CTAs per view carry it in
+// the grid's second dimension.
+constexpr uint32_t MAX_BATCH = 65'535;
+
 // Each view's splats by depth, on their own: all views in the same launches. (As one
 // sort of (view, depth) keys, 12 views of 300,000 took 190 us in five passes over 64-bit
 // keys, this way 135.)
@@ -320,7 +324,7 @@ dg_status views_render(dg_renderer* r, const dg_camera* cams, uint32_t count, co
   DG_TRY(check_views(r, cams, count));
   dg_context* ctx = r->ctx;
   dg_view_batch* b = batch_of(r);
-  batch = std::max(1u, std::min(batch ? batch : count, count));
+  batch = std::max(1u, std::min({batch ? batch : count, count, MAX_BATCH}));
   const size_t pixels = (size_t)cams[0].viewport[0] * (uint32_t)cams[0].viewport[1];
   for (uint32_t first = 0; first < count; first += batch) {
     const uint32_t n = std::min(batch, count - first);
