@@ -457,33 +457,50 @@ __global__ void __launch_bounds__(BIN_THREADS) bin_scatter_kernel(const Bins b,
   }
 }
 
+// Of `n` counts, consecutive ones per thread, the first whose running sum passes `left`
+// (their whole sum does): its place, and what of `left` remains before it. All threads get
+// it. count(i) is called once or twice per i.
+struct Passed {
+  uint32_t at, left;
+};
+template <class Count>
+__device__ __forceinline__ Passed first_past(uint32_t n, uint32_t left, Count count) {
+  __shared__ unsigned long long s_warp[SCAN_THREADS / 32];
+  __shared__ Passed s_passed;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t each = (n + SCAN_THREADS - 1) / SCAN_THREADS;
+  const uint32_t from = min(threadIdx.x * each, n), to = min(from + each, n);
+  unsigned long long mine = 0;
+  for (uint32_t i = from; i < to; i++) mine += count(i);
+  unsigned long long before = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned long long v = __shfl_up_sync(0xffffffffu, before, d);
+    if (lane >= d) before += v;
+  }
+  if (lane == 31) s_warp[warp] = before;
+  before -= mine;
+  __syncthreads();
+  for (uint32_t w = 0; w < warp; w++) before += s_warp[w];
+  if (before <= left && left < before + mine) {  // one thread
+    Passed p{from, left - (uint32_t)before};
+    for (uint32_t c = count(p.at); c <= p.left; c = count(++p.at)) p.left -= c;
+    s_passed = p;
+  }
+  __syncthreads();
+  const Passed p = s_passed;
+  __syncthreads();
+  return p;
+}
+
 // The chunk and splat at which the pairs reach `capacity` (there are more than
-// that). One call per CTA; rarely taken, so plain.
-__device__ Limit find_limit(const Bins& b, uint32_t capacity) {
-  __shared__ Limit s_limit;
-  __shared__ uint32_t s_pairs[SCAN_THREADS];
-  if (threadIdx.x == 0) {
-    uint32_t c = 0, left = capacity;
-    while (b.chunk_pairs[c] <= left) left -= b.chunk_pairs[c++];
-    s_limit = Limit{c, 0u, left, 0u};
-  }
-  __syncthreads();
-  const uint32_t c = s_limit.chunk, first = c % b.chunks * b.chunk, n = min(b.chunk, b.s.per_view - first);
-  const uint32_t* sorted = b.sorted + (size_t)(c / b.chunks) * b.s.per_view + first;
-  const uint32_t each = (b.chunk + SCAN_THREADS - 1) / SCAN_THREADS;  // consecutive splats per thread
-  uint32_t pairs = 0;
-  for (uint32_t i = threadIdx.x * each; i < min((threadIdx.x + 1) * each, n); i++) pairs += rect_area(sorted[i]);
-  s_pairs[threadIdx.x] = pairs;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0, left = s_limit.kept;
-    while (s_pairs[t] <= left) left -= s_pairs[t++];
-    uint32_t i = t * each;
-    while (rect_area(sorted[i]) <= left) left -= rect_area(sorted[i++]);
-    s_limit = Limit{c, i, left, 0u};
-  }
-  __syncthreads();
-  return s_limit;
+// that). One call per CTA.
+__device__ __forceinline__ Limit find_limit(const Bins& b, uint32_t capacity) {
+  const Passed row = first_past(b.s.views * b.chunks, capacity, [&](uint32_t c) { return b.chunk_pairs[c]; });
+  const uint32_t first = row.at % b.chunks * b.chunk, n = min(b.chunk, b.s.per_view - first);
+  const uint32_t* sorted = b.sorted + (size_t)(row.at / b.chunks) * b.s.per_view + first;
+  const Passed splat = first_past(n, row.left, [&](uint32_t i) { return rect_area(sorted[i]); });
+  return Limit{row.at, splat.at, splat.left, 0u};
 }
 
 // Each tile's counts over the chunks become exclusive prefixes, its total goes to
