@@ -15,7 +15,7 @@
 // (stable: warp-striped loads are ranked round by round), publishes its
 // per-digit counts, looks back over earlier tiles' counts (bounded waits), and
 // scatters through shared memory so each digit's run is written contiguously. Up to
-// 65,536 keys the passes run in one kernel instead (sort_cluster_kernel).
+// 65,536 u32 keys (43,000 u64) the passes run in one kernel instead (sort_cluster_kernel).
 #include "dg_common.cuh"
 #include "dg_scan.cuh"
 
@@ -336,12 +336,15 @@ __global__ void __launch_bounds__(SORT_THREADS, DG_SORT_MIN_BLOCKS)
 // warp, exchanges the CTAs' digit counts over distributed shared memory, and stores
 // each key straight into its new place, in whichever CTA that lies: two cluster
 // barriers instead of a launch, a ticket, a look-back and a trip through L2 each.
-// What bounds it: at a few thousand keys the barriers (15 us for 300 keys), beyond that
+// What bounds it: at a few thousand keys the barriers (12 us for 300 keys), beyond that
 // 16 SMs' shared memory and ranking (0.3 us per 1,000 keys).
-// Passes (clear and histogram with them) against one cluster, in us, without the 3 us
-// that timing one kernel adds: u32 keys in four passes, 5,000 36 and 18; 16,000 36 and
-// 20; 50,000 38 and 28; 65,536 39 and 32; 100,000 40 and 42. u64 keys in six, 5,000 54
-// and 24; 32,000 54 and 44; 50,000 61 and 54; 65,536 64 and 68; 100,000 66 and 95.
+// Passes (clear and histogram with them) against one cluster, in us, of sorts in a row of
+// keys in random order: u32 keys in four passes, 300 21 and 12; 5,000 27 and 13; 16,384 29
+// and 17; 32,768 31 and 22; 50,000 33 and 26; 65,536 33 and 30. u64 keys in six, 5,000 39
+// and 20; 16,384 43 and 29; 32,768 45 and 40; 40,000 47 and 44; 45,000 47 and 46; 50,000
+// 47 and 48; 65,536 49 and 62. In eight, 5,000 52 and 26; 16,384 57 and 38; 32,768 60 and
+// 54; 40,000 61 and 59; 45,000 62 and 63; 65,536 65 and 85. So u32 keys go to one cluster
+// up to its room, u64 keys up to 43,000.
 // 256 threads with the same room take as long, 1024 more (their bookkeeping); 8 CTAs 48
 // us where 16 take 38 (50,000 keys); putting a CTA's keys in digit order first, so that
 // its stores come in runs, changed nothing.
@@ -349,7 +352,9 @@ constexpr uint32_t CLUSTER = 16;
 constexpr uint32_t CLUSTER_THREADS = 512, CLUSTER_WARPS = CLUSTER_THREADS / 32;
 constexpr uint32_t CLUSTER_PARTS = CLUSTER_THREADS / RADIX;  // 2 threads share a digit's sums
 constexpr int CLUSTER_ITEMS = 8;
-constexpr uint32_t CLUSTER_KEYS = CLUSTER * CLUSTER_THREADS * CLUSTER_ITEMS;  // 65,536
+constexpr uint32_t CLUSTER_ROOM = CLUSTER * CLUSTER_THREADS * CLUSTER_ITEMS;  // 65,536
+template <int KW>
+constexpr uint32_t CLUSTER_KEYS = KW == 1 ? CLUSTER_ROOM : 43'000;
 
 template <int KW>
 struct ClusterShared {
@@ -638,7 +643,7 @@ dg_status launch_typed(dg_context* ctx, const SortPlan& plan, void* keys, uint32
   using K = typename KeyOf<KW>::type;
   // One cluster up to the sizes at which it still beats the passes (figures above
   // sort_cluster_kernel).
-  if (plan.segments <= (uint32_t)ctx->sort_clusters && plan.capacity <= CLUSTER_KEYS)
+  if (plan.segments <= (uint32_t)ctx->sort_clusters && plan.capacity <= CLUSTER_KEYS<KW>)
     return cluster_launch<KW>(ctx, plan, keys, values, keys_alt, values_alt, count);
   ScratchLayout l = layout_of(plan);
   char* s = static_cast<char*>(scratch);
