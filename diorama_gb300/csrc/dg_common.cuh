@@ -166,9 +166,9 @@ void timing_end(dg_context* ctx, const char* name);
 // placed while other kernels still hold an SM's shared memory, leave it divided as it
 // was (12 views 1007 -> 1162 us, a frame of 1.1M splats 775 -> 807); the loss gained
 // nothing.
-// Such a kernel runs while the one in front still writes, so none of its pointers is
-// __restrict__: a const one would be read through the path for data that does not change
-// while a kernel runs.
+// Such a kernel runs while the one in front still writes, so none of its pointers, and none
+// of those of the functions it calls, is __restrict__: a const one may be read through the
+// path for data that does not change while a kernel runs.
 // DG_CHAIN(ctx, "name", (kernel), grid, block, shared bytes, args...);
 #ifdef __CUDACC__
 namespace dg {

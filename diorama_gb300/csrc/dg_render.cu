@@ -40,7 +40,7 @@ struct Projected {
 };
 
 __device__ __forceinline__ Projected preprocess_one(const Camera& cam, const float (&g)[16], const float* shv,
-                                                    uint32_t basis_count, float4* __restrict__ out,
+                                                    uint32_t basis_count, float4* out,
                                                     uint32_t twl = 0, uint32_t thl = 0) {
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   auto culled = [&]() {
@@ -100,12 +100,12 @@ __device__ __forceinline__ Projected preprocess_one(const Camera& cam, const flo
 // Stages the SH coefficients of Gaussians [first, first + n) into shared memory
 // with coalesced loads (45 floats per Gaussian; the odd stride makes the
 // per-thread reads conflict-free). All threads of the CTA take part.
-__device__ __forceinline__ void stage_sh(float* s_sh, const float* __restrict__ sh, uint32_t first, uint32_t n) {
+__device__ __forceinline__ void stage_sh(float* s_sh, const float* sh, uint32_t first, uint32_t n) {
   stage_floats_async(s_sh, sh + (size_t)first * SH_REST_FLOATS, n * SH_REST_FLOATS);
   cp_async_wait_all();
 }
 
-__device__ __forceinline__ void load_gaussian(const float* __restrict__ gaussians, uint32_t i, float (&g)[16]) {
+__device__ __forceinline__ void load_gaussian(const float* gaussians, uint32_t i, float (&g)[16]) {
   const float4* gp = reinterpret_cast<const float4*>(gaussians + (size_t)i * FLOATS_PER_GAUSSIAN);
 #pragma unroll
   for (int k = 0; k < 4; k++) {

@@ -87,7 +87,7 @@ struct BackStage {
 // butterfly over the block's pixels (p + 16 first, p + 1 last). Pixel p is at
 // (corner_x + p % 8, corner_y + p / 8).
 __device__ __forceinline__ void add_gradients(const BackStage& st, uint32_t first, uint32_t n, uint32_t lane,
-                                              float corner_x, float corner_y, float* __restrict__ splat_grads) {
+                                              float corner_x, float corner_y, float* splat_grads) {
   const uint32_t s = lane & 15u, h = lane >> 4, e = first + s;
   const float* f = reinterpret_cast<const float*>(&st.pair[e / 2]) + (e & 1u);
   const float nx = f[0], ny = f[2], a = 2.0f * f[4], b = f[6], c = 2.0f * f[8];  // conic (a, b, c)
@@ -406,7 +406,7 @@ constexpr uint32_t PBWD_THREADS = DG_PBWD_THREADS;  // a multiple of 32
 
 // Copies n floats between global and shared memory, 16 bytes at a time where both
 // ends allow it; all threads of the CTA take part.
-__device__ __forceinline__ void copy_floats(float* __restrict__ dst, const float* __restrict__ src, uint32_t n) {
+__device__ __forceinline__ void copy_floats(float* dst, const float* src, uint32_t n) {
   if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
     const uint32_t vecs = n / 4;
     for (uint32_t k = threadIdx.x; k < vecs; k += blockDim.x)
@@ -423,9 +423,9 @@ __device__ __forceinline__ void copy_floats(float* __restrict__ dst, const float
 // gaussian: the Gaussian's 16 activated floats (16-byte aligned); radius: its
 // splat's radius (0 when it was not drawn); grads: its 9 splat gradients. shv
 // holds its SH coefficients and receives their gradients.
-__device__ __forceinline__ void preprocess_backward_one(const Camera& cam, const float* __restrict__ gaussian,
+__device__ __forceinline__ void preprocess_backward_one(const Camera& cam, const float* gaussian,
                                                         float* shv, uint32_t basis_count, float radius,
-                                                        const float* __restrict__ grads, float (&out)[16]) {
+                                                        const float* grads, float (&out)[16]) {
 #pragma unroll
   for (int k = 0; k < 16; k++) out[k] = 0.0f;
   if (radius == 0.0f) {
@@ -622,7 +622,7 @@ __device__ __forceinline__ void preprocess_backward_one(const Camera& cam, const
   out[14] = raw_grad[2];
 }
 
-__device__ __forceinline__ void store16(float* __restrict__ dst, const float (&v)[16]) {
+__device__ __forceinline__ void store16(float* dst, const float (&v)[16]) {
 #pragma unroll
   for (int k = 0; k < 4; k++)
     reinterpret_cast<float4*>(dst)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
