@@ -383,9 +383,14 @@ Window window_weights() {
 // that no strip waits for another's end; each strip costs 10 rows more. Six strips per
 // SM: 5 take 65 us at 1957x1091, 6 take 62, 7 take 68, 8 take 60; at 489x273 14 us for 6,
 // 15 for 7 and 8. At least 6 rows: at 251x187 10.6 us, 8 rows 11.5, 12 rows 12.3, 4 rows
-// no faster and at 489x273 1 us slower.
+// no faster and at 489x273 1 us slower. But 2 or 4 rows while there are no more than 2
+// strips per SM, where a strip's own chain of rows is all there is: the whole loss at 96x96
+// 22.2 us with 6 rows, 18.3 with 2 (21.5 with blocks); at 200x150 22.7 and 21.7 with 4
+// (21.6); with up to 3 strips per SM so, 160x120 takes 21.5 instead of 20.2.
 static int strip_rows(const dg_context* ctx, uint32_t width, uint32_t height) {
   const uint32_t across = ceil_div(width, COLS), room = (uint32_t)ctx->sm_count * STRIPS_PER_SM;
+  for (int rows = 2; rows < MIN_ROWS; rows += 2)
+    if (across * ceil_div(height, rows) <= 2 * (uint32_t)ctx->sm_count) return rows;
   const uint32_t down = std::max(1u, room / across);
   return std::max(MIN_ROWS, (int)(ceil_div(ceil_div(height, down), 2) * 2));
 }
