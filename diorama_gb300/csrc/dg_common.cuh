@@ -220,41 +220,6 @@ inline T* typed(dg_buffer* b) {
 // ---------------------------------------------------------------- device math
 namespace dg {
 
-// e^x by Cody-Waite reduction x = n ln2 + r (|r| <= ln2/2), e^r from its Taylor
-// series to degree 7 by Horner's rule, and scaling by 2^n through the exponent
-// bits, for -87 <= x <= 88 (the blend calls it only on powers between a splat's
-// cutoff, above ln(1/255) - 1e-3, and 0). The blend's forward and backward both
-// use it, so their alpha tests agree exactly; its error is about one ulp.
-__host__ __device__ __forceinline__ float exp_blend_core(float x) {
-  float n = rintf(x * 1.44269504088896341f);
-  float r = fmaf(n, -0.693145751953125f, x);
-  r = fmaf(n, -1.428606820309417232e-6f, r);
-  float p = 1.98412698412698413e-4f;
-  p = fmaf(p, r, 1.38888888888888889e-3f);
-  p = fmaf(p, r, 8.33333333333333333e-3f);
-  p = fmaf(p, r, 4.16666666666666667e-2f);
-  p = fmaf(p, r, 1.66666666666666667e-1f);
-  p = fmaf(p, r, 0.5f);
-  p = fmaf(p, r, 1.0f);
-  p = fmaf(p, r, 1.0f);
-  int32_t e = (int32_t)n + 127;
-#ifdef __CUDA_ARCH__
-  float scale = __int_as_float(e << 23);
-#else
-  float scale;
-  uint32_t bits = (uint32_t)e << 23;
-  std::memcpy(&scale, &bits, 4);
-#endif
-  return p * scale;
-}
-
-// exp_blend_core over the whole float range: 0 below -87, infinity above 88.
-__host__ __device__ __forceinline__ float exp_blend(float x) {
-  if (x < -87.0f) return 0.0f;
-  if (x > 88.0f) return INFINITY;
-  return exp_blend_core(x);
-}
-
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 
 #ifdef __CUDACC__  // device code below; host-only translation units skip it
@@ -338,9 +303,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
-// exp_blend_core of -q for two values at once, each lane of the pair its result bit for
-// bit where it is defined: the sign of the argument goes into every other coefficient.
-// The fused multiply-adds run as packed pairs, and rintf is the addition of 1.5 * 2^23,
+// e^-q for two values at once, for q from 0 to 87 (the blend's go from 0 to a splat's
+// cutoff, under 6 for opacities up to 1): Cody-Waite reduction -q = n ln2 + r
+// (|r| <= ln2/2), e^r from its Taylor series to degree 7 by Horner's rule, and scaling by
+// 2^n through the exponent bits; about one ulp. The forward and the backward blend both use
+// it, so their alpha tests agree exactly, and the oracle evaluates the same sequence for
+// x = -q, bit for bit: here r stands for -r, its sign in every other coefficient. The fused
+// multiply-adds run as packed pairs, and the rounding to n is the addition of 1.5 * 2^23,
 // whose sum holds the rounded integer in its low bits (and in 2^n's exponent when
 // shifted up by 23), which takes two conversions per value off the special-function unit.
 __device__ __forceinline__ F2 exp_blend_negated(F2 q) {

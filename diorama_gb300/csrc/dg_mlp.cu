@@ -190,7 +190,7 @@ __device__ __forceinline__ void forward16(const uint32_t (&ax)[4], const __nv_bf
 // accumulators share 64 tensor-memory columns, the next candidates' features load
 // during the products, and the GELU code is one loop body for both layers: inlined
 // 128 times (60 KB) it kept the warps waiting for instructions (59.6 us as 64, and
-// 62 with the weights staged per 128 candidates). 300,007 candidates: 62 -> 49 us;
+// 62 with the weights staged per 128 candidates). 300,007 candidates: 62 -> 47 us;
 // 1.1M: 198 -> 154. (A cheaper erf, however exact, moves values across BF16's
 // rounding boundaries, and scores by up to 3e-3.)
 constexpr uint32_t TC_ROWS = 128;     // candidates per CTA: the products' M

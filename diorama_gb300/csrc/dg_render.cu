@@ -195,8 +195,8 @@ uint32_t preprocess_grid(const dg_context* ctx, uint32_t count) {
 
 // The same for a batch of views sharing one viewport: each CTA stages its
 // Gaussians and their SH coefficients once and projects them into every view.
-// Splat (view v, Gaussian i) is number v * count + i; its depth-sort key puts
-// the view above the depth's bits, so one sort orders every view by depth.
+// Splat (view v, Gaussian i) is number v * count + i: each view's splats are a run of the
+// depth sort's keys, sorted on its own.
 __global__ void __launch_bounds__(PRE_THREADS) preprocess_views_kernel(
     const Camera* cameras, uint32_t views, const float* gaussians,
     const float* sh, uint32_t count, const uint32_t* scene_params,

@@ -110,7 +110,7 @@ struct BlendForward {
   uint32_t* pixel_last;
   float4* checkpoints;
   uint32_t* blend_mask;
-  uint32_t* counters;  // 4 words, cleared here
+  uint32_t* counters;  // 4 words, zero or cleared here (see cleared)
   BlendShape shape;
   bool splat_cutoffs;  // the splats carry their blend cutoff (this build's preprocess wrote them)
   bool cleared;        // the plan's header and the counters are zero (bin_launch cleared them)

@@ -213,7 +213,7 @@ __device__ __forceinline__ void sh_basis_gradient(const float d[3], float g[15][
 
 // A power below which alpha = opacity * exp(power) is certainly under 1/255, so
 // the exp can be skipped with the same outcome: ln(1 / (255 opacity)), lowered by
-// 1e-3 to cover the float error of exp_blend and of the product (~1e-7 relative).
+// 1e-3 to cover the float error of the exp and of the product (~1e-7 relative).
 __device__ __forceinline__ float blend_cutoff(float opacity) {
   return logf(1.0f / (255.0f * opacity)) - 1e-3f;
 }

@@ -1,7 +1,7 @@
 // Batched rendering of many views of one scene: every stage of the frame runs
 // once over all the views of a batch (one preprocess launch projecting each
-// Gaussian into every view, one depth sort over (view, depth) keys, one binning of
-// every view's splats into its tiles, one blend over all their tiles),
+// Gaussian into every view, one depth sort of every view's splats on their own, one binning
+// of them into the views' tiles, one blend over all their tiles),
 // and a batch whose pair count is known is replayed as one CUDA graph. Each view
 // gets exactly the pairs, order and blend of a single-view render, so its image
 // is bit-identical to GaussianRenderer.encode's. The views per batch, the
